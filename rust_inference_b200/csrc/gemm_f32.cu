@@ -1,0 +1,577 @@
+// out[M, N] = X[M, K] * W[N, K]^T for float32 operands with float32 results, in two kernels that between them take
+// every M (K a multiple of 4 and 16-byte aligned operands: rows are read 16 bytes at a time; `gemm_simt.cu` has the rest).
+//
+// Few rows of X (a decode step, up to FEW_MAX): the product is a read of W.  A warp owns a few rows of W, its lanes run
+// along K with 16-byte loads straight into registers, several steps ahead, and every loaded weight meets all rows of X,
+// which lie in shared memory; FFMA, float32 sums.  K is cut over the thread blocks of a cluster when N alone has too few
+// rows to keep the memory busy; the pieces meet through distributed shared memory in a fixed order, so a product's bits do
+// not change from run to run.
+//
+// More rows: the tensor cores, without giving up 32 bits.  A float32 number is the exact sum of three bfloat16 numbers
+// (its leading 8 significant bits, the next 8 and the last 8), so x * w is the sum of nine products of bfloat16 numbers,
+// each exact in the tensor core; the three smallest (mid * low, low * mid, low * low) are below 2^-24 of the whole and are
+// left out.  Eight warps read both operands, cut them and put the parts into shared memory as the MMA wants them
+// (128-byte swizzle); six MMAs per 16 steps of K, smallest products first, add up 64 steps of K in tensor memory; then
+// eight warps add that sum onto float32 registers and the next 64 steps start from zero, so that the tensor core's own
+// additions, which truncate, never run over more than 64 steps.  Against 64 bits (rows of N(0, 1) times rows of N(0, 1/K)) the
+// result is off by 1.3e-7 at K = 192, 1.4e-7 at 896, 1.5e-7 at 4,864 and 2.1e-7 at 18,944, where one running FFMA sum was off
+// by 2.5e-7, 5.3e-7, 1.2e-6 and 2.5e-6 (the kernel for few rows: 0.8e-7 to 1.8e-7).  A number that is infinite or NaN has no such parts: a tile that meets one computes
+// its piece again with FFMA, so that such numbers come out as the plain sum gives them.
+//
+// Epilogues as in `gemm_simt.cu` (0 and 1 are the same here: float32 with a bias): 2 out += acc, 3 gated, 4 an activation,
+// 5 silu for the first columns.
+#include "cluster.cuh"
+#include "tcgen05_common.cuh"
+
+using namespace ri;
+using namespace ri::tc;
+
+namespace {
+
+constexpr int SMS = 148;
+
+// weights: read once, kept out of L1 (a load that may stand before the wait for the kernel before)
+__device__ __forceinline__ float4 load_weight(const float* p) {
+    float4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+
+struct Forms {          // the epilogue's constants, loaded once per thread
+    GateForm gate;
+    ActForm act;
+    int silu_feats;
+};
+template <int MODE>
+__device__ __forceinline__ Forms load_forms(const float* bias) {
+    Forms f;
+    f.gate = load_gate_form(MODE == 3 ? bias : nullptr);
+    f.act = MODE == 4 ? load_act_form(bias) : ActForm{0.f, 0.f, 0.f};
+    f.silu_feats = MODE == 5 ? (int)bias[0] : 0;
+    return f;
+}
+template <int MODE>
+__device__ __forceinline__ void finish(float* out, size_t o, int f, float v, float up, const float* __restrict__ bias,
+                                       const Forms& forms) {
+    if (MODE == 1) out[o] = bias != nullptr ? v + bias[f] : v;
+    else if (MODE == 2) out[o] += v;
+    else if (MODE == 3) out[o] = gated_f32(v, up, forms.gate);
+    else if (MODE == 4) out[o] = act_f32(v, forms.act);
+    else out[o] = f < forms.silu_feats ? silu_f32(v) : v;
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// Few rows of X.
+//
+// Bound by the read of W.  Two blocks' worth of loads in flight per SM cover the memory's latency (8 warps x 4 KiB per
+// block).  A weight costs one FFMA per row of X and a 16-byte read of X from shared memory per RW of them: with RW = 2 up
+// to four rows and 4 beyond, both stay below what the memory delivers (23 bytes per clock and SM).
+// ---------------------------------------------------------------------------------------------------------------------
+constexpr int FEW_MAX = 16;
+constexpr int FEW_THREADS = 256, FEW_WARPS = FEW_THREADS / 32;
+constexpr int STEP = 128;                      // floats of K that a warp reads per step and row: 16 bytes per lane
+
+// a[0 .. n) of every lane, summed over the lanes: afterwards lane l holds in a[0 .. n/32) (n < 32: in a[0]) the sums number
+// `lane_first` .. ; every exchange halves what a lane still carries
+template <int N>
+__device__ __forceinline__ int reduce_lanes(float (&a)[N], int lane) {
+    int first = 0, n = N;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (n > 1) {
+            const int half = n / 2;
+            const bool upper = (lane & o) != 0;
+#pragma unroll
+            for (int i = 0; i < N / 2; ++i) {
+                if (i >= half) break;
+                const float give = upper ? a[i] : a[i + half], keep = upper ? a[i + half] : a[i];
+                a[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+            if (upper) first += half;
+            n = half;
+        } else {
+            a[0] += __shfl_xor_sync(0xffffffffu, a[0], o);
+        }
+    }
+    return first;
+}
+
+template <int MT, int RW, int U, int MODE>
+__global__ void __launch_bounds__(FEW_THREADS, MT > 8 ? 2 : 3)
+gemm_f32_few_kernel(const float* X, const float* __restrict__ W, const float* __restrict__ W2,
+                    const float* __restrict__ bias, float* out, int M, int N, int K, int steps, int splits) {
+    constexpr bool DUAL = MODE == 3;
+    constexpr int FEATS = DUAL ? RW / 2 : RW;                // features per warp (gated: a gate row and an up row each)
+    constexpr int GROUP = FEW_WARPS * FEATS;                 // features per block
+    constexpr int SUMS = FEW_WARPS * RW * MT;
+    extern __shared__ __align__(16) float xs[];              // [MT][this block's stretch of K]
+    __shared__ float sums[2][SUMS];
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = splits > 1 ? (int)cluster_rank() : 0;
+    const int first_step = (int)((long long)steps * rank / splits);
+    const int ns = (int)((long long)steps * (rank + 1) / splits) - first_step;      // >= 1: splits <= steps
+    const int ns_up = (ns + U - 1) / U * U;
+    const int k0 = first_step * STEP, width = ns * STEP;
+    const int groups = (N + GROUP - 1) / GROUP, stride = (int)gridDim.x / splits;
+
+    auto load = [&](float4 (&w)[RW], int group, int step) {
+        const int k = k0 + step * STEP + lane * 4;
+        const int f = group * GROUP + warp * FEATS;
+        const bool in = step < ns && k < K && group < groups;
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+            const int row = min(DUAL ? f + r / 2 : f + r, N - 1);
+            const float* base = (DUAL && (r & 1)) ? W2 : W;
+            w[r] = in ? load_weight(base + (size_t)row * K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+
+    let_next_kernel_start();
+    float4 w[U][RW];
+    int group = (int)blockIdx.x / splits;
+#pragma unroll
+    for (int u = 0; u < U; ++u) load(w[u], group, u);        // weights: written by no kernel
+    wait_for_previous_kernels();
+    for (int i = threadIdx.x * 4; i < MT * width; i += FEW_THREADS * 4) {
+        const int m = i / width, k = k0 + i - m * width;     // width is a multiple of 4: the four belong to one row
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (m < M && k < K) v = load_written(X + (size_t)m * K + k);
+        *reinterpret_cast<float4*>(xs + i) = v;
+    }
+    const Forms forms = load_forms<MODE>(bias);
+    __syncthreads();
+
+    for (int turn = 0; group < groups; group += stride, turn ^= 1) {
+        float acc[RW * MT];
+#pragma unroll
+        for (int i = 0; i < RW * MT; ++i) acc[i] = 0.f;
+        for (int s0 = 0; s0 < ns_up; s0 += U) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (s0 + u < ns) {
+                    const float* x0 = xs + (s0 + u) * STEP + lane * 4;
+#pragma unroll
+                    for (int m = 0; m < MT; ++m) {
+                        const float4 x = *reinterpret_cast<const float4*>(x0 + m * width);
+#pragma unroll
+                        for (int r = 0; r < RW; ++r) {
+                            float a = acc[r * MT + m];
+                            a = fmaf(w[u][r].x, x.x, a);
+                            a = fmaf(w[u][r].y, x.y, a);
+                            a = fmaf(w[u][r].z, x.z, a);
+                            a = fmaf(w[u][r].w, x.w, a);
+                            acc[r * MT + m] = a;
+                        }
+                    }
+                }
+                // the registers just used take the step U further on, of this group of rows or of the next
+                const int next = s0 + u + U;
+                if (next < ns_up) load(w[u], group, next);
+                else load(w[u], group + stride, next - ns_up);
+            }
+        }
+        const int at = reduce_lanes(acc, lane);
+        constexpr int HELD = RW * MT >= 32 ? RW * MT / 32 : 1;
+        if (RW * MT >= 32 || (lane & (32 / (RW * MT) - 1)) == 0) {
+#pragma unroll
+            for (int i = 0; i < HELD; ++i) sums[turn][warp * RW * MT + at + i] = acc[i];
+        }
+        if (splits > 1) cluster_sync(); else __syncthreads();
+        // outputs (feature of the group, row of X), the feature fastest; the cluster's blocks share them out
+        const int total = GROUP * MT, from = total * rank / splits, to = total * (rank + 1) / splits;
+        for (int i = from + threadIdx.x; i < to; i += FEW_THREADS) {
+            const int m = i / GROUP, fl = i - m * GROUP, f = group * GROUP + fl;
+            if (m >= M || f >= N) continue;
+            const int slot = ((fl / FEATS) * RW + (fl % FEATS) * (DUAL ? 2 : 1)) * MT + m;
+            float v = 0.f, up = 0.f;
+            if (splits > 1) {
+                for (int p = 0; p < splits; ++p) {
+                    v += peer_float(&sums[turn][slot], (uint32_t)p);
+                    if (DUAL) up += peer_float(&sums[turn][slot + MT], (uint32_t)p);
+                }
+            } else {
+                v = sums[turn][slot];
+                if (DUAL) up = sums[turn][slot + MT];
+            }
+            finish<MODE>(out, (size_t)m * N + f, f, v, up, bias, forms);
+        }
+        // the other half of `sums` is next: whoever writes this half again has passed the barrier of the turn between
+    }
+    if (splits > 1) cluster_sync();              // a peer may still be reading this block's sums
+}
+
+constexpr int FEW_SMEM_MAX = 200 * 1024;
+
+// How a product of few rows is cut: blocks along K (0: X does not fit shared memory in any cut).
+int few_splits(int rows, int group, int N, int K) {
+    const int steps = (K + STEP - 1) / STEP, groups = (N + group - 1) / group;
+    int best = 0;
+    long long best_cost = 0;
+    for (int s = 1; s <= 8 && s <= steps; s *= 2) {
+        const int per = (steps + s - 1) / s;
+        const long long smem = (long long)rows * per * STEP * 4;
+        if (smem > FEW_SMEM_MAX) continue;
+        const int resident = (smem > 100 * 1024 ? 1 : smem > 66 * 1024 || rows > 8 ? 2 : 3) * SMS / s;      // clusters
+        // rounds of the persistent grid times the steps of one, and what a round costs besides (about two steps; four
+        // where the pieces meet across blocks)
+        const long long rounds = (groups + resident - 1) / resident;
+        const long long cost = rounds * (per + (s > 1 ? 4 : 2));
+        if (best == 0 || cost < best_cost) { best = s; best_cost = cost; }
+    }
+    return best;
+}
+
+template <int MT, int RW, int U, int MODE>
+int launch_few(const float* X, const float* W, const float* W2, const float* bias, float* out, int M, int N, int K, int splits,
+               cudaStream_t stream) {
+    constexpr int GROUP = FEW_WARPS * (MODE == 3 ? RW / 2 : RW);
+    const int steps = (K + STEP - 1) / STEP, groups = (N + GROUP - 1) / GROUP;
+    const size_t smem = (size_t)MT * ((steps + splits - 1) / splits) * STEP * 4;
+    static PerDeviceOnce once;
+    if (int rc = raise_dynamic_smem(gemm_f32_few_kernel<MT, RW, U, MODE>, FEW_SMEM_MAX, once, "gemm_f32")) return rc;
+    const int per_sm = smem > 100 * 1024 ? 1 : smem > 66 * 1024 || MT > 8 ? 2 : 3;
+    const int clusters = max(1, min(groups, per_sm * SMS / splits));
+    return launch_cluster("gemm_f32 (few rows)", gemm_f32_few_kernel<MT, RW, U, MODE>, dim3(clusters * splits), FEW_THREADS, smem, splits,
+                          stream, X, W, W2, bias, out, M, N, K, steps, splits);
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// Many rows of X: three bfloat16 parts per operand on the tensor cores.
+//
+// A tile is 128 rows of W (gated: 64 gate rows and the 64 up rows of the same features) by TN rows of X.  What bounds a
+// block of 64 steps of K is shared memory (24 MMAs that read 4 KiB of W and TN * 32 bytes of X each, and the parts' writes: at
+// TN = 128 about 2,300 clocks against 1,536 of the tensor core, at TN = 64 1,730 against 768, so TN is 128 wherever a step has
+// that many rows) and the cutting, eight warps with a few dependent instructions per number.  Four warps instead of eight for
+// the additions made those the slowest part: 954 against 862 us at 333 x 151,936 x 896 (105 TFLOP/s of the product; the FFMA
+// kernel takes 2,950), 50 against 46 at 333 x 896 x 4,864 (345); sixteen warps for the cutting, 929 and 51.
+// ---------------------------------------------------------------------------------------------------------------------
+constexpr int ROWS = 128, BK = 64, PART = ROWS * BK * 2, STAGES = 2;
+constexpr int CUT_WARPS = 8, CUT_THREADS = CUT_WARPS * 32, ADD_WARPS = 8;
+constexpr int SPLIT_THREADS = CUT_THREADS + ADD_WARPS * 32;
+enum Status { ST_CUT_TIMEOUT = 41, ST_MMA_TIMEOUT = 42, ST_ADD_TIMEOUT = 43 };
+
+// x as three bfloat16 numbers that add up to it exactly, each the upper half of a float32: the leading 8 significant bits,
+// the next 8 and the rest.  `odd` becomes NaN if x is infinite or NaN.
+__device__ __forceinline__ void cut(float x, uint32_t& hi, uint32_t& mid, uint32_t& lo, float& odd) {
+    hi = __float_as_uint(x) & 0xffff0000u;
+    const float r = x - __uint_as_float(hi);
+    mid = __float_as_uint(r) & 0xffff0000u;
+    const float r2 = r - __uint_as_float(mid);
+    lo = __float_as_uint(r2);
+    odd = fmaf(r2, 0.f, odd);
+}
+__device__ __forceinline__ uint32_t upper_halves(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x7632); }
+__device__ __forceinline__ void store8(uint32_t addr, uint32_t a, uint32_t b) {
+    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
+}
+// four consecutive k of one row into the three parts
+__device__ __forceinline__ void put(uint32_t addr, uint32_t part_bytes, const float4& v, float& odd) {
+    uint32_t h[4], m[4], l[4];
+    cut(v.x, h[0], m[0], l[0], odd);
+    cut(v.y, h[1], m[1], l[1], odd);
+    cut(v.z, h[2], m[2], l[2], odd);
+    cut(v.w, h[3], m[3], l[3], odd);
+    store8(addr, upper_halves(h[0], h[1]), upper_halves(h[2], h[3]));
+    store8(addr + part_bytes, upper_halves(m[0], m[1]), upper_halves(m[2], m[3]));
+    store8(addr + 2 * part_bytes, upper_halves(l[0], l[1]), upper_halves(l[2], l[3]));
+}
+
+template <int TN, int MODE>
+__global__ void __launch_bounds__(SPLIT_THREADS, 1)
+gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* __restrict__ W2,
+                      const float* __restrict__ bias, float* out, int M, int N, int K, int splits, int* status) {
+    constexpr bool DUAL = MODE == 3;
+    constexpr int FEATS = DUAL ? ROWS / 2 : ROWS;
+    constexpr int X_PART = TN * BK * 2;
+    constexpr int STAGE = 3 * (PART + X_PART);
+    constexpr int TMEM_COLS = 2 * TN < 32 ? 32 : 2 * TN;
+    constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
+    __shared__ uint32_t tmem_slot;
+    __shared__ volatile int abort_flag, odd_flag;
+
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    float* pieces = reinterpret_cast<float*>(smem_raw + (base - smem_u32(smem_raw)));      // [TN][128], over the stages at the end
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = splits > 1 ? (int)cluster_rank() : 0;
+    const int tok_tiles = (M + TN - 1) / TN, tile = (int)blockIdx.x / splits;
+    const int t0 = (tile % tok_tiles) * TN, f0 = (tile / tok_tiles) * FEATS;        // rows of X fastest: W stays in L2
+    const int total_kb = (K + BK - 1) / BK;
+    const int kb0 = (int)((long long)total_kb * rank / splits);
+    const int n_kb = (int)((long long)total_kb * (rank + 1) / splits) - kb0;        // >= 1: splits <= total_kb
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(smem_u32(&full_bar[s]), CUT_WARPS);
+            mbar_init(smem_u32(&empty_bar[s]), 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(smem_u32(&acc_full[i]), 1);
+            mbar_init(smem_u32(&acc_empty[i]), ADD_WARPS);
+        }
+        abort_flag = 0;
+        odd_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == CUT_WARPS) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                     "r"((uint32_t)TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    let_next_kernel_start();
+
+    // row r of the tile: which row of which matrix (null beyond the matrix)
+    auto weight_row = [&](int r) -> const float* {
+        const int f = f0 + (DUAL ? r % FEATS : r);
+        return f < N ? (DUAL && r >= FEATS ? W2 : W) + (size_t)f * K : nullptr;
+    };
+
+    if (warp < CUT_WARPS) {
+        // ---- read, cut, store: 16 threads per row of 64 floats ----
+        const int k4 = threadIdx.x & 15, row = threadIdx.x >> 4;             // rows row, row + 16, ...
+        const uint32_t col = (uint32_t)(row * 128 + ((k4 * 8) ^ ((row & 7) << 4)));
+        constexpr int WN = ROWS / 16, XN = TN / 16;
+        // a thread's rows are 16 apart: one address per matrix, and a bit for every row that exists
+        const size_t stride = (size_t)16 * K;
+        const float* xp = X + (size_t)(t0 + row) * K;
+        const float* wp = W + (size_t)(f0 + row) * K;
+        const float* wp2 = DUAL ? W2 + (size_t)(f0 + row) * K : nullptr;
+        uint32_t w_has = 0, x_has = 0;
+#pragma unroll
+        for (int i = 0; i < WN; ++i) w_has |= (f0 + (row + 16 * i) % FEATS < N ? 1u : 0u) << i;
+#pragma unroll
+        for (int i = 0; i < XN; ++i) x_has |= (t0 + row + 16 * i < M ? 1u : 0u) << i;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        int k = kb0 * BK + k4 * 4;
+        auto load_w = [&](int i, bool in) {
+            const float* p = DUAL && i >= WN / 2 ? wp2 + (size_t)(i - WN / 2) * stride : wp + (size_t)i * stride;
+            return in && ((w_has >> i) & 1) ? load_weight(p + k) : zero;
+        };
+        auto load_x = [&](int i, bool in) {
+            return in && ((x_has >> i) & 1) ? load_written(xp + (size_t)i * stride + k) : zero;
+        };
+        float4 wv[WN], xv[XN];
+#pragma unroll
+        for (int i = 0; i < WN; ++i) wv[i] = load_w(i, k < K);
+        wait_for_previous_kernels();
+#pragma unroll
+        for (int i = 0; i < XN; ++i) xv[i] = load_x(i, k < K);
+        float odd = 0.f;
+        for (int b = 0; b < n_kb; ++b) {
+            const int s = b % STAGES;
+            if (!mbar_wait(smem_u32(&empty_bar[s]), (uint32_t)((b / STAGES) & 1) ^ 1u)) {
+                if (!abort_flag && lane == 0) report(status, ST_CUT_TIMEOUT);
+                abort_flag = 1;
+            }
+            if (abort_flag) break;
+            k += BK;
+            const bool more = b + 1 < n_kb && k < K;             // these registers take the next 64 of K as soon as they are cut
+            const uint32_t stage = base + (uint32_t)(s * STAGE) + col;
+#pragma unroll
+            for (int i = 0; i < WN; ++i) {
+                put(stage + (uint32_t)(i * 16 * 128), PART, wv[i], odd);
+                wv[i] = load_w(i, more);
+            }
+#pragma unroll
+            for (int i = 0; i < XN; ++i) {
+                put(stage + 3 * PART + (uint32_t)(i * 16 * 128), X_PART, xv[i], odd);
+                xv[i] = load_x(i, more);
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the MMA reads what was just stored
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&full_bar[s]));
+        }
+        if (odd != odd) odd_flag = 1;
+    } else {
+        // ---- add the sums of 64 steps onto float32 registers: a thread owns a row of W (a TMEM lane) ----
+        // The first of these warps also issues the MMAs, two blocks of K ahead of the one being added (a warp of its own for
+        // that would leave every thread fewer registers than the sums of 128 columns take).
+        constexpr int COLS = TN / 2;                             // four warps add the first half of the columns, four the second
+        const int q = warp & 3, part = (warp - CUT_WARPS) >> 2;  // q: the TMEM lanes this warp may read
+        const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(part * COLS);
+        const uint64_t a_desc = make_smem_desc(base), b_desc = make_smem_desc(base + 3 * PART);
+        auto issue = [&](int b) {                                // one lane
+            const int s = b % STAGES, buf = b & 1;
+            if (!(mbar_wait(smem_u32(&acc_empty[buf]), (uint32_t)((b >> 1) & 1) ^ 1u) &&
+                  mbar_wait(smem_u32(&full_bar[s]), (uint32_t)((b / STAGES) & 1)))) {
+                report(status, ST_MMA_TIMEOUT);
+                abort_flag = 1;
+                return;
+            }
+            tc_fence_after();
+            const uint64_t off = (uint64_t)((uint32_t)(s * STAGE) >> 4);
+            const uint32_t acc = tmem + (uint32_t)(buf * TN);
+            // (part of W, part of X), the smallest products first: the sum they start is rounded at their own size
+            constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+            for (int p = 0; p < 6; ++p)
+#pragma unroll
+                for (int k = 0; k < BK / 16; ++k)
+                    umma(acc, a_desc + off + (uint64_t)(PA[p] * (PART >> 4) + 2 * k), b_desc + off + (uint64_t)(PB[p] * (X_PART >> 4) + 2 * k),
+                         IDESC, p > 0 || k > 0);
+            umma_commit(smem_u32(&empty_bar[s]));
+            umma_commit(smem_u32(&acc_full[buf]));
+        };
+        if (warp == CUT_WARPS && lane == 0)
+            for (int b = 0; b < 2 && b < n_kb && !abort_flag; ++b) issue(b);
+        __syncwarp();
+        float acc[COLS];
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) acc[c] = 0.f;
+        for (int b = 0; b < n_kb; ++b) {
+            const int buf = b & 1;
+            const bool landed = !abort_flag && mbar_wait(smem_u32(&acc_full[buf]), (uint32_t)((b >> 1) & 1));
+            if (!landed && lane == 0) {
+                if (!abort_flag) report(status, ST_ADD_TIMEOUT);
+                abort_flag = 1;
+            }
+            __syncwarp();
+            if (abort_flag) break;
+            tc_fence_after();
+            // half of the columns at a time: a trip to tensor memory takes as long for 32 columns as for 16
+            constexpr int AT_ONCE = COLS < 32 ? COLS : 32;
+#pragma unroll
+            for (int c0 = 0; c0 < COLS; c0 += AT_ONCE) {
+                uint32_t v[AT_ONCE];
+#pragma unroll
+                for (int c = 0; c < AT_ONCE; c += 16) tmem_ld16(trow + (uint32_t)(buf * TN + c0 + c), v + c);
+                tmem_wait_ld();
+#pragma unroll
+                for (int j = 0; j < AT_ONCE; ++j) acc[c0 + j] += __uint_as_float(v[j]);
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(smem_u32(&acc_empty[buf]));
+                if (warp == CUT_WARPS && b + 2 < n_kb) issue(b + 2);
+            }
+            __syncwarp();
+        }
+        // the last MMAs have finished: nothing reads the stages any more
+        if (!abort_flag) {
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) pieces[(part * COLS + c) * ROWS + q * 32 + lane] = acc[c];
+        }
+    }
+    __syncwarp();
+    wait_for_previous_kernels();          // every thread may read and write `out` below
+    tc_fence_before();
+    __syncthreads();
+    if (warp == CUT_WARPS) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)TMEM_COLS) : "memory");
+    }
+    const bool failed = abort_flag != 0;
+    if (odd_flag && !failed) {
+        // infinite or NaN operands: this block's piece again, as a plain float32 sum
+        const int k_end = min(K, (kb0 + n_kb) * BK);
+        for (int i = threadIdx.x; i < TN * ROWS; i += SPLIT_THREADS) {
+            const int c = i / ROWS;
+            const float* wr = weight_row(i % ROWS);
+            float v = 0.f;
+            if (wr != nullptr && t0 + c < M)
+                for (int kk = kb0 * BK; kk < k_end; ++kk) v = fmaf(X[(size_t)(t0 + c) * K + kk], wr[kk], v);
+            pieces[i] = v;
+        }
+        __syncthreads();
+    }
+    if (splits > 1) cluster_sync();
+    const Forms forms = load_forms<MODE>(bias);
+    const int from = TN * FEATS / splits * rank, to = from + TN * FEATS / splits;      // TN * FEATS is a multiple of 8
+    for (int i = from + (int)threadIdx.x; i < to && !failed; i += SPLIT_THREADS) {
+        const int c = i / FEATS, fl = i - c * FEATS, f = f0 + fl;
+        if (t0 + c >= M || f >= N) continue;
+        const int at = c * ROWS + fl;
+        float v = 0.f, up = 0.f;
+        if (splits > 1) {
+            for (int p = 0; p < splits; ++p) {
+                v += peer_float(pieces + at, (uint32_t)p);
+                if (DUAL) up += peer_float(pieces + at + FEATS, (uint32_t)p);
+            }
+        } else {
+            v = pieces[at];
+            if (DUAL) up = pieces[at + FEATS];
+        }
+        finish<MODE>(out, (size_t)(t0 + c) * N + f, f, v, up, bias, forms);
+    }
+    if (splits > 1) cluster_sync();          // a peer may still be reading this block's pieces
+}
+
+template <int TN, int MODE>
+int launch_split(const float* X, const float* W, const float* W2, const float* bias, float* out, int M, int N, int K, int* status,
+                 cudaStream_t stream) {
+    constexpr int FEATS = MODE == 3 ? ROWS / 2 : ROWS;
+    constexpr int SMEM = STAGES * 3 * (PART + TN * BK * 2) + 1024;
+    static PerDeviceOnce once;
+    if (int rc = raise_dynamic_smem(gemm_f32_split_kernel<TN, MODE>, SMEM, once, "gemm_f32")) return rc;
+    const long long tiles = (long long)((M + TN - 1) / TN) * ((N + FEATS - 1) / FEATS);
+    const int total_kb = (K + BK - 1) / BK;
+    // K over the blocks of a cluster while that shortens the run of the fullest SM: rounds of the grid (one block per SM;
+    // clusters of eight leave some SMs out) times blocks of K, plus what a tile costs besides (about three blocks of K, one
+    // more where pieces meet)
+    int splits = 1;
+    long long best = 0;
+    for (int s = 1; s <= 8 && s <= total_kb; s *= 2) {
+        const long long at_once = s == 8 ? 128 : s == 4 ? 144 : SMS;
+        const long long cost = ((tiles * s + at_once - 1) / at_once) * ((total_kb + s - 1) / s + 3 + (s > 1));
+        if (s == 1 || cost < best) { splits = s; best = cost; }
+    }
+    if (tiles * splits > 0x7fffffffLL) return fail("gemm_f32: %lld tiles", tiles);
+    return launch_cluster("gemm_f32", gemm_f32_split_kernel<TN, MODE>, dim3((unsigned)(tiles * splits)), SPLIT_THREADS, SMEM, splits, stream, X, W,
+                          W2, bias, out, M, N, K, splits, status);
+}
+
+template <int MODE>
+int dispatch(const float* X, const float* W, const float* W2, const float* bias, float* out, int M, int N, int K, int* status,
+             int few_max, cudaStream_t stream) {
+    // Up to 16 rows the read of W past them is the faster one everywhere it was tried (us, few rows against tensor cores):
+    // 16 x 8,960 x 1,536 gated 37.7 / 42.3, 16 x 1,536 x 8,960 33.0 / 34.6, 16 x 151,936 x 896 153 / 234, 4 x 8,960 x 1,536 gated
+    // 22.5 / 41.7 (16.9 at the memory's rate; the FFMA kernel of square tiles: 160).
+    if (M <= few_max) {
+        const int rows = M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : M <= 8 ? 8 : 16;
+        const int rw = rows <= 4 ? 2 : 4;
+        const int splits = few_splits(rows, FEW_WARPS * (MODE == 3 ? rw / 2 : rw), N, K);
+        if (splits > 0) {
+            if (rows == 1) return launch_few<1, 2, 4, MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
+            if (rows == 2) return launch_few<2, 2, 4, MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
+            if (rows == 4) return launch_few<4, 2, 4, MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
+            if (rows == 8) return launch_few<8, 4, 2, MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
+            return launch_few<16, 4, 2, MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
+        }
+    }
+    if (M <= 32) return launch_split<32, MODE>(X, W, W2, bias, out, M, N, K, status, stream);
+    if (M <= 64) return launch_split<64, MODE>(X, W, W2, bias, out, M, N, K, status, stream);
+    return launch_split<128, MODE>(X, W, W2, bias, out, M, N, K, status, stream);
+}
+
+}  // namespace
+
+// `mode`: the epilogue; `few_max`: up to how many rows the kernel for few rows is taken (0: never; at most 16; negative:
+// the default).
+RI_API int ri_gemm_f32(const float* X, const float* W, const float* W2, const float* bias, float* out, int mode, int M, int N, int K,
+                       int few_max, int* status, cudaStream_t stream) {
+    if (M <= 0 || N <= 0) return 0;
+    if (K <= 0 || K % 4) return fail("gemm_f32: K must be a positive multiple of 4, found %d", K);
+    if (((uintptr_t)X | (uintptr_t)W | (uintptr_t)W2) % 16) return fail("gemm_f32: operands must be 16-byte aligned");
+    if (mode == 3 && W2 == nullptr) return fail("gemm_f32: the gated epilogue needs a second matrix");
+    if (mode == 2 && bias != nullptr) return fail("gemm_f32: the residual epilogue takes no bias");
+    if ((mode == 4 || mode == 5) && bias == nullptr) return fail("gemm_f32: epilogue %d needs its constants", mode);
+    if (few_max < 0 || few_max > FEW_MAX) few_max = FEW_MAX;
+    switch (mode) {
+        case 0:
+        case 1: return dispatch<1>(X, W, W2, bias, out, M, N, K, status, few_max, stream);
+        case 2: return dispatch<2>(X, W, W2, bias, out, M, N, K, status, few_max, stream);
+        case 3: return dispatch<3>(X, W, W2, bias, out, M, N, K, status, few_max, stream);
+        case 4: return dispatch<4>(X, W, W2, bias, out, M, N, K, status, few_max, stream);
+        case 5: return dispatch<5>(X, W, W2, bias, out, M, N, K, status, few_max, stream);
+    }
+    return fail("gemm_f32: unknown epilogue mode %d", mode);
+}
+
+RI_DEFINE_LAST_ERROR()

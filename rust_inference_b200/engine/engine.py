@@ -143,9 +143,8 @@ class Engine:
         """Raise if a kernel gave up on a bounded wait since the last check (meaningful after a
         synchronisation point: a device-to-host read of the step's result); in the checked build
         (RI_B200_CHECK_BOUNDS=1) also if a kernel met an index outside its table."""
-        if self.dtype == torch.bfloat16:
-            from ..kernels import tcgen05
-            tcgen05.check_status()
+        from ..kernels import tcgen05
+        tcgen05.check_status()
         from ..kernels import ops
         if ops.checked_build():
             found = ops.bounds_report()

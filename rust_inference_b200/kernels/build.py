@@ -25,6 +25,7 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 MODULES = {
     "elementwise": "elementwise.cu",
     "gemm_simt": "gemm_simt.cu",
+    "gemm_f32": "gemm_f32.cu",
     "attention_generic": "attention_generic.cu",
     "sampling": "sampling.cu",
     "gemm_tcgen05": "gemm_tcgen05.cu",

@@ -1,7 +1,9 @@
 """The contractions of the decoder, out = x @ W^T, each with its epilogue fused.
 
 Which kernel runs is decided here, by dtype and shape:
-  float32   always the FFMA kernel (`gemm_simt`): no tensor-core mode touches a 32-bit run;
+  float32   the kernels of `gemm_f32` (FFMA for a few tokens; beyond, three bfloat16 parts per operand on the
+            tensor cores, which together are the operand) when rows are whole 16-byte pieces, else the FFMA
+            kernel (`gemm_simt`);
   bfloat16  the tcgen05 kernel (`gemm_tcgen05`) when the shape meets its alignment rule,
             else the FFMA kernel on bf16 operands.  Either way accumulation is float32.
 """
@@ -31,6 +33,19 @@ def _use_tensor_cores(x: torch.Tensor, w: Weight) -> bool:
     return tcgen05.supports(x, w)
 
 
+# Three bfloat16 parts leave out products below 2^-24 of a term, which a sum of few terms shows: against 64 bits the tensor
+# cores' product errs by 1.0e-7 at K = 4 and 1.1e-7 at 36 (FFMA: 0.4e-7 and 1.1e-7), by 1.3e-7 at 192 and 1.5e-7 at 4,864
+# (FFMA: 2.5e-7 and 12e-7).
+F32_PARTS_MIN_K = 128
+
+
+def _plain(x, w: Weight, out, mode, w2: Weight | None = None, **constants):
+    """The product without bfloat16 tensor cores."""
+    t2 = w2.t if w2 is not None else None
+    run = ops.gemm_f32 if ops.gemm_f32_supports(x, w.t, t2) and (x.shape[0] <= 16 or w.k >= F32_PARTS_MIN_K) else ops.gemm_simt
+    return run(x, w.t, out, mode, w2=t2, **constants)
+
+
 on_tensor_cores = _use_tensor_cores      # for callers that choose their path by it
 
 
@@ -39,7 +54,7 @@ def project(x, w: Weight, out, ctx, bias=None):
     if _use_tensor_cores(x, w):
         from . import tcgen05
         return tcgen05.gemm(x, w, out, ops.EPI_STORE, ctx, bias=bias)
-    return ops.gemm_simt(x, w.t, out, ops.EPI_STORE, bias=bias)
+    return _plain(x, w, out, ops.EPI_STORE, bias=bias)
 
 
 def logits(x, w: Weight, out, ctx, silu_cols=None):
@@ -48,11 +63,11 @@ def logits(x, w: Weight, out, ctx, silu_cols=None):
         if _use_tensor_cores(x, w):
             from . import tcgen05
             return tcgen05.gemm(x, w, out, ops.EPI_SILU_F32, ctx, silu_cols=silu_cols)
-        return ops.gemm_simt(x, w.t, out, ops.EPI_SILU_F32, silu_cols=silu_cols)
+        return _plain(x, w, out, ops.EPI_SILU_F32, silu_cols=silu_cols)
     if _use_tensor_cores(x, w):
         from . import tcgen05
         return tcgen05.gemm(x, w, out, ops.EPI_STORE_F32, ctx)
-    return ops.gemm_simt(x, w.t, out, ops.EPI_STORE_F32)
+    return _plain(x, w, out, ops.EPI_STORE_F32)
 
 
 def into_residual(x, w: Weight, residual, ctx):
@@ -60,7 +75,7 @@ def into_residual(x, w: Weight, residual, ctx):
     if _use_tensor_cores(x, w):
         from . import tcgen05
         return tcgen05.gemm(x, w, residual, ops.EPI_RESIDUAL, ctx)
-    return ops.gemm_simt(x, w.t, residual, ops.EPI_RESIDUAL)
+    return _plain(x, w, residual, ops.EPI_RESIDUAL)
 
 
 def gated(x, w_gate: Weight, w_up: Weight, out, ctx, form=None):
@@ -70,7 +85,7 @@ def gated(x, w_gate: Weight, w_up: Weight, out, ctx, form=None):
     if _use_tensor_cores(x, w_gate):
         from . import tcgen05
         return tcgen05.gemm(x, w_gate, out, ops.EPI_SILU_MUL, ctx, w2=w_up, gate_form=form)
-    return ops.gemm_simt(x, w_gate.t, out, ops.EPI_SILU_MUL, w2=w_up.t, gate_form=form)
+    return _plain(x, w_gate, out, ops.EPI_SILU_MUL, w_up, gate_form=form)
 
 
 def activated(x, w: Weight, out, ctx, form):
@@ -79,7 +94,7 @@ def activated(x, w: Weight, out, ctx, form):
     if _use_tensor_cores(x, w):
         from . import tcgen05
         return tcgen05.gemm(x, w, out, ops.EPI_ACT, ctx, act_form=form)
-    return ops.gemm_simt(x, w.t, out, ops.EPI_ACT, act_form=form)
+    return _plain(x, w, out, ops.EPI_ACT, act_form=form)
 
 
 def accumulate_split(x, w: Weight, acc, ctx) -> bool:

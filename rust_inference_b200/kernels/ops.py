@@ -405,15 +405,9 @@ def whole_act_form(form: torch.Tensor) -> torch.Tensor:
     return form
 
 
-def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, *,
-              bias: torch.Tensor | None = None, w2: torch.Tensor | None = None,
-              gate_form: torch.Tensor | None = None, act_form: torch.Tensor | None = None,
-              silu_cols: torch.Tensor | None = None) -> torch.Tensor:
-    """out = x @ w.T with the chosen epilogue, on the FFMA pipe (float32 accumulate).  gate_form (gated
-    epilogue only): float32 [5] on the device (`gate_form`; the first three alone are accepted), {alpha, limit, shift, cubic, mult} of mult g' sigmoid(alpha g' (1 + cubic g'^2)) (u' + shift) with
-    g' = min(g, limit), u' = clamp(u, -limit, limit); None: SiLU(g) * u.  act_form (EPI_ACT only): float32 [4] on the
-    device, the activation's constants (`RELU_SQUARED_FORM`; two learned ones alone are accepted, `whole_act_form`).
-    silu_cols (EPI_SILU_F32 only): float32 [1] on the device, how many of the first columns become silu of themselves."""
+def _gemm_constants(x, w, out, mode, bias, w2, gate_form, act_form, silu_cols):
+    """Checks a product's arguments; the constants its epilogue takes (its bias, or those of a gate, an activation or the
+    activated columns, which travel in the bias's place)."""
     _need_cuda(x, w, out, bias, w2)
     m, k = x.shape
     n = w.shape[0]
@@ -441,8 +435,44 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, *,
         _need(bias is None and silu_cols.is_cuda and silu_cols.dtype == torch.float32 and silu_cols.numel() == 1,
               "gemm: the number of activated columns is one float32 on the device, and its epilogue takes no bias")
         bias = silu_cols
+    return bias
+
+
+def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, *,
+              bias: torch.Tensor | None = None, w2: torch.Tensor | None = None,
+              gate_form: torch.Tensor | None = None, act_form: torch.Tensor | None = None,
+              silu_cols: torch.Tensor | None = None) -> torch.Tensor:
+    """out = x @ w.T with the chosen epilogue, on the FFMA pipe (float32 accumulate).  gate_form (gated
+    epilogue only): float32 [5] on the device (`gate_form`; the first three alone are accepted), {alpha, limit, shift, cubic, mult} of mult g' sigmoid(alpha g' (1 + cubic g'^2)) (u' + shift) with
+    g' = min(g, limit), u' = clamp(u, -limit, limit); None: SiLU(g) * u.  act_form (EPI_ACT only): float32 [4] on the
+    device, the activation's constants (`RELU_SQUARED_FORM`; two learned ones alone are accepted, `whole_act_form`).
+    silu_cols (EPI_SILU_F32 only): float32 [1] on the device, how many of the first columns become silu of themselves."""
+    bias = _gemm_constants(x, w, out, mode, bias, w2, gate_form, act_form, silu_cols)
+    m, k = x.shape
     _call("gemm_simt", "ri_gemm_simt", _p(x), _p(w), _p(w2), _p(bias), _p(out), c_int(dtype_code(x.dtype)),
-          c_int(mode), c_int(m), c_int(n), c_int(k), _stream())
+          c_int(mode), c_int(m), c_int(w.shape[0]), c_int(k), _stream())
+    return out
+
+
+def gemm_f32_supports(x: torch.Tensor, w: torch.Tensor, w2: torch.Tensor | None = None) -> bool:
+    """What the float32 kernels ask for: rows of whole 16-byte pieces, 16-byte aligned operands."""
+    return (x.dtype == torch.float32 and w.dtype == torch.float32 and x.shape[1] % 4 == 0 and x.data_ptr() % 16 == 0
+            and w.data_ptr() % 16 == 0 and (w2 is None or w2.data_ptr() % 16 == 0))
+
+
+def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, *, bias: torch.Tensor | None = None,
+             w2: torch.Tensor | None = None, gate_form: torch.Tensor | None = None, act_form: torch.Tensor | None = None,
+             silu_cols: torch.Tensor | None = None, few_max: int = -1) -> torch.Tensor:
+    """`gemm_simt` for float32 operands that `gemm_f32_supports`: a kernel that streams w past a few rows of x, and for more
+    rows one whose operands are cut into three bfloat16 parts for the tensor cores (csrc/gemm_f32.cu).  few_max: up to how
+    many rows of x the first one is taken (at most 16; negative: the default), for comparisons and tests."""
+    bias = _gemm_constants(x, w, out, mode, bias, w2, gate_form, act_form, silu_cols)
+    _need(x.dtype == torch.float32, "gemm_f32: float32 operands")
+    m, k = x.shape
+    from . import tcgen05
+    st = tcgen05.status_word()
+    _call("gemm_f32", "ri_gemm_f32", _p(x), _p(w), _p(w2), _p(bias), _p(out), c_int(mode), c_int(m), c_int(w.shape[0]),
+          c_int(k), c_int(few_max), c_void_p(st.data_ptr()), _stream())
     return out
 
 

@@ -29,6 +29,9 @@ STATUS_TEXT = {
     32: "experts: the MMA issuer waited too long for a TMA load",
     33: "experts: the epilogue waited too long for the accumulator",
     34: "experts: a TMA load did not land before the CTA had to leave",
+    41: "float32 product: the reading warps waited too long for a free stage",
+    42: "float32 product: the MMA issuer waited too long for operands or for its accumulator",
+    43: "float32 product: the adding warps waited too long for the accumulator",
 }
 
 

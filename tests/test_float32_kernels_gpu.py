@@ -1,0 +1,97 @@
+"""The kernels of the 32-bit path alone: products by a few rows and by many (operands in three bfloat16 parts on the tensor
+cores), at the edges of their tiles."""
+import pytest
+import torch
+
+import plain_impl
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _ops():
+    from rust_inference_b200.kernels import ops
+    return ops
+
+
+def _check_status():
+    from rust_inference_b200.kernels import tcgen05
+    torch.cuda.synchronize()
+    tcgen05.check_status()
+
+
+@pytest.mark.parametrize("few_max", [-1, 0])          # the default choice; the tensor cores for few rows too
+@pytest.mark.parametrize("m", [1, 2, 3, 8, 9, 16, 17, 32, 33, 64, 65, 128, 130, 300])
+@pytest.mark.parametrize("n, k", [(7, 4), (100, 36), (391, 192), (130, 1032), (1152, 896), (264, 4864)])
+def test_product(m, n, k, few_max):
+    """Every epilogue against 64 bits.  The bound: a float32 sum of k products, each rounded (2^-24 of the running sum),
+    errs by about 2^-24 sqrt(k) of a typical result, and the largest of m n results lies a few times above typical;
+    2e-6 of the largest is what the FFMA kernel's test asks for."""
+    ops = _ops()
+    torch.manual_seed(m * 1000 + n)
+    x = torch.randn(m, k, device=DEV) * 0.5
+    w = torch.randn(n, k, device=DEV) * 0.1
+    w2 = torch.randn(n, k, device=DEV) * 0.1
+    bias = torch.randn(n, device=DEV)
+    ref, ref2 = x.double() @ w.double().t(), x.double() @ w2.double().t()
+    scale = ref.abs().max().item()
+    assert ops.gemm_f32_supports(x, w, w2)
+
+    def run(mode, start=None, **kw):
+        out = torch.full((m, n), 9.0, device=DEV) if start is None else start.clone()
+        ops.gemm_f32(x, w, out, mode, few_max=few_max, **kw)
+        again = torch.full((m, n), 7.0, device=DEV) if start is None else start.clone()
+        ops.gemm_f32(x, w, again, mode, few_max=few_max, **kw)
+        assert torch.equal(out, again)                                     # sums in a fixed order
+        return out.double()
+
+    assert (run(ops.EPI_STORE, bias=bias) - (ref + bias)).abs().max().item() <= 2e-6 * (scale + bias.abs().max().item())
+    assert (run(ops.EPI_STORE_F32) - ref).abs().max().item() <= 2e-6 * scale
+    before = torch.randn(m, n, device=DEV)
+    assert (run(ops.EPI_RESIDUAL, start=before) - (before + ref)).abs().max().item() <= 2e-6 * (scale + 4)
+    want = plain_impl.silu(ref) * ref2
+    assert (run(ops.EPI_SILU_MUL, w2=w2) - want).abs().max().item() <= 4e-6 * (want.abs().max().item() + 1e-3)
+    cols = torch.tensor([float(n // 2)], device=DEV)
+    want = torch.cat([plain_impl.silu(ref[:, :n // 2]), ref[:, n // 2:]], 1)
+    assert (run(ops.EPI_SILU_F32, silu_cols=cols) - want).abs().max().item() <= 2e-6 * (scale + 1e-3)
+    form = torch.tensor(ops.RELU_SQUARED_FORM, device=DEV)
+    want = ref.clamp_min(0) ** 2
+    assert (run(ops.EPI_ACT, act_form=form) - want).abs().max().item() <= 4e-6 * (want.abs().max().item() + 1e-3)
+    _check_status()
+
+
+@pytest.mark.parametrize("m", [3, 40, 200])
+def test_product_with_infinities(m):
+    """Infinite and NaN operands come out as the plain float32 sum gives them, and leave other rows alone."""
+    ops = _ops()
+    torch.manual_seed(5)
+    x, w = torch.randn(m, 640, device=DEV), torch.randn(200, 640, device=DEV)
+    clean = torch.empty(m, 200, device=DEV)
+    ops.gemm_f32(x, w, clean, ops.EPI_STORE_F32)
+    x[1, 100], x[2, 600] = float("inf"), float("nan")
+    w[3, 630] = float("-inf")
+    x[0, 0] = 3e38                        # its product with most weights overflows
+    w[4, :] = 0.0
+    got, want = torch.empty(m, 200, device=DEV), torch.empty(m, 200, device=DEV)
+    ops.gemm_f32(x, w, got, ops.EPI_STORE_F32)
+    ops.gemm_simt(x, w, want, ops.EPI_STORE_F32)
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    assert torch.equal(got[got.isinf()], want[got.isinf()])
+    rows = [r for r in range(3, m)]
+    cols = [c for c in range(200) if c not in (3, 4)]
+    if rows:
+        assert (got[rows][:, cols] - clean[rows][:, cols]).abs().max().item() <= 2e-6 * clean.abs().max().item()
+    _check_status()
+
+
+def test_product_with_small_and_large_numbers():
+    """Three parts hold a float32 number over its whole range: scaling the operands by powers of two scales the result."""
+    ops = _ops()
+    torch.manual_seed(6)
+    x, w = torch.randn(130, 256, device=DEV), torch.randn(140, 256, device=DEV)
+    base, out = torch.empty(130, 140, device=DEV), torch.empty(130, 140, device=DEV)
+    ops.gemm_f32(x, w, base, ops.EPI_STORE_F32)
+    for up, down in ((2.0 ** 100, 2.0 ** -60), (2.0 ** -80, 2.0 ** 70)):
+        ops.gemm_f32(x * up, w * down, out, ops.EPI_STORE_F32)
+        assert torch.equal(out, base * (up * down))
+    _check_status()
