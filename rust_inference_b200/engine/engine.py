@@ -144,7 +144,9 @@ class Engine:
         synchronisation point: a device-to-host read of the step's result); in the checked build
         (RI_B200_CHECK_BOUNDS=1) also if a kernel met an index outside its table."""
         from ..kernels import tcgen05
-        tcgen05.check_status()
+        if self.dtype == torch.bfloat16:
+            tcgen05.check_status()
+        tcgen05.check_f32_status()
         from ..kernels import ops
         if ops.checked_build():
             found = ops.bounds_report()

@@ -470,7 +470,7 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, *, 
     _need(x.dtype == torch.float32, "gemm_f32: float32 operands")
     m, k = x.shape
     from . import tcgen05
-    st = tcgen05.status_word()
+    st = tcgen05.f32_status_word()
     _call("gemm_f32", "ri_gemm_f32", _p(x), _p(w), _p(w2), _p(bias), _p(out), c_int(mode), c_int(m), c_int(w.shape[0]),
           c_int(k), c_int(few_max), c_void_p(st.data_ptr()), _stream())
     return out

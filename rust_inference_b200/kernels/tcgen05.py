@@ -10,6 +10,7 @@ from . import build, ops
 from .ops import KernelError, _call, _need, _need_cuda, _p, _stream
 
 _status = None     # host-visible word a kernel writes when one of its bounded waits ran out
+_f32_status = None # the same for the float32 products, which a 32-bit run looks at
 _x_maps: dict = {}  # tensor maps of activation buffers, by (pointer, rows, K, token tile)
 
 STATUS_TEXT = {
@@ -42,12 +43,28 @@ def status_word() -> torch.Tensor:
     return _status
 
 
+def f32_status_word() -> torch.Tensor:
+    global _f32_status
+    if _f32_status is None:
+        _f32_status = torch.zeros(1, dtype=torch.int32).pin_memory()
+    return _f32_status
+
+
 def check_status() -> None:
-    """Raise if any tensor-core kernel since the last check gave up on a wait.  Call after a
+    """Raise if any bfloat16 tensor-core kernel since the last check gave up on a wait.  Call after a
     synchronisation point (the word lives in pinned host memory the device writes to)."""
-    if _status is not None and int(_status[0]) != 0:
-        code = int(_status[0])
-        _status[0] = 0
+    _check(_status)
+
+
+def check_f32_status() -> None:
+    """The same for the float32 products."""
+    _check(_f32_status)
+
+
+def _check(word) -> None:
+    if word is not None and int(word[0]) != 0:
+        code = int(word[0])
+        word[0] = 0
         raise KernelError(f"a tensor-core kernel gave up: {STATUS_TEXT.get(code, f'code {code}')}")
 
 

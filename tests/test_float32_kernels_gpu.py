@@ -17,7 +17,7 @@ def _ops():
 def _check_status():
     from rust_inference_b200.kernels import tcgen05
     torch.cuda.synchronize()
-    tcgen05.check_status()
+    tcgen05.check_f32_status()
 
 
 @pytest.mark.parametrize("few_max", [-1, 0])          # the default choice; the tensor cores for few rows too
