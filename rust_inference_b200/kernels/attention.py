@@ -9,6 +9,8 @@
                                  a gate on the tcgen05 kernel
   bfloat16, head_dim 64 or 128,  values of 32, 64 or 128: the TMA-fed decode kernel and the tcgen05 prefill kernel, in their
   values of another size         instances for both sizes
+  float32, head_dim 64 or 128,   tiles of query rows over whole pages (`attention_f32`)
+  the plain form of the score
   anything else                  the generic kernel (`attention_generic`): any head size, any
                                  dtype, float32 arithmetic
 
@@ -51,6 +53,19 @@ def decode_splits(n_seqs: int, n_kv_heads: int, max_seq_len: int, page_size: int
     if os.environ.get("RI_B200_DECODE_SPLITS"):
         want = int(os.environ["RI_B200_DECODE_SPLITS"])
     return max(1, min(want, limit, -(-max_seq_len // page_size)))
+
+
+def f32_splits(n_seqs: int, max_new: int, n_heads: int, n_kv_heads: int, head_dim: int, longest: int, page_size: int) -> int:
+    """Thread blocks (1..8, a cluster) that share the pages of a tile of query rows in the float32 kernels: as many as keep
+    the step's tiles resident at once (an SM holds one block of 64 rows of 128 channels or three of 64, two of up to 8 rows,
+    one of 16), never more than the longest sequence has pages.  Tiles of 64 rows take two at most: merging 64 rows costs
+    more than it saves beyond (333 tokens, 14 heads of 64: 33 us with one, 21 with two, 28 with six)."""
+    rows = max_new * (n_heads // n_kv_heads)
+    few = rows <= 16
+    tiles = n_seqs * n_kv_heads * (1 if few else -(-rows // 64))
+    per_sm = (2 if rows <= 8 else 1) if few else (1 if head_dim == 128 else 3)
+    most = CLUSTER_SPLITS if few else 2
+    return max(1, min(most, per_sm * _sm_count() // tiles, -(-longest // page_size)))
 
 
 def decode_plan(n_seqs: int, n_kv_heads: int, max_seq_len: int, page_size: int, head_dim: int | None = None,
@@ -179,6 +194,14 @@ def attention(qkv, cache_layer, out, ctx, *, n_heads, n_kv_heads, head_dim, scal
             n_seqs=ctx.n_seqs, max_new=ctx.max_new, n_heads=n_heads, n_kv_heads=n_kv_heads, head_dim=head_dim,
             page_size=ctx.page_size, scale=scale, window=window or 0, softcap=softcap, keep_first=keep_first, sink=sink,
             dist=dist, gate=gate, out_scale=out_scale)
+    if (same_sizes and not (window and chunk) and plain
+            and ops.attention_f32_supports(qkv, q_ld, out, head_dim, ctx.page_size)):
+        longest = ctx.page_table.shape[1] * ctx.page_size if ctx.all_single else ctx.max_len
+        return ops.attention_f32(
+            qkv, q_ld, cache_layer.k, cache_layer.v, ctx.page_table, ctx.seq_slot, ctx.seq_start, ctx.cu_seqlens, out,
+            n_seqs=ctx.n_seqs, max_new=ctx.max_new, n_heads=n_heads, n_kv_heads=n_kv_heads, head_dim=head_dim,
+            page_size=ctx.page_size, scale=scale, span=span, out_scale=out_scale,
+            n_splits=f32_splits(ctx.n_seqs, ctx.max_new, n_heads, n_kv_heads, head_dim, longest, ctx.page_size))
     return ops.attention_generic(
         qkv, q_ld, cache_layer.k, cache_layer.v, ctx.page_table, ctx.token_pos, ctx.token_seq,
         ctx.seq_slot, out, n_tokens=qkv.shape[0], n_heads=n_heads, n_kv_heads=n_kv_heads,

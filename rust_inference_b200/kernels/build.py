@@ -27,6 +27,7 @@ MODULES = {
     "gemm_simt": "gemm_simt.cu",
     "gemm_f32": "gemm_f32.cu",
     "attention_generic": "attention_generic.cu",
+    "attention_f32": "attention_f32.cu",
     "sampling": "sampling.cu",
     "gemm_tcgen05": "gemm_tcgen05.cu",
     "attention_mma": "attention_mma.cu",

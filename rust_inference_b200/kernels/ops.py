@@ -476,6 +476,29 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, *, 
     return out
 
 
+def attention_f32_supports(q: torch.Tensor, q_ld: int, out: torch.Tensor, head_dim: int, page_size: int) -> bool:
+    """What the float32 attention kernel takes: heads of 64 or 128, pages of 64, rows of whole aligned 16-byte pieces."""
+    return (q.dtype == torch.float32 and out.dtype == torch.float32 and head_dim in (64, 128) and page_size == 64 and q_ld % 4 == 0
+            and out.shape[1] % 4 == 0 and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0)
+
+
+def attention_f32(q: torch.Tensor, q_ld: int, kcache, vcache, page_table, seq_slot, seq_start, cu_seqlens, out: torch.Tensor, *,
+                  n_seqs: int, max_new: int, n_heads: int, n_kv_heads: int, head_dim: int, page_size: int, scale: float,
+                  span: int = 0, out_scale: float = 1.0, n_splits: int = 1) -> torch.Tensor:
+    """Float32 attention of every token of the step over its slot's cached keys (`span` > 0: the last so many, < 0: its own block
+    of -span positions), times out_scale; n_splits (1..8): thread blocks that share the pages of a tile of query rows."""
+    _need_cuda(q, kcache, vcache, page_table, seq_slot, seq_start, cu_seqlens, out)
+    _need(q.dtype == kcache.dtype == vcache.dtype == out.dtype == torch.float32, "attention_f32: float32 only")
+    _need(kcache.is_contiguous() and vcache.is_contiguous() and kcache.shape[1:] == (n_kv_heads, page_size, head_dim)
+          and vcache.shape == kcache.shape, "attention_f32: cache layout")
+    _need(out.shape[1] >= n_heads * head_dim and q.shape[0] == out.shape[0], "attention_f32: bad shapes")
+    _call("attention_f32", "ri_attention_f32", _p(q), c_int(q_ld), _p(kcache), _p(vcache), _p(page_table), c_int(page_table.shape[1]),
+          _p(seq_slot), _p(seq_start), _p(cu_seqlens), _p(out), c_int(out.shape[1]), c_int(n_seqs), c_int(max_new), c_int(n_heads),
+          c_int(n_kv_heads), c_int(head_dim), c_int(page_size), c_float(scale), c_int(span), c_float(out_scale), c_int(n_splits),
+          _stream())
+    return out
+
+
 def attention_generic(q: torch.Tensor, q_ld: int, kcache, vcache, page_table, token_pos, token_seq,
                       seq_slot, out: torch.Tensor, *, n_tokens: int, n_heads: int, n_kv_heads: int,
                       head_dim: int, page_size: int, scale: float, window: int = 0, chunk: int = 0,

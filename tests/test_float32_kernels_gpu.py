@@ -1,5 +1,7 @@
 """The kernels of the 32-bit path alone: products by a few rows and by many (operands in three bfloat16 parts on the tensor
-cores), at the edges of their tiles."""
+cores) and attention in tiles of query rows, at the edges of their tiles."""
+import random
+
 import pytest
 import torch
 
@@ -95,3 +97,46 @@ def test_product_with_small_and_large_numbers():
         ops.gemm_f32(x * up, w * down, out, ops.EPI_STORE_F32)
         assert torch.equal(out, base * (up * down))
     _check_status()
+
+
+@pytest.mark.parametrize("splits", [1, 2, 5, 8])
+@pytest.mark.parametrize("span", [0, 50, -96])
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("heads, kv, starts, news", [
+    (14, 2, [0], [333]), (6, 2, [100, 0, 63, 700], [1, 1, 1, 1]), (8, 8, [5, 0], [70, 3]), (12, 2, [100, 0, 200], [40, 130, 1]),
+    (40, 2, [10, 300], [1, 1]), (16, 1, [127, 128, 0], [1, 1, 1])])
+def test_attention(hd, heads, kv, starts, news, span, splits):
+    """Against the generic kernel, which visits the same keys one by one; places beyond a sequence's end hold NaN."""
+    ops = _ops()
+    rng = random.Random(hd + heads + splits)
+    torch.manual_seed(heads)
+    need = [-(-(s + n) // 64) for s, n in zip(starts, news)]
+    order = list(range(sum(need) + 2))
+    rng.shuffle(order)
+    slots = list(range(len(starts)))
+    rng.shuffle(slots)
+    table = torch.zeros(len(starts), max(need), dtype=torch.int32)
+    kc, vc = torch.randn(len(order), kv, 64, hd), torch.randn(len(order), kv, 64, hd)
+    for b, pages in enumerate(need):
+        for j in range(pages):
+            table[slots[b], j] = order.pop()
+        end = starts[b] + news[b]
+        if end % 64:
+            last = int(table[slots[b], end // 64])
+            kc[last, :, end % 64:] = vc[last, :, end % 64:] = float("nan")
+    total = sum(news)
+    d = lambda t, kind=torch.int32: torch.as_tensor(t, dtype=kind).to(DEV)
+    kc, vc, table = kc.to(DEV), vc.to(DEV), table.to(DEV)
+    q = torch.randn(total, heads * hd + 8, device=DEV)
+    pos = d([s + i for s, n in zip(starts, news) for i in range(n)])
+    seq = d([b for b, n in enumerate(news) for _ in range(n)])
+    cu = d([sum(news[:i]) for i in range(len(news) + 1)])
+    slot, start = d(slots), d(starts)
+    want, got = torch.empty(total, heads * hd, device=DEV), torch.full((total, heads * hd), 7.0, device=DEV)
+    common = dict(n_heads=heads, n_kv_heads=kv, head_dim=hd, page_size=64, scale=hd ** -0.5, out_scale=0.7)
+    ops.attention_generic(q, q.shape[1], kc, vc, table, pos, seq, slot, want, n_tokens=total, window=max(span, 0),
+                          chunk=max(-span, 0), **common)
+    ops.attention_f32(q, q.shape[1], kc, vc, table, slot, start, cu, got, n_seqs=len(news), max_new=max(news), span=span,
+                      n_splits=splits, **common)
+    # two float32 sums over at most 701 keys in different orders
+    assert (got - want).abs().max().item() <= 5e-6 * want.abs().max().item()
