@@ -298,16 +298,27 @@ moe_arrange_kernel(const int* ids, int n_pairs, int experts, int tile_rows, int*
 }
 
 // xs[i, :] = x[order[i] / top, :]: the activations in the order of the list, 16 bytes at a time
-// (width a multiple of 8 bf16).
-__global__ void moe_gather_kernel(const uint4* x, uint4* __restrict__ xs, const int* order,
-                                  int n_pairs, int top, int vecs, const int* listed) {
+// (width a multiple of 8 bf16).  A warp per row: the row's place is looked up once, four pieces are on their way at a time (8,192
+// rows of 2,048: 7.6 us, 11.0 with a thread per piece).
+__global__ void __launch_bounds__(256)
+moe_gather_kernel(const uint4* x, uint4* xs, const int* order, int n_pairs, int top, int vecs, const int* listed) {
     let_next_kernel_start();
     wait_for_previous_kernels();
     // listed: the number of pairs in the lists (the last of the arrange kernel's offsets), where some pairs are in none
-    const size_t total = (size_t)(listed != nullptr ? min(n_pairs, *listed) : n_pairs) * vecs;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int r = (int)(i / vecs), c = (int)(i % vecs);
-        xs[i] = x[(size_t)(order[r] / top) * vecs + c];
+    const int rows = listed != nullptr ? min(n_pairs, *listed) : n_pairs;
+    const int warps = gridDim.x * (blockDim.x >> 5), lane = threadIdx.x & 31;
+    for (int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < rows; r += warps) {
+        const uint4* src = x + (size_t)(order[r] / top) * vecs;
+        uint4* dst = xs + (size_t)r * vecs;
+        for (int c0 = lane; c0 < vecs; c0 += 128) {
+            uint4 v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (c0 + 32 * i < vecs) v[i] = src[c0 + 32 * i];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (c0 + 32 * i < vecs) dst[c0 + 32 * i] = v[i];
+        }
     }
 }
 
@@ -393,26 +404,70 @@ moe_grouped_kernel(const T* X, const T* __restrict__ W, const T* __restrict__ W2
 }
 
 // ids / x / n_real (optional): a chosen id >= n_real hands the token's input row x[t] through instead of a row of y.
-template <typename T>
-__global__ void moe_combine_kernel(float* residual, const float* y, const float* weights, const float* shared_y,
-                                   const float* gate, const int* place, int n_tokens, int width, int top,
-                                   const int* ids, const T* x, int n_real, float scale) {
+// A block takes one token's channels: V at a time (4: whole, aligned 16-byte pieces of every row), the rows of up to four
+// experts read before the first of them is used.  Bound by its bytes, top + 2 float32 rows read and one written per token: 2,048
+// tokens of 2,048 channels and 4 experts (117 MB) 21.0 us, 38.6 with a channel per thread and one expert's row after the other.
+__device__ __forceinline__ float4 four_of(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 four_of(const __nv_bfloat16* p) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+template <typename T, int V>
+__global__ void __launch_bounds__(256)
+moe_combine_kernel(float* residual, const float* y, const float* weights, const float* shared_y, const float* gate, const int* place,
+                   int n_tokens, int width, int top, const int* ids, const T* x, int n_real, float scale) {
+    constexpr int AT_ONCE = 4;
     let_next_kernel_start();
     wait_for_previous_kernels();
-    const size_t total = (size_t)n_tokens * width;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int t = (int)(i / width), d = (int)(i % width);
-        float acc = 0.f;
-        for (int c = 0; c < top; ++c) {
-            const size_t p = (size_t)t * top + c;
-            if (ids != nullptr && ids[p] >= n_real) {
-                acc = fmaf(weights[p], to_f32<T>(x[i]), acc);
-                continue;
+    // blocks beyond one per token share its channels out (steps of few tokens)
+    const int parts = gridDim.y, part = blockIdx.y;
+    for (int t = blockIdx.x; t < n_tokens; t += gridDim.x) {
+        const size_t p0 = (size_t)t * top;
+        const float g = shared_y != nullptr && gate != nullptr ? gate[t] : 1.f;
+        for (int d = (part * (int)blockDim.x + (int)threadIdx.x) * V; d < width; d += parts * (int)blockDim.x * V) {
+            const size_t i = (size_t)t * width + d;
+            float acc[V], add[V], old[V];
+#pragma unroll
+            for (int v = 0; v < V; ++v) acc[v] = 0.f;
+            if (V == 4) {
+                *reinterpret_cast<float4*>(old) = four_of(residual + i);
+                if (shared_y != nullptr) *reinterpret_cast<float4*>(add) = four_of(shared_y + i);
+            } else {
+                old[0] = residual[i];
+                if (shared_y != nullptr) add[0] = shared_y[i];
             }
-            acc = fmaf(weights[p], y[(place != nullptr ? (size_t)place[p] : p) * width + d], acc);
+            for (int c0 = 0; c0 < top; c0 += AT_ONCE) {
+                float w[AT_ONCE], r[AT_ONCE][V];
+#pragma unroll
+                for (int k = 0; k < AT_ONCE; ++k) {
+                    if (c0 + k >= top) continue;
+                    const size_t p = p0 + c0 + k;
+                    w[k] = weights[p];
+                    if (ids != nullptr && ids[p] >= n_real) {
+                        if (V == 4) *reinterpret_cast<float4*>(r[k]) = four_of(x + i);
+                        else r[k][0] = to_f32<T>(x[i]);
+                    } else {
+                        const float* row = y + (place != nullptr ? (size_t)place[p] : p) * width + d;
+                        if (V == 4) *reinterpret_cast<float4*>(r[k]) = four_of(row);
+                        else r[k][0] = *row;
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < AT_ONCE; ++k)
+                    if (c0 + k < top)
+#pragma unroll
+                        for (int v = 0; v < V; ++v) acc[v] = fmaf(w[k], r[k][v], acc[v]);
+            }
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                if (shared_y != nullptr) acc[v] = gate != nullptr ? fmaf(g, add[v], acc[v]) : acc[v] + add[v];
+                old[v] += scale == 1.f ? acc[v] : scale * acc[v];
+            }
+            if (V == 4) *reinterpret_cast<float4*>(residual + i) = *reinterpret_cast<float4*>(old);
+            else residual[i] = old[0];
         }
-        if (shared_y != nullptr) acc = gate != nullptr ? fmaf(gate[t], shared_y[i], acc) : acc + shared_y[i];
-        residual[i] += scale == 1.f ? acc : scale * acc;
     }
 }
 
@@ -481,8 +536,7 @@ RI_API int ri_moe_gather(const void* x, void* xs, const int* order, int n_pairs,
                          cudaStream_t stream) {
     if (n_pairs <= 0) return 0;
     if (width % 8 || (uintptr_t)x % 16 || (uintptr_t)xs % 16) return fail("moe_gather: rows of %d bf16 are not 16-byte runs", width);
-    const size_t total = (size_t)n_pairs * (width / 8);
-    const int blocks = (int)((total + 255) / 256 < 8192 ? (total + 255) / 256 : 8192);
+    const int blocks = min((n_pairs + 7) / 8, 8192);
     cudaError_t e = launch_dependent(moe_gather_kernel, blocks, 256, 0, stream, (const uint4*)x, (uint4*)xs, order, n_pairs,
                                      top, width / 8, listed);
     return check_launch(e, "moe_gather");
@@ -514,17 +568,18 @@ RI_API int ri_moe_combine(float* residual, const float* y, const float* weights,
                           int n_real, float scale, cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
     if ((ids == nullptr) != (x == nullptr)) return fail("moe_combine: ids and the experts' input go together");
-    const size_t total = (size_t)n_tokens * width;
-    const int blocks = (int)((total + 255) / 256 < 8192 ? (total + 255) / 256 : 8192);
+    const bool vec = width % 4 == 0 && ((uintptr_t)residual | (uintptr_t)y | (uintptr_t)shared_y) % 16 == 0 &&
+                     (uintptr_t)x % (x_dtype == RI_BF16 ? 8 : 16) == 0;
+    // a block per token; a step of few tokens cuts a token's channels over as many blocks as its width has runs of 256 threads
+    const int runs = (width + (vec ? 1023 : 255)) / (vec ? 1024 : 256);
+    const dim3 grid(min(n_tokens, 65535), n_tokens < 148 ? min(runs, 64) : 1);
     cudaError_t e;
-    if (x == nullptr || x_dtype == RI_F32)
-        e = launch_dependent(moe_combine_kernel<float>, blocks, 256, 0, stream, residual, y, weights, shared_y, gate, place,
-                             n_tokens, width, top, ids, (const float*)x, n_real, scale);
-    else if (x_dtype == RI_BF16)
-        e = launch_dependent(moe_combine_kernel<__nv_bfloat16>, blocks, 256, 0, stream, residual, y, weights, shared_y, gate,
-                             place, n_tokens, width, top, ids, (const __nv_bfloat16*)x, n_real, scale);
-    else
-        return fail("moe_combine: unknown dtype %d", x_dtype);
+#define RI_COMBINE(T, V) launch_dependent(moe_combine_kernel<T, V>, grid, 256, 0, stream, residual, y, weights, shared_y, gate, place, \
+                                          n_tokens, width, top, ids, (const T*)x, n_real, scale)
+    if (x == nullptr || x_dtype == RI_F32) e = vec ? RI_COMBINE(float, 4) : RI_COMBINE(float, 1);
+    else if (x_dtype == RI_BF16) e = vec ? RI_COMBINE(__nv_bfloat16, 4) : RI_COMBINE(__nv_bfloat16, 1);
+    else return fail("moe_combine: unknown dtype %d", x_dtype);
+#undef RI_COMBINE
     return check_launch(e, "moe_combine");
 }
 

@@ -36,17 +36,34 @@ __device__ __forceinline__ float sigmoid_f32(float x) {
     return e / (1.f + e);
 }
 
-__global__ void recurrence_prepare_kernel(float* __restrict__ z, int ld, const float* __restrict__ bias,
-                                          const float* __restrict__ low, int n_tokens, int qdim) {
+// A block takes one token's channels after the other; VEC: four at a time (rows and channels then come in whole 16-byte pieces).
+// Bound by its bytes: 2,048 tokens of 2 x 1,024 channels (34 MB) 9.6 us, 14.1 one channel at a time over all blocks.
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+recurrence_prepare_kernel(float* z, int ld, const float* __restrict__ bias, const float* __restrict__ low, int n_tokens, int qdim) {
     let_next_kernel_start();
     wait_for_previous_kernels();
-    const size_t total = (size_t)n_tokens * qdim;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int t = (int)(i / qdim), c = (int)(i % qdim);
+    for (int t = blockIdx.x; t < n_tokens; t += gridDim.x) {
         float* row = z + (size_t)t * ld;
-        row[c] = silu_f32(row[c]);
-        const float l = low[c];
-        row[qdim + c] = l + (1.f - l) * sigmoid_f32(row[qdim + c] + bias[c]);
+        if (VEC) {
+            for (int c = threadIdx.x * 4; c < qdim; c += blockDim.x * 4) {
+                float4 q = *reinterpret_cast<float4*>(row + c), f = *reinterpret_cast<float4*>(row + qdim + c);
+                const float4 b = *reinterpret_cast<const float4*>(bias + c), l = *reinterpret_cast<const float4*>(low + c);
+                q.x = silu_f32(q.x); q.y = silu_f32(q.y); q.z = silu_f32(q.z); q.w = silu_f32(q.w);
+                f.x = l.x + (1.f - l.x) * sigmoid_f32(f.x + b.x);
+                f.y = l.y + (1.f - l.y) * sigmoid_f32(f.y + b.y);
+                f.z = l.z + (1.f - l.z) * sigmoid_f32(f.z + b.z);
+                f.w = l.w + (1.f - l.w) * sigmoid_f32(f.w + b.w);
+                *reinterpret_cast<float4*>(row + c) = q;
+                *reinterpret_cast<float4*>(row + qdim + c) = f;
+            }
+        } else {
+            for (int c = threadIdx.x; c < qdim; c += blockDim.x) {
+                row[c] = silu_f32(row[c]);
+                const float l = low[c];
+                row[qdim + c] = l + (1.f - l) * sigmoid_f32(row[qdim + c] + bias[c]);
+            }
+        }
     }
 }
 
@@ -290,37 +307,80 @@ __global__ void recurrence_carry_kernel(float* state, float* piece_state,
     if (!RI_IN_LIMIT(slot, RI_LIMIT_SLOTS, RI_CHECK_SLOT)) return;
     const size_t row = e / vdim;                                  // head * dim + channel
     float running = state[(size_t)slot * per_seq + e];
-    for (int c = 0; c < pieces; ++c) {
-        const size_t at = (size_t)(b * max_pieces + c);
-        const float local = piece_state[at * per_seq + e];
-        piece_state[at * per_seq + e] = running;
-        running = fmaf(piece_gates[at * heads * dim + row], running, local);
+    // Bound by the trips to memory: several pieces' loads are in flight before the first of their stores.  32 pieces of 8 heads'
+    // 128 x 128 states (34 MB): 8.9 us, 44.9 with one load at a time.
+    constexpr int AHEAD = 8;
+    const size_t gate_step = (size_t)heads * dim;
+    float* ps = piece_state + (size_t)b * max_pieces * per_seq + e;
+    const float* pg = piece_gates + (size_t)b * max_pieces * gate_step + row;
+    for (int c = 0; c < pieces; c += AHEAD) {
+        float local[AHEAD], keep[AHEAD];
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) {
+            local[i] = c + i < pieces ? ps[(size_t)(c + i) * per_seq] : 0.f;
+            keep[i] = c + i < pieces ? pg[(size_t)(c + i) * gate_step] : 1.f;
+        }
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i)
+            if (c + i < pieces) {
+                ps[(size_t)(c + i) * per_seq] = running;
+                running = fmaf(keep[i], running, local[i]);
+            }
     }
     state[(size_t)slot * per_seq + e] = running;
 }
 
 // One warp per (token, head): RMS norm over the head's vdim values with one weight shared by heads; with `gate`
 // (float32 rows of gate_ld values, the head's at gate_col + h * vdim) the result is also times silu(gate).
-template <typename T>
-__global__ void headwise_rmsnorm_kernel(const float* x, int ld, int col0, const float* __restrict__ w,
-                                        T* __restrict__ out, int out_ld, int n_tokens, int heads, int vdim,
-                                        float eps, float out_scale, const float* gate, int gate_ld, int gate_col) {
+// VEC: heads of up to 512 values in whole, aligned 16-byte pieces stay in registers between the two passes (2,048 tokens of 8
+// heads of 128: 5.4 us, 6.7 without).
+__device__ __forceinline__ void store_four(float* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void store_four(__nv_bfloat16* p, const float4& v) {
+    uint2 u;
+    *reinterpret_cast<__nv_bfloat162*>(&u.x) = __floats2bfloat162_rn(v.x, v.y);
+    *reinterpret_cast<__nv_bfloat162*>(&u.y) = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = u;
+}
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(256)
+headwise_rmsnorm_kernel(const float* x, int ld, int col0, const float* __restrict__ w, T* out, int out_ld, int n_tokens, int heads,
+                        int vdim, float eps, float out_scale, const float* gate, int gate_ld, int gate_col) {
     let_next_kernel_start();
     wait_for_previous_kernels();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= n_tokens * heads) return;
     const int t = warp / heads, h = warp % heads;
     const float* src = x + (size_t)t * ld + col0 + h * vdim;
-    float ss = 0.f;
-    for (int d = lane; d < vdim; d += 32) ss = fmaf(src[d], src[d], ss);
-    ss = warp_sum(ss);
-    const float inv = 1.0f / sqrtf(ss / (float)vdim + eps);
     T* dst = out + (size_t)t * out_ld + h * vdim;
-    if (gate != nullptr) {
-        const float* g = gate + (size_t)t * gate_ld + gate_col + h * vdim;
-        for (int d = lane; d < vdim; d += 32) dst[d] = from_f32<T>(src[d] * inv * w[d] * silu_f32(g[d]) * out_scale);
+    const float* g = gate != nullptr ? gate + (size_t)t * gate_ld + gate_col + h * vdim : nullptr;
+    float ss = 0.f;
+    if (VEC) {
+        constexpr int PER = 4;
+        float4 v[PER];
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const int d = (i * 32 + lane) * 4;
+            v[i] = d < vdim ? *reinterpret_cast<const float4*>(src + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+            ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
+        }
+        const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)vdim + eps);
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const int d = (i * 32 + lane) * 4;
+            if (d >= vdim) break;
+            const float4 u = *reinterpret_cast<const float4*>(w + d);
+            float4 r = make_float4(v[i].x * inv * u.x, v[i].y * inv * u.y, v[i].z * inv * u.z, v[i].w * inv * u.w);
+            if (g != nullptr) {
+                const float4 z = *reinterpret_cast<const float4*>(g + d);
+                r.x *= silu_f32(z.x); r.y *= silu_f32(z.y); r.z *= silu_f32(z.z); r.w *= silu_f32(z.w);
+            }
+            store_four(dst + d, make_float4(r.x * out_scale, r.y * out_scale, r.z * out_scale, r.w * out_scale));
+        }
     } else {
-        for (int d = lane; d < vdim; d += 32) dst[d] = from_f32<T>(src[d] * inv * w[d] * out_scale);
+        for (int d = lane; d < vdim; d += 32) ss = fmaf(src[d], src[d], ss);
+        const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)vdim + eps);
+        for (int d = lane; d < vdim; d += 32)
+            dst[d] = from_f32<T>(g != nullptr ? src[d] * inv * w[d] * silu_f32(g[d]) * out_scale : src[d] * inv * w[d] * out_scale);
     }
 }
 
@@ -456,16 +516,15 @@ int scan_and_norm(const float* z, int ld, const float* fz, ScanCols at, const fl
     }
     const long long warps = (long long)n_tokens * heads;
     const int blocks = (int)((warps * 32 + 255) / 256);
+    const bool whole = vdim % 4 == 0 && vdim <= 512 && gate_ld % 4 == 0 && gate_col % 4 == 0 &&
+                       ((uintptr_t)o_raw | (uintptr_t)norm_w | (uintptr_t)gate | (uintptr_t)out) % 16 == 0;
     cudaError_t e;
-    if (dtype == RI_F32)
-        e = launch_dependent(headwise_rmsnorm_kernel<float>, blocks, 256, 0, stream, (const float*)o_raw, heads * vdim, 0, norm_w,
-                             (float*)out, heads * vdim, n_tokens, heads, vdim, eps, out_scale, gate, gate_ld, gate_col);
-    else if (dtype == RI_BF16)
-        e = launch_dependent(headwise_rmsnorm_kernel<__nv_bfloat16>, blocks, 256, 0, stream, (const float*)o_raw, heads * vdim, 0,
-                             norm_w, (__nv_bfloat16*)out, heads * vdim, n_tokens, heads, vdim, eps, out_scale, gate, gate_ld,
-                             gate_col);
-    else
-        return fail("gated_recurrence: unknown dtype %d", dtype);
+#define RI_NORM(T, V) launch_dependent(headwise_rmsnorm_kernel<T, V>, blocks, 256, 0, stream, (const float*)o_raw, heads * vdim, 0, norm_w, \
+                                       (T*)out, heads * vdim, n_tokens, heads, vdim, eps, out_scale, gate, gate_ld, gate_col)
+    if (dtype == RI_F32) e = whole ? RI_NORM(float, true) : RI_NORM(float, false);
+    else if (dtype == RI_BF16) e = whole ? RI_NORM(__nv_bfloat16, true) : RI_NORM(__nv_bfloat16, false);
+    else return fail("gated_recurrence: unknown dtype %d", dtype);
+#undef RI_NORM
     return check_launch(e, "gated_recurrence (norm)");
 }
 
@@ -493,9 +552,9 @@ RI_API int ri_gated_recurrence(float* z, int ld, const float* bias, const float*
     if (piece > 0 && (max_pieces <= 0 || scratch == nullptr)) return fail("gated_recurrence: pieces need scratch");
     const int qdim = heads * dim;
     if (piece > 0) {                      // the one-pass scan applies the activations itself
-        const size_t total = (size_t)n_tokens * qdim;
-        const int blocks = (int)((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096);
-        cudaError_t e = launch_dependent(recurrence_prepare_kernel, blocks, 256, 0, stream, z, ld, bias, low, n_tokens, qdim);
+        const bool vec = qdim % 4 == 0 && ld % 4 == 0 && ((uintptr_t)z | (uintptr_t)bias | (uintptr_t)low) % 16 == 0;
+        const cudaError_t e = launch_dependent(vec ? recurrence_prepare_kernel<true> : recurrence_prepare_kernel<false>, min(n_tokens, 8192),
+                                               256, 0, stream, z, ld, bias, low, n_tokens, qdim);
         if (check_launch(e, "gated_recurrence (prepare)")) return 1;
     }
     const ScanCols at{0, qdim, 2 * qdim, 0, ld};
