@@ -30,6 +30,13 @@
 // walk then starts with the pages before the window that hold kept positions, and the mask lets keys below keep_first
 // pass; a sink, one more term exp(sink_h) in the row's sum, added where the row is divided by it.
 //
+// Expanded latent attention (template LATENT; prompts whose sequences start at position 0): keys of 192 channels, of which the
+// first 128 are a head's own and the last 64 one row shared by all heads, and values of 128, all of the step's own tokens
+// (nothing is read from the cache): a token's row holds, head by head, 128 key and 128 value channels (map_k, which map_v
+// equals), the shared part lies in rows of 64 (map_shared).  Two K buffers and one V buffer keep two CTAs on an SM (112 KiB);
+// the value page is asked for as soon as the product before it has finished, most of a softmax ahead of its own.  A head's
+// result is multiplied by the sigmoid of the token's gate, if there are gates, before it is rounded.
+//
 // All mbarrier waits are bounded; on a timeout the kernel records a code in the host-visible
 // status word and winds down.
 #include "tcgen05_common.cuh"
@@ -91,19 +98,21 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 }
 
 // VD: the size of a value head; one below 64 takes a tile of 64 columns that the copy fills up with zeros, and so does the product
-template <int HD, int VD, bool FORMS>
+template <int HD, int VD, bool FORMS, bool LATENT = false>
 __global__ void __launch_bounds__(THREADS, 2)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const int* __restrict__ page_table, int max_pages,
                        const int* __restrict__ seq_slot, const int* __restrict__ seq_start,
                        const int* __restrict__ cu_seqlens, int n_heads, int n_kv_heads, float scale_log2, int window,
                        float out_scale, __nv_bfloat16* __restrict__ out, int out_ld, uint32_t smem_bytes, int* status,
-                       float cap_log2, float scale_over_cap, int keep_first, const float* __restrict__ sink) {
+                       float cap_log2, float scale_over_cap, int keep_first, const float* __restrict__ sink,
+                       const __grid_constant__ CUtensorMap map_shared, const __nv_bfloat16* gate, int gate_ld) {
     constexpr int ATOMS = HD / 64;                       // 64-wide (128-byte) column tiles per row of head_dim
     constexpr int Q_BYTES = ATOMS * BM * 128;            // [atom][128 queries][64]
     constexpr int K_BYTES = ATOMS * BN * 128;            // one buffer: [atom][64 keys][64]
     constexpr int V_ATOMS = (VD + 63) / 64;
     constexpr int V_BYTES = V_ATOMS * BN * 128;
+    constexpr int V_BUFS = LATENT ? 1 : 2;
     constexpr int S_COL = 0, O_COL = 2 * BN;             // two score buffers, then the output accumulator
     constexpr int TMEM_COLS = 256;
     constexpr uint32_t IDESC_S = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
@@ -142,7 +151,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     const uint32_t q_smem = base, k_smem = q_smem + Q_BYTES, v_smem = k_smem + 2 * K_BYTES;
-    constexpr uint32_t TILE_BYTES = Q_BYTES + 2 * K_BYTES + 2 * V_BYTES;
+    constexpr uint32_t TILE_BYTES = Q_BYTES + 2 * K_BYTES + V_BUFS * V_BYTES;
     if (base - raw + TILE_BYTES + (uint32_t)sizeof(Sync) > smem_bytes) {          // uniform over the CTA
         if (threadIdx.x == 0) report(status, ST_ATTN_SMEM);
         return;
@@ -180,37 +189,63 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         // ---------------- TMA producer ----------------
         if (lane == 0) {
             wait_for_previous_kernels();           // q and the newest keys and values come from the kernel before
-            const int* pages = page_table + (size_t)seq_slot[b] * max_pages;
             mbar_expect_tx(smem_u32(&q_full), Q_BYTES);
             for (int a = 0; a < ATOMS; ++a)
                 tma_load_2d(q_smem + a * BM * 128, &map_q, smem_u32(&q_full), h * HD + a * 64, tok0 + q0);
             int k_issued = 0, v_issued = 0;
-            int page_next = pages[page_index(0)];                   // a page's number is fetched one turn ahead
-            for (int j = 0; j < n_pages; ++j) {
-                const int row = (page_next * n_kv_heads + kvh) * BN;
-                if (j + 1 < n_pages) page_next = pages[page_index(j + 1)];
-                const int kb = j & 1;
-                if (!mbar_wait(smem_u32(&k_empty[kb]), (uint32_t)((j >> 1) & 1) ^ 1u) || abort_flag) {
-                    report(status, ST_ATTN_PRODUCER); abort_flag = 1; break;
+            if constexpr (LATENT) {
+                // keys run a page ahead: a value page waits for the product before it, the next scores do not
+                for (int j = -1; j < n_pages; ++j) {
+                    if (j + 1 < n_pages) {
+                        const int kb = (j + 1) & 1, row = tok0 + page_index(j + 1) * BN;
+                        if (!mbar_wait(smem_u32(&k_empty[kb]), (uint32_t)(((j + 1) >> 1) & 1) ^ 1u) || abort_flag) {
+                            report(status, ST_ATTN_PRODUCER); abort_flag = 1; break;
+                        }
+                        mbar_expect_tx(smem_u32(&k_full[kb]), K_BYTES);
+                        for (int a = 0; a < ATOMS - 1; ++a)
+                            tma_load_2d(k_smem + kb * K_BYTES + a * BN * 128, &map_k, smem_u32(&k_full[kb]), h * (HD - 64 + VD) + a * 64, row);
+                        tma_load_2d(k_smem + kb * K_BYTES + (ATOMS - 1) * BN * 128, &map_shared, smem_u32(&k_full[kb]), 0, row);
+                        k_issued = j + 2;
+                    }
+                    if (j < 0) continue;
+                    if (!mbar_wait(smem_u32(&v_empty[0]), (uint32_t)(j & 1) ^ 1u) || abort_flag) {
+                        report(status, ST_ATTN_PRODUCER); abort_flag = 1; break;
+                    }
+                    mbar_expect_tx(smem_u32(&v_full[0]), V_BYTES);
+                    for (int a = 0; a < V_ATOMS; ++a)
+                        tma_load_2d(v_smem + a * BN * 128, &map_v, smem_u32(&v_full[0]), h * (HD - 64 + VD) + HD - 64 + a * 64,
+                                    tok0 + page_index(j) * BN);
+                    v_issued = j + 1;
                 }
-                mbar_expect_tx(smem_u32(&k_full[kb]), K_BYTES);
-                for (int a = 0; a < ATOMS; ++a)
-                    tma_load_2d(k_smem + kb * K_BYTES + a * BN * 128, &map_k, smem_u32(&k_full[kb]), a * 64, row);
-                k_issued = j + 1;
-                if (!mbar_wait(smem_u32(&v_empty[kb]), (uint32_t)((j >> 1) & 1) ^ 1u) || abort_flag) {
-                    report(status, ST_ATTN_PRODUCER); abort_flag = 1; break;
+            } else {
+                const int* pages = page_table + (size_t)seq_slot[b] * max_pages;
+                int page_next = pages[page_index(0)];                   // a page's number is fetched one turn ahead
+                for (int j = 0; j < n_pages; ++j) {
+                    const int row = (page_next * n_kv_heads + kvh) * BN;
+                    if (j + 1 < n_pages) page_next = pages[page_index(j + 1)];
+                    const int kb = j & 1;
+                    if (!mbar_wait(smem_u32(&k_empty[kb]), (uint32_t)((j >> 1) & 1) ^ 1u) || abort_flag) {
+                        report(status, ST_ATTN_PRODUCER); abort_flag = 1; break;
+                    }
+                    mbar_expect_tx(smem_u32(&k_full[kb]), K_BYTES);
+                    for (int a = 0; a < ATOMS; ++a)
+                        tma_load_2d(k_smem + kb * K_BYTES + a * BN * 128, &map_k, smem_u32(&k_full[kb]), a * 64, row);
+                    k_issued = j + 1;
+                    if (!mbar_wait(smem_u32(&v_empty[kb]), (uint32_t)((j >> 1) & 1) ^ 1u) || abort_flag) {
+                        report(status, ST_ATTN_PRODUCER); abort_flag = 1; break;
+                    }
+                    mbar_expect_tx(smem_u32(&v_full[kb]), V_BYTES);
+                    for (int a = 0; a < V_ATOMS; ++a)
+                        tma_load_2d(v_smem + kb * V_BYTES + a * BN * 128, &map_v, smem_u32(&v_full[kb]), a * 64, row);
+                    v_issued = j + 1;
                 }
-                mbar_expect_tx(smem_u32(&v_full[kb]), V_BYTES);
-                for (int a = 0; a < V_ATOMS; ++a)
-                    tma_load_2d(v_smem + kb * V_BYTES + a * BN * 128, &map_v, smem_u32(&v_full[kb]), a * 64, row);
-                v_issued = j + 1;
             }
             // do not leave while a copy into this CTA's shared memory may be in flight
             if (!mbar_wait(smem_u32(&q_full), 0)) report(status, ST_ATTN_DRAIN);
             for (int j = max(0, k_issued - 2); j < k_issued; ++j)
                 if (!mbar_wait(smem_u32(&k_full[j & 1]), (uint32_t)((j >> 1) & 1))) { report(status, ST_ATTN_DRAIN); break; }
-            for (int j = max(0, v_issued - 2); j < v_issued; ++j)
-                if (!mbar_wait(smem_u32(&v_full[j & 1]), (uint32_t)((j >> 1) & 1))) { report(status, ST_ATTN_DRAIN); break; }
+            for (int j = max(0, v_issued - V_BUFS); j < v_issued; ++j)
+                if (!mbar_wait(smem_u32(&v_full[j % V_BUFS]), (uint32_t)((j / V_BUFS) & 1))) { report(status, ST_ATTN_DRAIN); break; }
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
@@ -244,8 +279,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             for (int j = 0; j < n_pages && ok; ++j) {
                 // the buffer S(j+1) goes to was read by the softmax of page j-1, which arrived on p_full before PV(j-1)
                 if (j + 1 < n_pages && !issue_s(j + 1)) { report(status, ST_ATTN_MMA); abort_flag = 1; break; }
-                const uint32_t vb = (uint32_t)j & 1u;
-                if (!mbar_wait(p_full_a, vb) || !mbar_wait(v_full0 + 8u * vb, (uint32_t)((j >> 1) & 1))) {
+                const uint32_t pb = (uint32_t)j & 1u, vb = (uint32_t)(j % V_BUFS);
+                if (!mbar_wait(p_full_a, pb) || !mbar_wait(v_full0 + 8u * vb, (uint32_t)((j / V_BUFS) & 1))) {
                     report(status, ST_ATTN_MMA); abort_flag = 1; break;
                 }
                 tc_fence_after();
@@ -253,7 +288,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 #pragma unroll
                 for (int ks = 0; ks < BN / 16; ++ks)
                     // P of page j lies, two bf16 to a column, over the first half of the score buffer it came from
-                    umma_ts(tmem_base + O_COL, tmem_base + S_COL + vb * BN + ks * 8, vd + (uint64_t)(ks * 16 * 128 >> 4),
+                    umma_ts(tmem_base + O_COL, tmem_base + S_COL + pb * BN + ks * 8, vd + (uint64_t)(ks * 16 * 128 >> 4),
                             IDESC_PV, j > 0 || ks > 0);
                 umma_commit(v_empty0 + 8u * vb);
                 umma_commit(pv_done_a);
@@ -372,7 +407,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             wait_for_previous_kernels();          // `out` must not be written while an earlier kernel may read it
             // FORMS: a sink joins the row's sum as one more term exp(sink_h) without a value (2^x may overflow to infinity when
             // the sink outweighs every score: the result is then 0, as it should be)
-            const float inv = out_scale / ((FORMS && sink != nullptr) ? l + fast_exp2(fmaf(sink[h], 1.4426950408889634f, -m_used)) : l);
+            float inv = out_scale / ((FORMS && sink != nullptr) ? l + fast_exp2(fmaf(sink[h], 1.4426950408889634f, -m_used)) : l);
+            if (LATENT && gate != nullptr && r < rows)
+                inv = __fdividef(inv, 1.f + __expf(-__bfloat162float(gate[(size_t)(tok0 + q0 + r) * gate_ld + h])));
             __nv_bfloat16* dst = out + (size_t)(tok0 + q0 + r) * out_ld + (size_t)h * VD;
 #pragma unroll 1
             for (int c = 0; c < VD; c += 16) {
@@ -404,17 +441,18 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     }
 }
 
-template <int HD, int VD, bool FORMS>
+template <int HD, int VD, bool FORMS, bool LATENT = false>
 int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const int* page_table, int max_pages,
            const int* seq_slot, const int* seq_start, const int* cu_seqlens, int n_seqs, int max_new, int n_heads,
            int n_kv_heads, float scale, int window, float out_scale, void* out, int out_ld, int* status, cudaStream_t stream,
-           float softcap = 0.f, int keep_first = 0, const float* sink = nullptr) {
+           float softcap = 0.f, int keep_first = 0, const float* sink = nullptr, const CUtensorMap* shared = nullptr,
+           const void* gate = nullptr, int gate_ld = 0) {
     constexpr int ATOMS = HD / 64;
     // Q, two K and two V pages, P, the barriers; with head_dim 128 no room for alignment padding is left if
     // two CTAs are to share an SM (the kernel refuses, with a status code, a shared window that needs any)
-    constexpr int TILES = ATOMS * BM * 128 + 2 * (ATOMS + (VD + 63) / 64) * BN * 128;
+    constexpr int TILES = ATOMS * BM * 128 + (2 * ATOMS + (LATENT ? 1 : 2) * ((VD + 63) / 64)) * BN * 128;
     constexpr int SMEM = TILES + (HD >= 128 && VD >= 128 ? 256 : 1024 + 256);
-    auto kernel = attn_prefill_tc_kernel<HD, VD, FORMS>;
+    auto kernel = attn_prefill_tc_kernel<HD, VD, FORMS, LATENT>;
     static PerDeviceOnce configured;       // per device: the attribute belongs to a device's copy of the kernel
     if (int rc = raise_dynamic_smem(kernel, SMEM, configured, "attention_tcgen05")) return rc;
     // blocks are handed out x fastest: every head and sequence of the longest query tiles first, the short
@@ -424,7 +462,8 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, 
     cudaError_t e = launch_dependent(kernel, grid, dim3(THREADS), (size_t)SMEM, stream, mq, mk, mv, page_table, max_pages,
                                      seq_slot, seq_start, cu_seqlens, n_heads, n_kv_heads, scale_log2, window,
                                      out_scale, (__nv_bfloat16*)out, out_ld, (uint32_t)SMEM, status,
-                                     softcap * 1.4426950408889634f, softcap > 0.f ? scale / softcap : 0.f, keep_first, sink);
+                                     softcap * 1.4426950408889634f, softcap > 0.f ? scale / softcap : 0.f, keep_first, sink, shared != nullptr ? *shared : mk,
+                                     (const __nv_bfloat16*)gate, gate_ld);
     return check_launch(e, "attention_tcgen05");
 }
 
@@ -494,6 +533,27 @@ RI_API int ri_attention_tcgen05_prefill_forms(const void* map_q, const void* map
     RI_LAUNCH(64, 32); RI_LAUNCH(64, 64); RI_LAUNCH(64, 128); RI_LAUNCH(128, 32); RI_LAUNCH(128, 64); RI_LAUNCH(128, 128);
 #undef RI_LAUNCH
     return fail("attention_tcgen05: no kernel for heads of %d with values of %d", hd, v_hd);
+}
+
+// Expanded latent attention (`LATENT` above): queries of heads * 192 channels a row (map_q), rows of heads * (128 key + 128 value)
+// channels (map_kv) and of 64 shared key channels (map_shared), all of the step's tokens side by side; every sequence starts at
+// position 0.  gate (bfloat16 [tokens, gate_ld], or null): a gate per head; sink, window (>= 0): as above.
+RI_API int ri_attention_tcgen05_expanded(const void* map_q, const void* map_kv, const void* map_shared, const int* seq_slot,
+                                         const int* seq_start, const int* cu_seqlens, void* out, int out_ld, int n_seqs, int max_new,
+                                         int n_heads, float scale, int window, const float* sink, const void* gate, int gate_ld,
+                                         int* status, cudaStream_t stream) {
+    if (n_seqs <= 0 || max_new <= 0) return 0;
+    if (out_ld % 8 || (uintptr_t)out % 16) return fail("attention_tcgen05: out rows of %d are not aligned 16-byte pieces", out_ld);
+    if (window < 0 || n_heads <= 0 || n_heads > 65535 || n_seqs > 65535)
+        return fail("attention_tcgen05: %d heads, %d sequences, a window of %d", n_heads, n_seqs, window);
+    const CUtensorMap& mq = *reinterpret_cast<const CUtensorMap*>(map_q);
+    const CUtensorMap& mk = *reinterpret_cast<const CUtensorMap*>(map_kv);
+    const CUtensorMap* ms = reinterpret_cast<const CUtensorMap*>(map_shared);
+    if (sink != nullptr)
+        return launch<192, 128, true, true>(mq, mk, mk, nullptr, 0, seq_slot, seq_start, cu_seqlens, n_seqs, max_new, n_heads, n_heads, scale,
+                                            window, 1.f, out, out_ld, status, stream, 0.f, 0, sink, ms, gate, gate_ld);
+    return launch<192, 128, false, true>(mq, mk, mk, nullptr, 0, seq_slot, seq_start, cu_seqlens, n_seqs, max_new, n_heads, n_heads, scale,
+                                         window, 1.f, out, out_ld, status, stream, 0.f, 0, nullptr, ms, gate, gate_ld);
 }
 
 RI_DEFINE_LAST_ERROR()

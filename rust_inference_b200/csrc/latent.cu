@@ -14,6 +14,11 @@
 //              parts rotated into the wide query rows [T, heads, rank + rd]; and the lists that the grouped
 //              products want (every head is a group of T rows).
 //   widen      the per-head products' float32 results [heads, T, rank] into the wide query rows.
+//   expand     (instead of prepare, for prompts that start their sequences: keys and values are formed head by head and the
+//              cached rows are not the operands) rotates the queries' rotated parts where they were projected, writes the cache
+//              row as prepare does, and puts the token's latent and rotated key part, as the cache holds them, into rows of
+//              their own: the operand of the product that forms the heads' keys and values, and the key channels that all heads
+//              share.
 //   gate       out[t, h, :] = v[h, t, :] * sigmoid(g[t, h]): the heads' values (float32, head by head) times
 //              the output gate, token by token, in the run dtype.
 //
@@ -120,6 +125,113 @@ latent_prepare_kernel(TI* __restrict__ proj, int ld, const float* __restrict__ c
         dst[rank + i1] = from_f32<T>(x0 * s[k] + x1 * c[k]);
     }
     for (int j = rot + tid; j < rd; j += blockDim.x) dst[rank + j] = from_f32<T>(take(lat + rank + j));
+}
+
+// bfloat16, sizes in whole 16-byte pieces.  A block per token; a row is read once, eight values per thread and step.
+__device__ __forceinline__ void eight(const __nv_bfloat16* p, float* f) {
+    const uint4 u = *reinterpret_cast<const uint4*>(p);
+    const __nv_bfloat162* q = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 v = __bfloat1622float2(q[i]);
+        f[2 * i] = v.x;
+        f[2 * i + 1] = v.y;
+    }
+}
+__device__ __forceinline__ uint4 eight_of(const float* f) {
+    uint4 u;
+    __nv_bfloat162* q = reinterpret_cast<__nv_bfloat162*>(&u);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) q[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+    return u;
+}
+constexpr int EXPAND_THREADS = 128, EXPAND_PER = 4;      // latents of up to EXPAND_THREADS * 8 * EXPAND_PER channels
+
+__global__ void __launch_bounds__(EXPAND_THREADS)
+latent_expand_kernel(__nv_bfloat16* proj, int ld, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+                     const float* __restrict__ c_w, float eps, const int* __restrict__ token_pos, const int* __restrict__ token_seq,
+                     const int* __restrict__ seq_slot, const int* __restrict__ page_table, int max_pages, __nv_bfloat16* cache,
+                     __nv_bfloat16* c_rows, __nv_bfloat16* k_rows, int n_heads, int d, int rd, int rank, int rot, int style,
+                     int page_size, int own) {
+    __shared__ float scratch[33];
+    const int t = blockIdx.x, tid = threadIdx.x;
+    const int pos = token_pos[t], half = rot >> 1, qh = d + rd, wide = rank + rd;
+    const float* c = cos_t + (size_t)pos * half;
+    const float* s = sin_t + (size_t)pos * half;
+    let_next_kernel_start();
+    wait_for_previous_kernels();
+    __nv_bfloat16* row = proj + (size_t)t * ld;
+
+    // two channels that turn together belong to one thread: rotated where they stand
+    auto turn = [&](const __nv_bfloat16* src, __nv_bfloat16* dst, int k) {
+        const int i0 = style == 0 ? k : 2 * k, i1 = style == 0 ? k + half : 2 * k + 1;
+        const float x0 = __bfloat162float(src[i0]), x1 = __bfloat162float(src[i1]);
+        dst[i0] = __float2bfloat16_rn(x0 * c[k] - x1 * s[k]);
+        dst[i1] = __float2bfloat16_rn(x0 * s[k] + x1 * c[k]);
+    };
+    if (style == 0 && half % 8 == 0) {
+        const int runs = half >> 3;                       // pairs of runs of eight channels
+        for (int i = tid; i < n_heads * runs; i += EXPAND_THREADS) {
+            const int k = (i % runs) * 8;
+            __nv_bfloat16* at = row + (i / runs) * qh + d + k;
+            float lo[8], hi[8], a[8], b[8];
+            eight(at, lo);
+            eight(at + half, hi);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                a[e] = lo[e] * c[k + e] - hi[e] * s[k + e];
+                b[e] = lo[e] * s[k + e] + hi[e] * c[k + e];
+            }
+            *reinterpret_cast<uint4*>(at) = eight_of(a);
+            *reinterpret_cast<uint4*>(at + half) = eight_of(b);
+        }
+    } else {
+        for (int i = tid; i < n_heads * half; i += EXPAND_THREADS) {
+            __nv_bfloat16* at = row + (i / half) * qh + d;
+            turn(at, at, i % half);
+        }
+    }
+
+    const int slot = seq_slot[token_seq[t]];
+    // checked build: a slot, a page index or a page outside its range is recorded and nothing is written
+    if (!RI_BLOCK_IN_LIMIT(slot, RI_LIMIT_SLOTS, RI_CHECK_SLOT) || !RI_BLOCK_IN_RANGE(pos / page_size, max_pages, RI_CHECK_PAGE_INDEX)) return;
+    const int page = page_table[(size_t)slot * max_pages + pos / page_size];
+    if (!RI_BLOCK_IN_LIMIT(page, RI_LIMIT_PAGES, RI_CHECK_PAGE)) return;
+    __nv_bfloat16* kept = cache + ((size_t)page * page_size + (pos % page_size)) * wide;
+    __nv_bfloat16* c_out = c_rows + (size_t)t * rank;
+    __nv_bfloat16* k_out = k_rows + (size_t)t * rd;
+    if (!own) {                                            // the layer reads another layer's rows: gathered from its cache
+        for (int j = tid * 8; j < wide; j += EXPAND_THREADS * 8)
+            *reinterpret_cast<uint4*>(j < rank ? c_out + j : k_out + (j - rank)) = *reinterpret_cast<const uint4*>(kept + j);
+        return;
+    }
+    const __nv_bfloat16* lat = row + n_heads * qh;
+    float v[EXPAND_PER][8], ss = 0.f;
+#pragma unroll
+    for (int p = 0; p < EXPAND_PER; ++p) {
+        const int j = (p * EXPAND_THREADS + tid) * 8;
+        if (j >= rank) break;
+        eight(lat + j, v[p]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) ss += v[p][e] * v[p][e];
+    }
+    ss = block_sum(ss, scratch);
+    const float scale = 1.0f / sqrtf(ss / (float)rank + eps);
+#pragma unroll
+    for (int p = 0; p < EXPAND_PER; ++p) {
+        const int j = (p * EXPAND_THREADS + tid) * 8;
+        if (j >= rank) break;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[p][e] = v[p][e] * scale * c_w[j + e];
+        const uint4 u = eight_of(v[p]);
+        *reinterpret_cast<uint4*>(kept + j) = u;
+        *reinterpret_cast<uint4*>(c_out + j) = u;
+    }
+    for (int k = tid; k < half; k += EXPAND_THREADS) {
+        turn(lat + rank, k_out, k);
+        turn(lat + rank, kept + rank, k);
+    }
+    for (int j = rot + tid; j < rd; j += EXPAND_THREADS) k_out[j] = kept[rank + j] = lat[rank + j];
 }
 
 template <typename T>
@@ -248,6 +360,23 @@ RI_API int ri_latent_gate(const float* v, const void* gates, int gate_ld, void* 
     else if (dtype == RI_BF16) e = launch_dependent(latent_gate_kernel<__nv_bfloat16>, blocks, 256, 0, stream, v, (const __nv_bfloat16*)gates, gate_ld, (__nv_bfloat16*)out, n_tokens, n_heads, vd, vec);
     else return fail("latent_gate: unknown dtype %d", dtype);
     return check_launch(e, "latent_gate");
+}
+
+// proj: bfloat16 [n_tokens, ld] = [heads of d + rd query channels | latent of rank + rd, if `own`]; its rotated query channels are
+// rewritten in place.  c_rows [n_tokens, rank], k_rows [n_tokens, rd]: the tokens' cached rows in two parts.
+RI_API int ri_latent_expand(void* proj, int ld, const float* cos_t, const float* sin_t, const float* c_w, float eps,
+                            const int* token_pos, const int* token_seq, const int* seq_slot, const int* page_table, int max_pages,
+                            void* cache, void* c_rows, void* k_rows, int n_tokens, int n_heads, int d, int rd, int rank, int rot,
+                            int style, int page_size, int own, cudaStream_t stream) {
+    if (n_tokens <= 0) return 0;
+    if (d % 8 || rd % 8 || rank % 8 || ld % 8 || ((uintptr_t)proj | (uintptr_t)cache | (uintptr_t)c_rows | (uintptr_t)k_rows) % 16)
+        return fail("latent_expand: rows must be whole, aligned 16-byte pieces");
+    if (rank > EXPAND_THREADS * 8 * EXPAND_PER) return fail("latent_expand: a latent of %d channels exceeds %d", rank, EXPAND_THREADS * 8 * EXPAND_PER);
+    if (rot % 2 || rot > rd || rot < 0 || (style != 0 && style != 1)) return fail("latent_expand: %d rotated channels of %d, style %d", rot, rd, style);
+    cudaError_t e = launch_dependent(latent_expand_kernel, n_tokens, EXPAND_THREADS, 0, stream, (__nv_bfloat16*)proj, ld, cos_t, sin_t, c_w,
+                                     eps, token_pos, token_seq, seq_slot, page_table, max_pages, (__nv_bfloat16*)cache,
+                                     (__nv_bfloat16*)c_rows, (__nv_bfloat16*)k_rows, n_heads, d, rd, rank, rot, style, page_size, own);
+    return check_launch(e, "latent_expand");
 }
 
 RI_DEFINE_LAST_ERROR()

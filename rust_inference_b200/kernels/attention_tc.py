@@ -81,6 +81,38 @@ def prefill(qkv: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor, page_
     return out
 
 
+EXPANDED_SIZES = (128, 64, 128)      # a head's own key channels, the key channels shared by all heads, value channels
+
+
+def expanded(q: torch.Tensor, kv: torch.Tensor, shared: torch.Tensor, seq_slot, seq_start, cu_seqlens, out: torch.Tensor, *,
+             n_seqs: int, max_new: int, n_heads: int, scale: float, window: int = 0, sink: torch.Tensor | None = None,
+             gate: torch.Tensor | None = None) -> torch.Tensor:
+    """bf16 causal attention of prompts that start their sequences, over keys and values formed from the step's own tokens: q's
+    leading columns hold heads of 128 + 64 channels, kv [T, heads * (128 + 128)] a head's keys and values side by side, shared
+    [T, 64] the key channels that all heads share.  gate: a view [T, heads] of wider bfloat16 rows; the result of token t and
+    head h is multiplied by sigmoid(gate[t, h]).  sink, window: see `prefill`."""
+    _need_cuda(q, kv, shared, seq_slot, seq_start, cu_seqlens, out, sink, gate)
+    own, common, vd = EXPANDED_SIZES
+    n = q.shape[0]
+    _need(q.dtype == kv.dtype == shared.dtype == out.dtype == torch.bfloat16 and q.is_contiguous() and kv.is_contiguous()
+          and shared.is_contiguous() and out.is_contiguous(), "attention_tcgen05: bf16 contiguous tensors only")
+    _need(q.shape[1] >= n_heads * (own + common) and kv.shape == (n, n_heads * (own + vd)) and shared.shape == (n, common)
+          and out.shape[0] == n and out.shape[1] >= n_heads * vd, "attention_tcgen05: shapes of the expanded form")
+    _need(sink is None or (sink.dtype == torch.float32 and sink.is_contiguous() and sink.numel() == n_heads),
+          "attention_tcgen05: sink must be float32 [heads]")
+    _need(gate is None or (gate.dtype == torch.bfloat16 and gate.shape == (n, n_heads) and gate.stride(1) == 1),
+          "attention_tcgen05: gates are bfloat16 [tokens, heads]")
+    mq = _map(0, q, n, q.shape[1], q.shape[1])
+    mkv = _map(1, kv, n, kv.shape[1], kv.shape[1])
+    ms = _map(1, shared, n, common, common)
+    st = status_word()
+    _call("attention_tcgen05", "ri_attention_tcgen05_expanded", c_void_p(mq.data_ptr()), c_void_p(mkv.data_ptr()),
+          c_void_p(ms.data_ptr()), _p(seq_slot), _p(seq_start), _p(cu_seqlens), _p(out), c_int(out.shape[1]), c_int(n_seqs),
+          c_int(max_new), c_int(n_heads), c_float(scale), c_int(window), _p(sink), _p(gate),
+          c_int(gate.stride(0) if gate is not None else 0), c_void_p(st.data_ptr()), _stream())
+    return out
+
+
 def decode(q: torch.Tensor, q_ld: int, kcache: torch.Tensor, vcache: torch.Tensor, page_table, seq_slot, seq_len,
            cu_seqlens, out: torch.Tensor, *, n_seqs: int, n_heads: int, n_kv_heads: int, head_dim: int,
            page_size: int, scale: float, window: int, n_splits: int, part_o=None, part_ml=None) -> torch.Tensor:

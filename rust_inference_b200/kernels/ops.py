@@ -1059,6 +1059,30 @@ def latent_prepare(proj: torch.Tensor, cos, sin, latent_weight, eps: float, toke
           c_int(page_size), c_int(1 if write_kv else 0), c_int(tile_rows), _stream())
 
 
+def latent_expand(proj: torch.Tensor, cos, sin, latent_weight, eps: float, token_pos, token_seq, seq_slot, page_table, cache,
+                  c_rows: torch.Tensor, k_rows: torch.Tensor, *, n_heads: int, head_dim: int, rot_dim: int, rank: int,
+                  rot_dims: int, style: int, page_size: int, own: bool) -> None:
+    """From the bfloat16 projection [T, heads * (head_dim + rot_dim) (+ rank + rot_dim ...)]: the heads' rotated query channels
+    turned where they stand; the token's cached row (normalised latent, rotated key part), written to `cache` from the
+    projection when the layer owns its latent and read from there when not, in two parts into c_rows [T, rank] and k_rows
+    [T, rot_dim]."""
+    _need_cuda(proj, cos, sin, latent_weight, token_pos, token_seq, seq_slot, page_table, cache, c_rows, k_rows)
+    n, wide = proj.shape[0], rank + rot_dim
+    _need(proj.dtype == cache.dtype == c_rows.dtype == k_rows.dtype == torch.bfloat16 and proj.is_contiguous()
+          and proj.shape[1] >= n_heads * (head_dim + rot_dim) + (wide if own else 0), "latent_expand: the projection")
+    _need(c_rows.is_contiguous() and c_rows.shape == (n, rank) and k_rows.is_contiguous() and k_rows.shape == (n, rot_dim),
+          "latent_expand: rows")
+    _need(cache.is_contiguous() and tuple(cache.shape[1:]) == (1, page_size, wide), "latent_expand: cache shape")
+    _need(cos.dtype == torch.float32 and sin.dtype == torch.float32 and cos.shape[1] == rot_dims // 2 and cos.is_contiguous()
+          and sin.is_contiguous() and 0 < rot_dims <= rot_dim and rot_dims % 2 == 0, "latent_expand: rotation tables")
+    _need(not own or (latent_weight is not None and latent_weight.dtype == torch.float32 and latent_weight.numel() == rank),
+          "latent_expand: the latent's norm weight must be float32 [rank]")
+    _call("latent", "ri_latent_expand", _p(proj), c_int(proj.shape[1]), _p(cos), _p(sin), _p(latent_weight), c_float(eps),
+          _p(token_pos), _p(token_seq), _p(seq_slot), _p(page_table), c_int(page_table.shape[1]), _p(cache), _p(c_rows),
+          _p(k_rows), c_int(n), c_int(n_heads), c_int(head_dim), c_int(rot_dim), c_int(rank), c_int(rot_dims), c_int(style),
+          c_int(page_size), c_int(1 if own else 0), _stream())
+
+
 def latent_widen(q_lat: torch.Tensor, q_wide: torch.Tensor, *, n_tokens: int, n_heads: int, rank: int, rot_dim: int) -> None:
     """q_wide[t, h, :rank] = q_lat[h, t, :] (float32 [heads, T, rank] into the run dtype's wide query rows)."""
     _need_cuda(q_lat, q_wide)

@@ -63,7 +63,7 @@ class LatentAttention(Mixer):
             raise ValueError("latent attention: the position encoding must be built for the rotated part's size")
         self.q_dim = self.n_heads * (self.head_dim + self.rot_dim)
         self.wide = self.kv_rank + self.rot_dim
-        self.w_in = self.w_o = self.w_uk_t = self.w_uv = self.latent_norm = None
+        self.w_in = self.w_o = self.w_uk_t = self.w_uv = self.w_ukv = self.latent_norm = None
 
     # ---- tensors -----------------------------------------------------------------------------------------
     def tensor_specs(self):
@@ -97,6 +97,11 @@ class LatentAttention(Mixer):
         self.w_uk_t = tensors[nm["uk"]].view(H, self.head_dim, self.kv_rank).transpose(1, 2).contiguous()
         self.w_uv = tensors[nm["uv"]].view(H, self.v_head_dim, self.kv_rank).contiguous()
         self.w_o = linear.Weight(tensors[nm["o"]])
+        # the same maps in one matrix, a head's keys beside its values: what prompts form keys and values with
+        self.w_ukv = None
+        if self.dtype == torch.bfloat16 and self._expandable():
+            uk = tensors[nm["uk"]].view(H, self.head_dim, self.kv_rank)
+            self.w_ukv = linear.Weight(torch.cat([uk, self.w_uv], dim=1).view(-1, self.kv_rank))
 
     def get_tensors(self):
         nm, H = self.names, self.n_heads
@@ -122,6 +127,40 @@ class LatentAttention(Mixer):
     def cache_request(self):
         return KVRequest(1, self.wide, self.window, self.kv_rank, True)
 
+    # ---- prompts -------------------------------------------------------------------------------------------
+    def _expandable(self) -> bool:
+        from ..kernels import attention_tc
+        return ((self.head_dim, self.rot_dim, self.v_head_dim) == attention_tc.EXPANDED_SIZES and self.kv_rank % 8 == 0
+                and self.kv_rank <= 4096)
+
+    def _expands(self, ctx) -> bool:
+        """Prompts that start their sequences form every head's keys and values from the latents: a score then has head_dim +
+        rot_dim channels and a value v_head_dim, where the carried form has kv_rank + rot_dim and kv_rank for each (at 2,048
+        tokens, 16 heads and a latent of 512 a third of the multiply-adds, on the tcgen05 kernel).  Steps with cached positions
+        would have to form those positions' keys and values again, so they, and single tokens, stay with the carried form."""
+        return (self.w_ukv is not None and not ctx.all_single and ctx.host_starts is not None and not any(ctx.host_starts)
+                and ctx.page_size == 64)
+
+    def _forward_expanded(self, x, residual, ctx, cache_layer):
+        from ..kernels import attention_tc
+        n, H, d, rd, kr, vd = x.shape[0], self.n_heads, self.head_dim, self.rot_dim, self.kv_rank, self.v_head_dim
+        pos = self.position
+        proj = ctx.buffer("latent_proj", (n, self.w_in.n), self.dtype)
+        linear.project(x, self.w_in, proj, ctx)
+        c_rows = ctx.buffer("latent_rows", (n, kr), self.dtype)
+        k_rows = ctx.buffer("latent_rot_rows", (n, rd), self.dtype)
+        ops.latent_expand(proj, pos.cos, pos.sin, self.latent_norm, self.eps, ctx.token_pos, ctx.token_seq, ctx.seq_slot,
+                          ctx.page_table, cache_layer.k, c_rows, k_rows, n_heads=H, head_dim=d, rot_dim=rd, rank=kr,
+                          rot_dims=pos.rot_dims, style=pos.style, page_size=ctx.page_size, own=self.own_latent)
+        kv = ctx.buffer("latent_kv", (n, H * (d + vd)), self.dtype)
+        linear.project(c_rows, self.w_ukv, kv, ctx)
+        out = ctx.buffer("attn_out", (n, H * vd), self.dtype)
+        gates = proj[:, self.w_in.n - H:] if self.gated else None
+        attention_tc.expanded(proj, kv, k_rows, ctx.seq_slot, ctx.seq_start, ctx.cu_seqlens, out, n_seqs=ctx.n_seqs,
+                              max_new=ctx.max_new, n_heads=H, scale=self.scale, window=self.window or 0, sink=self.sinks,
+                              gate=gates)
+        linear.into_residual(out, self.w_o, residual, ctx)
+
     # ---- the step ------------------------------------------------------------------------------------------
     def _grouped(self, x, w, out, lists, n_rows):
         """out<float32>[rows of head h] = x[rows of head h] w[h]^T for every head: on the tensor cores when the
@@ -140,6 +179,9 @@ class LatentAttention(Mixer):
         pos = self.position
         if pos.cos is None or pos.cos.shape[0] < ctx.max_len:
             raise RuntimeError("rope tables do not cover the step's positions; call prepare() first")
+        if self._expands(ctx) and (self.w_in.n % 8) == 0:
+            self._forward_expanded(x, residual, ctx, cache_layer)
+            return
         if not self.gated and linear.wants_split(x, self.w_in):
             # a small step: the projection is split over K into float32 accumulators, which the preparing kernel reads and clears
             proj = ctx.zeroed_buffer("latent_proj_acc", (n, self.w_in.n), torch.float32)
