@@ -16,17 +16,23 @@ class Workspace:
     def __init__(self, device):
         self.device = torch.device(device)
         self._flat: dict = {}
+        self._views: dict = {}        # (name, dtype) -> (shape, view): what was asked for last
 
     def get(self, name: str, shape, dtype: torch.dtype) -> torch.Tensor:
+        key = (name, dtype)
+        last = self._views.get(key)
+        if last is not None and last[0] == shape:         # every layer of a step asks for the same
+            return last[1]
         n = 1
         for s in shape:
             n *= int(s)
-        key = (name, dtype)
         flat = self._flat.get(key)
         if flat is None or flat.numel() < n:
             flat = torch.empty(max(n, 1), dtype=dtype, device=self.device)
             self._flat[key] = flat
-        return flat[:n].view(*shape)
+        view = flat[:n].view(*shape)
+        self._views[key] = (tuple(shape), view)
+        return view
 
     def get_zeroed(self, name: str, shape, dtype: torch.dtype) -> torch.Tensor:
         """A buffer that holds zeros whenever it is handed out: it is zero-filled when made, and

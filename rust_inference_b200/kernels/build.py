@@ -190,6 +190,9 @@ def build(module: str, *, force: bool = False, verbose: bool = True, checked: bo
 
 def load(module: str) -> ctypes.CDLL:
     """The module's library, built first if need be.  Raises if it cannot be had."""
+    lib = _loaded.get(module)         # entered once it is ready to use
+    if lib is not None:
+        return lib
     with _lock:
         lib = _loaded.get(module)
         if lib is None:

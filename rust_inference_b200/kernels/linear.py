@@ -11,7 +11,7 @@ from __future__ import annotations
 
 import torch
 
-from . import ops
+from . import ops, tcgen05
 
 
 class Weight:
@@ -29,7 +29,6 @@ class Weight:
 def _use_tensor_cores(x: torch.Tensor, w: Weight) -> bool:
     if x.dtype != torch.bfloat16:
         return False
-    from . import tcgen05
     return tcgen05.supports(x, w)
 
 
@@ -52,7 +51,6 @@ on_tensor_cores = _use_tensor_cores      # for callers that choose their path by
 def project(x, w: Weight, out, ctx, bias=None):
     """out<run dtype> = x W^T + bias."""
     if _use_tensor_cores(x, w):
-        from . import tcgen05
         return tcgen05.gemm(x, w, out, ops.EPI_STORE, ctx, bias=bias)
     return _plain(x, w, out, ops.EPI_STORE, bias=bias)
 
@@ -61,11 +59,9 @@ def logits(x, w: Weight, out, ctx, silu_cols=None):
     """out<float32> = x W^T; with silu_cols (float32 [1] on the device) the first so many columns through silu."""
     if silu_cols is not None:
         if _use_tensor_cores(x, w):
-            from . import tcgen05
             return tcgen05.gemm(x, w, out, ops.EPI_SILU_F32, ctx, silu_cols=silu_cols)
         return _plain(x, w, out, ops.EPI_SILU_F32, silu_cols=silu_cols)
     if _use_tensor_cores(x, w):
-        from . import tcgen05
         return tcgen05.gemm(x, w, out, ops.EPI_STORE_F32, ctx)
     return _plain(x, w, out, ops.EPI_STORE_F32)
 
@@ -73,7 +69,6 @@ def logits(x, w: Weight, out, ctx, silu_cols=None):
 def into_residual(x, w: Weight, residual, ctx):
     """residual<float32> += x W^T."""
     if _use_tensor_cores(x, w):
-        from . import tcgen05
         return tcgen05.gemm(x, w, residual, ops.EPI_RESIDUAL, ctx)
     return _plain(x, w, residual, ops.EPI_RESIDUAL)
 
@@ -83,7 +78,6 @@ def gated(x, w_gate: Weight, w_up: Weight, out, ctx, form=None):
     limit, shift, cubic, mult) out = mult g' sigmoid(alpha g' (1 + cubic g'^2)) (u' + shift), g' = min(x Wg^T, limit),
     u' = clamp(x Wu^T, -limit, limit)."""
     if _use_tensor_cores(x, w_gate):
-        from . import tcgen05
         return tcgen05.gemm(x, w_gate, out, ops.EPI_SILU_MUL, ctx, w2=w_up, gate_form=form)
     return _plain(x, w_gate, out, ops.EPI_SILU_MUL, w_up, gate_form=form)
 
@@ -92,7 +86,6 @@ def activated(x, w: Weight, out, ctx, form):
     """out<run dtype> = act(x W^T), an activation with its four constants `form` (float32 on the device: `ops.xielu`'s
     two learned numbers through `ops.whole_act_form`, or `ops.RELU_SQUARED_FORM`), applied to the float32 accumulators in the product's epilogue."""
     if _use_tensor_cores(x, w):
-        from . import tcgen05
         return tcgen05.gemm(x, w, out, ops.EPI_ACT, ctx, act_form=form)
     return _plain(x, w, out, ops.EPI_ACT, act_form=form)
 
@@ -103,7 +96,6 @@ def accumulate_split(x, w: Weight, acc, ctx) -> bool:
     output has too few tiles to keep every SM streaming weights."""
     if not _use_tensor_cores(x, w):
         return False
-    from . import tcgen05
     tcgen05.gemm(x, w, acc, ops.EPI_RESIDUAL, ctx)
     return True
 
@@ -118,5 +110,4 @@ def wants_split(x, w: Weight) -> bool:
     """True for a small step whose projection would otherwise leave most SMs idle."""
     if not _use_tensor_cores(x, w) or x.shape[0] > SPLIT_MAX_TOKENS:
         return False
-    from . import tcgen05
     return tcgen05.pick_split(x.shape[0], w.n, w.k) > 1

@@ -34,8 +34,16 @@ def _p(t) -> c_void_p:
     return c_void_p(t.data_ptr()) if t is not None else c_void_p(0)
 
 
+# A launch costs the host a few microseconds in the driver; what surrounds it must not cost more, because a prompt of a few
+# hundred tokens is a couple of hundred launches of a few microseconds each: the current stream comes as the number that it is
+# (`torch.cuda.current_stream()` builds two objects and looks the device up by name, 4 us), messages are formatted only when
+# they are raised, and scratch buffers keep their last view.
+_current_raw_stream = torch._C._cuda_getCurrentRawStream
+_current_device = torch._C._cuda_getDevice
+
+
 def _stream() -> c_void_p:
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    return c_void_p(_current_raw_stream(_current_device()))
 
 
 def _need_cuda(*tensors) -> None:
@@ -414,7 +422,8 @@ def _gemm_constants(x, w, out, mode, bias, w2, gate_form, act_form, silu_cols):
     _need(w.shape[1] == k and x.dtype == w.dtype and x.is_contiguous() and w.is_contiguous()
           and out.is_contiguous() and out.shape == (m, n), "gemm: bad shapes")
     want_out = torch.float32 if mode in (EPI_STORE_F32, EPI_RESIDUAL, EPI_SILU_F32) else x.dtype
-    _need(out.dtype == want_out, f"gemm: epilogue {mode} writes {want_out}, out is {out.dtype}")
+    if out.dtype != want_out:
+        raise KernelError(f"gemm: epilogue {mode} writes {want_out}, out is {out.dtype}")
     if bias is not None:
         _need(bias.dtype == torch.float32 and bias.numel() == n, "gemm: bias must be float32 [N]")
     if w2 is not None:

@@ -144,7 +144,8 @@ def gemm(x: torch.Tensor, w, out: torch.Tensor, mode: int, ctx=None, bias=None, 
     _need(w.k == k and x.dtype == torch.bfloat16 and w.t.dtype == torch.bfloat16 and x.is_contiguous()
           and out.is_contiguous() and out.shape == (m, n), "gemm_tcgen05: bad shapes or dtypes")
     want_out = torch.float32 if mode in (ops.EPI_STORE_F32, ops.EPI_RESIDUAL, ops.EPI_SILU_F32) else torch.bfloat16
-    _need(out.dtype == want_out, f"gemm_tcgen05: epilogue {mode} writes {want_out}, out is {out.dtype}")
+    if out.dtype != want_out:
+        raise KernelError(f"gemm_tcgen05: epilogue {mode} writes {want_out}, out is {out.dtype}")
     if bias is not None:
         _need(bias.dtype == torch.float32 and bias.numel() == n, "gemm_tcgen05: bias must be float32 [N]")
     map_w2 = None
