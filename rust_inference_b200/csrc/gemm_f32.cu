@@ -15,8 +15,8 @@
 // eight warps add that sum onto float32 registers and the next 64 steps start from zero, so that the tensor core's own
 // additions, which truncate, never run over more than 64 steps.  Against 64 bits (rows of N(0, 1) times rows of N(0, 1/K)) the
 // result is off by 1.3e-7 at K = 192, 1.4e-7 at 896, 1.5e-7 at 4,864 and 2.1e-7 at 18,944, where one running FFMA sum was off
-// by 2.5e-7, 5.3e-7, 1.2e-6 and 2.5e-6 (the kernel for few rows: 0.8e-7 to 1.8e-7).  A number that is infinite or NaN has no such parts: a tile that meets one computes
-// its piece again with FFMA, so that such numbers come out as the plain sum gives them.
+// by 2.5e-7, 5.3e-7, 1.2e-6 and 2.5e-6 (the kernel for few rows: 0.8e-7 to 1.8e-7).  A number that is infinite or NaN has no such parts (they turn every sum that they meet
+// infinite or NaN): a tile with such a sum computes its piece again with FFMA, so that it comes out as the plain sum gives it.
 //
 // Epilogues as in `gemm_simt.cu` (0 and 1 are the same here: float32 with a bias): 2 out += acc, 3 gated, 4 an activation,
 // 5 silu for the first columns.
@@ -243,8 +243,9 @@ int launch_few(const float* X, const float* W, const float* W2, const float* bia
 // block of 64 steps of K is shared memory (24 MMAs that read 4 KiB of W and TN * 32 bytes of X each, and the parts' writes: at
 // TN = 128 about 2,300 clocks against 1,536 of the tensor core, at TN = 64 1,730 against 768, so TN is 128 wherever a step has
 // that many rows) and the cutting, eight warps with a few dependent instructions per number.  Four warps instead of eight for
-// the additions made those the slowest part: 954 against 862 us at 333 x 151,936 x 896 (105 TFLOP/s of the product; the FFMA
-// kernel takes 2,950), 50 against 46 at 333 x 896 x 4,864 (345); sixteen warps for the cutting, 929 and 51.
+// the additions made those the slowest part: 954 against 862 us at 333 x 151,936 x 896 (the FFMA kernel
+// takes 2,950), 50 against 46 at 333 x 896 x 4,864 (345); sixteen warps for the cutting, 929 and 51.
+// Looking for infinities and NaN in the sums instead of in every number that is cut: 837 (108 TFLOP/s of the product) and 45.
 // ---------------------------------------------------------------------------------------------------------------------
 constexpr int ROWS = 128, BK = 64, PART = ROWS * BK * 2, STAGES = 2;
 constexpr int CUT_WARPS = 8, CUT_THREADS = CUT_WARPS * 32, ADD_WARPS = 8;
@@ -252,26 +253,25 @@ constexpr int SPLIT_THREADS = CUT_THREADS + ADD_WARPS * 32;
 enum Status { ST_CUT_TIMEOUT = 41, ST_MMA_TIMEOUT = 42, ST_ADD_TIMEOUT = 43 };
 
 // x as three bfloat16 numbers that add up to it exactly, each the upper half of a float32: the leading 8 significant bits,
-// the next 8 and the rest.  `odd` becomes NaN if x is infinite or NaN.
-__device__ __forceinline__ void cut(float x, uint32_t& hi, uint32_t& mid, uint32_t& lo, float& odd) {
+// the next 8 and the rest.  An infinite x gives an infinity and two NaN, a NaN three.
+__device__ __forceinline__ void cut(float x, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
     hi = __float_as_uint(x) & 0xffff0000u;
     const float r = x - __uint_as_float(hi);
     mid = __float_as_uint(r) & 0xffff0000u;
     const float r2 = r - __uint_as_float(mid);
     lo = __float_as_uint(r2);
-    odd = fmaf(r2, 0.f, odd);
 }
 __device__ __forceinline__ uint32_t upper_halves(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x7632); }
 __device__ __forceinline__ void store8(uint32_t addr, uint32_t a, uint32_t b) {
     asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
 }
 // four consecutive k of one row into the three parts
-__device__ __forceinline__ void put(uint32_t addr, uint32_t part_bytes, const float4& v, float& odd) {
+__device__ __forceinline__ void put(uint32_t addr, uint32_t part_bytes, const float4& v) {
     uint32_t h[4], m[4], l[4];
-    cut(v.x, h[0], m[0], l[0], odd);
-    cut(v.y, h[1], m[1], l[1], odd);
-    cut(v.z, h[2], m[2], l[2], odd);
-    cut(v.w, h[3], m[3], l[3], odd);
+    cut(v.x, h[0], m[0], l[0]);
+    cut(v.y, h[1], m[1], l[1]);
+    cut(v.z, h[2], m[2], l[2]);
+    cut(v.w, h[3], m[3], l[3]);
     store8(addr, upper_halves(h[0], h[1]), upper_halves(h[2], h[3]));
     store8(addr + part_bytes, upper_halves(m[0], m[1]), upper_halves(m[2], m[3]));
     store8(addr + 2 * part_bytes, upper_halves(l[0], l[1]), upper_halves(l[2], l[3]));
@@ -362,7 +362,6 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
         wait_for_previous_kernels();
 #pragma unroll
         for (int i = 0; i < XN; ++i) xv[i] = load_x(i, k < K);
-        float odd = 0.f;
         for (int b = 0; b < n_kb; ++b) {
             const int s = b % STAGES;
             if (!mbar_wait(smem_u32(&empty_bar[s]), (uint32_t)((b / STAGES) & 1) ^ 1u)) {
@@ -375,19 +374,18 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
             const uint32_t stage = base + (uint32_t)(s * STAGE) + col;
 #pragma unroll
             for (int i = 0; i < WN; ++i) {
-                put(stage + (uint32_t)(i * 16 * 128), PART, wv[i], odd);
+                put(stage + (uint32_t)(i * 16 * 128), PART, wv[i]);
                 wv[i] = load_w(i, more);
             }
 #pragma unroll
             for (int i = 0; i < XN; ++i) {
-                put(stage + 3 * PART + (uint32_t)(i * 16 * 128), X_PART, xv[i], odd);
+                put(stage + 3 * PART + (uint32_t)(i * 16 * 128), X_PART, xv[i]);
                 xv[i] = load_x(i, more);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the MMA reads what was just stored
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&full_bar[s]));
         }
-        if (odd != odd) odd_flag = 1;
     } else {
         // ---- add the sums of 64 steps onto float32 registers: a thread owns a row of W (a TMEM lane) ----
         // The first of these warps also issues the MMAs, two blocks of K ahead of the one being added (a warp of its own for
@@ -455,8 +453,13 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
         }
         // the last MMAs have finished: nothing reads the stages any more
         if (!abort_flag) {
+            bool finite = true;
 #pragma unroll
-            for (int c = 0; c < COLS; ++c) pieces[(part * COLS + c) * ROWS + q * 32 + lane] = acc[c];
+            for (int c = 0; c < COLS; ++c) {
+                pieces[(part * COLS + c) * ROWS + q * 32 + lane] = acc[c];
+                finite &= fabsf(acc[c]) <= 3.402823466e38f;
+            }
+            if (!finite) odd_flag = 1;
         }
     }
     __syncwarp();
@@ -469,7 +472,7 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
     }
     const bool failed = abort_flag != 0;
     if (odd_flag && !failed) {
-        // infinite or NaN operands: this block's piece again, as a plain float32 sum
+        // infinite or NaN sums: this block's piece again, as a plain float32 sum
         const int k_end = min(K, (kb0 + n_kb) * BK);
         for (int i = threadIdx.x; i < TN * ROWS; i += SPLIT_THREADS) {
             const int c = i / ROWS;
