@@ -823,7 +823,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             const int t = t0 + rank * TM_TOK + lane_base + lane;
             const bool t_ok = t < n_tok;
             const uint32_t trow = tmem_base + ((uint32_t)lane_base << 16) + (uint32_t)(buf * TM_ROWS);
-            tm_write_tile<DUAL, MODE>(trow, t, t_ok, f0, n_feat, aligned, bias, out_, split_k > 1);
+            // adds without a returned value also where one item has the whole of K: reading the sums first kept the epilogue waiting
+            // for memory (1,845 x 1,536 x 1,536: 34.9 us, with two pieces 15)
+            tm_write_tile<DUAL, MODE>(trow, t, t_ok, f0, n_feat, aligned, bias, out_, true);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(acc_empty_first + 8u * (uint32_t)buf);
@@ -927,11 +929,6 @@ int launch_tm(const CUtensorMap& mw, const CUtensorMap& mw2, const CUtensorMap& 
 int g_pair_min_tokens = 512;     // steps of at least this many tokens may run on pairs of SMs (0: never)
 bool g_pair_always = false;      // ... whatever their tiles make of the grid (tests)
 
-// Whether a product runs on pairs of SMs.  Measured on a 3584-wide model at 512, 2,048 and 8,192 tokens: where
-// the pair tiles fill the grid's rounds as well as the single-CTA tiles do, pairs are 2-5% faster (SiLU-gate
-// projection 367 -> 357 us at 2,048 tokens, q/k/v 218 -> 208 us at 8,192); where they leave a round half
-// empty (o and down projections: 112 tiles of 256 x 256 on 74 pairs) they lose up to 15%.  The adding epilogue
-// cannot split K here, so it stays with the single-CTA kernel.
 // Pieces of K for the adding epilogue on pairs: the count that leaves the busiest pair the fewest k-blocks,
 // with a dozen per work item for its epilogue and ramp.
 int pair_split(int n_tok, int n_feat, int K) {
@@ -947,13 +944,26 @@ int pair_split(int n_tok, int n_feat, int K) {
     return split;
 }
 
-bool on_pairs(int n_tok, int n_feat, int mode) {
+// Whether a product runs on pairs of SMs.  Measured on a 3584-wide model at 512, 2,048 and 8,192 tokens: where
+// the pair tiles fill the grid's rounds as well as the single-CTA tiles do, pairs are 2-5% faster (SiLU-gate
+// projection 367 -> 357 us at 2,048 tokens, q/k/v 218 -> 208 us at 8,192); where they leave a round half
+// empty they lose up to 15%.  The adding epilogue can cut K into pieces, which fills rounds that whole tiles leave open
+// (`pair_split`); it adds without reading the sums first.  Over twelve steps of 512 to 7,999 tokens and ten shapes from 896 x 4,864
+// to 4,096 x 14,336 (us, single CTAs against pairs): 2,048 x 2,048 x 11,008 75.8 / 67.7, 3,000 x 1,536 x 8,960 67.0 / 60.0, 2,048 x
+// 3,584 x 18,944 226 / 212, 7,999 x 4,096 x 14,336 782 / 693; pairs are the faster ones by 1-14% from 1.4e10 multiply-adds on where
+// their rounds are at least 85% full (2,048 x 3,584 x 3,584, 76% full: 56.1 / 57.3), and lose up to 8% below that (777 x 1,536 x
+// 8,960: 25.3 / 26.5; 1,300 x 896 x 4,864: 17.7 / 18.9).
+bool on_pairs(int n_tok, int n_feat, int K, int mode) {
     if (g_pair_min_tokens <= 0 || n_tok < g_pair_min_tokens) return false;
     if (g_pair_always) return true;
-    if (mode == 2) return false;
     const long long feats = mode == 3 ? TM_ROWS / 2 : TM_ROWS;
-    const long long tiles = (long long)((n_tok + PAIR_TOK - 1) / PAIR_TOK) * ((n_feat + feats - 1) / feats);
+    long long tiles = (long long)((n_tok + PAIR_TOK - 1) / PAIR_TOK) * ((n_feat + feats - 1) / feats);
     const long long pairs = sm_count() / 2;
+    if (mode == 2) {
+        if ((double)n_tok * n_feat * K < 1.4e10) return false;
+        tiles *= pair_split(n_tok, n_feat, K);
+        return tiles * 100 >= (tiles + pairs - 1) / pairs * pairs * 85;
+    }
     const long long rounds = (tiles + pairs - 1) / pairs;
     return tiles * 100 >= rounds * pairs * 93;               // the last round at least ~93% full on average
 }
@@ -1041,7 +1051,7 @@ RI_API int ri_gemm_tcgen05_plan(int n_tok, int n_feat, int K, int mode, int* til
     const int total_kb = (K + BLOCK_K - 1) / BLOCK_K;
     const bool can_split = mode == 2;
     int tn = 16, sp = 1;
-    if (on_pairs(n_tok, n_feat, mode)) {
+    if (on_pairs(n_tok, n_feat, K, mode)) {
         tn = TM_TOK;                                              // pairs of SMs: each CTA's box holds 128 tokens
         if (mode == 2) sp = pair_split(n_tok, n_feat, K);
     } else if (n_tok <= 128) {
@@ -1110,7 +1120,7 @@ RI_API int ri_gemm_tcgen05(const void* map_x, const void* map_w, const void* map
     const CUtensorMap& mx = *reinterpret_cast<const CUtensorMap*>(map_x);
     // Measured at 2,048 tokens of a 3584-wide model: the SiLU-gate projection runs at 1,334 TFLOP/s
     // token-major against 1,145 feature-major; q/k/v, o and down are 3-12% faster feature-major.
-    if (on_pairs(n_tok, n_feat, mode)) {
+    if (on_pairs(n_tok, n_feat, K, mode)) {
         switch (mode) {
             case 0: return launch_pair<false, 0>(mw, mw2, mx, bias, out, n_tok, n_feat, K, 1, status, stream);
             case 1: return launch_pair<false, 1>(mw, mw2, mx, bias, out, n_tok, n_feat, K, 1, status, stream);

@@ -272,6 +272,22 @@ def test_gemm_tcgen05_token_tile_follows_the_grid(m, n, k):
     tcgen05.check_status()
 
 
+@pytest.mark.parametrize("m, n, k", [(1024, 2048, 8192), (1000, 1990, 8200), (7999, 1536, 1544), (2048, 3584, 18944)])
+def test_gemm_tcgen05_adds_on_pairs_of_sms_by_itself(m, n, k):
+    """Large products that add onto float32 sums run on pairs of SMs where their pieces fill the pairs' rounds; ragged sizes."""
+    ops = _ops()
+    from rust_inference_b200.kernels import linear, tcgen05
+    assert tcgen05.plan(m, n, k, ops.EPI_RESIDUAL)[0] == 128          # a pair's box: 128 tokens per CTA
+    x = (torch.randn(m, k, device=DEV) * 0.5).bfloat16()
+    w = linear.Weight((torch.randn(n, k, device=DEV) * 0.1).bfloat16())
+    res = torch.randn(m, n, device=DEV)
+    ref = res.double() + x.double() @ w.t.double().t()
+    tcgen05.gemm(x, w, res, ops.EPI_RESIDUAL)
+    assert (res.double() - ref).abs().max().item() <= 1e-5 * ref.abs().max().item()
+    torch.cuda.synchronize()
+    tcgen05.check_status()
+
+
 @pytest.mark.parametrize("m, n, k", [(512, 512, 256), (300, 1000, 520), (1111, 264, 72), (256, 3000, 64), (40, 384, 128),
                                      (2048, 1184, 1096)])
 def test_gemm_tcgen05_on_pairs_of_sms(m, n, k):
