@@ -1,7 +1,7 @@
 // out[M, N] = X[M, K] * W[N, K]^T on the FFMA pipe, float32 accumulation, any M, N, K.
 //
-// This is the true 32-bit contraction (no tensor-core mode of any kind touches the
-// operands), and the fallback of the bf16 path for shapes the tensor-core kernel refuses.
+// The fallback: 32-bit contractions whose rows are no whole 16-byte pieces or whose sums have few terms (`gemm_f32.cu` has the
+// others), and bf16 ones whose shapes the tensor-core kernel refuses.
 // It restates the reference's mat-vec, y_r = sum_c W[r, c] x_c over a row-major [out, in]
 // matrix (quant.rs:178-206, math.rs:212-229), for a batch of rows of X at once.
 //
