@@ -249,7 +249,8 @@ __device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepc
 
 // Sixteen bytes that an earlier kernel of the stream writes, read behind `wait_for_previous_kernels()`.  A plain load through a
 // `const __restrict__` pointer promises that nobody writes the data while the kernel lives, and the compiler may move such a
-// load above the wait (seen: products read the rows of two kernels ago); this one stays where it is written.
+// load above the wait (seen: products that were right alone and wrong behind the kernel that writes their rows); this one stays
+// where it is written.
 __device__ __forceinline__ float4 load_written(const float* p) {
     float4 v;
     asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
