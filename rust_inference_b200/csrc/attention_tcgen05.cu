@@ -34,7 +34,8 @@
 // first 128 are a head's own and the last 64 one row shared by all heads, and values of 128, all of the step's own tokens
 // (nothing is read from the cache): a token's row holds, head by head, 128 key and 128 value channels (map_k, which map_v
 // equals), the shared part lies in rows of 64 (map_shared).  Two K buffers and one V buffer keep two CTAs on an SM (112 KiB);
-// the value page is asked for as soon as the product before it has finished, most of a softmax ahead of its own.  A head's
+// the value page is asked for as soon as the product before it has finished, most of a softmax ahead of its own.  A sequence's
+// last page reaches into the rows of the next one; its value rows are zeroed there before the product.  A head's
 // result is multiplied by the sigmoid of the token's gate, if there are gates, before it is rounded.
 //
 // All mbarrier waits are bounded; on a timeout the kernel records a code in the host-visible
@@ -387,6 +388,22 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             }
             l = l * alpha + sum;
             m_used = m_new;
+            if (LATENT && key0 + BN > n_new) {
+                // the rows beyond the sequence's last one are the next sequence's first tokens: their weights are 0, but 0 times
+                // an infinity or a NaN is NaN, so they are made zeros before the product reads them (whole 128-byte rows, which
+                // the swizzle keeps together)
+                if (!mbar_wait(smem_u32(&v_full[0]), (uint32_t)(j & 1)) || abort_flag) {
+                    if (lane == 0) { report(status, ST_ATTN_SOFTMAX); abort_flag = 1; }
+                    ok = false;
+                    break;
+                }
+                uint4* const v_rows = reinterpret_cast<uint4*>(smem_raw + (v_smem - raw));
+                const int from = n_new - key0;
+                for (int i = r; i < (BN - from) * 8; i += BM)
+#pragma unroll
+                    for (int a = 0; a < V_ATOMS; ++a) v_rows[(a * BN + from) * 8 + i] = make_uint4(0u, 0u, 0u, 0u);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            }
             // P goes back to tensor memory, over the scores it was made from (this thread has read its row of
             // them): the product P V takes its A operand from there, so P never passes through shared memory
 #pragma unroll

@@ -93,3 +93,32 @@ def test_kernel(window, sink, gated, lengths):
             got = out[rows, h * 128:(h + 1) * 128].double()
             assert (got - want).abs().max().item() <= 2 ** -7 * want.abs().max().item()
         at += n
+
+
+@pytest.mark.parametrize("first", [1, 63, 65, 130, 200])         # the last page holds 63, 1, 63, 62 and 56 rows of the next prompt
+@pytest.mark.parametrize("gated", [False, True])
+def test_neighbours_with_infinities(first, gated):
+    """A prompt's result does not depend on what stands in the prompt packed behind it, infinities and NaN included: to the
+    bit what it is alone."""
+    from rust_inference_b200.kernels import attention_tc, tcgen05
+    heads, second = 3, 100
+    g = torch.Generator(device="cuda").manual_seed(first)
+    draw = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    total = first + second
+    q, kv, shared, gates = draw(total, heads * 192), draw(total, heads * 256), draw(total, 64), draw(total, 8)
+    for t in (q, kv, shared):
+        t[first::3], t[first + 1::3], t[first + 2::3] = float("nan"), float("inf"), float("-inf")
+
+    def run(n, lengths):
+        cu = torch.tensor([sum(lengths[:i]) for i in range(len(lengths) + 1)], dtype=torch.int32, device="cuda")
+        zeros = torch.zeros(len(lengths), dtype=torch.int32, device="cuda")
+        out = torch.full((n, heads * 128), 7.0, dtype=torch.bfloat16, device="cuda")
+        attention_tc.expanded(q[:n], kv[:n], shared[:n], zeros, zeros, cu, out, n_seqs=len(lengths), max_new=max(lengths), n_heads=heads,
+                              scale=192 ** -0.5, gate=gates[:n, 2:2 + heads] if gated else None)
+        torch.cuda.synchronize()
+        tcgen05.check_status()
+        return out
+
+    alone, beside = run(first, [first]), run(total, [first, second])
+    assert bool(alone.isfinite().all())
+    assert torch.equal(beside[:first], alone)
