@@ -35,7 +35,8 @@
 // (nothing is read from the cache): a token's row holds, head by head, 128 key and 128 value channels (map_k, which map_v
 // equals), the shared part lies in rows of 64 (map_shared).  Two K buffers and one V buffer keep two CTAs on an SM (112 KiB);
 // the value page is asked for as soon as the product before it has finished, most of a softmax ahead of its own.  A sequence's
-// last page reaches into the rows of the next one; its value rows are zeroed there before the product.  A head's
+// last page reaches into the rows of the next one; its value rows are zeroed there before the product.  LATENT == 2: values in two
+// bfloat16 terms (map_low: the second ones), which leaves one CTA on an SM (128 KiB).  A head's
 // result is multiplied by the sigmoid of the token's gate, if there are gates, before it is rounded.
 //
 // All mbarrier waits are bounded; on a timeout the kernel records a code in the host-visible
@@ -99,7 +100,7 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 }
 
 // VD: the size of a value head; one below 64 takes a tile of 64 columns that the copy fills up with zeros, and so does the product
-template <int HD, int VD, bool FORMS, bool LATENT = false>
+template <int HD, int VD, bool FORMS, int LATENT = 0>
 __global__ void __launch_bounds__(THREADS, 2)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const int* __restrict__ page_table, int max_pages,
@@ -107,12 +108,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                        const int* __restrict__ cu_seqlens, int n_heads, int n_kv_heads, float scale_log2, int window,
                        float out_scale, __nv_bfloat16* __restrict__ out, int out_ld, uint32_t smem_bytes, int* status,
                        float cap_log2, float scale_over_cap, int keep_first, const float* __restrict__ sink,
-                       const __grid_constant__ CUtensorMap map_shared, const __nv_bfloat16* gate, int gate_ld) {
+                       const __grid_constant__ CUtensorMap map_shared, const __grid_constant__ CUtensorMap map_low, const __nv_bfloat16* gate,
+                       int gate_ld) {
     constexpr int ATOMS = HD / 64;                       // 64-wide (128-byte) column tiles per row of head_dim
     constexpr int Q_BYTES = ATOMS * BM * 128;            // [atom][128 queries][64]
     constexpr int K_BYTES = ATOMS * BN * 128;            // one buffer: [atom][64 keys][64]
     constexpr int V_ATOMS = (VD + 63) / 64;
-    constexpr int V_BYTES = V_ATOMS * BN * 128;
+    constexpr int V_TERM = V_ATOMS * BN * 128;           // one buffer of values; LATENT == 2: the lower terms lie behind the upper ones
+    constexpr int V_BYTES = (LATENT == 2 ? 2 : 1) * V_TERM;
     constexpr int V_BUFS = LATENT ? 1 : 2;
     constexpr int S_COL = 0, O_COL = 2 * BN;             // two score buffers, then the output accumulator
     constexpr int TMEM_COLS = 256;
@@ -216,6 +219,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     for (int a = 0; a < V_ATOMS; ++a)
                         tma_load_2d(v_smem + a * BN * 128, &map_v, smem_u32(&v_full[0]), h * (HD - 64 + VD) + HD - 64 + a * 64,
                                     tok0 + page_index(j) * BN);
+                    if constexpr (LATENT == 2)
+                        for (int a = 0; a < V_ATOMS; ++a)
+                            tma_load_2d(v_smem + V_TERM + a * BN * 128, &map_low, smem_u32(&v_full[0]), h * VD + a * 64, tok0 + page_index(j) * BN);
                     v_issued = j + 1;
                 }
             } else {
@@ -291,6 +297,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     // P of page j lies, two bf16 to a column, over the first half of the score buffer it came from
                     umma_ts(tmem_base + O_COL, tmem_base + S_COL + pb * BN + ks * 8, vd + (uint64_t)(ks * 16 * 128 >> 4),
                             IDESC_PV, j > 0 || ks > 0);
+                if constexpr (LATENT == 2)
+#pragma unroll
+                    for (int ks = 0; ks < BN / 16; ++ks)
+                        umma_ts(tmem_base + O_COL, tmem_base + S_COL + pb * BN + ks * 8,
+                                vd + (uint64_t)(V_TERM >> 4) + (uint64_t)(ks * 16 * 128 >> 4), IDESC_PV, true);
                 umma_commit(v_empty0 + 8u * vb);
                 umma_commit(pv_done_a);
             }
@@ -401,7 +412,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 const int from = n_new - key0;
                 for (int i = r; i < (BN - from) * 8; i += BM)
 #pragma unroll
-                    for (int a = 0; a < V_ATOMS; ++a) v_rows[(a * BN + from) * 8 + i] = make_uint4(0u, 0u, 0u, 0u);
+                    for (int a = 0; a < V_BYTES / (BN * 128); ++a) v_rows[(a * BN + from) * 8 + i] = make_uint4(0u, 0u, 0u, 0u);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             }
             // P goes back to tensor memory, over the scores it was made from (this thread has read its row of
@@ -426,7 +437,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             // the sink outweighs every score: the result is then 0, as it should be)
             float inv = out_scale / ((FORMS && sink != nullptr) ? l + fast_exp2(fmaf(sink[h], 1.4426950408889634f, -m_used)) : l);
             if (LATENT && gate != nullptr && r < rows)
-                inv = __fdividef(inv, 1.f + __expf(-__bfloat162float(gate[(size_t)(tok0 + q0 + r) * gate_ld + h])));
+                inv = inv / (1.f + expf(-__bfloat162float(gate[(size_t)(tok0 + q0 + r) * gate_ld + h])));
             __nv_bfloat16* dst = out + (size_t)(tok0 + q0 + r) * out_ld + (size_t)h * VD;
 #pragma unroll 1
             for (int c = 0; c < VD; c += 16) {
@@ -458,16 +469,16 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     }
 }
 
-template <int HD, int VD, bool FORMS, bool LATENT = false>
+template <int HD, int VD, bool FORMS, int LATENT = 0>
 int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const int* page_table, int max_pages,
            const int* seq_slot, const int* seq_start, const int* cu_seqlens, int n_seqs, int max_new, int n_heads,
            int n_kv_heads, float scale, int window, float out_scale, void* out, int out_ld, int* status, cudaStream_t stream,
            float softcap = 0.f, int keep_first = 0, const float* sink = nullptr, const CUtensorMap* shared = nullptr,
-           const void* gate = nullptr, int gate_ld = 0) {
+           const CUtensorMap* low = nullptr, const void* gate = nullptr, int gate_ld = 0) {
     constexpr int ATOMS = HD / 64;
     // Q, two K and two V pages, P, the barriers; with head_dim 128 no room for alignment padding is left if
     // two CTAs are to share an SM (the kernel refuses, with a status code, a shared window that needs any)
-    constexpr int TILES = ATOMS * BM * 128 + (2 * ATOMS + (LATENT ? 1 : 2) * ((VD + 63) / 64)) * BN * 128;
+    constexpr int TILES = ATOMS * BM * 128 + (2 * ATOMS + (LATENT == 1 ? 1 : 2) * ((VD + 63) / 64)) * BN * 128;
     constexpr int SMEM = TILES + (HD >= 128 && VD >= 128 ? 256 : 1024 + 256);
     auto kernel = attn_prefill_tc_kernel<HD, VD, FORMS, LATENT>;
     static PerDeviceOnce configured;       // per device: the attribute belongs to a device's copy of the kernel
@@ -480,6 +491,7 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, 
                                      seq_slot, seq_start, cu_seqlens, n_heads, n_kv_heads, scale_log2, window,
                                      out_scale, (__nv_bfloat16*)out, out_ld, (uint32_t)SMEM, status,
                                      softcap * 1.4426950408889634f, softcap > 0.f ? scale / softcap : 0.f, keep_first, sink, shared != nullptr ? *shared : mk,
+                                     low != nullptr ? *low : mk,
                                      (const __nv_bfloat16*)gate, gate_ld);
     return check_launch(e, "attention_tcgen05");
 }
@@ -554,11 +566,12 @@ RI_API int ri_attention_tcgen05_prefill_forms(const void* map_q, const void* map
 
 // Expanded latent attention (`LATENT` above): queries of heads * 192 channels a row (map_q), rows of heads * (128 key + 128 value)
 // channels (map_kv) and of 64 shared key channels (map_shared), all of the step's tokens side by side; every sequence starts at
-// position 0.  gate (bfloat16 [tokens, gate_ld], or null): a gate per head; sink, window (>= 0): as above.
-RI_API int ri_attention_tcgen05_expanded(const void* map_q, const void* map_kv, const void* map_shared, const int* seq_slot,
-                                         const int* seq_start, const int* cu_seqlens, void* out, int out_ld, int n_seqs, int max_new,
-                                         int n_heads, float scale, int window, const float* sink, const void* gate, int gate_ld,
-                                         int* status, cudaStream_t stream) {
+// position 0.  map_low (or null): rows of heads * 128 channels, the values' second terms.  gate (bfloat16 [tokens, gate_ld], or
+// null): a gate per head; sink, window (>= 0): as above.
+RI_API int ri_attention_tcgen05_expanded(const void* map_q, const void* map_kv, const void* map_shared, const void* map_low,
+                                         const int* seq_slot, const int* seq_start, const int* cu_seqlens, void* out, int out_ld,
+                                         int n_seqs, int max_new, int n_heads, float scale, int window, const float* sink,
+                                         const void* gate, int gate_ld, int* status, cudaStream_t stream) {
     if (n_seqs <= 0 || max_new <= 0) return 0;
     if (out_ld % 8 || (uintptr_t)out % 16) return fail("attention_tcgen05: out rows of %d are not aligned 16-byte pieces", out_ld);
     if (window < 0 || n_heads <= 0 || n_heads > 65535 || n_seqs > 65535)
@@ -566,11 +579,17 @@ RI_API int ri_attention_tcgen05_expanded(const void* map_q, const void* map_kv, 
     const CUtensorMap& mq = *reinterpret_cast<const CUtensorMap*>(map_q);
     const CUtensorMap& mk = *reinterpret_cast<const CUtensorMap*>(map_kv);
     const CUtensorMap* ms = reinterpret_cast<const CUtensorMap*>(map_shared);
-    if (sink != nullptr)
-        return launch<192, 128, true, true>(mq, mk, mk, nullptr, 0, seq_slot, seq_start, cu_seqlens, n_seqs, max_new, n_heads, n_heads, scale,
-                                            window, 1.f, out, out_ld, status, stream, 0.f, 0, sink, ms, gate, gate_ld);
-    return launch<192, 128, false, true>(mq, mk, mk, nullptr, 0, seq_slot, seq_start, cu_seqlens, n_seqs, max_new, n_heads, n_heads, scale,
-                                         window, 1.f, out, out_ld, status, stream, 0.f, 0, nullptr, ms, gate, gate_ld);
+    const CUtensorMap* ml = reinterpret_cast<const CUtensorMap*>(map_low);
+#define RI_EXPANDED(FORMS, TERMS)                                                                                                         \
+    return launch<192, 128, FORMS, TERMS>(mq, mk, mk, nullptr, 0, seq_slot, seq_start, cu_seqlens, n_seqs, max_new, n_heads, n_heads,     \
+                                          scale, window, 1.f, out, out_ld, status, stream, 0.f, 0, sink, ms, ml, gate, gate_ld)
+    if (sink != nullptr) {
+        if (ml != nullptr) RI_EXPANDED(true, 2);
+        RI_EXPANDED(true, 1);
+    }
+    if (ml != nullptr) RI_EXPANDED(false, 2);
+    RI_EXPANDED(false, 1);
+#undef RI_EXPANDED
 }
 
 RI_DEFINE_LAST_ERROR()

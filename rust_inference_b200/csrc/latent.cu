@@ -13,6 +13,8 @@
 //              head (a head's tokens consecutive: the rows of the per-head products), the rotated query
 //              parts rotated into the wide query rows [T, heads, rank + rd]; and the lists that the grouped
 //              products want (every head is a group of T rows).
+//   terms      the keys and values formed so, where the product left them in float32 (short prompts): keys in bfloat16, values in
+//              two bfloat16 terms.
 //   widen      the per-head products' float32 results [heads, T, rank] into the wide query rows.
 //   expand     (instead of prepare, for prompts that start their sequences: keys and values are formed head by head and the
 //              cached rows are not the operands) rotates the queries' rotated parts where they were projected, writes the cache
@@ -234,6 +236,29 @@ latent_expand_kernel(__nv_bfloat16* proj, int ld, const float* __restrict__ cos_
     for (int j = rot + tid; j < rd; j += EXPAND_THREADS) k_out[j] = kept[rank + j] = lat[rank + j];
 }
 
+// A token's keys and values, float32, head by head (d key, vd value channels), in bfloat16; of a value also what that leaves,
+// rounded once more.
+__global__ void latent_terms_kernel(const float* kv32, __nv_bfloat16* kv, __nv_bfloat16* low, int n_tokens, int n_heads, int d, int vd) {
+    let_next_kernel_start();
+    wait_for_previous_kernels();
+    const int per = (d + vd) / 8;
+    const size_t total = (size_t)n_tokens * n_heads * per;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+        const size_t th = i / per;
+        const int c = (int)(i % per) * 8;
+        const float4* src = reinterpret_cast<const float4*>(kv32 + th * (d + vd) + c);
+        const float4 a = src[0], b = src[1];
+        float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}, up[8];
+        const uint4 upper = eight_of(v);
+        *reinterpret_cast<uint4*>(kv + th * (d + vd) + c) = upper;
+        if (c < d) continue;
+        eight(reinterpret_cast<const __nv_bfloat16*>(&upper), up);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = fabsf(up[e]) <= 3.402823466e38f ? v[e] - up[e] : 0.f;      // an infinite or NaN value has no second term
+        *reinterpret_cast<uint4*>(low + th * vd + (c - d)) = eight_of(v);
+    }
+}
+
 template <typename T>
 __global__ void latent_widen_kernel(const float* __restrict__ q_lat, T* __restrict__ q_wide, int n_tokens, int n_heads,
                                     int rank, int rd, int vec) {
@@ -377,6 +402,17 @@ RI_API int ri_latent_expand(void* proj, int ld, const float* cos_t, const float*
                                      eps, token_pos, token_seq, seq_slot, page_table, max_pages, (__nv_bfloat16*)cache,
                                      (__nv_bfloat16*)c_rows, (__nv_bfloat16*)k_rows, n_heads, d, rd, rank, rot, style, page_size, own);
     return check_launch(e, "latent_expand");
+}
+
+// kv32 float32 [n_tokens, n_heads * (d + vd)] into kv (bfloat16, the same rows) and low (bfloat16 [n_tokens, n_heads * vd]): kv + low
+// holds a value to 16 bits.
+RI_API int ri_latent_terms(const float* kv32, void* kv, void* low, int n_tokens, int n_heads, int d, int vd, cudaStream_t stream) {
+    if (n_tokens <= 0) return 0;
+    if (d % 8 || vd % 8 || ((uintptr_t)kv32 | (uintptr_t)kv | (uintptr_t)low) % 16)
+        return fail("latent_terms: rows must be whole, aligned 16-byte pieces");
+    const cudaError_t e = launch_dependent(latent_terms_kernel, blocks_for((size_t)n_tokens * n_heads * ((d + vd) / 8)), 256, 0, stream, kv32,
+                                           (__nv_bfloat16*)kv, (__nv_bfloat16*)low, n_tokens, n_heads, d, vd);
+    return check_launch(e, "latent_terms");
 }
 
 RI_DEFINE_LAST_ERROR()

@@ -86,12 +86,13 @@ EXPANDED_SIZES = (128, 64, 128)      # a head's own key channels, the key channe
 
 def expanded(q: torch.Tensor, kv: torch.Tensor, shared: torch.Tensor, seq_slot, seq_start, cu_seqlens, out: torch.Tensor, *,
              n_seqs: int, max_new: int, n_heads: int, scale: float, window: int = 0, sink: torch.Tensor | None = None,
-             gate: torch.Tensor | None = None) -> torch.Tensor:
+             gate: torch.Tensor | None = None, low: torch.Tensor | None = None) -> torch.Tensor:
     """bf16 causal attention of prompts that start their sequences, over keys and values formed from the step's own tokens: q's
     leading columns hold heads of 128 + 64 channels, kv [T, heads * (128 + 128)] a head's keys and values side by side, shared
     [T, 64] the key channels that all heads share.  gate: a view [T, heads] of wider bfloat16 rows; the result of token t and
-    head h is multiplied by sigmoid(gate[t, h]).  sink, window: see `prefill`."""
-    _need_cuda(q, kv, shared, seq_slot, seq_start, cu_seqlens, out, sink, gate)
+    head h is multiplied by sigmoid(gate[t, h]).  low [T, heads * 128]: what is added to the values (their second terms).  sink,
+    window: see `prefill`."""
+    _need_cuda(q, kv, shared, seq_slot, seq_start, cu_seqlens, out, sink, gate, low)
     own, common, vd = EXPANDED_SIZES
     n = q.shape[0]
     _need(q.dtype == kv.dtype == shared.dtype == out.dtype == torch.bfloat16 and q.is_contiguous() and kv.is_contiguous()
@@ -102,13 +103,16 @@ def expanded(q: torch.Tensor, kv: torch.Tensor, shared: torch.Tensor, seq_slot, 
           "attention_tcgen05: sink must be float32 [heads]")
     _need(gate is None or (gate.dtype == torch.bfloat16 and gate.shape == (n, n_heads) and gate.stride(1) == 1),
           "attention_tcgen05: gates are bfloat16 [tokens, heads]")
+    _need(low is None or (low.dtype == torch.bfloat16 and low.is_contiguous() and low.shape == (n, n_heads * vd)),
+          "attention_tcgen05: the values' second terms are bfloat16 [tokens, heads * value channels]")
     mq = _map(0, q, n, q.shape[1], q.shape[1])
     mkv = _map(1, kv, n, kv.shape[1], kv.shape[1])
     ms = _map(1, shared, n, common, common)
+    ml = _map(1, low, n, low.shape[1], low.shape[1]) if low is not None else None
     st = status_word()
     _call("attention_tcgen05", "ri_attention_tcgen05_expanded", c_void_p(mq.data_ptr()), c_void_p(mkv.data_ptr()),
-          c_void_p(ms.data_ptr()), _p(seq_slot), _p(seq_start), _p(cu_seqlens), _p(out), c_int(out.shape[1]), c_int(n_seqs),
-          c_int(max_new), c_int(n_heads), c_float(scale), c_int(window), _p(sink), _p(gate),
+          c_void_p(ms.data_ptr()), _p(ml), _p(seq_slot), _p(seq_start), _p(cu_seqlens), _p(out), c_int(out.shape[1]),
+          c_int(n_seqs), c_int(max_new), c_int(n_heads), c_float(scale), c_int(window), _p(sink), _p(gate),
           c_int(gate.stride(0) if gate is not None else 0), c_void_p(st.data_ptr()), _stream())
     return out
 

@@ -1092,6 +1092,17 @@ def latent_expand(proj: torch.Tensor, cos, sin, latent_weight, eps: float, token
           c_int(page_size), c_int(1 if own else 0), _stream())
 
 
+def latent_terms(kv32: torch.Tensor, kv: torch.Tensor, low: torch.Tensor, *, n_heads: int, head_dim: int, v_head_dim: int) -> None:
+    """kv32 (float32 [T, heads * (head_dim + v_head_dim)], a head's keys beside its values) rounded into kv (bfloat16, the same
+    shape), and what the rounding took off the values into low (bfloat16 [T, heads * v_head_dim])."""
+    _need_cuda(kv32, kv, low)
+    n = kv32.shape[0]
+    _need(kv32.dtype == torch.float32 and kv.dtype == low.dtype == torch.bfloat16 and kv32.is_contiguous() and kv.is_contiguous()
+          and low.is_contiguous() and kv32.shape == kv.shape == (n, n_heads * (head_dim + v_head_dim))
+          and low.shape == (n, n_heads * v_head_dim), "latent_terms: shapes")
+    _call("latent", "ri_latent_terms", _p(kv32), _p(kv), _p(low), c_int(n), c_int(n_heads), c_int(head_dim), c_int(v_head_dim), _stream())
+
+
 def latent_widen(q_lat: torch.Tensor, q_wide: torch.Tensor, *, n_tokens: int, n_heads: int, rank: int, rot_dim: int) -> None:
     """q_wide[t, h, :rank] = q_lat[h, t, :] (float32 [heads, T, rank] into the run dtype's wide query rows)."""
     _need_cuda(q_lat, q_wide)

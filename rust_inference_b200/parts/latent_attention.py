@@ -133,13 +133,21 @@ class LatentAttention(Mixer):
         return ((self.head_dim, self.rot_dim, self.v_head_dim) == attention_tc.EXPANDED_SIZES and self.kv_rank % 8 == 0
                 and self.kv_rank <= 4096)
 
-    def _expands(self, ctx) -> bool:
+    # Steps whose shortest prompt has fewer tokens than this hold their values in two bfloat16 terms.  Rounding every value instead
+    # of the weighted latents costs accuracy while few keys are averaged.  How far the layer's output is from 64 bits, 1e-3, in
+    # one term / in two / in the carried form (1,024 wide, a latent of 256, eight seeds): 2 tokens 3.52 / 3.12 / 3.32, 16 tokens
+    # 3.86 / 3.51 / 3.82, 64 tokens 4.02 / 3.72 / 4.02, 256 tokens 3.96 / 3.70 / 4.01, 400 tokens 3.87 / 3.62 / 3.95 (2,048 wide, a
+    # latent of 512: 16 tokens 3.90 / 3.55 / 3.83, 192 tokens 4.09 / 3.79 / 4.09, 256 tokens 4.06 / 3.78 / 4.08).
+    TWO_TERMS_BELOW = 256
+
+    def _expands(self, x, ctx) -> bool:
         """Prompts that start their sequences form every head's keys and values from the latents: a score then has head_dim +
         rot_dim channels and a value v_head_dim, where the carried form has kv_rank + rot_dim and kv_rank for each (at 2,048
         tokens, 16 heads and a latent of 512 a third of the multiply-adds, on the tcgen05 kernel).  Steps with cached positions
-        would have to form those positions' keys and values again, so they, and single tokens, stay with the carried form."""
+        would have to form those positions' keys and values again, so they, and single tokens, stay with the carried form; so do
+        the small steps without gates whose projection is added up and kept in float32."""
         return (self.w_ukv is not None and not ctx.all_single and ctx.host_starts is not None and not any(ctx.host_starts)
-                and ctx.page_size == 64)
+                and ctx.page_size == 64 and self.w_in.n % 8 == 0 and (self.gated or not linear.wants_split(x, self.w_in)))
 
     def _forward_expanded(self, x, residual, ctx, cache_layer):
         from ..kernels import attention_tc
@@ -153,12 +161,19 @@ class LatentAttention(Mixer):
                           ctx.page_table, cache_layer.k, c_rows, k_rows, n_heads=H, head_dim=d, rot_dim=rd, rank=kr,
                           rot_dims=pos.rot_dims, style=pos.style, page_size=ctx.page_size, own=self.own_latent)
         kv = ctx.buffer("latent_kv", (n, H * (d + vd)), self.dtype)
-        linear.project(c_rows, self.w_ukv, kv, ctx)
+        low = None
+        if min(ctx.host_counts) < self.TWO_TERMS_BELOW:
+            kv32 = ctx.buffer("latent_kv32", (n, H * (d + vd)), torch.float32)
+            linear.logits(c_rows, self.w_ukv, kv32, ctx)
+            low = ctx.buffer("latent_v_low", (n, H * vd), self.dtype)
+            ops.latent_terms(kv32, kv, low, n_heads=H, head_dim=d, v_head_dim=vd)
+        else:
+            linear.project(c_rows, self.w_ukv, kv, ctx)
         out = ctx.buffer("attn_out", (n, H * vd), self.dtype)
         gates = proj[:, self.w_in.n - H:] if self.gated else None
         attention_tc.expanded(proj, kv, k_rows, ctx.seq_slot, ctx.seq_start, ctx.cu_seqlens, out, n_seqs=ctx.n_seqs,
                               max_new=ctx.max_new, n_heads=H, scale=self.scale, window=self.window or 0, sink=self.sinks,
-                              gate=gates)
+                              gate=gates, low=low)
         linear.into_residual(out, self.w_o, residual, ctx)
 
     # ---- the step ------------------------------------------------------------------------------------------
@@ -179,7 +194,7 @@ class LatentAttention(Mixer):
         pos = self.position
         if pos.cos is None or pos.cos.shape[0] < ctx.max_len:
             raise RuntimeError("rope tables do not cover the step's positions; call prepare() first")
-        if self._expands(ctx) and (self.w_in.n % 8) == 0:
+        if self._expands(x, ctx):
             self._forward_expanded(x, residual, ctx, cache_layer)
             return
         if not self.gated and linear.wants_split(x, self.w_in):

@@ -122,3 +122,64 @@ def test_neighbours_with_infinities(first, gated):
     alone, beside = run(first, [first]), run(total, [first, second])
     assert bool(alone.isfinite().all())
     assert torch.equal(beside[:first], alone)
+
+
+@pytest.mark.parametrize("lengths", [[2], [16, 5], [70, 128]])
+def test_values_in_two_terms(lengths):
+    """Short prompts hold a value as the sum of two bfloat16 numbers: the float32 values come back to 2^-16, and the attention over
+    them is as close to 64 bits over the float32 values as its rounded weights and result (2^-8 each at most) allow; where a
+    token sees one key (weight 1), only the result is rounded."""
+    from rust_inference_b200.kernels import attention_tc, ops, tcgen05
+    heads, total = 3, sum(lengths)
+    g = torch.Generator(device="cuda").manual_seed(total)
+    kv32 = torch.randn(total, heads * 256, device="cuda", generator=g)
+    q, shared = (torch.randn(total, n, device="cuda", generator=g).bfloat16() for n in (heads * 192, 64))
+    kv, low = torch.empty(total, heads * 256, dtype=torch.bfloat16, device="cuda"), torch.empty(total, heads * 128, dtype=torch.bfloat16, device="cuda")
+    ops.latent_terms(kv32, kv, low, n_heads=heads, head_dim=128, v_head_dim=128)
+    assert torch.equal(kv, kv32.bfloat16())
+    values = kv32.view(total, heads, 256)[:, :, 128:].double()
+    terms = kv.view(total, heads, 256)[:, :, 128:].double() + low.view(total, heads, 128).double()
+    assert ((terms - values).abs() <= 2.0 ** -16 * values.abs()).all()
+    cu = torch.tensor([sum(lengths[:i]) for i in range(len(lengths) + 1)], dtype=torch.int32, device="cuda")
+    zeros = torch.zeros(len(lengths), dtype=torch.int32, device="cuda")
+    out = torch.empty(total, heads * 128, dtype=torch.bfloat16, device="cuda")
+    attention_tc.expanded(q, kv, shared, zeros, zeros, cu, out, n_seqs=len(lengths), max_new=max(lengths), n_heads=heads,
+                          scale=192 ** -0.5, low=low)
+    torch.cuda.synchronize()
+    tcgen05.check_status()
+    at = 0
+    for n in lengths:
+        rows = slice(at, at + n)
+        hidden = torch.ones(n, n, dtype=torch.bool, device="cuda").triu(1)
+        for h in range(heads):
+            k = torch.cat([kv[rows, h * 256:h * 256 + 128], shared[rows]], 1).double()
+            s = (q[rows, h * 192:(h + 1) * 192].double() @ k.T * 192 ** -0.5).masked_fill(hidden, -math.inf)
+            want = torch.softmax(s, 1) @ values[rows, h]
+            got = out[rows, h * 128:(h + 1) * 128].double()
+            assert ((got[0] - want[0]).abs() <= 2.0 ** -8 * (1 + 2.0 ** -7) * want[0].abs()).all()
+            assert (got - want).abs().max().item() <= 2 ** -7 * want.abs().max().item()
+        at += n
+
+
+def test_short_prompts_take_two_terms(monkeypatch):
+    """The shortest prompt of a step decides."""
+    from rust_inference_b200 import config_from_dict
+    from rust_inference_b200.config.registry import get_architecture
+    from rust_inference_b200.engine.engine import Engine
+    from rust_inference_b200.engine.model import DecoderModel
+    from rust_inference_b200.kernels import attention_tc
+    cfg = _config(8, 64, [None])
+    config = config_from_dict(cfg)
+    model = DecoderModel(get_architecture(config.architecture).build_spec(config), dtype=torch.bfloat16, device="cuda")
+    model.load(plain_vadodra.random_weights(cfg, seed=1).items())
+    eng = Engine(model, max_tokens=2048, max_seq_len=1024, n_slots=4)
+    taken = []
+    expanded = attention_tc.expanded
+    monkeypatch.setattr(attention_tc, "expanded", lambda *a, **k: taken.append(k["low"] is not None) or expanded(*a, **k))
+    for lengths in ([255], [256], [300, 256], [300, 2]):
+        slots = [eng.alloc_slot() for _ in lengths]
+        eng.step(slots, [random_tokens(n, cfg["vocab"], seed=n) for n in lengths], "last")
+        for slot in slots:
+            eng.free_slot(slot)
+    eng.check_device_status()
+    assert taken == [True, False, False, True]
