@@ -4,6 +4,7 @@ tokens, unequal batches, slots and pages used again, keys at the edges of chunks
 decoding, and greedy generation through `Model.generate`."""
 import math
 
+import numpy as np
 import pytest
 import torch
 
@@ -196,6 +197,35 @@ def test_recurrence_in_portions_and_slots(heads, dim, vdim, lens, cuts):
         got = run(portions)
         for b in range(2):
             assert rel_err(got[b], want[b]) < 2e-5, (portions, b)
+
+
+@pytest.mark.parametrize("vdim", [24, 33, 64, 128, 130, 200, 512, 516])
+def test_head_norm_adds_in_one_order(vdim):
+    """The norm over a head's read-out, to the bit: lane l of a warp adds the squares of the values l, l + 32, ... one after the
+    other, then the lanes meet in a tree."""
+    from rust_inference_b200.kernels import ops
+    heads, dim, n, eps, scale = 2, 8, 7, 1e-5, 0.6
+    g = torch.Generator().manual_seed(vdim)
+    z = torch.randn(n, heads * (2 * dim + vdim), generator=g)
+    w = 1 + torch.randn(vdim, generator=g) * 0.2
+    raw, out = torch.empty(n, heads * vdim, device=DEV), torch.empty(n, heads * vdim, device=DEV)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    ops.gated_recurrence(d(z), torch.zeros(heads * dim, device=DEV), torch.zeros(heads * dim, device=DEV), d(w),
+                         torch.zeros(1, heads, dim, vdim, device=DEV), i32([0, n]), i32([0]), out, n_seqs=1, heads=heads, dim=dim,
+                         vdim=vdim, eps=eps, out_scale=scale, o_raw=raw)
+    o = raw.cpu().view(n, heads, vdim).numpy()
+    padded = np.zeros((n, heads, -(-vdim // 32) * 32), dtype=np.float32)
+    padded[..., :vdim] = o
+    lanes = np.zeros((n, heads, 32), dtype=np.float32)
+    for row in np.moveaxis(padded.reshape(n, heads, -1, 32), 2, 0):
+        # a fused multiply-add: the product whole, one rounding (64 bits hold the sum but for cases rarer than one in 2^30)
+        lanes = (row.astype(np.longdouble) * row + lanes).astype(np.float32)
+    for step in (16, 8, 4, 2, 1):
+        lanes = lanes + lanes[..., np.arange(32) ^ step]
+    inv = np.float32(1) / np.sqrt(lanes[..., :1] / np.float32(vdim) + np.float32(eps))
+    want = o * inv * w.numpy() * np.float32(scale)
+    assert want.dtype == np.float32
+    assert np.array_equal(out.cpu().view(n, heads, vdim).numpy(), want)
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
