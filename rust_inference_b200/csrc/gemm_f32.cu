@@ -9,14 +9,18 @@
 //
 // More rows: the tensor cores, without giving up 32 bits.  A float32 number is the exact sum of three bfloat16 numbers
 // (its leading 8 significant bits, the next 8 and the last 8), so x * w is the sum of nine products of bfloat16 numbers,
-// each exact in the tensor core; the three smallest (mid * low, low * mid, low * low) are below 2^-24 of the whole and are
-// left out.  Eight warps read both operands, cut them and put the parts into shared memory as the MMA wants them
-// (128-byte swizzle); six MMAs per 16 steps of K, smallest products first, add up 64 steps of K in tensor memory; then
-// eight warps add that sum onto float32 registers and the next 64 steps start from zero, so that the tensor core's own
-// additions, which truncate, never run over more than 64 steps.  Against 64 bits (rows of N(0, 1) times rows of N(0, 1/K)) the
-// result is off by 1.3e-7 at K = 192, 1.4e-7 at 896, 1.5e-7 at 4,864 and 2.1e-7 at 18,944, where one running FFMA sum was off
-// by 2.5e-7, 5.3e-7, 1.2e-6 and 2.5e-6 (the kernel for few rows: 0.8e-7 to 1.8e-7).  A number that is infinite or NaN has no such parts (they turn every sum that they meet
-// infinite or NaN): a tile with such a sum computes its piece again with FFMA, so that it comes out as the plain sum gives it.
+// each exact in the tensor core.  The last one (low * low) is below 2^-30 of the whole and is left out; the other eight are added.
+// Eight warps read both operands, cut them and put the parts into shared memory as the MMA wants them (128-byte swizzle); eight
+// MMAs per 16 steps of K add up 64 steps of K in tensor memory, the seven small products in a sum of their own: the tensor
+// core's additions truncate, which would cost the large product's sum its last bits with every small one.  Then eight warps
+// add both sums onto float32 registers and the next 64 steps start from zero, so that truncated sums never run over more.
+// Off from 64 bits (root mean square over that of the results; in brackets one running FFMA sum, `gemm_simt.cu`), rows of
+// N(0, 1) times rows of N(0, 1/K): 0.75e-7 at K = 128 (2.0e-7), 0.94e-7 at 896 (5.4e-7), 1.1e-7 at 4,864 (12e-7), 1.4e-7 at 18,944
+// (25e-7); all-positive rows 0.81e-7 at 896 (4.2e-7), where sums are too small by 0.67e-7 on average; rows with one entry 0.25e-7
+// (0.25e-7), with 2 of 896 0.36e-7 (0.31e-7: every block's sum is rounded for itself), with 4 0.46e-7 (0.41e-7), with 16 0.62e-7
+// (0.76e-7).  The kernel for few rows: 0.7e-7 to 1.8e-7 dense, 0.25e-7, 0.38e-7, 0.49e-7 and 0.64e-7 for those few entries.
+// A number that is infinite or NaN has no such parts (they turn every sum that they meet infinite or NaN): a tile with
+// such a sum computes its piece again with FFMA, so that it comes out as the plain sum gives it.
 //
 // Epilogues as in `gemm_simt.cu` (0 and 1 are the same here: float32 with a bias): 2 out += acc, 3 gated, 4 an activation,
 // 5 silu for the first columns.
@@ -240,41 +244,49 @@ int launch_few(const float* X, const float* W, const float* W2, const float* bia
 // Many rows of X: three bfloat16 parts per operand on the tensor cores.
 //
 // A tile is 128 rows of W (gated: 64 gate rows and the 64 up rows of the same features) by TN rows of X.  What bounds a
-// block of 64 steps of K is shared memory (24 MMAs that read 4 KiB of W and TN * 32 bytes of X each, and the parts' writes: at
-// TN = 128 about 2,300 clocks against 1,536 of the tensor core, at TN = 64 1,730 against 768, so TN is 128 wherever a step has
-// that many rows) and the cutting, eight warps with a few dependent instructions per number.  Four warps instead of eight for
-// the additions made those the slowest part: 954 against 862 us at 333 x 151,936 x 896 (the FFMA kernel
-// takes 2,950), 50 against 46 at 333 x 896 x 4,864 (345); sixteen warps for the cutting, 929 and 51.
-// Looking for infinities and NaN in the sums instead of in every number that is cut: 837 (108 TFLOP/s of the product) and 45.
+// block of 64 steps of K is shared memory (32 MMAs that read 4 KiB of W and TN * 32 bytes of X each, and the parts' writes: at
+// TN = 128 about 2,800 clocks against 2,048 of the tensor core, at TN = 64 2,100 against 1,024, so TN is 128 wherever a step has
+// that many rows) and the cutting, eight warps with a few dependent instructions per number.  333 x 151,936 x 896 takes 997 us (90
+// TFLOP/s of the product; the FFMA kernel 2,950), 333 x 896 x 4,864 52 (345).  Tried on the way there, with six products in one
+// sum: four warps instead of eight for the additions 954 against 862, sixteen for the cutting 929; looking for infinities and NaN
+// in the sums instead of in every number that is cut 837.  The two further products and the sum of their own cost 15% of
+// that and are what makes the result as close to 64 bits as a plain float32 sum for any rows; parts rounded instead of cut off,
+// with six products, took as long and left a single product off by up to 1.4 x 2^-24.
 // ---------------------------------------------------------------------------------------------------------------------
 constexpr int ROWS = 128, BK = 64, PART = ROWS * BK * 2, STAGES = 2;
 constexpr int CUT_WARPS = 8, CUT_THREADS = CUT_WARPS * 32, ADD_WARPS = 8;
 constexpr int SPLIT_THREADS = CUT_THREADS + ADD_WARPS * 32;
 enum Status { ST_CUT_TIMEOUT = 41, ST_MMA_TIMEOUT = 42, ST_ADD_TIMEOUT = 43 };
 
-// x as three bfloat16 numbers that add up to it exactly, each the upper half of a float32: the leading 8 significant bits,
-// the next 8 and the rest.  An infinite x gives an infinity and two NaN, a NaN three.
-__device__ __forceinline__ void cut(float x, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-    hi = __float_as_uint(x) & 0xffff0000u;
-    const float r = x - __uint_as_float(hi);
-    mid = __float_as_uint(r) & 0xffff0000u;
-    const float r2 = r - __uint_as_float(mid);
-    lo = __float_as_uint(r2);
+// x * 2^16 as three bfloat16 numbers that add up to it exactly, each the upper half of a float32: the leading 8 significant
+// bits, the next 8 and the rest.  The factor keeps the parts of every float32 number, the denormal ones too, among the numbers
+// bfloat16 has (without it numbers below 2^-110 lose bits); the sums are divided by both operands' factors at the end.  From
+// 2^112 on the parts become infinite or NaN, as those of an infinity or a NaN are.
+constexpr float UP = 65536.f, DOWN = 1.f / (UP * UP);
+__device__ __forceinline__ float2 two(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 leading(const float2& v) {
+    return make_float2(__uint_as_float(__float_as_uint(v.x) & 0xffff0000u), __uint_as_float(__float_as_uint(v.y) & 0xffff0000u));
 }
-__device__ __forceinline__ uint32_t upper_halves(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x7632); }
+__device__ __forceinline__ uint32_t upper_halves(const float2& v) { return __byte_perm(__float_as_uint(v.x), __float_as_uint(v.y), 0x7632); }
+__device__ __forceinline__ void cut(float2 v, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+    v = __fmul2_rn(v, two(UP));
+    hi = upper_halves(v);
+    v = __ffma2_rn(leading(v), two(-1.f), v);
+    mid = upper_halves(v);
+    v = __ffma2_rn(leading(v), two(-1.f), v);
+    lo = upper_halves(v);
+}
 __device__ __forceinline__ void store8(uint32_t addr, uint32_t a, uint32_t b) {
     asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
 }
 // four consecutive k of one row into the three parts
 __device__ __forceinline__ void put(uint32_t addr, uint32_t part_bytes, const float4& v) {
-    uint32_t h[4], m[4], l[4];
-    cut(v.x, h[0], m[0], l[0]);
-    cut(v.y, h[1], m[1], l[1]);
-    cut(v.z, h[2], m[2], l[2]);
-    cut(v.w, h[3], m[3], l[3]);
-    store8(addr, upper_halves(h[0], h[1]), upper_halves(h[2], h[3]));
-    store8(addr + part_bytes, upper_halves(m[0], m[1]), upper_halves(m[2], m[3]));
-    store8(addr + 2 * part_bytes, upper_halves(l[0], l[1]), upper_halves(l[2], l[3]));
+    uint32_t h[2], m[2], l[2];
+    cut(make_float2(v.x, v.y), h[0], m[0], l[0]);
+    cut(make_float2(v.z, v.w), h[1], m[1], l[1]);
+    store8(addr, h[0], h[1]);
+    store8(addr + part_bytes, m[0], m[1]);
+    store8(addr + 2 * part_bytes, l[0], l[1]);
 }
 
 template <int TN, int MODE>
@@ -285,7 +297,8 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
     constexpr int FEATS = DUAL ? ROWS / 2 : ROWS;
     constexpr int X_PART = TN * BK * 2;
     constexpr int STAGE = 3 * (PART + X_PART);
-    constexpr int TMEM_COLS = 2 * TN < 32 ? 32 : 2 * TN;
+    constexpr int ACC = 2 * TN;                  // tensor memory columns of a block of K: the large products' sums, the small ones'
+    constexpr int TMEM_COLS = 2 * ACC;
     constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
@@ -404,15 +417,17 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
             }
             tc_fence_after();
             const uint64_t off = (uint64_t)((uint32_t)(s * STAGE) >> 4);
-            const uint32_t acc = tmem + (uint32_t)(buf * TN);
-            // (part of W, part of X), the smallest products first: the sum they start is rounded at their own size
-            constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
+            const uint32_t acc = tmem + (uint32_t)(buf * ACC);
+            // (part of W, part of X), the smallest products first; the last is the large one
+            constexpr int PRODUCTS = 8, PA[PRODUCTS] = {1, 2, 2, 0, 1, 1, 0, 0}, PB[PRODUCTS] = {2, 1, 0, 2, 1, 0, 1, 0};
 #pragma unroll
-            for (int p = 0; p < 6; ++p)
+            for (int p = 0; p < PRODUCTS; ++p) {
+                const bool large = p == PRODUCTS - 1;
 #pragma unroll
                 for (int k = 0; k < BK / 16; ++k)
-                    umma(acc, a_desc + off + (uint64_t)(PA[p] * (PART >> 4) + 2 * k), b_desc + off + (uint64_t)(PB[p] * (X_PART >> 4) + 2 * k),
-                         IDESC, p > 0 || k > 0);
+                    umma(large ? acc : acc + TN, a_desc + off + (uint64_t)(PA[p] * (PART >> 4) + 2 * k),
+                         b_desc + off + (uint64_t)(PB[p] * (X_PART >> 4) + 2 * k), IDESC, (p > 0 && !large) || k > 0);
+            }
             umma_commit(smem_u32(&empty_bar[s]));
             umma_commit(smem_u32(&acc_full[buf]));
         };
@@ -432,16 +447,14 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
             __syncwarp();
             if (abort_flag) break;
             tc_fence_after();
-            // half of the columns at a time: a trip to tensor memory takes as long for 32 columns as for 16
-            constexpr int AT_ONCE = COLS < 32 ? COLS : 32;
 #pragma unroll
-            for (int c0 = 0; c0 < COLS; c0 += AT_ONCE) {
-                uint32_t v[AT_ONCE];
-#pragma unroll
-                for (int c = 0; c < AT_ONCE; c += 16) tmem_ld16(trow + (uint32_t)(buf * TN + c0 + c), v + c);
+            for (int c0 = 0; c0 < COLS; c0 += 16) {
+                uint32_t large[16], small[16];
+                tmem_ld16(trow + (uint32_t)(buf * ACC + c0), large);
+                tmem_ld16(trow + (uint32_t)(buf * ACC + TN + c0), small);
                 tmem_wait_ld();
 #pragma unroll
-                for (int j = 0; j < AT_ONCE; ++j) acc[c0 + j] += __uint_as_float(v[j]);
+                for (int j = 0; j < 16; ++j) acc[c0 + j] += __uint_as_float(large[j]) + __uint_as_float(small[j]);
             }
             tc_fence_before();
             __syncwarp();
@@ -456,7 +469,7 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
             bool finite = true;
 #pragma unroll
             for (int c = 0; c < COLS; ++c) {
-                pieces[(part * COLS + c) * ROWS + q * 32 + lane] = acc[c];
+                pieces[(part * COLS + c) * ROWS + q * 32 + lane] = acc[c] * DOWN;
                 finite &= fabsf(acc[c]) <= 3.402823466e38f;
             }
             if (!finite) odd_flag = 1;

@@ -2,8 +2,8 @@
 
 Which kernel runs is decided here, by dtype and shape:
   float32   the kernels of `gemm_f32` (FFMA for a few tokens; beyond, three bfloat16 parts per operand on the
-            tensor cores, which together are the operand) when rows are whole 16-byte pieces, else the FFMA
-            kernel (`gemm_simt`);
+            tensor cores, which together are the operand: sums as close to 64 bits as the FFMA kernel's) when rows are
+            whole 16-byte pieces, else the FFMA kernel (`gemm_simt`);
   bfloat16  the tcgen05 kernel (`gemm_tcgen05`) when the shape meets its alignment rule,
             else the FFMA kernel on bf16 operands.  Either way accumulation is float32.
 """
@@ -32,9 +32,8 @@ def _use_tensor_cores(x: torch.Tensor, w: Weight) -> bool:
     return tcgen05.supports(x, w)
 
 
-# Three bfloat16 parts leave out products below 2^-24 of a term, which a sum of few terms shows: against 64 bits the tensor
-# cores' product errs by 1.0e-7 at K = 4 and 1.1e-7 at 36 (FFMA: 0.4e-7 and 1.1e-7), by 1.3e-7 at 192 and 1.5e-7 at 4,864
-# (FFMA: 2.5e-7 and 12e-7).
+# Shorter sums are left to the FFMA kernel, which has them sooner: a block of the tensor cores' kernel is 64 steps of K long and
+# costs about 4.5 us to start (us, FFMA / tensor cores, N = 512: 17 rows of K = 96 5.9 / 6.4, of K = 128 7.3 / 6.4).
 F32_PARTS_MIN_K = 128
 
 
