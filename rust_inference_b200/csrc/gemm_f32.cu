@@ -19,8 +19,8 @@
 // (25e-7); all-positive rows 0.81e-7 at 896 (4.2e-7), where sums are too small by 0.67e-7 on average; rows with one entry 0.25e-7
 // (0.25e-7), with 2 of 896 0.36e-7 (0.31e-7: every block's sum is rounded for itself), with 4 0.46e-7 (0.41e-7), with 16 0.62e-7
 // (0.76e-7).  The kernel for few rows: 0.7e-7 to 1.8e-7 dense, 0.25e-7, 0.38e-7, 0.49e-7 and 0.64e-7 for those few entries.
-// A number that is infinite or NaN has no such parts (they turn every sum that they meet infinite or NaN): a tile with
-// such a sum computes its piece again with FFMA, so that it comes out as the plain sum gives it.
+// A number that is infinite or NaN has no such parts (they turn every sum that they meet infinite or NaN): sums that came out
+// so are computed again with FFMA, as a plain float32 sum; finite ones beside them keep their bits.
 //
 // Epilogues as in `gemm_simt.cu` (0 and 1 are the same here: float32 with a bias): 2 out += acc, 3 gated, 4 an activation,
 // 5 silu for the first columns.
@@ -339,11 +339,8 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
     const uint32_t tmem = tmem_slot;
     let_next_kernel_start();
 
-    // row r of the tile: which row of which matrix (null beyond the matrix)
-    auto weight_row = [&](int r) -> const float* {
-        const int f = f0 + (DUAL ? r % FEATS : r);
-        return f < N ? (DUAL && r >= FEATS ? W2 : W) + (size_t)f * K : nullptr;
-    };
+    // row r of the tile (one that exists): which row of which matrix
+    auto weight_row = [&](int r) { return (DUAL && r >= FEATS ? W2 : W) + (size_t)(f0 + (DUAL ? r % FEATS : r)) * K; };
 
     if (warp < CUT_WARPS) {
         // ---- read, cut, store: 16 threads per row of 64 floats ----
@@ -485,15 +482,56 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
     }
     const bool failed = abort_flag != 0;
     if (odd_flag && !failed) {
-        // infinite or NaN sums: this block's piece again, as a plain float32 sum
+        // infinite or NaN sums are computed again, as plain float32 sums over this block's piece of K; the others stay what they
+        // are.  A warp looks at 32 neighbouring features of four rows of X and takes four features at a time that are to be done
+        // for any of the rows, its lanes along K, so that both operands are read in whole lines and each once for four sums
+        // (333 x 151,936 x 896 with one row of NaN: 1,262 us, 986 without; with NaN in every row 7,505, the FFMA kernel 2,962).
         const int k_end = min(K, (kb0 + n_kb) * BK);
-        for (int i = threadIdx.x; i < TN * ROWS; i += SPLIT_THREADS) {
-            const int c = i / ROWS;
-            const float* wr = weight_row(i % ROWS);
-            float v = 0.f;
-            if (wr != nullptr && t0 + c < M)
-                for (int kk = kb0 * BK; kk < k_end; ++kk) v = fmaf(X[(size_t)(t0 + c) * K + kk], wr[kk], v);
-            pieces[i] = v;
+        for (int g = warp; g < TN / 4 * (ROWS / 32); g += SPLIT_THREADS / 32) {
+            const int c0 = g / (ROWS / 32) * 4, r0 = g % (ROWS / 32) * 32;
+            const bool exists = f0 + (r0 + lane) % FEATS < N;        // zeros in the place of a row may have met an infinity too
+            const float* x[4];
+            uint32_t odd[4], todo = 0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const bool row = t0 + c0 + i < M;
+                x[i] = X + (size_t)(row ? t0 + c0 + i : t0) * K;
+                odd[i] = __ballot_sync(0xffffffffu, row && exists && !(fabsf(pieces[(c0 + i) * ROWS + r0 + lane]) <= 3.402823466e38f));
+                todo |= odd[i];
+            }
+            while (todo != 0) {
+                const float* w[4];
+                int r[4];
+                float sum[4][4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {                        // fewer than four left: the first again
+                    r[j] = todo != 0 ? __ffs(todo) - 1 : r[0];
+                    w[j] = weight_row(r0 + r[j]);
+                    todo &= todo - 1;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) sum[i][j] = 0.f;
+                }
+#pragma unroll 2
+                for (int k = kb0 * BK + lane * 4; k < k_end; k += 128) {
+                    float4 a[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) a[i] = load_written(x[i] + k);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float4 b = load_weight(w[j] + k);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            sum[i][j] = fmaf(a[i].w, b.w, fmaf(a[i].z, b.z, fmaf(a[i].y, b.y, fmaf(a[i].x, b.x, sum[i][j]))));
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float v = warp_sum(sum[i][j]);
+                        if (lane == 0 && ((odd[i] >> r[j]) & 1)) pieces[(c0 + i) * ROWS + r0 + r[j]] = v;
+                    }
+            }
         }
         __syncthreads();
     }

@@ -86,6 +86,37 @@ def test_product_with_infinities(m):
     _check_status()
 
 
+@pytest.mark.parametrize("m, n, k", [(20, 200, 640), (40, 130, 100), (200, 200, 640), (130, 391, 4864)])
+@pytest.mark.parametrize("mode", ["store", "gated"])
+def test_product_keeps_finite_sums_beside_infinite_ones(mode, m, n, k):
+    """Sums that do not meet an infinity, a NaN or an overflow keep their bits; those that do come out as the plain float32 sum's
+    infinities and NaN.  Rows and features at the matrices' ends, whose tiles are filled up with zeros, are among them."""
+    ops = _ops()
+    torch.manual_seed(m)
+    x, w, w2 = torch.randn(m, k, device=DEV), torch.randn(n, k, device=DEV), torch.randn(n, k, device=DEV)
+
+    def run(kernel, **kw):
+        out = torch.full((m, n), 9.0, device=DEV)
+        if mode == "gated":
+            kernel(x, w, out, ops.EPI_SILU_MUL, w2=w2, **kw)
+        else:
+            kernel(x, w, out, ops.EPI_STORE_F32, **kw)
+        return out
+
+    clean = run(ops.gemm_f32, few_max=0)
+    rows, cols = [1, 2, m - 1], [3, n - 1]
+    x[1, k // 3], x[2, k - 1], x[m - 1, 0] = float("inf"), float("nan"), 3e38
+    w[3, k - 2], w[n - 1, 5] = float("-inf"), float("nan")
+    got, want = run(ops.gemm_f32, few_max=0), run(ops.gemm_simt)
+    _check_status()
+    same = torch.ones(m, n, dtype=torch.bool, device=DEV)
+    same[rows] = False
+    same[:, cols] = False
+    assert torch.equal(got[same], clean[same])
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    assert torch.equal(got[got.isinf()], want[got.isinf()])
+
+
 def test_product_with_small_and_large_numbers():
     """Three parts hold a float32 number over its whole range: scaling the operands by powers of two scales the result."""
     ops = _ops()
