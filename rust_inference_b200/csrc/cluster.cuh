@@ -13,6 +13,9 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// the two halves of a meeting point, for one that nobody has to wait at: arrive early, wait late
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // the float at the same place in the shared memory of the cluster's block `rank`
 __device__ __forceinline__ float peer_float(const float* own, uint32_t rank) {
     uint32_t there;
@@ -28,6 +31,16 @@ __device__ __forceinline__ float4 peer_float4(const float* own, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"((uint32_t)__cvta_generic_to_shared(own)), "r"(rank));
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(there) : "memory");
     return v;
+}
+// Sets an int of the shared memory, which lies at the same place in every block, in all of the cluster's `blocks`.  Other blocks
+// must have set up theirs (a meeting point before) and look at it behind the next `cluster_sync`.
+__device__ __forceinline__ void set_in_all(volatile int* own, int blocks) {
+    for (int p = 0; p < blocks; ++p) {
+        uint32_t there;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there)
+                     : "r"((uint32_t)__cvta_generic_to_shared(const_cast<int*>(own))), "r"(p));
+        asm volatile("st.shared::cluster.s32 [%0], 1;" ::"r"(there) : "memory");
+    }
 }
 
 // A launch that may start under the kernel before it (`launch_dependent`), its blocks in clusters of `cluster` along x.

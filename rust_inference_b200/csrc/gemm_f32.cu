@@ -303,7 +303,7 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
-    __shared__ volatile int abort_flag, odd_flag;
+    __shared__ volatile int abort_flag, odd_flag, any_failed;
 
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     float* pieces = reinterpret_cast<float*>(smem_raw + (base - smem_u32(smem_raw)));      // [TN][128], over the stages at the end
@@ -325,7 +325,7 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
             mbar_init(smem_u32(&acc_empty[i]), ADD_WARPS);
         }
         abort_flag = 0;
-        odd_flag = 0;
+        odd_flag = any_failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == CUT_WARPS) {
@@ -337,6 +337,7 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
+    if (splits > 1) cluster_arrive();            // flags and barriers are set up
     let_next_kernel_start();
 
     // row r of the tile (one that exists): which row of which matrix
@@ -404,6 +405,7 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
         const int q = warp & 3, part = (warp - CUT_WARPS) >> 2;  // q: the TMEM lanes this warp may read
         const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(part * COLS);
         const uint64_t a_desc = make_smem_desc(base), b_desc = make_smem_desc(base + 3 * PART);
+        int issued = 0;
         auto issue = [&](int b) {                                // one lane
             const int s = b % STAGES, buf = b & 1;
             if (!(mbar_wait(smem_u32(&acc_empty[buf]), (uint32_t)((b >> 1) & 1) ^ 1u) &&
@@ -427,6 +429,7 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
             }
             umma_commit(smem_u32(&empty_bar[s]));
             umma_commit(smem_u32(&acc_full[buf]));
+            issued = b + 1;
         };
         if (warp == CUT_WARPS && lane == 0)
             for (int b = 0; b < 2 && b < n_kb && !abort_flag; ++b) issue(b);
@@ -442,7 +445,12 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
                 abort_flag = 1;
             }
             __syncwarp();
-            if (abort_flag) break;
+            if (abort_flag) {
+                // the MMAs on their way have to finish before tensor memory is given back
+                if (warp == CUT_WARPS && lane == 0)
+                    for (int i = max(0, issued - 2); i < issued; ++i) mbar_wait(smem_u32(&acc_full[i & 1]), (uint32_t)((i >> 1) & 1));
+                break;
+            }
             tc_fence_after();
 #pragma unroll
             for (int c0 = 0; c0 < COLS; c0 += 16) {
@@ -480,7 +488,7 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)TMEM_COLS) : "memory");
     }
-    const bool failed = abort_flag != 0;
+    bool failed = abort_flag != 0;
     if (odd_flag && !failed) {
         // infinite or NaN sums are computed again, as plain float32 sums over this block's piece of K; the others stay what they
         // are.  A warp looks at 32 neighbouring features of four rows of X and takes four features at a time that are to be done
@@ -535,7 +543,12 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
         }
         __syncthreads();
     }
-    if (splits > 1) cluster_sync();
+    if (splits > 1) {
+        cluster_wait();                          // the peers have started
+        if (failed && threadIdx.x == 0) set_in_all(&any_failed, splits);
+        cluster_sync();
+        failed = any_failed != 0;                // one block without its piece: none writes a sum that lacks it
+    }
     const Forms forms = load_forms<MODE>(bias);
     const int from = TN * FEATS / splits * rank, to = from + TN * FEATS / splits;      // TN * FEATS is a multiple of 8
     for (int i = from + (int)threadIdx.x; i < to && !failed; i += SPLIT_THREADS) {

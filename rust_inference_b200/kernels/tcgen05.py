@@ -78,6 +78,16 @@ def wait_probe(limit: int = 2000, code: int = 2, arrive_first: bool = False) -> 
           c_void_p(st.data_ptr()), _stream())
 
 
+def wait_probe_cluster(blocks: int, failing: int, limit: int = 2000, code: int = 43) -> torch.Tensor:
+    """The same in block `failing` (-1: none) of a cluster of `blocks` blocks, with the float32 products' status word; int32 [blocks],
+    whether a block knows, as those products make known before they write, that one of the cluster gave up."""
+    st = f32_status_word()
+    seen = torch.full((max(blocks, 1),), -1, dtype=torch.int32, device="cuda")
+    _call("wait_probe", "ri_wait_probe_cluster", c_int(limit), c_int(code), c_int(blocks), c_int(failing), _p(seen),
+          c_void_p(st.data_ptr()), _stream())
+    return seen
+
+
 def supports(x: torch.Tensor, w) -> bool:
     """The kernel's alignment rule: bf16, K a multiple of 8 (16-byte rows for TMA)."""
     return x.dtype == torch.bfloat16 and w.t.dtype == torch.bfloat16 and w.k % 8 == 0 and w.k >= 8

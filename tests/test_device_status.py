@@ -72,3 +72,34 @@ def test_a_wait_that_runs_out_reports_and_the_device_goes_on(model_factory):
     got = eng.step([s], [toks], "all")
     assert rel_err(got, model.plain_logits(toks)) <= TOL["bfloat16"]
     eng.check_device_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("blocks", [1, 2, 4, 8])
+def test_a_cluster_learns_that_one_of_its_blocks_gave_up(blocks):
+    """The pieces of a float32 product that is cut over a cluster are added only if every block has its own."""
+    assert tcgen05.wait_probe_cluster(blocks, -1).tolist() == [0] * blocks
+    torch.cuda.synchronize()
+    tcgen05.check_f32_status()
+    for failing in range(blocks):
+        assert tcgen05.wait_probe_cluster(blocks, failing).tolist() == [1] * blocks
+        torch.cuda.synchronize()
+        with pytest.raises(KernelError, match="adding warps"):
+            tcgen05.check_f32_status()
+    with pytest.raises(KernelError, match="block 1 of 1"):
+        tcgen05.wait_probe_cluster(1, 1)
+
+
+def test_float32_products_tell_their_cluster_before_they_write():
+    """Read from the source: a block that gave up says so before the pieces meet, and nothing is read from them or stored otherwise."""
+    import os
+    from rust_inference_b200.kernels import build
+    with open(os.path.join(build.CSRC, "gemm_f32.cu")) as f:
+        kernel = f.read().split("gemm_f32_split_kernel(", 1)[1].split("int launch_split(", 1)[0]
+    told = kernel.index("if (failed && threadIdx.x == 0) set_in_all(&any_failed, splits);")
+    meet = kernel.rindex("failed = any_failed != 0;")
+    assert "cluster_sync();" in kernel[told:meet]
+    assert kernel.index("finish<MODE>(") > meet and kernel.rindex("peer_float(") > meet
+    assert "!failed" in kernel[meet:kernel.index("finish<MODE>(")]
+    # tensor memory is given back behind the wait for every MMA that was issued
+    assert kernel.index("for (int i = max(0, issued - 2); i < issued; ++i)") < kernel.index("tcgen05.dealloc")
