@@ -27,6 +27,11 @@ __device__ __forceinline__ void copy16(float* dst, const float* src) {
 __device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// The weight of a key that the row does not see: such a key may hold anything, NaN too, and its value is left out.  A key that is
+// seen and whose weight is so small that it is 0 takes part (0 times an infinity is NaN): its weight is never the negative zero.
+constexpr float UNSEEN = -0.f;
+__device__ __forceinline__ bool unseen(float weight) { return __float_as_uint(weight) == 0x80000000u; }
+
 // over the 16 threads that share a row
 __device__ __forceinline__ float row_max(float v) {
 #pragma unroll
@@ -180,10 +185,12 @@ attn_f32_kernel(const float* q, int q_ld, const float* __restrict__ kcache, cons
 #pragma unroll
         for (int i = 0; i < RI; ++i) {
             float top = -INFINITY;
+            bool seen[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int key = page * KEYS + tx + 16 * j;
-                s[i][j] = key <= pos[i] && key >= low[i] ? s[i][j] * scale : -INFINITY;
+                seen[j] = key <= pos[i] && key >= low[i];
+                s[i][j] = seen[j] ? s[i][j] * scale : -INFINITY;
                 top = fmaxf(top, s[i][j]);
             }
             const float m_new = fmaxf(m[i], row_max(top));
@@ -191,7 +198,7 @@ attn_f32_kernel(const float* q, int q_ld, const float* __restrict__ kcache, cons
             float sum = 0.f;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const float p = expf(s[i][j] - ref);
+                const float p = seen[j] ? expf(s[i][j] - ref) : UNSEEN;
                 ps[(ty + 16 * i) * LP + tx + 16 * j] = p;
                 sum += p;
             }
@@ -220,7 +227,7 @@ attn_f32_kernel(const float* q, int q_ld, const float* __restrict__ kcache, cons
 #pragma unroll
                 for (int i = 0; i < RI; ++i) {
                     const float w = u == 0 ? p[i].x : u == 1 ? p[i].y : u == 2 ? p[i].z : p[i].w;
-                    if (w != 0.f) {              // a key that the row does not see may hold anything, NaN too
+                    if (!unseen(w)) {
 #pragma unroll
                         for (int j = 0; j < CJ; ++j) {
                             o[i][j][0] = fmaf(w, v[j].x, o[i][j][0]);
@@ -373,10 +380,12 @@ attn_f32_few_kernel(const float* q, int q_ld, const float* __restrict__ kcache, 
             if (r >= n_rows) continue;           // uniform over the warp
             const int pos = start + r / n_rep, low = first_visible_key(pos, span);
             float s[2], top = -INFINITY;
+            bool seen[2];
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
                 const int k = page * KEYS + lane + 32 * j;
-                s[j] = k <= pos && k >= low ? p[r * LP + lane + 32 * j] * scale : -INFINITY;
+                seen[j] = k <= pos && k >= low;
+                s[j] = seen[j] ? p[r * LP + lane + 32 * j] * scale : -INFINITY;
                 top = fmaxf(top, s[j]);
             }
             const float m_new = fmaxf(m[i], warp_max(top));
@@ -384,7 +393,7 @@ attn_f32_few_kernel(const float* q, int q_ld, const float* __restrict__ kcache, 
             float sum = 0.f;
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                const float e = expf(s[j] - ref);
+                const float e = seen[j] ? expf(s[j] - ref) : UNSEEN;
                 p[r * LP + lane + 32 * j] = e;
                 sum += e;
             }
@@ -403,7 +412,7 @@ attn_f32_few_kernel(const float* q, int q_ld, const float* __restrict__ kcache, 
 #pragma unroll
             for (int i = 0; i < VN; ++i) {
                 const float w = p[r * LP + group * VN + i];
-                if (w != 0.f) {                  // a key that the row does not see may hold anything, NaN too
+                if (!unseen(w)) {
                     o[r][0] = fmaf(w, vr[i].x, o[r][0]);
                     o[r][1] = fmaf(w, vr[i].y, o[r][1]);
                     o[r][2] = fmaf(w, vr[i].z, o[r][2]);

@@ -215,3 +215,32 @@ def test_attention(hd, heads, kv, starts, news, span, splits):
                       n_splits=splits, **common)
     # two float32 sums over at most 701 keys in different orders
     assert (got - want).abs().max().item() <= 5e-6 * want.abs().max().item()
+
+
+@pytest.mark.parametrize("splits", [1, 3])
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("heads, kv, start, new", [(6, 2, 150, 1), (4, 4, 20, 3), (14, 2, 0, 200)])
+def test_attention_with_infinite_values(hd, heads, kv, start, new, splits):
+    """A value that is infinite or NaN reaches every row that sees its key, also where the key's weight is so small that it is 0
+    (0 times an infinity is NaN), and no other row: as in the generic kernel, which visits the seen keys only."""
+    ops = _ops()
+    torch.manual_seed(hd + heads)
+    end, page = start + new, 64
+    pages = -(-end // page)
+    kc, vc = torch.randn(pages, kv, page, hd), torch.randn(pages, kv, page, hd)
+    kc[0, :, 9] = -40.0                        # its scores lie hundreds below the others'
+    vc[0, 0, 9, 5], vc[0, -1, 9, 7] = float("inf"), float("nan")
+    if new > 100:
+        vc[1, 0, 50, 2] = float("-inf")         # seen by the later rows, with an ordinary weight
+    q = torch.randn(new, heads * hd).abs() + 1.0
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    table, slot, first = i32([list(range(pages))]), i32([0]), i32([start])
+    kc, vc, q = kc.to(DEV), vc.to(DEV), q.to(DEV)
+    want, got = torch.empty(new, heads * hd, device=DEV), torch.full((new, heads * hd), 7.0, device=DEV)
+    common = dict(n_heads=heads, n_kv_heads=kv, head_dim=hd, page_size=page, scale=hd ** -0.5)
+    ops.attention_generic(q, q.shape[1], kc, vc, table, i32(list(range(start, end))), i32([0] * new), slot, want, n_tokens=new, **common)
+    ops.attention_f32(q, q.shape[1], kc, vc, table, slot, first, i32([0, new]), got, n_seqs=1, max_new=new, n_splits=splits, **common)
+    assert bool(want.isnan().any()) and not bool(want.isnan().all())
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    fine = want.isfinite()
+    assert (got[fine] - want[fine]).abs().max().item() <= 5e-6 * want[fine].abs().max().item()
