@@ -195,7 +195,8 @@ def attention(qkv, cache_layer, out, ctx, *, n_heads, n_kv_heads, head_dim, scal
             page_size=ctx.page_size, scale=scale, window=window or 0, softcap=softcap, keep_first=keep_first, sink=sink,
             dist=dist, gate=gate, out_scale=out_scale)
     if (same_sizes and not (window and chunk) and plain
-            and ops.attention_f32_supports(qkv, q_ld, out, head_dim, ctx.page_size)):
+            and ops.attention_f32_supports(qkv, q_ld, cache_layer.k, cache_layer.v, out, n_seqs=ctx.n_seqs, n_kv_heads=n_kv_heads,
+                                           head_dim=head_dim, page_size=ctx.page_size)):
         longest = ctx.page_table.shape[1] * ctx.page_size if ctx.all_single else ctx.max_len
         return ops.attention_f32(
             qkv, q_ld, cache_layer.k, cache_layer.v, ctx.page_table, ctx.seq_slot, ctx.seq_start, ctx.cu_seqlens, out,

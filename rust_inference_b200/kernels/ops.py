@@ -485,10 +485,13 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, *, 
     return out
 
 
-def attention_f32_supports(q: torch.Tensor, q_ld: int, out: torch.Tensor, head_dim: int, page_size: int) -> bool:
-    """What the float32 attention kernel takes: heads of 64 or 128, pages of 64, rows of whole aligned 16-byte pieces."""
+def attention_f32_supports(q: torch.Tensor, q_ld: int, kcache: torch.Tensor, vcache: torch.Tensor, out: torch.Tensor, *, n_seqs: int,
+                           n_kv_heads: int, head_dim: int, page_size: int) -> bool:
+    """What the float32 attention kernel takes: heads of 64 or 128, pages of 64, rows of whole aligned 16-byte pieces, as many
+    sequences and kv heads as a launch grid's second and third axis hold."""
     return (q.dtype == torch.float32 and out.dtype == torch.float32 and head_dim in (64, 128) and page_size == 64 and q_ld % 4 == 0
-            and out.shape[1] % 4 == 0 and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0)
+            and out.shape[1] % 4 == 0 and all(t.data_ptr() % 16 == 0 for t in (q, kcache, vcache, out))
+            and kcache.is_contiguous() and vcache.is_contiguous() and max(n_seqs, n_kv_heads) <= 65535)
 
 
 def attention_f32(q: torch.Tensor, q_ld: int, kcache, vcache, page_table, seq_slot, seq_start, cu_seqlens, out: torch.Tensor, *,

@@ -56,3 +56,30 @@ def test_the_kernel_can_be_forced(plan, monkeypatch):
     assert plan(64, 4, 8192) == ("cp_async", 1)
     monkeypatch.setattr(attention, "_DECODE", "tma")
     assert plan(8, 4, 8192) == ("tma", 9)
+
+
+def test_float32_attention_leaves_to_the_generic_kernel_what_the_tiles_do_not_take(monkeypatch):
+    """More sequences than a launch grid's third axis holds, caches that are no whole aligned 16-byte pieces, other pages and heads."""
+    from types import SimpleNamespace
+
+    import torch
+    from rust_inference_b200.kernels import attention, ops
+    monkeypatch.setattr(attention, "_sm_count", lambda: 148)
+    taken = []
+    monkeypatch.setattr(ops, "attention_f32", lambda *a, **k: taken.append("tiles"))
+    monkeypatch.setattr(ops, "attention_generic", lambda *a, **k: taken.append("generic"))
+
+    def route(n_seqs=2, kv=2, hd=64, page=64, offset=0):
+        floats = torch.zeros(3 * kv * page * hd + 64)
+        floats = floats[-(floats.data_ptr() // 4) % 4:]            # a 16-byte boundary
+        k = floats[offset:offset + 3 * kv * page * hd].view(3, kv, page, hd)
+        q = torch.zeros(4, 2 * kv * hd)
+        none = torch.zeros(1, dtype=torch.int32)
+        ctx = SimpleNamespace(n_seqs=n_seqs, max_new=1, max_len=100, all_single=True, page_size=page, page_table=torch.zeros(2, 3),
+                              token_pos=none, token_seq=none, seq_slot=none, seq_start=none, cu_seqlens=none)
+        taken.clear()
+        attention.attention(q, SimpleNamespace(k=k, v=k), torch.zeros_like(q), ctx, n_heads=2 * kv, n_kv_heads=kv, head_dim=hd, scale=0.1)
+        return taken[0]
+
+    assert route() == route(hd=128) == route(n_seqs=65535) == route(offset=4) == "tiles"
+    assert route(n_seqs=65536) == route(offset=1) == route(hd=80) == route(page=32) == "generic"
