@@ -97,7 +97,9 @@ class LatentAttention(Mixer):
         self.w_uk_t = tensors[nm["uk"]].view(H, self.head_dim, self.kv_rank).transpose(1, 2).contiguous()
         self.w_uv = tensors[nm["uv"]].view(H, self.v_head_dim, self.kv_rank).contiguous()
         self.w_o = linear.Weight(tensors[nm["o"]])
-        # the same maps in one matrix, a head's keys beside its values: what prompts form keys and values with
+        # the same maps in one matrix, a head's keys beside its values: what prompts form keys and values with.  A second copy,
+        # heads * (head_dim + v_head_dim) * kv_rank bfloat16 numbers per layer (4 MiB with 16 heads and a latent of 512), kept
+        # only where a prompt can take it.
         self.w_ukv = None
         if self.dtype == torch.bfloat16 and self._expandable():
             uk = tensors[nm["uk"]].view(H, self.head_dim, self.kv_rank)
@@ -131,7 +133,7 @@ class LatentAttention(Mixer):
     def _expandable(self) -> bool:
         from ..kernels import attention_tc
         return ((self.head_dim, self.rot_dim, self.v_head_dim) == attention_tc.EXPANDED_SIZES and self.kv_rank % 8 == 0
-                and self.kv_rank <= 4096)
+                and self.kv_rank <= 4096 and self.w_in.n % 8 == 0)       # rows of whole 16-byte pieces
 
     # Steps whose shortest prompt has fewer tokens than this hold their values in two bfloat16 terms.  Rounding every value instead
     # of the weighted latents costs accuracy while few keys are averaged.  How far the layer's output is from 64 bits, 1e-3, in
@@ -147,7 +149,7 @@ class LatentAttention(Mixer):
         would have to form those positions' keys and values again, so they, and single tokens, stay with the carried form; so do
         the small steps without gates whose projection is added up and kept in float32."""
         return (self.w_ukv is not None and not ctx.all_single and ctx.host_starts is not None and not any(ctx.host_starts)
-                and ctx.page_size == 64 and self.w_in.n % 8 == 0 and (self.gated or not linear.wants_split(x, self.w_in)))
+                and ctx.page_size == 64 and (self.gated or not linear.wants_split(x, self.w_in)))
 
     def _forward_expanded(self, x, residual, ctx, cache_layer):
         from ..kernels import attention_tc

@@ -125,3 +125,16 @@ def test_latent_scores_equal_scores_over_expanded_keys():
     direct = torch.einsum("ihd,jhd->hij", q, (c @ uk.T).view(7, H, d))
     carried = torch.einsum("ihr,jr->hij", torch.einsum("ihd,hdr->ihr", q, uk.view(H, d, r)), c)
     assert torch.allclose(direct, carried)
+
+
+@pytest.mark.parametrize("heads, rank, gated, kept", [(8, 64, True, True), (3, 64, True, False), (3, 64, False, True), (8, 60, True, False)])
+def test_latent_maps_are_kept_twice_only_where_prompts_take_them(heads, rank, gated, kept):
+    """The matrix that prompts form keys and values with needs projected rows of whole 16-byte pieces (with gates: a number of
+    heads that is a multiple of eight) and such a latent."""
+    from rust_inference_b200.parts.latent_attention import LatentAttention
+    from rust_inference_b200.parts.spec import PartSpec
+    mixer = LatentAttention(n_heads=heads, head_dim=128, rot_dim=64, v_head_dim=128, kv_rank=rank, eps=1e-5, gated=gated, hidden_size=64,
+                            dtype=torch.bfloat16, device="cpu",
+                            position=PartSpec("rope", {"head_dim": 64, "base": 10000.0}))
+    mixer.set_tensors({name: torch.zeros(s.shape, dtype=torch.bfloat16) for name, s in mixer.tensor_specs().items()})
+    assert (mixer.w_ukv is not None) == kept
