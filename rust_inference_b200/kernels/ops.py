@@ -38,12 +38,16 @@ def _p(t) -> c_void_p:
 # hundred tokens is a couple of hundred launches of a few microseconds each: the current stream comes as the number that it is
 # (`torch.cuda.current_stream()` builds two objects and looks the device up by name, 4 us), messages are formatted only when
 # they are raised, and scratch buffers keep their last view.
-_current_raw_stream = torch._C._cuda_getCurrentRawStream
-_current_device = torch._C._cuda_getDevice
+if hasattr(torch._C, "_cuda_getCurrentRawStream") and hasattr(torch._C, "_cuda_getDevice"):
+    _current_raw_stream = torch._C._cuda_getCurrentRawStream
+    _current_device = torch._C._cuda_getDevice
 
+    def _stream() -> c_void_p:
+        return c_void_p(_current_raw_stream(_current_device()))
+else:                                            # a torch without these two (built without CUDA): the module still imports
 
-def _stream() -> c_void_p:
-    return c_void_p(_current_raw_stream(_current_device()))
+    def _stream() -> c_void_p:
+        return c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
 def _need_cuda(*tensors) -> None:

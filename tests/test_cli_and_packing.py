@@ -135,3 +135,19 @@ def test_flags_of_the_random_weights_mode(tmp_path):
     ]:
         with pytest.raises(CliError, match=word):
             parse_args(argv)
+
+
+def test_the_package_imports_on_a_torch_without_cuda():
+    """A torch that was built without CUDA lacks the functions that tell the current stream as a number."""
+    import os
+    import subprocess
+    import sys
+    code = ("import torch\n"
+            "for name in ('_cuda_getCurrentRawStream', '_cuda_getDevice'):\n"
+            "    if hasattr(torch._C, name): delattr(torch._C, name)\n"
+            "import rust_inference_b200\n"
+            "from rust_inference_b200.kernels import ops\n"
+            "assert callable(ops._stream)\n")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr
