@@ -3,7 +3,7 @@
 Which kernel runs is decided here, by dtype and shape:
   float32   the kernels of `gemm_f32` (FFMA for a few tokens; beyond, three bfloat16 parts per operand on the
             tensor cores, which together are the operand: sums as close to 64 bits as the FFMA kernel's) when rows are
-            whole 16-byte pieces, else the FFMA kernel (`gemm_simt`);
+            whole 16-byte pieces and sums not short (`_in_parts`), else the FFMA kernel (`gemm_simt`);
   bfloat16  the tcgen05 kernel (`gemm_tcgen05`) when the shape meets its alignment rule,
             else the FFMA kernel on bf16 operands.  Either way accumulation is float32.
 """
@@ -12,6 +12,7 @@ from __future__ import annotations
 import torch
 
 from . import ops, tcgen05
+from .attention import _sm_count
 
 
 class Weight:
@@ -32,15 +33,24 @@ def _use_tensor_cores(x: torch.Tensor, w: Weight) -> bool:
     return tcgen05.supports(x, w)
 
 
-# Shorter sums are left to the FFMA kernel, which has them sooner: a block of the tensor cores' kernel is 64 steps of K long and
-# costs about 4.5 us to start (us, FFMA / tensor cores, N = 512: 17 rows of K = 96 5.9 / 6.4, of K = 128 7.3 / 6.4).
-F32_PARTS_MIN_K = 128
+# Sums of fewer than 128 terms are left to the FFMA kernel, and up to 256 products of more than 32 rows whose tiles of 64 x 64 it
+# does in one round: it has them sooner, because a block of the tensor cores' kernel is 64 steps of K long and costs 4.5 to 9 us to
+# start.  (us, FFMA / tensor cores.  N = 512: 17 rows of K = 96 5.9 / 6.4, of 128 7.3 / 6.4; 64 rows of 128 7.6 / 8.4, of 160 9.2 / 10.3,
+# of 256 13.8 / 7.3, which is the first to be cut over a cluster; 333 rows of 128 7.7 / 11.8, of 192 10.7 / 13.7, of 256 13.8 / 9.9.
+# Two rounds, N = 4,096: 333 rows of 128 16.3 / 12.5.)
+F32_PARTS_MIN_K, F32_PARTS_ALWAYS_K = 128, 256
+
+
+def _in_parts(m: int, n: int, k: int) -> bool:
+    if k < F32_PARTS_MIN_K or k >= F32_PARTS_ALWAYS_K:
+        return k >= F32_PARTS_MIN_K
+    return m <= 32 or -(-m // 64) * -(-n // 64) > _sm_count()
 
 
 def _plain(x, w: Weight, out, mode, w2: Weight | None = None, **constants):
     """The product without bfloat16 tensor cores."""
     t2 = w2.t if w2 is not None else None
-    run = ops.gemm_f32 if ops.gemm_f32_supports(x, w.t, t2) and (x.shape[0] <= 16 or w.k >= F32_PARTS_MIN_K) else ops.gemm_simt
+    run = ops.gemm_f32 if ops.gemm_f32_supports(x, w.t, t2) and (x.shape[0] <= 16 or _in_parts(x.shape[0], w.n, w.k)) else ops.gemm_simt
     return run(x, w.t, out, mode, w2=t2, **constants)
 
 

@@ -83,3 +83,23 @@ def test_float32_attention_leaves_to_the_generic_kernel_what_the_tiles_do_not_ta
 
     assert route() == route(hd=128) == route(n_seqs=65535) == route(offset=4) == "tiles"
     assert route(n_seqs=65536) == route(offset=1) == route(hd=80) == route(page=32) == "generic"
+
+
+def test_short_float32_sums_stay_with_the_ffma_kernel(monkeypatch):
+    import torch
+    from rust_inference_b200.kernels import linear, ops
+    monkeypatch.setattr(linear, "_sm_count", lambda: 148)
+    taken = []
+    monkeypatch.setattr(ops, "gemm_f32", lambda *a, **k: taken.append("parts"))
+    monkeypatch.setattr(ops, "gemm_simt", lambda *a, **k: taken.append("ffma"))
+
+    def route(m, n, k):
+        taken.clear()
+        linear._plain(torch.zeros(m, k), linear.Weight(torch.zeros(n, k)), torch.zeros(m, n), ops.EPI_STORE)
+        return taken[0]
+
+    assert [route(16, 512, k) for k in (4, 128, 2048)] == ["parts"] * 3            # few rows: a kernel of their own
+    assert [route(17, 512, k) for k in (124, 128, 256)] == ["ffma", "parts", "parts"]
+    assert [route(33, 512, k) for k in (128, 252, 256)] == ["ffma", "ffma", "parts"]
+    assert [route(333, n, 128) for n in (512, 24 * 64, 25 * 64)] == ["ffma", "ffma", "parts"]      # 6 x 24 = 144 tiles, 150
+    assert route(333, 512, 130) == route(333, 512, 2050) == "ffma"                  # rows of no whole 16-byte pieces
