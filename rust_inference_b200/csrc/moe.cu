@@ -428,7 +428,7 @@ moe_combine_kernel(float* residual, const float* y, const float* weights, const 
         const float g = shared_y != nullptr && gate != nullptr ? gate[t] : 1.f;
         for (int d = (part * (int)blockDim.x + (int)threadIdx.x) * V; d < width; d += parts * (int)blockDim.x * V) {
             const size_t i = (size_t)t * width + d;
-            float acc[V], add[V], old[V];
+            __align__(16) float acc[V], add[V], old[V];          // written four at a time
 #pragma unroll
             for (int v = 0; v < V; ++v) acc[v] = 0.f;
             if (V == 4) {
@@ -439,7 +439,8 @@ moe_combine_kernel(float* residual, const float* y, const float* weights, const 
                 if (shared_y != nullptr) add[0] = shared_y[i];
             }
             for (int c0 = 0; c0 < top; c0 += AT_ONCE) {
-                float w[AT_ONCE], r[AT_ONCE][V];
+                float w[AT_ONCE];
+                __align__(16) float r[AT_ONCE][V];
 #pragma unroll
                 for (int k = 0; k < AT_ONCE; ++k) {
                     if (c0 + k >= top) continue;

@@ -199,6 +199,52 @@ def test_recurrence_in_portions_and_slots(heads, dim, vdim, lens, cuts):
             assert rel_err(got[b], want[b]) < 2e-5, (portions, b)
 
 
+@pytest.mark.parametrize("width", [1, 3, 4, 70, 73, 128, 257, 1030, 1032])          # four channels at a time, and one where they do not divide
+@pytest.mark.parametrize("tokens, top", [(1, 1), (5, 3), (150, 4), (149, 6)])           # a token's channels over several blocks, or one block
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_experts_rows_are_summed(width, tokens, top, dtype):
+    """The weighted sum of the experts' rows onto the stream against 64 bits, in every form: rows in the pairs' or another order, a
+    shared result with and without a gate, experts that hand their input through, a factor."""
+    from rust_inference_b200.kernels import ops
+    g = torch.Generator().manual_seed(width + tokens)
+    draw = lambda *s: torch.randn(*s, generator=g)
+    stream, y, weights = draw(tokens, width), draw(tokens * top, width), draw(tokens, top)
+    shared, gate, x = draw(tokens, width), draw(tokens), draw(tokens, width).to(dtype)
+    place = torch.randperm(tokens * top, generator=g).to(torch.int32)
+    ids = torch.randint(0, 8, (tokens, top), generator=g, dtype=torch.int32)
+    for with_place, with_shared, with_gate, real, scale in ((0, 0, 0, None, 1.0), (1, 1, 0, None, 1.0), (1, 1, 1, 5, 0.7), (0, 0, 0, 0, 1.3)):
+        rows = y[place.long()] if with_place else y
+        rows = rows.view(tokens, top, width).double()
+        if real is not None:
+            rows = torch.where((ids >= real)[..., None], x.double()[:, None], rows)
+        want = (weights.double()[..., None] * rows).sum(1)
+        if with_shared:
+            want += (gate.double()[:, None] if with_gate else 1.0) * shared.double()
+        want = stream.double() + scale * want
+        residual = d(stream.clone())
+        ops.moe_combine(residual, d(y), d(weights), top=top, place=d(place) if with_place else None, shared_y=d(shared) if with_shared else None,
+                        gate=d(gate) if with_gate else None, ids=d(ids) if real is not None else None, x=d(x) if real is not None else None,
+                        n_real=real or 0, scale=scale)
+        # top + 3 float32 roundings of numbers below about 5 each
+        assert (residual.cpu().double() - want).abs().max().item() <= (top + 3) * 2.0 ** -24 * 20
+
+
+@pytest.mark.parametrize("width", [8, 64, 1016, 1024, 1032, 2056])          # runs of 128 pieces of 16 bytes, and what is left
+def test_rows_are_gathered(width):
+    from rust_inference_b200.kernels import ops
+    g = torch.Generator().manual_seed(width)
+    tokens, top = 37, 3
+    x = torch.randn(tokens, width, generator=g).to(torch.bfloat16)
+    order = torch.randperm(tokens * top, generator=g).to(torch.int32)
+    want = x[(order // top).long()]
+    for listed in (None, 0, 50, tokens * top):
+        xs = torch.full((tokens * top, width), 9.0, dtype=torch.bfloat16, device=DEV)
+        ops.moe_gather(d(x), xs, d(order), n_pairs=tokens * top, top=top,
+                       listed=torch.tensor([listed], dtype=torch.int32, device=DEV) if listed is not None else None)
+        n = tokens * top if listed is None else listed
+        assert torch.equal(xs[:n].cpu(), want[:n]) and bool((xs[n:] == 9.0).all())
+
+
 @pytest.mark.parametrize("vdim", [24, 33, 64, 128, 130, 200, 512, 516])
 def test_head_norm_adds_in_one_order(vdim):
     """The norm over a head's read-out, to the bit: lane l of a warp adds the squares of the values l, l + 32, ... one after the
