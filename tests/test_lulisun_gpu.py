@@ -245,6 +245,33 @@ def test_rows_are_gathered(width):
         assert torch.equal(xs[:n].cpu(), want[:n]) and bool((xs[n:] == 9.0).all())
 
 
+@pytest.mark.parametrize("pieces", [1, 2, 7, 8, 9, 16, 17])                 # eight pieces' loads are on their way at a time
+@pytest.mark.parametrize("heads, dim, vdim", [(2, 32, 24), (1, 30, 33)])     # four channels at a time, and one
+def test_recurrence_in_pieces_side_by_side(pieces, heads, dim, vdim):
+    """Sequences cut into so many pieces, and into fewer beside it, against the scan in one pass, from a state that is not zero."""
+    from rust_inference_b200.kernels import ops
+    g = torch.Generator().manual_seed(pieces)
+    piece = 16
+    lens = [pieces * piece - 3, max(1, pieces // 2 * piece), 1]
+    n = sum(lens)
+    z = torch.randn(n, heads * (2 * dim + vdim), generator=g)
+    bias, low, w = torch.randn(heads * dim, generator=g), torch.rand(heads * dim, generator=g) * 0.9, 1 + torch.randn(vdim, generator=g) * 0.2
+    start = torch.randn(4, heads, dim, vdim, generator=g)
+    cu = torch.tensor([0, lens[0], lens[0] + lens[1], n], dtype=torch.int32, device=DEV)
+    slots = torch.tensor([3, 0, 2], dtype=torch.int32, device=DEV)
+    results = []
+    for cut in (0, piece):
+        state, out = d(start.clone()), torch.empty(n, heads * vdim, device=DEV)
+        ops.gated_recurrence(d(z.clone()), d(bias), d(low), d(w), state, cu, slots, out, n_seqs=3, heads=heads, dim=dim, vdim=vdim, eps=1e-5,
+                             piece=cut, max_pieces=pieces if cut else 1, longest_run=max(lens))
+        results.append((out, state))
+    (want, want_state), (got, got_state) = results
+    assert torch.equal(got_state[1], d(start)[1])                            # no sequence's slot
+    assert rel_err(got, want.cpu().double()) < 2e-5
+    # a state row is a sum whose terms may have cancelled: float32 roundings of numbers of the largest state's size, not of the row's
+    assert (got_state - want_state).abs().max().item() <= 2e-6 * want_state.abs().max().item()
+
+
 @pytest.mark.parametrize("vdim", [24, 33, 64, 128, 130, 200, 512, 516])
 def test_head_norm_adds_in_one_order(vdim):
     """The norm over a head's read-out, to the bit: lane l of a warp adds the squares of the values l, l + 32, ... one after the
@@ -386,6 +413,55 @@ def test_two_norms_in_one_kernel(dtype, rows, n):
     tol = 1e-5 if dtype == torch.float32 else 1e-2
     assert rel_err(a, plain_lulisun.plain_rmsnorm(x.double(), wa.double(), 1e-5)) < tol
     assert rel_err(b, plain_lulisun.plain_rmsnorm(x.double(), wb.double(), 1e-5)) < tol
+
+
+@pytest.mark.parametrize("style", [0, 1])
+@pytest.mark.parametrize("heads, kvh, hd, vhd, rot, more", [
+    (16, 4, 128, 128, 64, 0), (3, 1, 64, 64, 16, 8), (5, 2, 48, 40, 32, 0), (2, 2, 64, 128, 64, 0), (4, 1, 32, 8, 0, 16), (28, 4, 128, 64, 128, 0),
+    (3, 1, 24, 24, 16, 0), (2, 1, 64, 64, 24, 0), (2, 1, 64, 36, 32, 0), (2, 1, 64, 64, 32, 4)])      # the last four: element by element
+def test_partial_rotation_in_bfloat16(style, heads, kvh, hd, vhd, rot, more):
+    """Sixteen bytes at a time: heads of which only the first channels turn (or none), values of another size, rows that hold more,
+    against the rotation in 64 bits rounded once; what does not turn is copied bit by bit, and nothing else is touched."""
+    from rust_inference_b200.kernels import ops
+    from rust_inference_b200.parts.rope import rope_tables
+    n, page, bf = 70, 64, torch.bfloat16
+    g = torch.Generator().manual_seed(hd + rot)
+    qkv = torch.randn(n, (heads + kvh) * hd + kvh * vhd + more, generator=g).to(bf)
+    cos, sin = (torch.from_numpy(t) for t in rope_tables(rot, 321.0, 256, exact_angles=True)) if rot else (None, None)
+    pos = torch.arange(100, 100 + n, dtype=torch.int32)
+    table = [9, 1, 4, 2]
+    half = rot // 2
+    want = qkv.double()
+    if rot:
+        at = torch.arange(half)
+        a, b = (at, at + half) if style == 0 else (2 * at, 2 * at + 1)
+        c, s = cos[pos.long()].double()[:, None], sin[pos.long()].double()[:, None]
+        turned = want[:, :(heads + kvh) * hd].view(n, heads + kvh, hd)
+        x, y = turned[..., a].clone(), turned[..., b].clone()
+        turned[..., a], turned[..., b] = x * c - y * s, x * s + y * c
+    for write in (True, False):
+        kc, vc = torch.full((10, kvh, page, hd), 77.0, dtype=bf, device=DEV), torch.full((10, kvh, page, vhd), 77.0, dtype=bf, device=DEV)
+        row = d(qkv.clone())
+        ops.rope_cache_write(row, d(cos) if rot else None, d(sin) if rot else None, d(pos), torch.zeros(n, dtype=torch.int32, device=DEV),
+                             torch.zeros(1, dtype=torch.int32, device=DEV), torch.tensor([table], dtype=torch.int32, device=DEV), kc, vc,
+                             n_heads=heads, n_kv_heads=kvh, head_dim=hd, page_size=page, style=style, write_kv=write, rot_dims=rot,
+                             v_head_dim=vhd)
+        row, kc, vc = row.cpu(), kc.cpu(), vc.cpu()
+        close = lambda got, ref: bool(((got.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5).all())
+        q = row[:, :heads * hd].view(n, heads, hd)
+        assert close(q, want[:, :heads * hd].view(n, heads, hd))
+        assert torch.equal(q[..., rot:], qkv[:, :heads * hd].view(n, heads, hd)[..., rot:])
+        assert torch.equal(row[:, (heads + kvh) * hd:], qkv[:, (heads + kvh) * hd:])
+        if not write:
+            assert bool((kc == 77.0).all()) and bool((vc == 77.0).all())
+            continue
+        pages, offset = torch.tensor(table)[pos.long() // page], pos.long() % page
+        k, v = kc[pages, :, offset], vc[pages, :, offset]
+        assert close(k, want[:, heads * hd:(heads + kvh) * hd].view(n, kvh, hd))
+        assert torch.equal(k[..., rot:], qkv[:, heads * hd:(heads + kvh) * hd].view(n, kvh, hd)[..., rot:])
+        assert torch.equal(v, qkv[:, (heads + kvh) * hd:(heads + kvh) * hd + kvh * vhd].view(n, kvh, vhd))
+        kc[pages, :, offset], vc[pages, :, offset] = 77.0, 77.0
+        assert bool((kc == 77.0).all()) and bool((vc == 77.0).all())
 
 
 def test_partial_rotation_and_value_cache():
