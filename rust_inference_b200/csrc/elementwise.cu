@@ -527,23 +527,6 @@ __global__ void rope_cache_write_kernel(T* __restrict__ qkv, int ld, const float
 // thread takes 8 consecutive elements of a head (and, for the half-split pairing, their 8 partners half the rotated channels
 // on), rotates them in float32 and writes them back the same way; channels behind the rotated ones are copied for keys and
 // stay where they are for queries.  (2,048 tokens of 16 + 4 heads of 128 with 64 rotated channels: 7.9 us, 11.5 element by element.)
-__device__ __forceinline__ void unpack8(const uint4& v, float* f) {
-    const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float2 x = __bfloat1622float2(p[i]);
-        f[2 * i] = x.x;
-        f[2 * i + 1] = x.y;
-    }
-}
-__device__ __forceinline__ uint4 pack8(const float* f) {
-    uint4 v;
-    __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&v);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) p[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
-    return v;
-}
-
 __global__ void rope_cache_write_vec_kernel(__nv_bfloat16* __restrict__ qkv, int ld, const float* __restrict__ cos_t,
                                             const float* __restrict__ sin_t, const int* __restrict__ token_pos,
                                             const int* __restrict__ token_seq, const int* __restrict__ seq_slot,

@@ -32,8 +32,6 @@ using namespace ri::tc;
 
 namespace {
 
-constexpr int SMS = 148;
-
 // weights: read once, kept out of L1 (a load that may stand before the wait for the kernel before)
 __device__ __forceinline__ float4 load_weight(const float* p) {
     float4 v;
@@ -216,7 +214,7 @@ int few_splits(int rows, int group, int N, int K) {
         const int per = (steps + s - 1) / s;
         const long long smem = (long long)rows * per * STEP * 4;
         if (smem > FEW_SMEM_MAX) continue;
-        const int resident = (smem > 100 * 1024 ? 1 : smem > 66 * 1024 || rows > 8 ? 2 : 3) * SMS / s;      // clusters
+        const int resident = (smem > 100 * 1024 ? 1 : smem > 66 * 1024 || rows > 8 ? 2 : 3) * sm_count() / s;      // clusters
         // rounds of the persistent grid times the steps of one, and what a round costs besides (about two steps; four
         // where the pieces meet across blocks)
         const long long rounds = (groups + resident - 1) / resident;
@@ -235,7 +233,7 @@ int launch_few(const float* X, const float* W, const float* W2, const float* bia
     static PerDeviceOnce once;
     if (int rc = raise_dynamic_smem(gemm_f32_few_kernel<MT, RW, U, MODE>, FEW_SMEM_MAX, once, "gemm_f32")) return rc;
     const int per_sm = smem > 100 * 1024 ? 1 : smem > 66 * 1024 || MT > 8 ? 2 : 3;
-    const int clusters = max(1, min(groups, per_sm * SMS / splits));
+    const int clusters = max(1, min(groups, per_sm * sm_count() / splits));
     return launch_cluster("gemm_f32 (few rows)", gemm_f32_few_kernel<MT, RW, U, MODE>, dim3(clusters * splits), FEW_THREADS, smem, splits,
                           stream, X, W, W2, bias, out, M, N, K, steps, splits);
 }
@@ -585,7 +583,7 @@ int launch_split(const float* X, const float* W, const float* W2, const float* b
     int splits = 1;
     long long best = 0;
     for (int s = 1; s <= 8 && s <= total_kb; s *= 2) {
-        const long long at_once = s == 8 ? 128 : s == 4 ? 144 : SMS;
+        const long long at_once = s == 8 ? 128 : s == 4 ? 144 : sm_count();
         const long long cost = ((tiles * s + at_once - 1) / at_once) * ((total_kb + s - 1) / s + 3 + (s > 1));
         if (s == 1 || cost < best) { splits = s; best = cost; }
     }

@@ -42,6 +42,7 @@
 // TMA needs 16-byte row strides: K must be a multiple of 8.  Everything else (tokens,
 // features, K not a multiple of the tile) is handled by TMA's zero fill and by bounds
 // checks in the epilogue.
+#include "cluster.cuh"
 #include "tcgen05_common.cuh"
 
 using namespace ri;
@@ -363,8 +364,7 @@ constexpr int TM_STAGE_BYTES = (TM_TOK + TM_ROWS) * BLOCK_K * 2;     // 48 KiB
 // from the accumulator at `trow` (SiLU-gate: gate values in the first 128 columns, up values in the second).
 template <bool DUAL, int MODE>
 __device__ __forceinline__ void tm_write_tile(uint32_t trow, int t, bool t_ok, int f0, int n_feat, bool aligned,
-                                              const float* __restrict__ bias, void* __restrict__ out_,
-                                              bool pieces = false) {     // MODE 2: other work items add to the same tile
+                                              const float* __restrict__ bias, void* __restrict__ out_) {
     constexpr int FEATS = DUAL ? TM_ROWS / 2 : TM_ROWS;
     const GateForm gf = load_gate_form(MODE == 3 ? bias : nullptr);     // the gated epilogue's constants come in `bias`
     const ActForm af = MODE == 4 ? load_act_form(bias) : ActForm{0.f, 0.f, 0.f};     // so do the activation's
@@ -404,14 +404,12 @@ __device__ __forceinline__ void tm_write_tile(uint32_t trow, int t, bool t_ok, i
 #pragma unroll
                 for (int q4 = 0; q4 < 4; ++q4) {
                     float4 x = make_float4(r[4 * q4], r[4 * q4 + 1], r[4 * q4 + 2], r[4 * q4 + 3]);
-                    if (MODE == 2 && pieces) {           // four adds in one reduction, no value returned
+                    // four adds in one reduction without a returned value, also where one item has the whole of K: reading the
+                    // sums first kept the epilogue waiting for memory (1,845 x 1,536 x 1,536: 34.9 us, with two pieces 15)
+                    if (MODE == 2) {
                         asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + q4), "f"(x.x),
                                      "f"(x.y), "f"(x.z), "f"(x.w) : "memory");
                         continue;
-                    }
-                    if (MODE == 2) {                     // K is not split: a plain read-add-write
-                        const float4 old = dst[q4];
-                        x.x += old.x; x.y += old.y; x.z += old.z; x.w += old.w;
                     }
                     dst[q4] = x;
                 }
@@ -421,8 +419,7 @@ __device__ __forceinline__ void tm_write_tile(uint32_t trow, int t, bool t_ok, i
                 if (f0 + c0 + j < n_feat) {
                     if (MODE == 0 || MODE == 3 || MODE == 4) reinterpret_cast<__nv_bfloat16*>(out_)[o0 + j] = __float2bfloat16_rn(r[j]);
                     else if (MODE == 1 || MODE == 5) reinterpret_cast<float*>(out_)[o0 + j] = r[j];
-                    else if (pieces) atomicAdd(reinterpret_cast<float*>(out_) + o0 + j, r[j]);
-                    else reinterpret_cast<float*>(out_)[o0 + j] += r[j];
+                    else atomicAdd(reinterpret_cast<float*>(out_) + o0 + j, r[j]);
                 }
         }
     }
@@ -625,20 +622,11 @@ gemm_tm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 constexpr int PAIR_STAGE_BYTES = 2 * A_BYTES;       // 128 tokens + 128 W rows per CTA and k-block: 32 KiB
 constexpr int PAIR_TOK = 2 * TM_TOK;                // tokens per pair tile
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
 // The address, in the cluster's shared window, of the first CTA's copy of a shared variable of this CTA.
 __device__ __forceinline__ uint32_t in_first_cta(uint32_t local_addr) {
     uint32_t a;
     asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(local_addr));
     return a;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // A tile into this CTA's shared memory whose arrival is counted by a barrier of the pair's first CTA.
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t cluster_bar, int x, int y) {
@@ -711,7 +699,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
-    cluster_sync_all();                                        // the partner's barriers stand before anything arrives there
+    cluster_sync();                                        // the partner's barriers stand before anything arrives there
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_slot;
     const uint32_t full0 = smem_u32(&full_bar[0]), empty0 = smem_u32(&empty_bar[0]);
@@ -823,9 +811,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             const int t = t0 + rank * TM_TOK + lane_base + lane;
             const bool t_ok = t < n_tok;
             const uint32_t trow = tmem_base + ((uint32_t)lane_base << 16) + (uint32_t)(buf * TM_ROWS);
-            // adds without a returned value also where one item has the whole of K: reading the sums first kept the epilogue waiting
-            // for memory (1,845 x 1,536 x 1,536: 34.9 us, with two pieces 15)
-            tm_write_tile<DUAL, MODE>(trow, t, t_ok, f0, n_feat, aligned, bias, out_, true);
+            tm_write_tile<DUAL, MODE>(trow, t, t_ok, f0, n_feat, aligned, bias, out_);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(acc_empty_first + 8u * (uint32_t)buf);
@@ -834,7 +820,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
 
     // nothing of the pair's tensor or shared memory is freed while the partner may still use it
     tc_fence_before();
-    cluster_sync_all();
+    cluster_sync();
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)TMEM_COLS)
@@ -860,16 +846,6 @@ int make_map(CUtensorMap* map, const void* ptr, long long rows, long long K, int
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail("gemm_tcgen05: cuTensorMapEncodeTiled failed for %s (code %d)", what, (int)r);
     return 0;
-}
-
-int sm_count() {
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-    }
-    return n;
 }
 
 template <int TN, bool DUAL, int MODE>

@@ -130,23 +130,6 @@ latent_prepare_kernel(TI* __restrict__ proj, int ld, const float* __restrict__ c
 }
 
 // bfloat16, sizes in whole 16-byte pieces.  A block per token; a row is read once, eight values per thread and step.
-__device__ __forceinline__ void eight(const __nv_bfloat16* p, float* f) {
-    const uint4 u = *reinterpret_cast<const uint4*>(p);
-    const __nv_bfloat162* q = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float2 v = __bfloat1622float2(q[i]);
-        f[2 * i] = v.x;
-        f[2 * i + 1] = v.y;
-    }
-}
-__device__ __forceinline__ uint4 eight_of(const float* f) {
-    uint4 u;
-    __nv_bfloat162* q = reinterpret_cast<__nv_bfloat162*>(&u);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) q[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
-    return u;
-}
 constexpr int EXPAND_THREADS = 128, EXPAND_PER = 4;      // latents of up to EXPAND_THREADS * 8 * EXPAND_PER channels
 
 __global__ void __launch_bounds__(EXPAND_THREADS)
@@ -177,15 +160,15 @@ latent_expand_kernel(__nv_bfloat16* proj, int ld, const float* __restrict__ cos_
             const int k = (i % runs) * 8;
             __nv_bfloat16* at = row + (i / runs) * qh + d + k;
             float lo[8], hi[8], a[8], b[8];
-            eight(at, lo);
-            eight(at + half, hi);
+            unpack8(*reinterpret_cast<const uint4*>(at), lo);
+            unpack8(*reinterpret_cast<const uint4*>(at + half), hi);
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
                 a[e] = lo[e] * c[k + e] - hi[e] * s[k + e];
                 b[e] = lo[e] * s[k + e] + hi[e] * c[k + e];
             }
-            *reinterpret_cast<uint4*>(at) = eight_of(a);
-            *reinterpret_cast<uint4*>(at + half) = eight_of(b);
+            *reinterpret_cast<uint4*>(at) = pack8(a);
+            *reinterpret_cast<uint4*>(at + half) = pack8(b);
         }
     } else {
         for (int i = tid; i < n_heads * half; i += EXPAND_THREADS) {
@@ -213,7 +196,7 @@ latent_expand_kernel(__nv_bfloat16* proj, int ld, const float* __restrict__ cos_
     for (int p = 0; p < EXPAND_PER; ++p) {
         const int j = (p * EXPAND_THREADS + tid) * 8;
         if (j >= rank) break;
-        eight(lat + j, v[p]);
+        unpack8(*reinterpret_cast<const uint4*>(lat + j), v[p]);
 #pragma unroll
         for (int e = 0; e < 8; ++e) ss += v[p][e] * v[p][e];
     }
@@ -225,7 +208,7 @@ latent_expand_kernel(__nv_bfloat16* proj, int ld, const float* __restrict__ cos_
         if (j >= rank) break;
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[p][e] = v[p][e] * scale * c_w[j + e];
-        const uint4 u = eight_of(v[p]);
+        const uint4 u = pack8(v[p]);
         *reinterpret_cast<uint4*>(kept + j) = u;
         *reinterpret_cast<uint4*>(c_out + j) = u;
     }
@@ -249,13 +232,13 @@ __global__ void latent_terms_kernel(const float* kv32, __nv_bfloat16* kv, __nv_b
         const float4* src = reinterpret_cast<const float4*>(kv32 + th * (d + vd) + c);
         const float4 a = src[0], b = src[1];
         float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}, up[8];
-        const uint4 upper = eight_of(v);
+        const uint4 upper = pack8(v);
         *reinterpret_cast<uint4*>(kv + th * (d + vd) + c) = upper;
         if (c < d) continue;
-        eight(reinterpret_cast<const __nv_bfloat16*>(&upper), up);
+        unpack8(upper, up);
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[e] = fabsf(up[e]) <= 3.402823466e38f ? v[e] - up[e] : 0.f;      // an infinite or NaN value has no second term
-        *reinterpret_cast<uint4*>(low + th * vd + (c - d)) = eight_of(v);
+        *reinterpret_cast<uint4*>(low + th * vd + (c - d)) = pack8(v);
     }
 }
 

@@ -814,19 +814,6 @@ sample_cluster_kernel(float* __restrict__ logits, int vocab, int per_cta, int* o
 int g_cluster_min_vocab = 32768;
 int g_cluster_any_rows = 0;            // 1: clusters however many rows there are (for tests and comparisons)
 
-// SMs of the current device (asked once per device)
-static int sm_count() {
-    static std::atomic<int> known[64];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-    int n = known[dev].load(std::memory_order_relaxed);
-    if (n == 0) {
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-        known[dev].store(n, std::memory_order_relaxed);
-    }
-    return n;
-}
-
 // logits: float32 [rows, vocab], overwritten.  out: int32 [rows].
 // recent (may be null): int32 [rows, recent_ld] with recent_count[r] valid ids per row, oldest first.
 // row_stream / row_counter: int32 [rows], which sequence a row is and how many tokens it has drawn;
