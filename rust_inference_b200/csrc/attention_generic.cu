@@ -1,5 +1,6 @@
 // Attention over the paged cache for any head size, any number of heads and groups and
-// any mix of query lengths: the 32-bit path's kernel for what `attention_f32.cu` does not take, and the bf16 path's fallback.
+// any mix of query lengths: the 32-bit path's kernel for what `attention_f32.cu` does not take and for its shortest prompts, and the
+// bf16 path's fallback.
 //
 // One block per (query token, query head).  The token at position p of its sequence
 // sees the cached keys 0..p of its slot, nothing else: causal by construction, as in

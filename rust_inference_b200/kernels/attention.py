@@ -9,7 +9,7 @@
                                  a gate on the tcgen05 kernel
   bfloat16, head_dim 64 or 128,  values of 32, 64 or 128: the TMA-fed decode kernel and the tcgen05 prefill kernel, in their
   values of another size         instances for both sizes
-  float32, head_dim 64 or 128,   tiles of query rows over whole pages (`attention_f32`)
+  float32, head_dim 64 or 128,   tiles of query rows over whole pages (`attention_f32`), but for short prompts (`f32_few_keys`)
   the plain form of the score
   anything else                  the generic kernel (`attention_generic`): any head size, any
                                  dtype, float32 arithmetic
@@ -59,13 +59,25 @@ def f32_splits(n_seqs: int, max_new: int, n_heads: int, n_kv_heads: int, head_di
     """Thread blocks (1..8, a cluster) that share the pages of a tile of query rows in the float32 kernels: as many as keep
     the step's tiles resident at once (an SM holds one block of 64 rows of 128 channels or three of 64, two of up to 8 rows,
     one of 16), never more than the longest sequence has pages.  Tiles of 64 rows take two at most: merging 64 rows costs
-    more than it saves beyond (333 tokens, 14 heads of 64: 33 us with one, 21 with two, 28 with six)."""
+    more than it saves beyond for a prompt (333 tokens, 14 heads of 64: 33 us with one, 21 with two, 28 with six).  A few new tokens
+    behind a long sequence would gain from more (12 heads of 128 over 2, 3 tokens behind 8,000: 1,088 with one, 551 with two,
+    150 with eight; the generic kernel 893)."""
     rows = max_new * (n_heads // n_kv_heads)
     few = rows <= 16
     tiles = n_seqs * n_kv_heads * (1 if few else -(-rows // 64))
     per_sm = (2 if rows <= 8 else 1) if few else (1 if head_dim == 128 else 3)
     most = CLUSTER_SPLITS if few else 2
     return max(1, min(most, per_sm * _sm_count() // tiles, -(-longest // page_size)))
+
+
+def f32_few_keys(n_tokens: int, max_new: int, n_heads: int, n_kv_heads: int, longest: int) -> bool:
+    """Float32 steps that the generic kernel has sooner than the tiles of 64 rows: a block per (token, head) reads a few keys in
+    less time than a tile takes to bring a whole page and its queries through shared memory, while all of its blocks are
+    resident together.  (us, generic / tiles, prompts without cached positions.  14 heads of 64 over 2 kv heads: 3 tokens 10.2 / 12.3,
+    24 tokens 12.2 / 14.3, 64 tokens 20.5 / 14.3; 12 heads of 128 over 2: 3 tokens 11.2 / 16.4, 24 tokens 14.3 / 18.5, 64 tokens
+    26.6 / 18.5, four prompts of 24 19.4 / 19.2; 28 heads over 4, four prompts of 6 12.3 / 18.4, of 24 36.9 / 18.7.)  Up to 16
+    rows there is a kernel for few rows, which is as fast as the generic one or faster there."""
+    return max_new * (n_heads // n_kv_heads) > 16 and longest <= 32 and n_tokens * n_heads <= 8 * _sm_count()
 
 
 def decode_plan(n_seqs: int, n_kv_heads: int, max_seq_len: int, page_size: int, head_dim: int | None = None,
@@ -194,10 +206,11 @@ def attention(qkv, cache_layer, out, ctx, *, n_heads, n_kv_heads, head_dim, scal
             n_seqs=ctx.n_seqs, max_new=ctx.max_new, n_heads=n_heads, n_kv_heads=n_kv_heads, head_dim=head_dim,
             page_size=ctx.page_size, scale=scale, window=window or 0, softcap=softcap, keep_first=keep_first, sink=sink,
             dist=dist, gate=gate, out_scale=out_scale)
+    longest = ctx.page_table.shape[1] * ctx.page_size if ctx.all_single else ctx.max_len
     if (same_sizes and not (window and chunk) and plain
             and ops.attention_f32_supports(qkv, q_ld, cache_layer.k, cache_layer.v, out, n_seqs=ctx.n_seqs, n_kv_heads=n_kv_heads,
-                                           head_dim=head_dim, page_size=ctx.page_size)):
-        longest = ctx.page_table.shape[1] * ctx.page_size if ctx.all_single else ctx.max_len
+                                           head_dim=head_dim, page_size=ctx.page_size)
+            and not f32_few_keys(qkv.shape[0], ctx.max_new, n_heads, n_kv_heads, longest)):
         return ops.attention_f32(
             qkv, q_ld, cache_layer.k, cache_layer.v, ctx.page_table, ctx.seq_slot, ctx.seq_start, ctx.cu_seqlens, out,
             n_seqs=ctx.n_seqs, max_new=ctx.max_new, n_heads=n_heads, n_kv_heads=n_kv_heads, head_dim=head_dim,

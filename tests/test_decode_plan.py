@@ -85,6 +85,34 @@ def test_float32_attention_leaves_to_the_generic_kernel_what_the_tiles_do_not_ta
     assert route(n_seqs=65536) == route(offset=1) == route(hd=80) == route(page=32) == "generic"
 
 
+def test_float32_prompts_of_few_keys_stay_with_the_generic_kernel(monkeypatch):
+    """Where a tile's fixed time is longer than a block per token and head takes for its few keys."""
+    from types import SimpleNamespace
+
+    import torch
+    from rust_inference_b200.kernels import attention, ops
+    monkeypatch.setattr(attention, "_sm_count", lambda: 148)
+    taken = []
+    monkeypatch.setattr(ops, "attention_f32", lambda *a, **k: taken.append("tiles"))
+    monkeypatch.setattr(ops, "attention_generic", lambda *a, **k: taken.append("generic"))
+    monkeypatch.setattr(ops, "attention_f32_supports", lambda *a, **k: True)
+
+    def route(new, cached=0, seqs=1, heads=12, kv=2, single=False):
+        none = torch.zeros(1, dtype=torch.int32)
+        q = torch.zeros(new * seqs, 1)
+        ctx = SimpleNamespace(n_seqs=seqs, max_new=new, max_len=new + cached, all_single=single, page_size=64,
+                              page_table=torch.zeros(2, 1), token_pos=none, token_seq=none, seq_slot=none, seq_start=none, cu_seqlens=none)
+        taken.clear()
+        attention.attention(q, SimpleNamespace(k=q, v=q), q, ctx, n_heads=heads, n_kv_heads=kv, head_dim=128, scale=0.1)
+        return taken[0]
+
+    assert [route(n) for n in (2, 3, 32, 33, 64)] == ["tiles", "generic", "generic", "tiles", "tiles"]     # 12 rows: the kernel for few
+    assert [route(3, cached=c) for c in (29, 30)] == ["generic", "tiles"]
+    assert [route(24, seqs=n) for n in (4, 5)] == ["generic", "tiles"]             # 1,152 and 1,440 blocks on 8 x 148
+    assert route(1, heads=40, kv=2, single=True) == "tiles"                        # a captured step: by the cache's geometry
+    assert route(16, heads=8, kv=8) == "tiles" and route(17, heads=8, kv=8) == "generic"
+
+
 def test_short_float32_sums_stay_with_the_ffma_kernel(monkeypatch):
     import torch
     from rust_inference_b200.kernels import linear, ops
