@@ -96,8 +96,8 @@ def test_kernel(window, sink, gated, lengths):
 
 
 @pytest.mark.parametrize("first", [1, 63, 65, 130, 200])         # the last page holds 63, 1, 63, 62 and 56 rows of the next prompt
-@pytest.mark.parametrize("gated", [False, True])
-def test_neighbours_with_infinities(first, gated):
+@pytest.mark.parametrize("gated, terms", [(False, 1), (True, 1), (False, 2)])
+def test_neighbours_with_infinities(first, gated, terms):
     """A prompt's result does not depend on what stands in the prompt packed behind it, infinities and NaN included: to the
     bit what it is alone."""
     from rust_inference_b200.kernels import attention_tc, tcgen05
@@ -106,7 +106,8 @@ def test_neighbours_with_infinities(first, gated):
     draw = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
     total = first + second
     q, kv, shared, gates = draw(total, heads * 192), draw(total, heads * 256), draw(total, 64), draw(total, 8)
-    for t in (q, kv, shared):
+    low = draw(total, heads * 128) * 2.0 ** -8 if terms == 2 else None
+    for t in (q, kv, shared) + ((low,) if terms == 2 else ()):
         t[first::3], t[first + 1::3], t[first + 2::3] = float("nan"), float("inf"), float("-inf")
 
     def run(n, lengths):
@@ -114,7 +115,7 @@ def test_neighbours_with_infinities(first, gated):
         zeros = torch.zeros(len(lengths), dtype=torch.int32, device="cuda")
         out = torch.full((n, heads * 128), 7.0, dtype=torch.bfloat16, device="cuda")
         attention_tc.expanded(q[:n], kv[:n], shared[:n], zeros, zeros, cu, out, n_seqs=len(lengths), max_new=max(lengths), n_heads=heads,
-                              scale=192 ** -0.5, gate=gates[:n, 2:2 + heads] if gated else None)
+                              scale=192 ** -0.5, gate=gates[:n, 2:2 + heads] if gated else None, low=low[:n] if terms == 2 else None)
         torch.cuda.synchronize()
         tcgen05.check_status()
         return out
