@@ -24,6 +24,12 @@ __device__ __forceinline__ float peer_float(const float* own, uint32_t rank) {
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(there) : "memory");
     return v;
 }
+// ... and a store to it
+__device__ __forceinline__ void store_peer_float(const float* own, uint32_t rank, float v) {
+    uint32_t there;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"((uint32_t)__cvta_generic_to_shared(own)), "r"(rank));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(there), "f"(v) : "memory");
+}
 // four of them (16-byte aligned)
 __device__ __forceinline__ float4 peer_float4(const float* own, uint32_t rank) {
     uint32_t there;

@@ -56,6 +56,8 @@ constexpr int A_BYTES = BLOCK_F * BLOCK_K * 2;     // 16 KiB
 constexpr int MAX_STAGES = 8;
 constexpr int THREADS = 192;
 constexpr int SMEM_BUDGET = 200 * 1024;
+constexpr int CLUSTER_MAX_TOK = 16;                // tokens of a product whose K is cut over clusters
+constexpr int CLUSTER_RECV_MAX = 24 * 1024;        // bytes of sums that a CTA takes from its cluster, at most
 
 enum Status { ST_OK = 0, ST_PRODUCER_TIMEOUT = 1, ST_MMA_TIMEOUT = 2, ST_EPILOGUE_TIMEOUT = 3, ST_DRAIN_TIMEOUT = 4 };
 
@@ -109,7 +111,7 @@ template <int TN, bool DUAL, int MODE>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2,
                const __grid_constant__ CUtensorMap map_x, const float* __restrict__ bias, void* __restrict__ out_,
-               int n_tok, int n_feat, int K, int kb_per_split, int split_k, int stages, int tn, int* status) {
+               int n_tok, int n_feat, int K, int kb_per_split, int split_k, int cluster, int stages, int tn, int* status) {
     // TN is the widest token tile this instance holds (shared memory and tensor memory are laid out
     // for it); tn <= TN, a multiple of 16, is the width it runs: the box of map_x has tn rows.
     constexpr int B_BYTES = TN * BLOCK_K * 2;
@@ -125,16 +127,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     __shared__ __align__(8) uint64_t acc_full[2];
     __shared__ __align__(8) uint64_t acc_empty[2];
     __shared__ uint32_t tmem_base_slot;
-    __shared__ volatile int abort_flag;
+    __shared__ volatile int abort_flag, any_failed;
 
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;     // swizzled tiles want 1024-byte alignment
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int total_kb = (K + BLOCK_K - 1) / BLOCK_K;
+    // The gated product of a few tokens may have its K cut over the CTAs of a cluster (`cluster` > 1; one tile per
+    // cluster, one token tile): see the end of the kernel.
+    const bool clustered = DUAL && cluster > 1;
+    const int rank = clustered ? (int)cluster_rank() : 0;
     // Tiles are numbered with the token tile fastest, so that CTAs running together share a weight
     // tile in L2; a CTA takes tiles blockIdx.x, blockIdx.x + gridDim.x, ...
     const int n_tok_tiles = (n_tok + tn - 1) / tn, n_feat_tiles = (n_feat + BLOCK_F - 1) / BLOCK_F;
     const int total_tiles = n_tok_tiles * n_feat_tiles * split_k;
-    const int my_tiles = ((int)blockIdx.x < total_tiles) ? (total_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    const int my_tiles = clustered ? 1
+                         : ((int)blockIdx.x < total_tiles) ? (total_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < stages; ++s) {
@@ -145,7 +152,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             mbar_init(smem_u32(&acc_full[i]), 1);
             mbar_init(smem_u32(&acc_empty[i]), 4);             // one arrival per epilogue warp
         }
-        abort_flag = 0;
+        abort_flag = any_failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -159,10 +166,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_slot;
     const uint32_t full0 = smem_u32(&full_bar[0]), empty0 = smem_u32(&empty_bar[0]);
+    if (clustered) cluster_arrive();                   // "this CTA runs, its flags are set": waited for before anything is sent
     let_next_kernel_start();
 
     // coordinates of the CTA's i-th tile
     auto tile_coords = [&](int i, int& f0, int& t0, int& kb_begin, int& n_kb) {
+        if (clustered) {
+            f0 = ((int)blockIdx.x / cluster) * BLOCK_F;
+            t0 = 0;
+            kb_begin = total_kb * rank / cluster;
+            n_kb = total_kb * (rank + 1) / cluster - kb_begin;             // >= 1: cluster <= total_kb
+            return;
+        }
         const int tile = (int)blockIdx.x + i * (int)gridDim.x;
         const int tt = tile % n_tok_tiles, rest = tile / n_tok_tiles;
         const int ft = rest % n_feat_tiles, sp = rest / n_feat_tiles;
@@ -295,6 +310,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             }
             tc_fence_after();
             if (!landed || abort_flag) break;
+            if (clustered) break;                                  // the pieces of K meet below
             const int f = f0 + lane_base + lane;
             const bool f_ok = f < n_feat;
             const float b = MODE == 5 ? (f < (int)bias[0] ? 1.f : 0.f)
@@ -331,6 +347,54 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&acc_empty[buf]));
+        }
+    }
+
+    if constexpr (DUAL) {
+        if (clustered) {
+            // Token c is finished by the CTA of rank c % cluster: everybody sends it its sums of that token, gate and up, into
+            // `recv` [rank of the sender][c / cluster][gate, up][128] (behind the ring), and it adds them in the order of the
+            // ranks.  A CTA that gave up says so first; then none of the cluster writes.
+            const int held = (n_tok + cluster - 1) / cluster;
+            float* recv = reinterpret_cast<float*>(smem_raw + (smem_base - smem_u32(smem_raw)) + (size_t)stages * STAGE_BYTES);
+            const int fl = (warp & 3) * 32 + lane;
+            __syncwarp();
+            cluster_wait();                                        // the peers run
+            if (abort_flag && lane == 0) set_in_all(&any_failed, cluster);
+            if (warp >= 2 && !abort_flag) {
+                const uint32_t trow = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+                const float* mine = recv + (size_t)rank * held * 2 * BLOCK_F + fl;
+#pragma unroll 1
+                for (int c0 = 0; c0 < n_tok; c0 += 16) {
+                    uint32_t v[16], u[16];
+                    tmem_ld16(trow + c0, v);
+                    tmem_ld16(trow + TN + c0, u);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        const int c = c0 + j;
+                        if (c >= n_tok) break;
+                        const int to = c % cluster, at = (c / cluster) * 2 * BLOCK_F;
+                        store_peer_float(mine + at, (uint32_t)to, __uint_as_float(v[j]));
+                        store_peer_float(mine + at + BLOCK_F, (uint32_t)to, __uint_as_float(u[j]));
+                    }
+                }
+            }
+            __syncwarp();
+            cluster_sync();                                        // everything sent has arrived
+            const int f = ((int)blockIdx.x / cluster) * BLOCK_F + fl;
+            if (warp >= 2 && !any_failed && f < n_feat) {
+                const GateForm gf = load_gate_form(MODE == 3 ? bias : nullptr);
+                for (int i = 0, c = rank; c < n_tok; ++i, c += cluster) {
+                    const float* from = recv + (size_t)i * 2 * BLOCK_F + fl;
+                    float g = 0.f, up = 0.f;
+                    for (int p = 0; p < cluster; ++p, from += (size_t)held * 2 * BLOCK_F) {
+                        g += from[0];
+                        up += from[BLOCK_F];
+                    }
+                    store_result<MODE>(out_, (size_t)c * n_feat + f, g, 0.f, up, gf, ActForm{0.f, 0.f, 0.f});
+                }
+            }
         }
     }
 
@@ -853,21 +917,30 @@ int launch(int tn, const CUtensorMap& mw, const CUtensorMap& mw2, const CUtensor
            int n_tok, int n_feat, int K, int split_k, int* status, cudaStream_t stream) {
     constexpr int STAGE_BYTES = (DUAL ? 2 : 1) * A_BYTES + TN * BLOCK_K * 2;
     const int total_kb = (K + BLOCK_K - 1) / BLOCK_K;
+    if (split_k < 1) split_k = 1;
+    if (split_k > total_kb) split_k = total_kb;
+    const int cluster = DUAL ? split_k : 1;                          // the gated epilogue's pieces of K meet in a cluster
+    const long long cluster_ctas = (long long)((n_feat + BLOCK_F - 1) / BLOCK_F) * cluster;
+    const int recv = cluster > 1 ? cluster * ((n_tok + cluster - 1) / cluster) * 2 * BLOCK_F * 4 : 0;
     // Small token tiles (decode) leave room for a second CTA on the SM, so that the next kernel's
     // CTAs can settle in and prefetch their weights while this one drains.
-    const int budget = (3 * STAGE_BYTES <= 108 * 1024 && TN <= 64) ? 108 * 1024 : SMEM_BUDGET;
+    int budget = (3 * STAGE_BYTES <= 108 * 1024 && TN <= 64) ? 108 * 1024 : SMEM_BUDGET;
+    if (cluster > 1 && cluster_ctas > sm_count()) budget = 111 * 1024 - recv;         // two of these CTAs on an SM
     int stages = budget / STAGE_BYTES;
     if (stages > MAX_STAGES) stages = MAX_STAGES;
     if (stages > total_kb) stages = total_kb;
     if (stages < 1) stages = 1;
-    const size_t smem = (size_t)stages * STAGE_BYTES + 1024;
-    if (split_k < 1) split_k = 1;
-    if (split_k > total_kb) split_k = total_kb;
+    const size_t smem = (size_t)stages * STAGE_BYTES + 1024 + recv;
     int kb_per_split = (total_kb + split_k - 1) / split_k;
-    split_k = (total_kb + kb_per_split - 1) / kb_per_split;          // no empty split
+    if (!DUAL) split_k = (total_kb + kb_per_split - 1) / kb_per_split;          // no empty split
     auto kernel = gemm_tc_kernel<TN, DUAL, MODE>;
     static PerDeviceOnce configured;       // per device: the attribute belongs to a device's copy of the kernel
-    if (int rc = raise_dynamic_smem(kernel, SMEM_BUDGET + 1024, configured, "gemm_tcgen05")) return rc;
+    if (int rc = raise_dynamic_smem(kernel, SMEM_BUDGET + 1024 + CLUSTER_RECV_MAX, configured, "gemm_tcgen05")) return rc;
+    if (cluster > 1) {
+        if (cluster_ctas > 0x7fffffffLL) return fail("gemm_tcgen05: %lld CTAs exceed the grid limit", cluster_ctas);
+        return launch_cluster("gemm_tcgen05 (cluster)", kernel, dim3((unsigned)cluster_ctas), THREADS, smem, cluster, stream, mw, mw2, mx, bias,
+                              out, n_tok, n_feat, K, kb_per_split, 1, cluster, stages, tn, status);
+    }
     const long long total_tiles = (long long)((n_tok + tn - 1) / tn) * ((n_feat + BLOCK_F - 1) / BLOCK_F) * split_k;
     if (total_tiles > 0x7fffffffLL) return fail("gemm_tcgen05: %lld tiles exceed the index range", total_tiles);
     // a persistent grid: as many CTAs as fit the GPU at once (two per SM when the ring is small and
@@ -878,7 +951,7 @@ int launch(int tn, const CUtensorMap& mw, const CUtensorMap& mw2, const CUtensor
     if (ctas > total_tiles) ctas = total_tiles;
     dim3 grid((unsigned)ctas);
     cudaError_t e = launch_dependent(kernel, grid, dim3(THREADS), smem, stream, mw, mw2, mx, bias, out, n_tok, n_feat, K,
-                                     kb_per_split, split_k, stages, tn, status);
+                                     kb_per_split, split_k, 1, stages, tn, status);
     return check_launch(e, "gemm_tcgen05");
 }
 
@@ -998,6 +1071,29 @@ int pick_tile(int tn, const CUtensorMap& mw, const CUtensorMap& mw2, const CUten
 
 }  // namespace
 
+// Over how many CTAs of a cluster K is cut for the gated product of a few tokens.  Such a product is a read of its weights, and a CTA,
+// whose ring holds 102 KB of them on their way, takes about 64 GB/s, so a product with few tiles leaves most of the memory's rate
+// unused.  Cut in four where that makes about one CTA per SM: most of a CTA's weights are then asked for before its wait.  Otherwise
+// in two or three, whichever leaves the SMs more evenly filled, as long as all CTAs are resident together (two to an SM).
+// Whole decode steps, us, not cut / 2 / 3 / 4: 38 tiles of K = 896 (24 layers), 1 token 690 / 648 / 650 / 633, 8 tokens 757 / 713 / 692 /
+// 675; 70 tiles of 1,536 (28), 1 token 1,059 / 985 / 1,025 / 1,000, 12 tokens 1,140 / 1,130 / 1,144 / 1,203; 86 tiles of 2,048 (36), 1 token
+// 1,629 / 1,604 / 1,576 / 1,758; 112 tiles of 4,096 (32), 1 token 2,835 / 2,670 / 2,925 / 2,828.
+int gated_cluster(int n_tok, int n_feat, int K) {
+    const int total_kb = (K + BLOCK_K - 1) / BLOCK_K, sms = sm_count();
+    const long long tiles = (n_feat + BLOCK_F - 1) / BLOCK_F;
+    if (n_tok > CLUSTER_MAX_TOK || total_kb < 8) return 1;
+    if (tiles * 4 * 100 <= sms * 108LL) return 4;
+    int cluster = 1;
+    long long filled = 0;                                            // of 1,000 places, on the SMs as full as the fullest
+    for (int cl = 2; cl <= 3; ++cl) {
+        const long long ctas = tiles * cl, rounds = (ctas + sms - 1) / sms;
+        if (ctas > 2 * (sms - 6)) break;                             // clusters leave some SMs out
+        const long long share = ctas * 1000 / (rounds * sms);
+        if (share > filled) { filled = share; cluster = cl; }
+    }
+    return cluster;
+}
+
 // Steps of at least n_tok tokens may run on pairs of SMs (0: never); with always != 0 they do, whatever
 // their tiles make of the grid.  For comparisons and tests; plans made before the call no longer hold.
 RI_API int ri_gemm_tcgen05_set_pairs(int n_tok, int always) {
@@ -1032,6 +1128,7 @@ RI_API int ri_gemm_tcgen05_plan(int n_tok, int n_feat, int K, int mode, int* til
         if (mode == 2) sp = pair_split(n_tok, n_feat, K);
     } else if (n_tok <= 128) {
         tn = n_tok <= 16 ? 16 : (n_tok + 15) / 16 * 16;
+        if (mode == 3) sp = gated_cluster(n_tok, n_feat, K);
         if (can_split && feat_tiles < ctas) {
             // every piece ends in tn x 128 atomic adds, so wider steps want longer pieces: at least a tenth of
             // the tile's width in k-blocks (128 tokens, K = 3584: 4-5 pieces, 11 us, against 10 pieces, 13 us)
@@ -1086,7 +1183,9 @@ RI_API int ri_gemm_tcgen05(const void* map_x, const void* map_w, const void* map
     if (mode == 5 && bias == nullptr) return fail("gemm_tcgen05: the partly activated epilogue needs its number of features");
     if (mode == 3 && map_w2 == nullptr) return fail("gemm_tcgen05: the SiLU-gate epilogue needs a second matrix");
     if (mode == 2 && bias != nullptr) return fail("gemm_tcgen05: the residual epilogue takes no bias");
-    if (mode != 2 && split_k > 1) return fail("gemm_tcgen05: only the residual epilogue can split K");
+    if (mode == 3 && split_k > 1 && (split_k > 8 || n_tok > CLUSTER_MAX_TOK))
+        return fail("gemm_tcgen05: no cluster of %d CTAs for the gated epilogue of %d tokens", split_k, n_tok);
+    if (mode != 2 && mode != 3 && split_k > 1) return fail("gemm_tcgen05: only the residual and the gated epilogue can split K");
     const bool dual = mode == 3;
     int tn = 0, planned_split = 1;
     ri_gemm_tcgen05_plan(n_tok, n_feat, K, mode, &tn, &planned_split);

@@ -1,0 +1,33 @@
+"""The gated product of a few tokens whose K is cut over the blocks of a cluster, against 64 bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 7, 8, 9, 16])
+@pytest.mark.parametrize("n, k", [(128, 512), (391, 192), (1000, 2056)])
+@pytest.mark.parametrize("cluster", [1, 2, 3, 8])
+def test_gated_product_cut_over_a_cluster(m, n, k, cluster):
+    from rust_inference_b200.kernels import linear, ops, tcgen05
+    cluster = min(cluster, -(-k // 64))
+    x = (torch.randn(m, k, device=DEV) * 0.5).bfloat16()
+    w, w2 = (linear.Weight((torch.randn(n, k, device=DEV) * 0.1).bfloat16()) for _ in range(2))
+    gate, up = (x.double() @ t.t.double().t() for t in (w, w2))
+    want = gate * torch.sigmoid(gate) * up
+    out = torch.full((m, n), 9.0, device=DEV, dtype=torch.bfloat16)
+    tcgen05.gemm(x, w, out, ops.EPI_SILU_MUL, w2=w2, split_k=cluster)
+    # one rounding to bfloat16 (2^-9) of each result, and float32 sums of k products (k * 2^-24 of their size)
+    assert float(((out.double() - want).norm() / want.norm())) <= 2.0 ** -8
+    torch.cuda.synchronize()
+    tcgen05.check_status()
+
+
+def test_gated_product_refuses_clusters_it_cannot_form():
+    from rust_inference_b200.kernels import linear, ops, tcgen05
+    w = linear.Weight(torch.zeros(128, 1024, device=DEV, dtype=torch.bfloat16))
+    for m, cluster in ((17, 2), (200, 2), (4, 9)):
+        x = torch.zeros(m, 1024, device=DEV, dtype=torch.bfloat16)
+        with pytest.raises(ops.KernelError, match="no cluster"):
+            tcgen05.gemm(x, w, torch.zeros(m, 128, device=DEV, dtype=torch.bfloat16), ops.EPI_SILU_MUL, w2=w, split_k=cluster)
