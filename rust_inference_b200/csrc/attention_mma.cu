@@ -239,7 +239,7 @@ constexpr int CLUSTER_RECV_FLOATS = 16 * HD + 4 * MAX_CLUSTER_SPLITS + MAX_CLUST
 template <int HD, int NT>
 __device__ __forceinline__ void cluster_merge(const float* so, const float* sml, float* recv, int n_rep, int n_splits,
                                               int split, int token, int kvh, __nv_bfloat16* __restrict__ out,
-                                              int out_ld, bool ok) {
+                                              int out_ld, bool ok, float out_scale = 1.f) {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     const int total = n_rep * HD;
@@ -289,7 +289,7 @@ __device__ __forceinline__ void cluster_merge(const float* so, const float* sml,
                     acc.z += f * x.z;
                     acc.w += f * x.w;
                 }
-            const float inv = 1.0f / L;
+            const float inv = out_scale / L;
             store_bf16x4(out + (size_t)token * out_ld + (size_t)(kvh * n_rep + r) * HD + d, acc.x * inv, acc.y * inv,
                          acc.z * inv, acc.w * inv, wide);
         }
@@ -302,10 +302,12 @@ __device__ __forceinline__ void cluster_merge(const float* so, const float* sml,
 template <int HD>
 __device__ __forceinline__ void write_merged(const float* so, const float* sml, int r, int d, int b, int h, int token,
                                              int n_heads, int n_splits, int split, float* __restrict__ part_o,
-                                             float* __restrict__ part_ml, __nv_bfloat16* __restrict__ out, int out_ld) {
+                                             float* __restrict__ part_ml, __nv_bfloat16* __restrict__ out, int out_ld,
+                                             float out_scale = 1.f) {
     float M, L;
-    const float4 acc = merge_warps<HD>(so, sml, r, d, M, L);
+    float4 acc = merge_warps<HD>(so, sml, r, d, M, L);
     if (n_splits == 1) {
+        if (out_scale != 1.f) { acc.x *= out_scale; acc.y *= out_scale; acc.z *= out_scale; acc.w *= out_scale; }
         const bool wide = ((reinterpret_cast<uintptr_t>(out) & 7) == 0) && ((out_ld & 3) == 0);
         store_bf16x4(out + (size_t)token * out_ld + (size_t)h * HD + d, acc.x / L, acc.y / L, acc.z / L, acc.w / L, wide);
     } else {
@@ -501,21 +503,148 @@ __device__ __forceinline__ void pv_16keys_atoms(const uint32_t* p, uint32_t vtil
     }
 }
 
+// The heads of the new position as the kernel forms them itself (FORM), instead of a kernel of its own before it: from the float32
+// sums of the K-split projection, acc[token] = [q heads | k heads (| v heads)], each plus the bias, the q and k heads RMS-normed
+// (q_w, k_w: one weight of HD values each; null: no norm), their first `rot` channels turned by the position's angles.  Every block of
+// a (sequence, kv head) forms the queries; the one that has the sequence's last page also the key and the value, which it writes
+// to the cache and into its copy of that page.  Without v columns (`v_from_k`) the value is the key as projected.
+struct Fresh {
+    float* acc;
+    int ld;
+    const float* bias;
+    const float* cos_t;
+    const float* sin_t;                 // [positions, rot / 2]
+    const float* q_w;
+    const float* k_w;
+    float eps;
+    int style, rot, v_from_k;           // style 0: channels (i, i + rot / 2) turn together, 1: (2 i, 2 i + 1)
+    __nv_bfloat16* kcache;
+    __nv_bfloat16* vcache;
+};
+
+// What the block's 128 compute threads do to form them: an item is eight channels of a head (the two fours of a pair of halves, or
+// eight in a row), a thread has up to two of them, whose loads go out together; what no kernel of the step writes (bias, angles,
+// weights) is read before the wait.  8 sequences of 28 heads of 128 over 4 kv heads: 0.5 us of the kernel, in place of one of 3.2 us.
+template <int HD>
+__device__ __forceinline__ void form_heads(const Fresh& f, int token, int pos, int kvh, int n_rep, int n_heads, int n_kv_heads,
+                                           bool with_kv, int cache_row, uint8_t* q_tile, __nv_bfloat16* new_k, __nv_bfloat16* new_v) {
+    constexpr int PER_HEAD = HD / 8, SLOTS = 2;
+    const int q_items = n_rep * PER_HEAD, items = q_items + (with_kv ? 2 * PER_HEAD : 0);
+    const float* row = f.acc + (size_t)token * f.ld;
+    const float* cs = f.cos_t + (size_t)pos * (f.rot >> 1);
+    const float* sn = f.sin_t + (size_t)pos * (f.rot >> 1);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int base = 0; base < items; base += SLOTS * 128) {
+        float4 lo[SLOTS], hi[SLOTS], b_lo[SLOTS], b_hi[SLOTS], c[SLOTS], s[SLOTS];
+        int kind[SLOTS], col[SLOTS], c0[SLOTS], c1[SLOTS];           // kind 0 a query, 1 the key, 2 the value, 3 nothing
+        bool turned[SLOTS];
+#pragma unroll
+        for (int u = 0; u < SLOTS; ++u) {
+            const int it = base + u * 128 + (int)threadIdx.x, j = it % PER_HEAD;
+            kind[u] = it < q_items ? 0 : it < q_items + PER_HEAD ? 1 : 2;
+            if (it >= items) kind[u] = 3;
+            col[u] = kind[u] == 0 ? (kvh * n_rep + it / PER_HEAD) * HD
+                     : kind[u] == 1 || f.v_from_k ? (n_heads + kvh) * HD : (n_heads + n_kv_heads + kvh) * HD;
+            turned[u] = kind[u] < 2 && j < f.rot / 8;
+            c0[u] = turned[u] && f.style == 0 ? 4 * j : 8 * j;
+            c1[u] = turned[u] && f.style == 0 ? 4 * j + f.rot / 2 : 8 * j + 4;
+            b_lo[u] = b_hi[u] = c[u] = s[u] = zero;
+            if (kind[u] < 3 && f.bias != nullptr) {
+                b_lo[u] = *reinterpret_cast<const float4*>(f.bias + col[u] + c0[u]);
+                b_hi[u] = *reinterpret_cast<const float4*>(f.bias + col[u] + c1[u]);
+            }
+            if (turned[u]) {
+                c[u] = *reinterpret_cast<const float4*>(cs + 4 * j);
+                s[u] = *reinterpret_cast<const float4*>(sn + 4 * j);
+            }
+        }
+        if (base == 0) wait_for_previous_kernels();                  // the sums come from the kernel before
+#pragma unroll
+        for (int u = 0; u < SLOTS; ++u) {
+            lo[u] = kind[u] < 3 ? load_written(row + col[u] + c0[u]) : zero;
+            hi[u] = kind[u] < 3 ? load_written(row + col[u] + c1[u]) : zero;
+        }
+#pragma unroll
+        for (int u = 0; u < SLOTS; ++u) {
+            float a[4] = {lo[u].x + b_lo[u].x, lo[u].y + b_lo[u].y, lo[u].z + b_lo[u].z, lo[u].w + b_lo[u].w};
+            float b[4] = {hi[u].x + b_hi[u].x, hi[u].y + b_hi[u].y, hi[u].z + b_hi[u].z, hi[u].w + b_hi[u].w};
+            if (f.q_w != nullptr) {                                  // PER_HEAD neighbouring threads have a head
+                float ss = 0.f;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) ss += a[i] * a[i] + b[i] * b[i];
+#pragma unroll
+                for (int o = PER_HEAD / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                if (kind[u] < 2) {
+                    const float inv = 1.0f / sqrtf(ss / (float)HD + f.eps);
+                    const float* w = kind[u] == 0 ? f.q_w : f.k_w;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        a[i] *= inv * w[c0[u] + i];
+                        b[i] *= inv * w[c1[u] + i];
+                    }
+                }
+            }
+            if (kind[u] == 3) continue;
+            const float cc[4] = {c[u].x, c[u].y, c[u].z, c[u].w}, sc[4] = {s[u].x, s[u].y, s[u].z, s[u].w};
+            if (turned[u] && f.style == 0) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float x = a[i], y = b[i];
+                    a[i] = x * cc[i] - y * sc[i];
+                    b[i] = x * sc[i] + y * cc[i];
+                }
+            } else if (turned[u]) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    float x = a[2 * i], y = a[2 * i + 1];
+                    a[2 * i] = x * cc[i] - y * sc[i];
+                    a[2 * i + 1] = x * sc[i] + y * cc[i];
+                    x = b[2 * i];
+                    y = b[2 * i + 1];
+                    b[2 * i] = x * cc[2 + i] - y * sc[2 + i];
+                    b[2 * i + 1] = x * sc[2 + i] + y * cc[2 + i];
+                }
+            }
+            uint2 p0, p1;
+            p0.x = pack_bf16(a[0], a[1]);
+            p0.y = pack_bf16(a[2], a[3]);
+            p1.x = pack_bf16(b[0], b[1]);
+            p1.y = pack_bf16(b[2], b[3]);
+            if (kind[u] == 0) {
+                const int r = (base + u * 128 + (int)threadIdx.x) / PER_HEAD;
+                *reinterpret_cast<uint2*>(q_tile + tile_off<HD>(r, c0[u] >> 3) + (c0[u] & 4) * 2) = p0;
+                *reinterpret_cast<uint2*>(q_tile + tile_off<HD>(r, c1[u] >> 3) + (c1[u] & 4) * 2) = p1;
+            } else {
+                __nv_bfloat16* near = kind[u] == 1 ? new_k : new_v;
+                *reinterpret_cast<uint2*>(near + c0[u]) = p0;
+                *reinterpret_cast<uint2*>(near + c1[u]) = p1;
+                if (cache_row >= 0) {
+                    __nv_bfloat16* far = (kind[u] == 1 ? f.kcache : f.vcache) + (size_t)cache_row * HD;
+                    *reinterpret_cast<uint2*>(far + c0[u]) = p0;
+                    *reinterpret_cast<uint2*>(far + c1[u]) = p1;
+                }
+            }
+        }
+    }
+}
+
 // VD: the size of a value head; 32 takes tiles of 64 columns whose upper half the copy fills with zeros
-template <int HD, int VD, bool CLUSTER>
+template <int HD, int VD, bool CLUSTER, bool FORM>
 __global__ void __launch_bounds__(DECODE_TMA_THREADS)
 attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                        const __nv_bfloat16* __restrict__ q, int q_ld, const int* __restrict__ page_table,
                        int max_pages, const int* __restrict__ seq_slot, const int* __restrict__ seq_len,
                        const int* __restrict__ cu_seqlens, int n_heads, int n_kv_heads, float scale, int window,
                        int n_splits, float* __restrict__ part_o, float* __restrict__ part_ml,
-                       __nv_bfloat16* __restrict__ out, int out_ld, int* status) {
+                       __nv_bfloat16* __restrict__ out, int out_ld, const Fresh fresh, float out_scale, int* status) {
+    static_assert(!FORM || HD == VD, "heads are formed for values of the keys' size");
     constexpr int ATOMS = HD / 64, V_ATOMS = (VD + 63) / 64;
     constexpr int K_TILE = PAGE * HD * 2, V_TILE = V_ATOMS * PAGE * 128;      // bytes of a K and of a V page tile
     constexpr int STAGE = K_TILE + V_TILE;
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[RING], empty_bar[RING];
     __shared__ volatile int abort_flag;
+    __shared__ __align__(16) __nv_bfloat16 new_k[FORM ? HD : 1], new_v[FORM ? HD : 1];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);      // swizzled tiles: 1024-byte aligned
     const uint32_t kv_base = smem_u32(smem);            // [RING][K tile, V tile], then the Q tile [16][HD]
     const uint32_t q_tile = kv_base + RING * STAGE;
@@ -559,7 +688,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                 const int j = pg - pg_begin, s = j % RING;
                 const int page_now = page_next;
                 if (pg + 1 < pg_end) page_next = pages[pg + 1];
-                if (pg == pg_hi - 1) wait_for_previous_kernels();      // the page the new key and value went to
+                if (!FORM && pg == pg_hi - 1) wait_for_previous_kernels();      // the page the new key and value went to
                 if (!tc::mbar_wait(smem_u32(&empty_bar[s]), (uint32_t)((j / RING) & 1) ^ 1u) || abort_flag) {
                     tc::report(status, 21);
                     abort_flag = 1;
@@ -581,12 +710,27 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         }
     } else {
         // ---------------- compute: warp w takes keys 16w .. 16w+15 of every page ----------------
-        wait_for_previous_kernels();          // q comes from the kernel before
+        if (!FORM) wait_for_previous_kernels();          // q comes from the kernel before
         for (int idx = threadIdx.x; idx < 16 * (HD / 8); idx += 128) {
             const int r = idx / (HD / 8), c = idx % (HD / 8);
+            if (FORM && r < n_rep) continue;
             uint4 v = make_uint4(0, 0, 0, 0);
             if (r < n_rep) v = *reinterpret_cast<const uint4*>(q + (size_t)token * q_ld + (size_t)(kvh * n_rep + r) * HD + c * 8);
             *reinterpret_cast<uint4*>(smem + RING * STAGE + tile_off<HD>(r, c)) = v;
+        }
+        if constexpr (FORM) {
+            const bool with_kv = pg_begin < pg_end && pg_end == pg_hi;
+            int cache_row = -1;
+            if (with_kv) {
+                const int slot = seq_slot[b];
+                // checked build: a slot, a page index or a page outside its range is recorded and nothing is written
+                if (RI_BLOCK_IN_LIMIT(slot, RI_LIMIT_SLOTS, RI_CHECK_SLOT) && RI_BLOCK_IN_RANGE(pg_hi - 1, max_pages, RI_CHECK_PAGE_INDEX)) {
+                    const int page = page_table[(size_t)slot * max_pages + pg_hi - 1];
+                    if (RI_BLOCK_IN_LIMIT(page, RI_LIMIT_PAGES, RI_CHECK_PAGE))
+                        cache_row = (page * n_kv_heads + kvh) * PAGE + (n_keys - 1) % PAGE;
+                }
+            }
+            form_heads<HD>(fresh, token, n_keys - 1, kvh, n_rep, n_heads, n_kv_heads, with_kv, cache_row, smem + RING * STAGE, new_k, new_v);
         }
         asm volatile("bar.sync 1, 128;" ::: "memory");          // the four compute warps: Q tile written
         RI_PHASE(0);
@@ -606,6 +750,15 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             const uint32_t ktile = kv_base + s * STAGE, vtile = ktile + K_TILE;
             const int kbase = warp * 16;
             const int key0 = pg * PAGE + kbase;
+            if (FORM && pg == pg_hi - 1 && warp == (n_keys - 1) % PAGE / 16) {
+                // the new key and value join the page as it was before the step; this warp alone reads their row
+                const int at = lane % (HD / 8), row = (n_keys - 1) % PAGE;
+                if (lane < 2 * (HD / 8)) {
+                    const uint4 v = *reinterpret_cast<const uint4*>((lane < HD / 8 ? new_k : new_v) + at * 8);
+                    *reinterpret_cast<uint4*>(smem + s * STAGE + (lane < HD / 8 ? 0 : K_TILE) + atom_off<HD>(row, at)) = v;
+                }
+                __syncwarp();
+            }
             if (key0 < n_keys && key0 + 16 > first_key) {
                 float sc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
                 qk_16keys_atoms<HD>(qf, ktile, kbase, sc);
@@ -648,16 +801,28 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         }
     }
     __syncthreads();
+    // the sums hold zeros again for the next projection once every block that forms heads from them has read them
+    auto clear_sums = [&]() {
+        const int width = n_rep * HD, kv = fresh.v_from_k ? HD : 2 * HD;
+        float* row = fresh.acc + (size_t)token * fresh.ld;
+        for (int i = 4 * (split * DECODE_TMA_THREADS + (int)threadIdx.x); i < width + kv; i += 4 * n_splits * DECODE_TMA_THREADS) {
+            const int col = i < width ? kvh * width + i
+                            : i < width + HD ? (n_heads + kvh) * HD + i - width : (n_heads + n_kv_heads + kvh) * HD + i - width - HD;
+            *reinterpret_cast<float4*>(row + col) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
     if constexpr (CLUSTER) {
         // the splits of this (sequence, kv head) are the CTAs of one cluster: merged here, no scratch, no second kernel
         float* recv = reinterpret_cast<float*>(smem + RING * STAGE + 16 * HD * 2);
-        cluster_merge<VD, DECODE_TMA_THREADS>(so, sml, recv, n_rep, n_splits, split, token, kvh, out, out_ld, !abort_flag);
+        cluster_merge<VD, DECODE_TMA_THREADS>(so, sml, recv, n_rep, n_splits, split, token, kvh, out, out_ld, !abort_flag, out_scale);
+        if constexpr (FORM) clear_sums();                 // behind the cluster's meeting point
         return;
     }
+    if constexpr (FORM) clear_sums();                     // one block per (sequence, kv head)
     if (abort_flag) return;
     for (int it = threadIdx.x; it < n_rep * (VD / 4); it += DECODE_TMA_THREADS) {
         const int r = it / (VD / 4), d = (it % (VD / 4)) * 4;
-        write_merged<VD>(so, sml, r, d, b, kvh * n_rep + r, token, n_heads, n_splits, split, part_o, part_ml, out, out_ld);
+        write_merged<VD>(so, sml, r, d, b, kvh * n_rep + r, token, n_heads, n_splits, split, part_o, part_ml, out, out_ld, out_scale);
     }
 }
 
@@ -1202,20 +1367,20 @@ int launch_decode(const void* q, int q_ld, const void* kc, const void* vc, const
 template <int HD, int VD>
 constexpr int decode_ring_bytes() { return RING * (PAGE * HD * 2 + (VD + 63) / 64 * PAGE * 128); }
 
-template <int HD, int VD>
+template <int HD, int VD, bool FORM = false>
 int launch_decode_tma(const CUtensorMap& mk, const CUtensorMap& mv, const void* q, int q_ld, const int* page_table,
                       int max_pages, const int* seq_slot, const int* seq_len, const int* cu_seqlens, int n_seqs,
                       int n_heads, int n_kv_heads, float scale, int window, int n_splits, float* part_o,
-                      float* part_ml, void* out, int out_ld, int* status, cudaStream_t stream) {
+                      float* part_ml, void* out, int out_ld, const Fresh& fresh, float out_scale, int* status, cudaStream_t stream) {
     constexpr int SMEM = decode_ring_bytes<HD, VD>() + 16 * HD * 2 + 1024;
     static_assert((4 * 16 * (VD + 4) + 4 * 16 * 2 + 4 * 16 + 16 * 2) * 4 <= decode_ring_bytes<HD, VD>(), "merge area must fit the ring");
     static PerDeviceOnce configured;       // per device: the attribute belongs to a device's copy of the kernel
-    if (int rc = raise_dynamic_smem(attn_decode_tma_kernel<HD, VD, false>, SMEM, configured, "attention")) return rc;
+    if (int rc = raise_dynamic_smem(attn_decode_tma_kernel<HD, VD, false, FORM>, SMEM, configured, "attention")) return rc;
     dim3 grid(n_seqs, n_kv_heads, n_splits);
     cudaError_t e = launch_dependent(
-        attn_decode_tma_kernel<HD, VD, false>, grid, dim3(DECODE_TMA_THREADS), (size_t)SMEM, stream, mk, mv, (const __nv_bfloat16*)q,
+        attn_decode_tma_kernel<HD, VD, false, FORM>, grid, dim3(DECODE_TMA_THREADS), (size_t)SMEM, stream, mk, mv, (const __nv_bfloat16*)q,
         q_ld, page_table, max_pages, seq_slot, seq_len, cu_seqlens, n_heads, n_kv_heads, scale, window, n_splits, part_o,
-        part_ml, (__nv_bfloat16*)out, out_ld, status);
+        part_ml, (__nv_bfloat16*)out, out_ld, fresh, out_scale, status);
     if (int rc = check_launch(e, "attn_decode_tma")) return rc;
     if (n_splits > 1) {
         e = launch_dependent(attn_combine_kernel, dim3(n_seqs, n_heads), dim3(VD >= 128 ? 128 : 64), (size_t)0, stream,
@@ -1232,7 +1397,7 @@ constexpr int tma_cluster_smem_bytes() {
     return decode_ring_bytes<HD, VD>() + 16 * HD * 2 + CLUSTER_RECV_FLOATS<VD> * 4 + 1024;
 }
 
-template <int HD, int VD>
+template <int HD, int VD, bool FORM = false>
 PerDeviceOnce& tma_cluster_configured() {
     static PerDeviceOnce once;
     return once;
@@ -1256,26 +1421,26 @@ void tma_cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int 
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
 }
 
-template <int HD, int VD>
+template <int HD, int VD, bool FORM = false>
 int launch_decode_tma_cluster(const CUtensorMap& mk, const CUtensorMap& mv, const void* q, int q_ld, const int* page_table,
                               int max_pages, const int* seq_slot, const int* seq_len, const int* cu_seqlens, int n_seqs,
                               int n_heads, int n_kv_heads, float scale, int window, int n_splits, void* out, int out_ld,
-                              int* status, cudaStream_t stream) {
-    auto kernel = attn_decode_tma_kernel<HD, VD, true>;
-    if (int rc = raise_dynamic_smem(kernel, tma_cluster_smem_bytes<HD, VD>(), tma_cluster_configured<HD, VD>(), "attention")) return rc;
+                              const Fresh& fresh, float out_scale, int* status, cudaStream_t stream) {
+    auto kernel = attn_decode_tma_kernel<HD, VD, true, FORM>;
+    if (int rc = raise_dynamic_smem(kernel, tma_cluster_smem_bytes<HD, VD>(), tma_cluster_configured<HD, VD, FORM>(), "attention")) return rc;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
     tma_cluster_config<HD, VD>(cfg, attr, n_seqs, n_kv_heads, n_splits, stream);
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, mk, mv, (const __nv_bfloat16*)q, q_ld, page_table, max_pages, seq_slot,
                                        seq_len, cu_seqlens, n_heads, n_kv_heads, scale, window, n_splits, (float*)nullptr,
-                                       (float*)nullptr, (__nv_bfloat16*)out, out_ld, status);
+                                       (float*)nullptr, (__nv_bfloat16*)out, out_ld, fresh, out_scale, status);
     return check_launch(e, "attn_decode_tma_cluster");
 }
 
 // How many clusters of n_splits CTAs of that kernel the device holds at once.
 template <int HD, int VD>
 int decode_tma_cluster_capacity(int n_splits, int* clusters) {
-    auto kernel = attn_decode_tma_kernel<HD, VD, true>;
+    auto kernel = attn_decode_tma_kernel<HD, VD, true, false>;
     if (int rc = raise_dynamic_smem(kernel, tma_cluster_smem_bytes<HD, VD>(), tma_cluster_configured<HD, VD>(), "attention")) return rc;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
@@ -1390,8 +1555,9 @@ RI_API int ri_attention_decode_tma(const void* map_k, const void* map_v, const v
     RI_CHECK_VALUES();
     const CUtensorMap& mk = *reinterpret_cast<const CUtensorMap*>(map_k);
     const CUtensorMap& mv = *reinterpret_cast<const CUtensorMap*>(map_v);
+    const Fresh none{};
 #define ARGS (mk, mv, q, q_ld, page_table, max_pages, seq_slot, seq_len, cu_seqlens, n_seqs, n_heads, n_kv_heads, \
-              scale, window, n_splits, part_o, part_ml, out, out_ld, status, stream)
+              scale, window, n_splits, part_o, part_ml, out, out_ld, none, 1.f, status, stream)
     RI_HEAD_SIZES(launch_decode_tma);
 #undef ARGS
 }
@@ -1412,10 +1578,48 @@ RI_API int ri_attention_decode_tma_cluster(const void* map_k, const void* map_v,
     RI_CHECK_VALUES();
     const CUtensorMap& mk = *reinterpret_cast<const CUtensorMap*>(map_k);
     const CUtensorMap& mv = *reinterpret_cast<const CUtensorMap*>(map_v);
+    const Fresh none{};
 #define ARGS (mk, mv, q, q_ld, page_table, max_pages, seq_slot, seq_len, cu_seqlens, n_seqs, n_heads, n_kv_heads, \
-              scale, window, n_splits, out, out_ld, status, stream)
+              scale, window, n_splits, out, out_ld, none, 1.f, status, stream)
     RI_HEAD_SIZES(launch_decode_tma_cluster);
 #undef ARGS
+}
+
+// The two kernels above with the new position's heads formed inside them (`Fresh`): acc float32 [n_seqs, ld] holds the projection's
+// sums and is left zeroed, keys and values also go to the cache (kcache, vcache: the layer's pages, the memory behind the maps).
+// n_splits 1: one block per (sequence, kv head); 2..8: a cluster of blocks.  The result is times out_scale.  Rows and the biases,
+// tables and weights are read sixteen bytes at a time: ld and rot multiples of 8, all of them 16-byte aligned.
+RI_API int ri_attention_decode_tma_form(const void* map_k, const void* map_v, float* acc, int ld, const float* bias, const float* cos_t,
+                                        const float* sin_t, const float* q_w, const float* k_w, float eps, int style, int rot,
+                                        int v_from_k, void* kcache, void* vcache, const int* page_table, int max_pages,
+                                        const int* seq_slot, const int* seq_len, const int* cu_seqlens, void* out, int out_ld,
+                                        int n_seqs, int n_heads, int n_kv_heads, int hd, int page_size, float scale, int window,
+                                        int n_splits, float out_scale, int* status, cudaStream_t stream) {
+    if (n_seqs <= 0) return 0;
+    if (int rc = check_common(hd, page_size, n_heads, n_kv_heads, ld, out_ld, acc, out)) return rc;
+    if (n_heads / n_kv_heads > 16) return fail("attention_decode: %d query heads per kv head exceed 16", n_heads / n_kv_heads);
+    if (n_splits < 1 || n_splits > MAX_CLUSTER_SPLITS)
+        return fail("attention_decode: heads are formed in 1 to %d blocks of a sequence, not %d", MAX_CLUSTER_SPLITS, n_splits);
+    if (n_kv_heads > 65535) return fail("attention_decode: %d kv heads exceed the grid limit", n_kv_heads);
+    if (ld < (n_heads + (v_from_k ? 1 : 2) * n_kv_heads) * hd) return fail("attention_decode: rows of %d sums are too short", ld);
+    if (style != 0 && style != 1) return fail("attention_decode: unknown style %d", style);
+    if (rot <= 0 || rot > hd || rot % 8) return fail("attention_decode: %d of %d channels turn", rot, hd);
+    if ((q_w == nullptr) != (k_w == nullptr)) return fail("attention_decode: one of two norm weights");
+    if (((uintptr_t)bias | (uintptr_t)cos_t | (uintptr_t)sin_t | (uintptr_t)q_w | (uintptr_t)k_w | (uintptr_t)kcache | (uintptr_t)vcache) % 16)
+        return fail("attention_decode: heads are formed from 16-byte aligned arrays");
+    const CUtensorMap& mk = *reinterpret_cast<const CUtensorMap*>(map_k);
+    const CUtensorMap& mv = *reinterpret_cast<const CUtensorMap*>(map_v);
+    const Fresh fresh{acc, ld, bias, cos_t, sin_t, q_w, k_w, eps, style, rot, v_from_k, (__nv_bfloat16*)kcache, (__nv_bfloat16*)vcache};
+#define RI_FORM(H)                                                                                                                       \
+    return n_splits == 1 ? launch_decode_tma<H, H, true>(mk, mv, nullptr, 0, page_table, max_pages, seq_slot, seq_len, cu_seqlens,       \
+                                                         n_seqs, n_heads, n_kv_heads, scale, window, 1, nullptr, nullptr, out, out_ld,   \
+                                                         fresh, out_scale, status, stream)                                               \
+                         : launch_decode_tma_cluster<H, H, true>(mk, mv, nullptr, 0, page_table, max_pages, seq_slot, seq_len,           \
+                                                                 cu_seqlens, n_seqs, n_heads, n_kv_heads, scale, window, n_splits, out,  \
+                                                                 out_ld, fresh, out_scale, status, stream)
+    if (hd == 64) RI_FORM(64);
+    RI_FORM(128);
+#undef RI_FORM
 }
 
 // clusters[0] = how many clusters of n_splits CTAs of that kernel the current device holds at the same time

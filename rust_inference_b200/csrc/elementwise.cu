@@ -1243,14 +1243,14 @@ RI_API int ri_fill_normal(void* out, int dtype, long long n, unsigned long long 
 // already hold what the sampler drew.  Optionally (null pointers switch a part off): the
 // sampler's per-row draw counters grow by 1; the drawn tokens are copied into slot
 // (*turn % host_slots) of a ring in pinned host memory and into slot (*turn % log_slots) of a
-// ring on the device; then *turn grows by 1.  One thread block; it runs last in the step.
+// ring on the device; then *turn grows by 1.  One thread block; it runs last in the step, and lets the next step's first kernel start
+// only when it is done: a step's kernels read positions, lengths and the cache's older rows before their wait.
 // ---------------------------------------------------------------------------------------
 __global__ void advance_decode_kernel(int* __restrict__ token_pos, int* __restrict__ seq_start,
                                       int* __restrict__ seq_len, int n, const int* __restrict__ token_ids,
                                       int* __restrict__ draw_counter, int* __restrict__ turn,
                                       int* __restrict__ host_ring, int host_slots, int* __restrict__ log_ring,
                                       int log_slots) {
-    let_next_kernel_start();
     wait_for_previous_kernels();          // every kernel of the step has read the arrays; the sampler has written the tokens
     const int t = turn ? *turn : 0;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -1267,6 +1267,8 @@ __global__ void advance_decode_kernel(int* __restrict__ token_pos, int* __restri
     if (host_ring) __threadfence_system();
     __syncthreads();                      // everyone has read *turn
     if (threadIdx.x == 0 && turn) *turn = t + 1;
+    __threadfence();
+    let_next_kernel_start();
 }
 
 RI_API int ri_advance_decode(int* token_pos, int* seq_start, int* seq_len, int n, const int* token_ids,

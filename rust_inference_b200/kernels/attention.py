@@ -224,6 +224,42 @@ def attention(qkv, cache_layer, out, ctx, *, n_heads, n_kv_heads, head_dim, scal
         gate=gate)
 
 
+class FormedHeads:
+    """A decode step's attention that forms the new position's heads itself from the float32 sums of their projection, instead of
+    behind a kernel that does (`attention_tc.decode_form`): made by `formed_heads`, run by the position encoding, which brings the
+    sums, the angles and the cache."""
+
+    def __init__(self, ctx, out, n_splits, sizes, scale, span, out_scale, rot_dims, norm=(None, None, 0.0), values_from_keys=False):
+        self.ctx, self.out, self.n_splits, self.sizes, self.scale, self.span = ctx, out, n_splits, sizes, scale, span
+        self.out_scale, self.rot_dims, self.norm, self.values_from_keys = out_scale, rot_dims, norm, values_from_keys
+
+    def run(self, acc, bias, cos, sin, kcache, vcache, *, style: int):
+        from . import attention_tc
+        ctx, (n_heads, n_kv_heads, head_dim) = self.ctx, self.sizes
+        q_weight, k_weight, eps = self.norm
+        return attention_tc.decode_form(
+            acc, bias, cos, sin, q_weight, k_weight, eps, kcache, vcache, ctx.page_table, ctx.seq_slot, ctx.seq_len, ctx.cu_seqlens,
+            self.out, n_seqs=ctx.n_seqs, n_heads=n_heads, n_kv_heads=n_kv_heads, head_dim=head_dim, page_size=ctx.page_size,
+            scale=self.scale, window=self.span, n_splits=self.n_splits, style=style, rot_dims=self.rot_dims,
+            values_from_keys=self.values_from_keys, out_scale=self.out_scale)
+
+
+def formed_heads(out, ctx, width, *, n_heads, n_kv_heads, head_dim, rot_dims, scale, window=0, chunk=0, out_scale=1.0,
+                 norm=(None, None, 0.0), values_from_keys=False):
+    """What runs a decode step's attention straight from its projection's sums (rows of `width` floats), or None where the kernel that
+    does so takes no such step: bfloat16 steps of one token per sequence whose runs of pages meet in a cluster (or that have one
+    run), plain scores, heads of 64 or 128."""
+    if not ctx.all_single or ctx.dtype != torch.bfloat16 or (window and chunk) or rot_dims <= 0 or rot_dims % 8 or width % 8:
+        return None
+    if not ops.attention_mma_supports(head_dim, ctx.page_size, n_heads, n_kv_heads, True):
+        return None
+    name, splits = decode_plan(ctx.n_seqs, n_kv_heads, ctx.page_table.shape[1] * ctx.page_size, ctx.page_size, head_dim)
+    if not (name == "cluster" or (name == "tma" and splits == 1)):
+        return None
+    return FormedHeads(ctx, out, splits, (n_heads, n_kv_heads, head_dim), scale, window if window else -int(chunk or 0), out_scale,
+                       rot_dims, norm, values_from_keys)
+
+
 def _own_value_size(qkv, cache_layer, out, ctx, *, n_heads, n_kv_heads, head_dim, v_head_dim, scale, span, out_scale):
     """`attention` on the tensor cores for values of another head size than the keys'; None where no kernel takes the sizes."""
     from . import attention_tc

@@ -162,6 +162,37 @@ def decode_cluster(q: torch.Tensor, q_ld: int, kcache: torch.Tensor, vcache: tor
     return out
 
 
+def decode_form(acc: torch.Tensor, bias, cos, sin, q_weight, k_weight, eps: float, kcache: torch.Tensor, vcache: torch.Tensor, page_table,
+                seq_slot, seq_len, cu_seqlens, out: torch.Tensor, *, n_seqs: int, n_heads: int, n_kv_heads: int, head_dim: int,
+                page_size: int, scale: float, window: int, n_splits: int, style: int, rot_dims: int, values_from_keys: bool = False,
+                out_scale: float = 1.0) -> torch.Tensor:
+    """`decode` (n_splits 1) and `decode_cluster` (2..8) from the float32 sums of a projection, acc [n_seqs, ld] = [q heads | k heads |
+    v heads] without their bias: the kernel adds it, norms the q and k heads (q_weight, k_weight; None: not), turns their first
+    rot_dims channels by their position's angles, puts the position's key and value into the cache, attends, and leaves acc zeroed.
+    values_from_keys: no v columns, a value is the key as projected.  The result is times out_scale."""
+    _need_cuda(acc, bias, cos, sin, q_weight, k_weight, kcache, vcache, page_table, seq_slot, seq_len, cu_seqlens, out)
+    _need(acc.dtype == torch.float32 and acc.is_contiguous() and acc.shape[0] == n_seqs
+          and acc.shape[1] >= (n_heads + (1 if values_from_keys else 2) * n_kv_heads) * head_dim, "attention_decode: accumulator shape")
+    _need(bias is None or (bias.dtype == torch.float32 and bias.is_contiguous() and bias.numel() == acc.shape[1]), "attention_decode: bias")
+    _need(kcache.dtype == torch.bfloat16 and vcache.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and kcache.is_contiguous()
+          and vcache.is_contiguous() and kcache.shape == vcache.shape and tuple(kcache.shape[1:]) == (n_kv_heads, page_size, head_dim)
+          and out.shape[1] >= n_heads * head_dim, "attention_decode: bf16 contiguous cache and result")
+    _need(cos.dtype == torch.float32 and sin.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
+          and cos.shape[1] == rot_dims // 2 and sin.shape == cos.shape, "attention_decode: angle tables")
+    for w in (q_weight, k_weight):
+        _need(w is None or (w.dtype == torch.float32 and w.is_contiguous() and w.numel() == head_dim), "attention_decode: head norms")
+    rows = kcache.shape[0] * kcache.shape[1] * kcache.shape[2]
+    mk = _map(1, kcache, rows, head_dim, head_dim)
+    mv = _map(1, vcache, rows, head_dim, head_dim)
+    st = status_word()
+    _call("attention_mma", "ri_attention_decode_tma_form", c_void_p(mk.data_ptr()), c_void_p(mv.data_ptr()), _p(acc), c_int(acc.shape[1]),
+          _p(bias), _p(cos), _p(sin), _p(q_weight), _p(k_weight), c_float(eps), c_int(style), c_int(rot_dims),
+          c_int(1 if values_from_keys else 0), _p(kcache), _p(vcache), _p(page_table), c_int(page_table.shape[1]), _p(seq_slot),
+          _p(seq_len), _p(cu_seqlens), _p(out), c_int(out.shape[1]), c_int(n_seqs), c_int(n_heads), c_int(n_kv_heads), c_int(head_dim),
+          c_int(page_size), c_float(scale), c_int(window), c_int(n_splits), c_float(out_scale), c_void_p(st.data_ptr()), _stream())
+    return out
+
+
 _capacity: dict = {}
 
 

@@ -355,9 +355,14 @@ def rope_cache_write(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, to
 
 def rope_cache_write_acc(acc: torch.Tensor, bias, q_out: torch.Tensor, cos, sin, token_pos, token_seq, seq_slot,
                          page_table, kcache, vcache, *, n_heads: int, n_kv_heads: int, head_dim: int,
-                         page_size: int, style: int, write_kv: bool) -> None:
+                         page_size: int, style: int, write_kv: bool, attend=None) -> None:
     """The rotary + cache-write kernel fed from float32 accumulators acc[T, (heads + 2 kv heads) * head_dim]
-    (+ bias): q goes to q_out[T, heads * head_dim], k and v to the cache, and `acc` is zeroed again."""
+    (+ bias): q goes to q_out[T, heads * head_dim], k and v to the cache, and `acc` is zeroed again.
+    `attend` (`attention.FormedHeads`, a decode step): the decode attention does all of that itself; q_out is None then."""
+    if attend is not None:
+        _need(q_out is None and write_kv, "rope_cache_write_acc: the attention keeps the queries and writes the cache")
+        attend.run(acc, bias, cos, sin, kcache, vcache, style=style)
+        return
     _need_cuda(acc, bias, q_out, cos, sin, token_pos, token_seq, seq_slot, page_table, kcache, vcache)
     n = acc.shape[0]
     _need(acc.dtype == torch.float32 and acc.is_contiguous()

@@ -284,6 +284,8 @@ class GQAttention(Mixer):
         special = self.values_from_keys or self.qk_norm_eps is not None or self.value_mix is not None
         usual = (self.v_head_dim == self.head_dim and not getattr(self.position, "partial", False) and not special
                  and not self.extended)
+        if self._formed_in_attention(x, width, residual, ctx, cache_layer, writes_cache):
+            return
         from_acc = getattr(self.position, "apply_and_store_from_accumulators", None) if usual else None
         if from_acc is not None and linear.wants_split(x, self.w_qkv):
             # a small step: the projection is split over K into float32 accumulators, and the
@@ -325,6 +327,28 @@ class GQAttention(Mixer):
                                               write_kv=writes_cache and self.own_kv, **extra)
         self._attend(qkv, gate_col, residual, ctx, cache_layer)
 
+    def _formed_in_attention(self, x, width, residual, ctx, cache_layer, writes_cache) -> bool:
+        """A decode step whose projection is split over K: the attention's own kernel adds the bias to the sums, norms and turns the
+        heads and writes the cache.  False (nothing done) where it does not take the step."""
+        if (not ctx.all_single or self.extended or self.value_mix is not None or not writes_cache or self.v_head_dim != self.head_dim
+                or not hasattr(self.position, "apply_and_store_from_accumulators") or not linear.wants_split(x, self.w_qkv)):
+            return False
+        mixed = ctx.buffer("attn_out", (x.shape[0], self.o_dim), self.dtype)
+        attend = attn_kernels.formed_heads(
+            mixed, ctx, width, n_heads=self.n_heads, n_kv_heads=self.n_kv_heads, head_dim=self.head_dim,
+            rot_dims=self.position.rot_dims, scale=self.scale, window=self.window or 0, chunk=self.chunk or 0,
+            out_scale=self.out_scale, values_from_keys=self.values_from_keys,
+            norm=(None, None, 0.0) if self.qk_norm_eps is None else (self.q_norm, self.k_norm, self.qk_norm_eps))
+        if attend is None:
+            return False
+        acc = ctx.zeroed_buffer("qkv_acc", (x.shape[0], width), torch.float32)
+        linear.accumulate_split(x, self.w_qkv, acc, ctx)
+        self.position.apply_and_store_from_accumulators(
+            acc, self.b_qkv, None, ctx, cache_layer, n_heads=self.n_heads, n_kv_heads=self.n_kv_heads, head_dim=self.head_dim,
+            write_kv=True, attend=attend)
+        self._project_out(mixed, residual, ctx)
+        return True
+
     def _blend(self, ctx, n, own):
         """What the values are blended with, (lambda, rows, column), or None.  `own`: rows and column of the layer's own projected
         values, which later layers of the step read if this one is the first."""
@@ -349,6 +373,9 @@ class GQAttention(Mixer):
         if self.out_gate:
             # the gates of the projection's last columns, the mixer's factor with them (float32, one rounding)
             ops.sigmoid_gate_(mixed, qkv, gate_col, self.out_scale)
+        self._project_out(mixed, residual, ctx)
+
+    def _project_out(self, mixed, residual, ctx):
         linear.into_residual(mixed, self.w_o, residual, ctx)
         if self.o_bias and not self.hands_over_bias:
             ops.add_row_bias(residual, self.b_o_scaled)
