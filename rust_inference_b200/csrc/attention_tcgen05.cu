@@ -70,12 +70,13 @@ __device__ __forceinline__ uint64_t make_smem_desc_mn(uint32_t addr, uint32_t at
 
 // D[tmem] (+)= A[tmem] * B[smem]: the A operand (128 rows x 16 bf16, two to a 32-bit column, 8 columns) comes from
 // tensor memory, where the softmax threads put the probabilities.
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t idesc, bool accumulate) {
+__device__ __forceinline__ void umma_ts(uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t idesc, bool accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate), "r"(leader)
         : "memory");
 }
 
@@ -256,12 +257,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            bool ok = mbar_wait(smem_u32(&q_full), 0);
-            if (!ok) { report(status, ST_ATTN_MMA); abort_flag = 1; }
-            // One thread issues every MMA, and a lone thread gets a dependent instruction out only every few
-            // cycles: the descriptors are built once, and a page's MMAs add constants to their address field
-            // (shared memory ends below 256 KiB, so the 14-bit field never carries).
+        {                                                        // the whole warp goes through, one lane issues
+            const uint32_t leader = elect_one();
+            bool ok = mbar_wait_warp(smem_u32(&q_full), 0);
+            if (!ok) { if (lane == 0) report(status, ST_ATTN_MMA); abort_flag = 1; }
+            // The descriptors are built once, and a page's MMAs add constants to their address field (shared memory
+            // ends below 256 KiB, so the 14-bit field never carries).
             const uint64_t q_desc = make_smem_desc(q_smem), k_desc = make_smem_desc(k_smem);
             const uint64_t v_desc = make_smem_desc_mn(v_smem, BN * 128);
             const uint32_t k_full0 = smem_u32(&k_full[0]), k_empty0 = smem_u32(&k_empty[0]), s_full0 = smem_u32(&s_full[0]);
@@ -270,40 +271,40 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             // scores of page j go to buffer j & 1, so S(j+1) is computed while the softmax of page j runs
             auto issue_s = [&](int j) -> bool {
                 const uint32_t kb = (uint32_t)j & 1u;
-                if (!mbar_wait(k_full0 + 8u * kb, (uint32_t)((j >> 1) & 1))) return false;
+                if (!mbar_wait_warp(k_full0 + 8u * kb, (uint32_t)((j >> 1) & 1))) return false;
                 tc_fence_after();
                 const uint64_t kd = k_desc + (uint64_t)(kb * (uint32_t)(K_BYTES >> 4));
                 const uint32_t s_acc = tmem_base + S_COL + kb * BN;
 #pragma unroll
                 for (int ks = 0; ks < HD / 16; ++ks)
-                    umma(s_acc, q_desc + (uint64_t)(((ks / 4) * BM * 128 + (ks % 4) * 32) >> 4),
-                         kd + (uint64_t)(((ks / 4) * BN * 128 + (ks % 4) * 32) >> 4), IDESC_S, ks > 0);
-                umma_commit(k_empty0 + 8u * kb);
-                umma_commit(s_full0 + 8u * kb);
+                    umma_by(leader, s_acc, q_desc + (uint64_t)(((ks / 4) * BM * 128 + (ks % 4) * 32) >> 4),
+                            kd + (uint64_t)(((ks / 4) * BN * 128 + (ks % 4) * 32) >> 4), IDESC_S, ks > 0);
+                umma_commit_by(leader, k_empty0 + 8u * kb);
+                umma_commit_by(leader, s_full0 + 8u * kb);
                 return true;
             };
-            if (ok && !issue_s(0)) { report(status, ST_ATTN_MMA); abort_flag = 1; ok = false; }
+            if (ok && !issue_s(0)) { if (lane == 0) report(status, ST_ATTN_MMA); abort_flag = 1; ok = false; }
             for (int j = 0; j < n_pages && ok; ++j) {
                 // the buffer S(j+1) goes to was read by the softmax of page j-1, which arrived on p_full before PV(j-1)
-                if (j + 1 < n_pages && !issue_s(j + 1)) { report(status, ST_ATTN_MMA); abort_flag = 1; break; }
+                if (j + 1 < n_pages && !issue_s(j + 1)) { if (lane == 0) report(status, ST_ATTN_MMA); abort_flag = 1; break; }
                 const uint32_t pb = (uint32_t)j & 1u, vb = (uint32_t)(j % V_BUFS);
-                if (!mbar_wait(p_full_a, pb) || !mbar_wait(v_full0 + 8u * vb, (uint32_t)((j / V_BUFS) & 1))) {
-                    report(status, ST_ATTN_MMA); abort_flag = 1; break;
+                if (!mbar_wait_warp(p_full_a, pb) || !mbar_wait_warp(v_full0 + 8u * vb, (uint32_t)((j / V_BUFS) & 1))) {
+                    if (lane == 0) report(status, ST_ATTN_MMA); abort_flag = 1; break;
                 }
                 tc_fence_after();
                 const uint64_t vd = v_desc + (uint64_t)(vb * (uint32_t)(V_BYTES >> 4));
 #pragma unroll
                 for (int ks = 0; ks < BN / 16; ++ks)
                     // P of page j lies, two bf16 to a column, over the first half of the score buffer it came from
-                    umma_ts(tmem_base + O_COL, tmem_base + S_COL + pb * BN + ks * 8, vd + (uint64_t)(ks * 16 * 128 >> 4),
+                    umma_ts(leader, tmem_base + O_COL, tmem_base + S_COL + pb * BN + ks * 8, vd + (uint64_t)(ks * 16 * 128 >> 4),
                             IDESC_PV, j > 0 || ks > 0);
                 if constexpr (LATENT == 2)
 #pragma unroll
                     for (int ks = 0; ks < BN / 16; ++ks)
-                        umma_ts(tmem_base + O_COL, tmem_base + S_COL + pb * BN + ks * 8,
+                        umma_ts(leader, tmem_base + O_COL, tmem_base + S_COL + pb * BN + ks * 8,
                                 vd + (uint64_t)(V_TERM >> 4) + (uint64_t)(ks * 16 * 128 >> 4), IDESC_PV, true);
-                umma_commit(v_empty0 + 8u * vb);
-                umma_commit(pv_done_a);
+                umma_commit_by(leader, v_empty0 + 8u * vb);
+                umma_commit_by(leader, pv_done_a);
             }
         }
     } else {

@@ -25,42 +25,14 @@
 // Epilogues as in `gemm_simt.cu` (0 and 1 are the same here: float32 with a bias): 2 out += acc, 3 gated, 4 an activation,
 // 5 silu for the first columns.
 #include "cluster.cuh"
+#include "gemm_f32_common.cuh"
 #include "tcgen05_common.cuh"
 
 using namespace ri;
+using namespace ri::f32;
 using namespace ri::tc;
 
 namespace {
-
-// weights: read once, kept out of L1 (a load that may stand before the wait for the kernel before)
-__device__ __forceinline__ float4 load_weight(const float* p) {
-    float4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
-    return v;
-}
-
-struct Forms {          // the epilogue's constants, loaded once per thread
-    GateForm gate;
-    ActForm act;
-    int silu_feats;
-};
-template <int MODE>
-__device__ __forceinline__ Forms load_forms(const float* bias) {
-    Forms f;
-    f.gate = load_gate_form(MODE == 3 ? bias : nullptr);
-    f.act = MODE == 4 ? load_act_form(bias) : ActForm{0.f, 0.f, 0.f};
-    f.silu_feats = MODE == 5 ? (int)bias[0] : 0;
-    return f;
-}
-template <int MODE>
-__device__ __forceinline__ void finish(float* out, size_t o, int f, float v, float up, const float* __restrict__ bias,
-                                       const Forms& forms) {
-    if (MODE == 1) out[o] = bias != nullptr ? v + bias[f] : v;
-    else if (MODE == 2) out[o] += v;
-    else if (MODE == 3) out[o] = gated_f32(v, up, forms.gate);
-    else if (MODE == 4) out[o] = act_f32(v, forms.act);
-    else out[o] = f < forms.silu_feats ? silu_f32(v) : v;
-}
 
 // ---------------------------------------------------------------------------------------------------------------------
 // Few rows of X.
@@ -256,37 +228,6 @@ constexpr int CUT_WARPS = 8, CUT_THREADS = CUT_WARPS * 32, ADD_WARPS = 8;
 constexpr int SPLIT_THREADS = CUT_THREADS + ADD_WARPS * 32;
 enum Status { ST_CUT_TIMEOUT = 41, ST_MMA_TIMEOUT = 42, ST_ADD_TIMEOUT = 43 };
 
-// x * 2^16 as three bfloat16 numbers that add up to it exactly, each the upper half of a float32: the leading 8 significant
-// bits, the next 8 and the rest.  The factor keeps the parts of every float32 number, the denormal ones too, among the numbers
-// bfloat16 has (without it numbers below 2^-110 lose bits); the sums are divided by both operands' factors at the end.  From
-// 2^112 on the parts become infinite or NaN, as those of an infinity or a NaN are.
-constexpr float UP = 65536.f, DOWN = 1.f / (UP * UP);
-__device__ __forceinline__ float2 two(float v) { return make_float2(v, v); }
-__device__ __forceinline__ float2 leading(const float2& v) {
-    return make_float2(__uint_as_float(__float_as_uint(v.x) & 0xffff0000u), __uint_as_float(__float_as_uint(v.y) & 0xffff0000u));
-}
-__device__ __forceinline__ uint32_t upper_halves(const float2& v) { return __byte_perm(__float_as_uint(v.x), __float_as_uint(v.y), 0x7632); }
-__device__ __forceinline__ void cut(float2 v, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-    v = __fmul2_rn(v, two(UP));
-    hi = upper_halves(v);
-    v = __ffma2_rn(leading(v), two(-1.f), v);
-    mid = upper_halves(v);
-    v = __ffma2_rn(leading(v), two(-1.f), v);
-    lo = upper_halves(v);
-}
-__device__ __forceinline__ void store8(uint32_t addr, uint32_t a, uint32_t b) {
-    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
-}
-// four consecutive k of one row into the three parts
-__device__ __forceinline__ void put(uint32_t addr, uint32_t part_bytes, const float4& v) {
-    uint32_t h[2], m[2], l[2];
-    cut(make_float2(v.x, v.y), h[0], m[0], l[0]);
-    cut(make_float2(v.z, v.w), h[1], m[1], l[1]);
-    store8(addr, h[0], h[1]);
-    store8(addr + part_bytes, m[0], m[1]);
-    store8(addr + 2 * part_bytes, l[0], l[1]);
-}
-
 template <int TN, int MODE>
 __global__ void __launch_bounds__(SPLIT_THREADS, 1)
 gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* __restrict__ W2,
@@ -404,11 +345,12 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
         const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(part * COLS);
         const uint64_t a_desc = make_smem_desc(base), b_desc = make_smem_desc(base + 3 * PART);
         int issued = 0;
-        auto issue = [&](int b) {                                // one lane
+        const uint32_t leader = elect_one();
+        auto issue = [&](int b) {                                // the whole warp goes through, one lane issues
             const int s = b % STAGES, buf = b & 1;
-            if (!(mbar_wait(smem_u32(&acc_empty[buf]), (uint32_t)((b >> 1) & 1) ^ 1u) &&
-                  mbar_wait(smem_u32(&full_bar[s]), (uint32_t)((b / STAGES) & 1)))) {
-                report(status, ST_MMA_TIMEOUT);
+            if (!(mbar_wait_warp(smem_u32(&acc_empty[buf]), (uint32_t)((b >> 1) & 1) ^ 1u) &&
+                  mbar_wait_warp(smem_u32(&full_bar[s]), (uint32_t)((b / STAGES) & 1)))) {
+                if (lane == 0) report(status, ST_MMA_TIMEOUT);
                 abort_flag = 1;
                 return;
             }
@@ -422,15 +364,15 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
                 const bool large = p == PRODUCTS - 1;
 #pragma unroll
                 for (int k = 0; k < BK / 16; ++k)
-                    umma(large ? acc : acc + TN, a_desc + off + (uint64_t)(PA[p] * (PART >> 4) + 2 * k),
-                         b_desc + off + (uint64_t)(PB[p] * (X_PART >> 4) + 2 * k), IDESC, (p > 0 && !large) || k > 0);
+                    umma_by(leader, large ? acc : acc + TN, a_desc + off + (uint64_t)(PA[p] * (PART >> 4) + 2 * k),
+                            b_desc + off + (uint64_t)(PB[p] * (X_PART >> 4) + 2 * k), IDESC, (p > 0 && !large) || k > 0);
             }
-            umma_commit(smem_u32(&empty_bar[s]));
-            umma_commit(smem_u32(&acc_full[buf]));
+            umma_commit_by(leader, smem_u32(&empty_bar[s]));
+            umma_commit_by(leader, smem_u32(&acc_full[buf]));
             issued = b + 1;
         };
-        if (warp == CUT_WARPS && lane == 0)
-            for (int b = 0; b < 2 && b < n_kb && !abort_flag; ++b) issue(b);
+        if (warp == CUT_WARPS)
+            for (int b = 0; b < 2 && b < n_kb && !__any_sync(0xffffffffu, abort_flag); ++b) issue(b);
         __syncwarp();
         float acc[COLS];
 #pragma unroll
@@ -442,8 +384,7 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
                 if (!abort_flag) report(status, ST_ADD_TIMEOUT);
                 abort_flag = 1;
             }
-            __syncwarp();
-            if (abort_flag) {
+            if (__any_sync(0xffffffffu, abort_flag)) {
                 // the MMAs on their way have to finish before tensor memory is given back
                 if (warp == CUT_WARPS && lane == 0)
                     for (int i = max(0, issued - 2); i < issued; ++i) mbar_wait(smem_u32(&acc_full[i & 1]), (uint32_t)((i >> 1) & 1));
@@ -461,10 +402,8 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(smem_u32(&acc_empty[buf]));
-                if (warp == CUT_WARPS && b + 2 < n_kb) issue(b + 2);
-            }
+            if (lane == 0) mbar_arrive(smem_u32(&acc_empty[buf]));
+            if (warp == CUT_WARPS && b + 2 < n_kb) issue(b + 2);
             __syncwarp();
         }
         // the last MMAs have finished: nothing reads the stages any more

@@ -253,7 +253,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        {                                                        // the whole warp goes through, one lane issues
+            const uint32_t leader = elect_one();
             int s = 0;
             uint32_t ph = 0;
             bool alive = true;
@@ -266,16 +267,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 tile_coords(i, f0, t0, kb_begin, n_kb);
                 const int buf = i & 1;
                 // the epilogue must have emptied this accumulator buffer (two tiles ago)
-                if (!mbar_wait(smem_u32(&acc_empty[buf]), (uint32_t)((i >> 1) & 1) ^ 1u)) {
-                    report(status, ST_MMA_TIMEOUT);
+                if (!mbar_wait_warp(smem_u32(&acc_empty[buf]), (uint32_t)((i >> 1) & 1) ^ 1u)) {
+                    if (lane == 0) report(status, ST_MMA_TIMEOUT);
                     abort_flag = 1;
                     break;
                 }
                 tc_fence_after();
                 const uint32_t acc = tmem_base + (uint32_t)(buf * ACC_COLS);
                 for (int kb = 0; kb < n_kb; ++kb) {
-                    if (!mbar_wait(full0 + 8u * s, ph)) {
-                        report(status, ST_MMA_TIMEOUT);
+                    if (!mbar_wait_warp(full0 + 8u * s, ph)) {
+                        if (lane == 0) report(status, ST_MMA_TIMEOUT);
                         abort_flag = 1;
                         alive = false;
                         break;
@@ -286,13 +287,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 #pragma unroll
                     for (int k = 0; k < BLOCK_K / 16; ++k) {
                         // 16 bf16 = 32 bytes further along K inside the swizzled row: 2 in the address field
-                        umma(acc, a0 + 2 * k, b0 + 2 * k, IDESC, kb > 0 || k > 0);
-                        if (DUAL) umma(acc + TN, a0 + (A_BYTES >> 4) + 2 * k, b0 + 2 * k, IDESC, kb > 0 || k > 0);
+                        umma_by(leader, acc, a0 + 2 * k, b0 + 2 * k, IDESC, kb > 0 || k > 0);
+                        if (DUAL) umma_by(leader, acc + TN, a0 + (A_BYTES >> 4) + 2 * k, b0 + 2 * k, IDESC, kb > 0 || k > 0);
                     }
-                    umma_commit(empty0 + 8u * s);              // frees the stage once these MMAs have read it
+                    umma_commit_by(leader, empty0 + 8u * s);              // frees the stage once these MMAs have read it
                     if (++s == stages) { s = 0; ph ^= 1u; }
                 }
-                umma_commit(smem_u32(&acc_full[buf]));         // accumulator complete (or aborted: flag says which)
+                umma_commit_by(leader, smem_u32(&acc_full[buf]));         // accumulator complete (or aborted: flag says which)
             }
         }
     } else {
@@ -601,23 +602,24 @@ gemm_tm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {                                                        // the whole warp goes through, one lane issues
+            const uint32_t leader = elect_one();
             int s = 0;
             uint32_t ph = 0;
             bool alive = true;
             const uint64_t desc_x0 = make_smem_desc(smem_base), desc_w0 = make_smem_desc(smem_base + X_BYTES);
             for (int i = 0; i < my_tiles && alive; ++i) {
                 const int buf = i & 1;
-                if (!mbar_wait(smem_u32(&acc_empty[buf]), ((uint32_t)(i >> 1) & 1u) ^ 1u)) {
-                    report(status, ST_MMA_TIMEOUT);
+                if (!mbar_wait_warp(smem_u32(&acc_empty[buf]), ((uint32_t)(i >> 1) & 1u) ^ 1u)) {
+                    if (lane == 0) report(status, ST_MMA_TIMEOUT);
                     abort_flag = 1;
                     break;
                 }
                 tc_fence_after();
                 const uint32_t acc = tmem_base + (uint32_t)(buf * TM_ROWS);
                 for (int kb = 0; kb < n_kb; ++kb) {
-                    if (!mbar_wait(full0 + 8u * s, ph)) {
-                        report(status, ST_MMA_TIMEOUT);
+                    if (!mbar_wait_warp(full0 + 8u * s, ph)) {
+                        if (lane == 0) report(status, ST_MMA_TIMEOUT);
                         abort_flag = 1;
                         alive = false;
                         break;
@@ -626,11 +628,11 @@ gemm_tm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                     const uint64_t off = (uint64_t)((uint32_t)s * (uint32_t)(TM_STAGE_BYTES >> 4));
 #pragma unroll
                     for (int k = 0; k < BLOCK_K / 16; ++k)
-                        umma(acc, desc_x0 + off + 2 * k, desc_w0 + off + 2 * k, IDESC, kb > 0 || k > 0);
-                    umma_commit(empty0 + 8u * s);
+                        umma_by(leader, acc, desc_x0 + off + 2 * k, desc_w0 + off + 2 * k, IDESC, kb > 0 || k > 0);
+                    umma_commit_by(leader, empty0 + 8u * s);
                     if (++s == stages) { s = 0; ph ^= 1u; }
                 }
-                umma_commit(smem_u32(&acc_full[buf]));
+                umma_commit_by(leader, smem_u32(&acc_full[buf]));
             }
         }
     } else {
@@ -699,18 +701,22 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
         ::"r"(dst), "l"(map), "r"(cluster_bar), "r"(x), "r"(y)
         : "memory");
 }
-__device__ __forceinline__ void umma_pair(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate) {
+__device__ __forceinline__ void umma_pair(uint32_t leader, uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate), "r"(leader)
         : "memory");
 }
 // Arrives at the barrier at this address in both CTAs of the pair once the MMAs issued so far are done.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(bar), "h"((uint16_t)3) : "memory");
+__device__ __forceinline__ void umma_commit_pair(uint32_t leader, uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %2, 0;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+        ::"r"(bar), "h"((uint16_t)3), "r"(leader) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
@@ -821,7 +827,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer (first CTA) ----------------
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {                                         // the whole warp goes through, one lane issues
+            const uint32_t leader = elect_one();
             int s = 0;
             uint32_t ph = 0;
             bool alive = true;
@@ -830,16 +837,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                 int f0, t0, kb_begin, kb_end;
                 tile_coords(i, f0, t0, kb_begin, kb_end);
                 const int buf = i & 1;
-                if (!mbar_wait(smem_u32(&acc_empty[buf]), ((uint32_t)(i >> 1) & 1u) ^ 1u)) {
-                    report(status, ST_MMA_TIMEOUT);
+                if (!mbar_wait_warp(smem_u32(&acc_empty[buf]), ((uint32_t)(i >> 1) & 1u) ^ 1u)) {
+                    if (lane == 0) report(status, ST_MMA_TIMEOUT);
                     abort_flag = 1;
                     break;
                 }
                 tc_fence_after();
                 const uint32_t acc = tmem_base + (uint32_t)(buf * TM_ROWS);
                 for (int kb = kb_begin; kb < kb_end; ++kb) {
-                    if (!mbar_wait(full0 + 8u * s, ph)) {
-                        report(status, ST_MMA_TIMEOUT);
+                    if (!mbar_wait_warp(full0 + 8u * s, ph)) {
+                        if (lane == 0) report(status, ST_MMA_TIMEOUT);
                         abort_flag = 1;
                         alive = false;
                         break;
@@ -848,11 +855,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                     const uint64_t off = (uint64_t)((uint32_t)s * (uint32_t)(PAIR_STAGE_BYTES >> 4));
 #pragma unroll
                     for (int k = 0; k < BLOCK_K / 16; ++k)
-                        umma_pair(acc, desc_x0 + off + 2 * k, desc_w0 + off + 2 * k, IDESC, kb > kb_begin || k > 0);
-                    umma_commit_pair(empty0 + 8u * s);           // frees the stage in both CTAs
+                        umma_pair(leader, acc, desc_x0 + off + 2 * k, desc_w0 + off + 2 * k, IDESC, kb > kb_begin || k > 0);
+                    umma_commit_pair(leader, empty0 + 8u * s);           // frees the stage in both CTAs
                     if (++s == stages) { s = 0; ph ^= 1u; }
                 }
-                umma_commit_pair(smem_u32(&acc_full[buf]));
+                umma_commit_pair(leader, smem_u32(&acc_full[buf]));
             }
         }
     } else {

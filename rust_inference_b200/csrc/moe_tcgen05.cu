@@ -200,23 +200,24 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {                                                        // the whole warp goes through, one lane issues
+            const uint32_t leader = elect_one();
             int s = 0;
             uint32_t ph = 0;
             bool alive = true;
             const uint64_t desc_x0 = make_smem_desc(smem_base), desc_w0 = make_smem_desc(smem_base + X_BYTES);
             for (int i = 0; i < my_tiles && alive; ++i) {
                 const int buf = i & 1;
-                if (!mbar_wait(smem_u32(&acc_empty[buf]), ((uint32_t)(i >> 1) & 1u) ^ 1u)) {
-                    report(status, ST_MMA_TIMEOUT);
+                if (!mbar_wait_warp(smem_u32(&acc_empty[buf]), ((uint32_t)(i >> 1) & 1u) ^ 1u)) {
+                    if (lane == 0) report(status, ST_MMA_TIMEOUT);
                     abort_flag = 1;
                     break;
                 }
                 tc_fence_after();
                 const uint32_t acc = tmem_base + (uint32_t)(buf * TM_ROWS);
                 for (int kb = 0; kb < n_kb; ++kb) {
-                    if (!mbar_wait(full0 + 8u * s, ph)) {
-                        report(status, ST_MMA_TIMEOUT);
+                    if (!mbar_wait_warp(full0 + 8u * s, ph)) {
+                        if (lane == 0) report(status, ST_MMA_TIMEOUT);
                         abort_flag = 1;
                         alive = false;
                         break;
@@ -225,11 +226,11 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                     const uint64_t off = (uint64_t)((uint32_t)s * (uint32_t)(STAGE_BYTES >> 4));
 #pragma unroll
                     for (int k = 0; k < BLOCK_K / 16; ++k)
-                        umma(acc, desc_x0 + off + 2 * k, desc_w0 + off + 2 * k, IDESC, kb > 0 || k > 0);
-                    umma_commit(empty0 + 8u * s);
+                        umma_by(leader, acc, desc_x0 + off + 2 * k, desc_w0 + off + 2 * k, IDESC, kb > 0 || k > 0);
+                    umma_commit_by(leader, empty0 + 8u * s);
                     if (++s == stages) { s = 0; ph ^= 1u; }
                 }
-                umma_commit(smem_u32(&acc_full[buf]));
+                umma_commit_by(leader, smem_u32(&acc_full[buf]));
             }
         }
     } else {
