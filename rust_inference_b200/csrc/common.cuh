@@ -148,14 +148,11 @@ __device__ __forceinline__ float act_quick_f32(float z, const ActForm& f) {
     return fmaf(f.an, t, f.lin * z);
 }
 
-// The reference's SiLU, stable on both sides (math.rs:137-146).
+// The reference's SiLU, stable on both sides (math.rs:137-146): x / (1 + e^-x) from 0 on, x e^x / (1 + e^x) below.  Both sides through
+// the same instructions, so that a warp whose lanes lie on both goes through them once.
 __device__ __forceinline__ float silu_f32(float x) {
-    if (x >= 0.f) {
-        return x / (1.f + expf(-x));
-    } else {
-        float e = expf(x);
-        return x * e / (1.f + e);
-    }
+    const float e = expf(-fabsf(x));
+    return (x >= 0.f ? x : x * e) / (1.f + e);
 }
 
 // The gated activation with accurate exponentials (the 32-bit path); alpha 1 without limit and shift is silu_f32(g) * u.
@@ -163,8 +160,8 @@ __device__ __forceinline__ float gated_f32(float g, float u, const GateForm& f) 
     g = fminf(g, f.limit);
     u = fmaxf(fminf(u, f.limit), -f.limit) + f.shift;
     if (f.alpha == 1.f && f.cubic == 0.f) return silu_f32(g) * u * f.mult;
-    const float z = f.alpha * g * fmaf(f.cubic * g, g, 1.f);
-    const float sig = z >= 0.f ? 1.f / (1.f + expf(-z)) : expf(z) / (1.f + expf(z));
+    const float z = f.alpha * g * fmaf(f.cubic * g, g, 1.f), e = expf(-fabsf(z));
+    const float sig = (z >= 0.f ? 1.f : e) / (1.f + e);
     return g * sig * u * f.mult;
 }
 

@@ -7,7 +7,7 @@
 // rows to keep the memory busy; the pieces meet through distributed shared memory in a fixed order, so a product's bits do
 // not change from run to run.
 //
-// More rows: the tensor cores, without giving up 32 bits.  A float32 number is the exact sum of three bfloat16 numbers
+// More rows (up to 64; beyond, `gemm_f32_wide.cu`): the tensor cores, without giving up 32 bits.  A float32 number is the exact sum of three bfloat16 numbers
 // (its leading 8 significant bits, the next 8 and the last 8), so x * w is the sum of nine products of bfloat16 numbers,
 // each exact in the tensor core.  The last one (low * low) is below 2^-30 of the whole and is left out; the other eight are added.
 // Eight warps read both operands, cut them and put the parts into shared memory as the MMA wants them (128-byte swizzle); eight
@@ -213,15 +213,12 @@ int launch_few(const float* X, const float* W, const float* W2, const float* bia
 // ---------------------------------------------------------------------------------------------------------------------
 // Many rows of X: three bfloat16 parts per operand on the tensor cores.
 //
-// A tile is 128 rows of W (gated: 64 gate rows and the 64 up rows of the same features) by TN rows of X.  What bounds a
-// block of 64 steps of K is shared memory (32 MMAs that read 4 KiB of W and TN * 32 bytes of X each, and the parts' writes: at
-// TN = 128 about 2,800 clocks against 2,048 of the tensor core, at TN = 64 2,100 against 1,024, so TN is 128 wherever a step has
-// that many rows) and the cutting, eight warps with a few dependent instructions per number.  333 x 151,936 x 896 takes 997 us (90
-// TFLOP/s of the product; the FFMA kernel 2,950), 333 x 896 x 4,864 52 (345).  Tried on the way there, with six products in one
-// sum: four warps instead of eight for the additions 954 against 862, sixteen for the cutting 929; looking for infinities and NaN
-// in the sums instead of in every number that is cut 837.  The two further products and the sum of their own cost 15% of
-// that and are what makes the result as close to 64 bits as a plain float32 sum for any rows; parts rounded instead of cut off,
-// with six products, took as long and left a single product off by up to 1.4 x 2^-24.
+// A tile is 128 rows of W (gated: 64 gate rows and the 64 up rows of the same features) by TN rows of X, up to 64 (beyond, the kernel of
+// `gemm_f32_wide.cu` puts less work into a multiply-add: X is cut here once for every tile of rows of W).  What bounds a
+// block of 64 steps of K is the cutting, eight warps with a few dependent instructions per number, and shared memory (32 MMAs that
+// read 4 KiB of W and TN * 32 bytes of X each, and the parts' writes: at TN = 64 2,100 clocks against 1,024 of the tensor core).
+// 64 x 4,864 x 896 gated takes 29 us, 64 x 896 x 4,864 24.  Parts rounded instead of cut off, with six products, took as long and left
+// a single product off by up to 1.4 x 2^-24.
 // ---------------------------------------------------------------------------------------------------------------------
 constexpr int ROWS = 128, BK = 64, PART = ROWS * BK * 2, STAGES = 2;
 constexpr int CUT_WARPS = 8, CUT_THREADS = CUT_WARPS * 32, ADD_WARPS = 8;
@@ -550,8 +547,7 @@ int dispatch(const float* X, const float* W, const float* W2, const float* bias,
         }
     }
     if (M <= 32) return launch_split<32, MODE>(X, W, W2, bias, out, M, N, K, status, stream);
-    if (M <= 64) return launch_split<64, MODE>(X, W, W2, bias, out, M, N, K, status, stream);
-    return launch_split<128, MODE>(X, W, W2, bias, out, M, N, K, status, stream);
+    return launch_split<64, MODE>(X, W, W2, bias, out, M, N, K, status, stream);
 }
 
 }  // namespace

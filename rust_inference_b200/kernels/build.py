@@ -26,6 +26,7 @@ MODULES = {
     "elementwise": "elementwise.cu",
     "gemm_simt": "gemm_simt.cu",
     "gemm_f32": "gemm_f32.cu",
+    "gemm_f32_wide": "gemm_f32_wide.cu",
     "attention_generic": "attention_generic.cu",
     "attention_f32": "attention_f32.cu",
     "sampling": "sampling.cu",

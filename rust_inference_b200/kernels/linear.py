@@ -47,11 +47,15 @@ def _in_parts(m: int, n: int, k: int) -> bool:
     return m <= 32 or -(-m // 64) * -(-n // 64) > _sm_count()
 
 
-def _plain(x, w: Weight, out, mode, w2: Weight | None = None, **constants):
+def _plain(x, w: Weight, out, mode, w2: Weight | None = None, ctx=None, **constants):
     """The product without bfloat16 tensor cores."""
     t2 = w2.t if w2 is not None else None
-    run = ops.gemm_f32 if ops.gemm_f32_supports(x, w.t, t2) and (x.shape[0] <= 16 or _in_parts(x.shape[0], w.n, w.k)) else ops.gemm_simt
-    return run(x, w.t, out, mode, w2=t2, **constants)
+    m = x.shape[0]
+    if not (ops.gemm_f32_supports(x, w.t, t2) and (m <= 16 or _in_parts(m, w.n, w.k))):
+        return ops.gemm_simt(x, w.t, out, mode, w2=t2, **constants)
+    if ctx is not None and ops.gemm_f32_takes_wide(m, w.n, w.k):
+        constants["parts"] = ctx.buffer("f32_parts", ops.gemm_f32_wide_scratch(m, w.k), torch.bfloat16)
+    return ops.gemm_f32(x, w.t, out, mode, w2=t2, **constants)
 
 
 on_tensor_cores = _use_tensor_cores      # for callers that choose their path by it
@@ -61,7 +65,7 @@ def project(x, w: Weight, out, ctx, bias=None):
     """out<run dtype> = x W^T + bias."""
     if _use_tensor_cores(x, w):
         return tcgen05.gemm(x, w, out, ops.EPI_STORE, ctx, bias=bias)
-    return _plain(x, w, out, ops.EPI_STORE, bias=bias)
+    return _plain(x, w, out, ops.EPI_STORE, ctx=ctx, bias=bias)
 
 
 def logits(x, w: Weight, out, ctx, silu_cols=None):
@@ -69,17 +73,17 @@ def logits(x, w: Weight, out, ctx, silu_cols=None):
     if silu_cols is not None:
         if _use_tensor_cores(x, w):
             return tcgen05.gemm(x, w, out, ops.EPI_SILU_F32, ctx, silu_cols=silu_cols)
-        return _plain(x, w, out, ops.EPI_SILU_F32, silu_cols=silu_cols)
+        return _plain(x, w, out, ops.EPI_SILU_F32, ctx=ctx, silu_cols=silu_cols)
     if _use_tensor_cores(x, w):
         return tcgen05.gemm(x, w, out, ops.EPI_STORE_F32, ctx)
-    return _plain(x, w, out, ops.EPI_STORE_F32)
+    return _plain(x, w, out, ops.EPI_STORE_F32, ctx=ctx)
 
 
 def into_residual(x, w: Weight, residual, ctx):
     """residual<float32> += x W^T."""
     if _use_tensor_cores(x, w):
         return tcgen05.gemm(x, w, residual, ops.EPI_RESIDUAL, ctx)
-    return _plain(x, w, residual, ops.EPI_RESIDUAL)
+    return _plain(x, w, residual, ops.EPI_RESIDUAL, ctx=ctx)
 
 
 def gated(x, w_gate: Weight, w_up: Weight, out, ctx, form=None):
@@ -88,7 +92,7 @@ def gated(x, w_gate: Weight, w_up: Weight, out, ctx, form=None):
     u' = clamp(x Wu^T, -limit, limit)."""
     if _use_tensor_cores(x, w_gate):
         return tcgen05.gemm(x, w_gate, out, ops.EPI_SILU_MUL, ctx, w2=w_up, gate_form=form)
-    return _plain(x, w_gate, out, ops.EPI_SILU_MUL, w_up, gate_form=form)
+    return _plain(x, w_gate, out, ops.EPI_SILU_MUL, w_up, ctx=ctx, gate_form=form)
 
 
 def activated(x, w: Weight, out, ctx, form):
@@ -96,7 +100,7 @@ def activated(x, w: Weight, out, ctx, form):
     two learned numbers through `ops.whole_act_form`, or `ops.RELU_SQUARED_FORM`), applied to the float32 accumulators in the product's epilogue."""
     if _use_tensor_cores(x, w):
         return tcgen05.gemm(x, w, out, ops.EPI_ACT, ctx, act_form=form)
-    return _plain(x, w, out, ops.EPI_ACT, act_form=form)
+    return _plain(x, w, out, ops.EPI_ACT, ctx=ctx, act_form=form)
 
 
 def accumulate_split(x, w: Weight, acc, ctx) -> bool:

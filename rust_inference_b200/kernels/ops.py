@@ -480,10 +480,13 @@ def gemm_f32_supports(x: torch.Tensor, w: torch.Tensor, w2: torch.Tensor | None 
 
 def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, *, bias: torch.Tensor | None = None,
              w2: torch.Tensor | None = None, gate_form: torch.Tensor | None = None, act_form: torch.Tensor | None = None,
-             silu_cols: torch.Tensor | None = None, few_max: int = -1) -> torch.Tensor:
+             silu_cols: torch.Tensor | None = None, few_max: int = -1, parts: torch.Tensor | None = None) -> torch.Tensor:
     """`gemm_simt` for float32 operands that `gemm_f32_supports`: a kernel that streams w past a few rows of x, and for more
-    rows one whose operands are cut into three bfloat16 parts for the tensor cores (csrc/gemm_f32.cu).  few_max: up to how
-    many rows of x the first one is taken (at most 16; negative: the default), for comparisons and tests."""
+    rows two whose operands are cut into three bfloat16 parts for the tensor cores, up to 64 rows of x inside the kernel
+    (csrc/gemm_f32.cu) and beyond in memory (`gemm_f32_wide`, which takes `parts`).  few_max: up to how many rows of x the first one
+    is taken (at most 16; negative: the default), for comparisons and tests."""
+    if gemm_f32_takes_wide(x.shape[0], w.shape[0], w.shape[1]):
+        return gemm_f32_wide(x, w, out, mode, bias=bias, w2=w2, gate_form=gate_form, act_form=act_form, silu_cols=silu_cols, parts=parts)
     bias = _gemm_constants(x, w, out, mode, bias, w2, gate_form, act_form, silu_cols)
     _need(x.dtype == torch.float32, "gemm_f32: float32 operands")
     m, k = x.shape
@@ -491,6 +494,42 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, *, 
     st = tcgen05.f32_status_word()
     _call("gemm_f32", "ri_gemm_f32", _p(x), _p(w), _p(w2), _p(bias), _p(out), c_int(mode), c_int(m), c_int(w.shape[0]),
           c_int(k), c_int(few_max), c_void_p(st.data_ptr()), _stream())
+    return out
+
+
+# Up to 64 rows a product of few weights has less to gain from the wide kernel's tiles than the kernel that cuts x for it costs
+# (us, kernel for few more rows / wide: 40 rows 896 x 896 9.8 / 12.2, 1,536 x 1,536 12.2 / 13.3, 2,048 x 1,536 21.9 / 15.4, 896 x 4,864 23.6 / 21.3,
+# gated 4,864 x 896 30.0 / 25.5; up to 32 rows it is the faster one for most: 896 x 4,864 20.4 / 23.0, gated 4,864 x 896 25.7 / 24.4,
+# gated 8,960 x 1,536 41.0 / 41.5).  Beyond 64 rows wide is: 128 rows 896 x 896 13.6 / 12.8, 100 rows 2,048 x 1,536 28.6 / 17.5.
+F32_WIDE_ROWS, F32_WIDE_MANY_ROWS, F32_WIDE_WEIGHTS = 32, 64, 3_000_000
+
+
+def gemm_f32_takes_wide(m: int, n: int, k: int) -> bool:
+    return m > F32_WIDE_MANY_ROWS or (m > F32_WIDE_ROWS and n * k >= F32_WIDE_WEIGHTS)
+
+
+def gemm_f32_wide_scratch(m: int, k: int) -> tuple:
+    """Shape of the bfloat16 scratch that `gemm_f32_wide` cuts x into."""
+    return 3, m, -(-k // 8) * 8
+
+
+def gemm_f32_wide(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, *, bias: torch.Tensor | None = None,
+                  w2: torch.Tensor | None = None, gate_form: torch.Tensor | None = None, act_form: torch.Tensor | None = None,
+                  silu_cols: torch.Tensor | None = None, parts: torch.Tensor | None = None, tile: int = 0, splits: int = 0) -> torch.Tensor:
+    """`gemm_f32` for many rows of x, which are cut into their bfloat16 parts once, in memory (csrc/gemm_f32_wide.cu).  parts: bfloat16
+    scratch (`gemm_f32_wide_scratch`; made here if None); tile, splits: rows of x per tile and blocks along K (0: the kernel's own
+    plan), for comparisons and tests."""
+    bias = _gemm_constants(x, w, out, mode, bias, w2, gate_form, act_form, silu_cols)
+    _need(x.dtype == torch.float32, "gemm_f32: float32 operands")
+    m, k = x.shape
+    if parts is None:
+        parts = torch.empty(gemm_f32_wide_scratch(m, k), dtype=torch.bfloat16, device=x.device)
+    _need(parts.dtype == torch.bfloat16 and parts.is_contiguous() and tuple(parts.shape) == gemm_f32_wide_scratch(m, k) and parts.is_cuda,
+          "gemm_f32: scratch for the parts of x")
+    from . import tcgen05
+    st = tcgen05.f32_status_word()
+    _call("gemm_f32_wide", "ri_gemm_f32_wide", _p(x), _p(w), _p(w2), _p(bias), _p(out), _p(parts), c_int(mode), c_int(m),
+          c_int(w.shape[0]), c_int(k), c_int(tile), c_int(splits), c_void_p(st.data_ptr()), _stream())
     return out
 
 
