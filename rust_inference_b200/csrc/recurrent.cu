@@ -68,9 +68,14 @@ recurrence_prepare_kernel(float* z, int ld, const float* __restrict__ bias, cons
 }
 
 // Threads of a warp: lane = column_in_warp * R + r.  Thread (r, j) keeps ROWS consecutive rows
-// (r * ROWS ...) of columns j and j + 32 of the state in registers (its gates and query values, read once
-// per token from shared memory, serve both columns: the scan is bound by those reads); the sum over rows of S[i, j] q[i] is finished by
-// log2(R) shuffles inside the warp.  The tokens' q, f and v come through shared memory in tiles of up to 64
+// (r * ROWS ...) of CPT columns j, j + 32, ... of the state in registers (its gates and query values, read once
+// per token from shared memory, serve all of them); the sum over rows of S[i, j] q[i] is finished by
+// log2(R) shuffles inside the warp.  Two neighbouring rows go through one instruction of two multiply-adds.  Steps of few tokens keep two
+// columns per thread, pieces of long runs four where the registers allow it: a token's reads and shuffles then serve twice the work.
+// What bounds it: 3 multiply-adds per state element and token (22 us at the SMs' rate for 32 pieces of 64 tokens, 8 heads of 128 x 128)
+// with twelve warps on an SM to hide their latency, and the reads from shared memory (68% of their rate).  Those sizes, end states and
+// outputs: 38 and 55 us (one multiply-add per instruction and two columns: 50 and 67); all five kernels of a prompt of 2,048 tokens
+// 130 -> 102, of 700 69 -> 66 (four columns there, 88 blocks: 92), of 2,048 with 8 heads of 64 x 128 82 -> 68.  The tokens' q, f and v come through shared memory in tiles of up to 64
 // tokens, fetched by all threads at once with cp.async (a token's gates are shared by the block's columns),
 // so the loop over a tile's tokens touches no global memory but its one store of o.
 //
@@ -82,16 +87,15 @@ recurrence_prepare_kernel(float* z, int ld, const float* __restrict__ bias, cons
 // A short run (one piece per sequence: decode steps, small portions) is one pass, WHOLE: from the
 // slot's state, writing o and the slot's state.
 constexpr int R = 8;                 // row slices per column
-constexpr int CPT = 2;               // value columns per thread: a thread's gates serve both
-constexpr int COLS = 32 * CPT;       // value columns per block
 constexpr int SCAN_THREADS = R * 32;
 enum ScanMode { WHOLE = 0, LOCAL = 1, FINAL = 2 };
 
 // Shared memory of the scan: tiles of up to `tile_t` tokens, per token f and q as [R][ROWS + 4] (a slice of
 // ROWS channels per row slice, padded so that the eight slices' 16-byte reads fall into different banks;
 // channels beyond `dim` stay zero) and the block's COLS values of v.
-template <int ROWS, bool KEYED = false>
+template <int ROWS, bool KEYED, int CPT>
 struct ScanTile {
+    static constexpr int COLS = 32 * CPT;                       // value columns per block
     static constexpr int SLICE = ROWS + 4;
     static constexpr int V_AT = (KEYED ? 3 : 2) * R * SLICE;    // f, q (, k), then the values
     static constexpr int TOKEN = V_AT + COLS;                   // floats per token
@@ -111,13 +115,14 @@ struct ScanCols { int q_col, f_col, v_col, k_col, f_ld; };
 // of z, and q times q_scale.  w2 == nullptr: the gates come from memory as they are.
 struct KeyedPrep { const float* w2; const float* bias; int rank, a_col; float inv_tau, q_scale; };
 
-template <int ROWS, bool VEC, int mode, bool KEYED>
+template <int ROWS, bool VEC, int mode, bool KEYED, int CPT>
 __global__ void __launch_bounds__(SCAN_THREADS)
 recurrence_scan_kernel(const float* z, int ld, const float* fz, ScanCols at, float* __restrict__ o_raw, float* state,
                        float* piece_state, float* piece_gates, const int* __restrict__ cu_seqlens,
                        const int* __restrict__ seq_slot, int heads, int dim, int vdim, int piece, int max_pieces,
                        int tile_t, const float* __restrict__ prep_bias, const float* __restrict__ prep_low, KeyedPrep keyed) {
-    using Tile = ScanTile<ROWS, KEYED>;
+    using Tile = ScanTile<ROWS, KEYED, CPT>;
+    constexpr int COLS = Tile::COLS;
     const bool forms_decays = KEYED && mode == WHOLE && keyed.w2 != nullptr;
     extern __shared__ __align__(16) float tile[];
     const int b = blockIdx.x / max_pieces, c = blockIdx.x % max_pieces, h = blockIdx.y;
@@ -140,17 +145,17 @@ recurrence_scan_kernel(const float* z, int ld, const float* fz, ScanCols at, flo
         S = piece_state + (((size_t)blockIdx.x * heads + h) * dim) * vdim;
     }
     bool live[CPT];
-    float s[CPT][ROWS], g[ROWS];
+    float2 s[CPT][ROWS / 2], g[ROWS / 2];                         // rows 2 k and 2 k + 1 of the thread's
 #pragma unroll
     for (int cc = 0; cc < CPT; ++cc) {
         const int j = j0 + jj + 32 * cc;
         live[cc] = j < vdim;
+        auto start = [&](int k) { return (mode != LOCAL && live[cc] && i0 + k < dim) ? S[(size_t)(i0 + k) * vdim + j] : 0.f; };
 #pragma unroll
-        for (int k = 0; k < ROWS; ++k)
-            s[cc][k] = (mode != LOCAL && live[cc] && i0 + k < dim) ? S[(size_t)(i0 + k) * vdim + j] : 0.f;
+        for (int k = 0; k < ROWS / 2; ++k) s[cc][k] = make_float2(start(2 * k), start(2 * k + 1));
     }
 #pragma unroll
-    for (int k = 0; k < ROWS; ++k) g[k] = 1.f;
+    for (int k = 0; k < ROWS / 2; ++k) g[k] = make_float2(1.f, 1.f);
     const int q_off = at.q_col + h * dim, f_off = at.f_col + h * dim, v_off = at.v_col + h * vdim + j0;
     const int k_off = at.k_col + h * dim, f_ld = at.f_ld;
     const int cols = min(COLS, vdim - j0);
@@ -237,39 +242,40 @@ recurrence_scan_kernel(const float* z, int ld, const float* fz, ScanCols at, flo
             const float4* f4 = reinterpret_cast<const float4*>(base + r * Tile::SLICE);
             const float4* q4 = reinterpret_cast<const float4*>(base + R * Tile::SLICE + r * Tile::SLICE);
             const float4* k4 = reinterpret_cast<const float4*>(base + 2 * R * Tile::SLICE + r * Tile::SLICE);   // KEYED only
-            float v[CPT], acc0[CPT], acc1[CPT];
+            float2 v[CPT], acc[CPT];
 #pragma unroll
             for (int cc = 0; cc < CPT; ++cc) {
-                v[cc] = base[Tile::V_AT + jj + 32 * cc];             // columns beyond vdim: zero, never stored
-                acc0[cc] = acc1[cc] = 0.f;
+                const float x = base[Tile::V_AT + jj + 32 * cc];     // columns beyond vdim: zero, never stored
+                v[cc] = make_float2(x, x);
+                acc[cc] = make_float2(0.f, 0.f);
             }
 #pragma unroll
             for (int k4i = 0; k4i < ROWS / 4; ++k4i) {
                 const float4 fv = f4[k4i], qv = mode != LOCAL ? q4[k4i] : make_float4(0.f, 0.f, 0.f, 0.f);
                 const float4 kv = KEYED ? k4[k4i] : make_float4(0.f, 0.f, 0.f, 0.f);
-                const float ff[4] = {fv.x, fv.y, fv.z, fv.w}, qq[4] = {qv.x, qv.y, qv.z, qv.w}, kk[4] = {kv.x, kv.y, kv.z, kv.w};
+                const float2 ff[2] = {make_float2(fv.x, fv.y), make_float2(fv.z, fv.w)};
+                const float2 qq[2] = {make_float2(qv.x, qv.y), make_float2(qv.z, qv.w)};
+                const float2 kk[2] = {make_float2(kv.x, kv.y), make_float2(kv.z, kv.w)};
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int k = 4 * k4i + u;
-                    if (mode == LOCAL) g[k] *= ff[u];
+                for (int u = 0; u < 2; ++u) {
+                    const int k = 2 * k4i + u;
+                    const float2 not_f = make_float2(-ff[u].x, -ff[u].y);
+                    if (mode == LOCAL) g[k] = __fmul2_rn(g[k], ff[u]);
 #pragma unroll
                     for (int cc = 0; cc < CPT; ++cc) {
                         // f s + (1 - f) v, or with a key f s + k v; channels beyond dim: f = 0, q = 0, k = 0
-                        s[cc][k] = KEYED ? fmaf(ff[u], s[cc][k], kk[u] * v[cc])
-                                         : fmaf(ff[u], s[cc][k], fmaf(-ff[u], v[cc], v[cc]));
-                        if (mode != LOCAL) {
-                            if (u & 1) acc1[cc] = fmaf(s[cc][k], qq[u], acc1[cc]); else acc0[cc] = fmaf(s[cc][k], qq[u], acc0[cc]);
-                        }
+                        s[cc][k] = __ffma2_rn(ff[u], s[cc][k], KEYED ? __fmul2_rn(kk[u], v[cc]) : __ffma2_rn(not_f, v[cc], v[cc]));
+                        if (mode != LOCAL) acc[cc] = __ffma2_rn(s[cc][k], qq[u], acc[cc]);
                     }
                 }
             }
             if (mode != LOCAL) {
 #pragma unroll
                 for (int cc = 0; cc < CPT; ++cc) {
-                    float acc = acc0[cc] + acc1[cc];
+                    float sum = acc[cc].x + acc[cc].y;
 #pragma unroll
-                    for (int o = R / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-                    if (live[cc] && r == 0) o_raw[(size_t)(tb + tok) * o_ld + h * vdim + j0 + jj + 32 * cc] = acc;
+                    for (int o = R / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                    if (live[cc] && r == 0) o_raw[(size_t)(tb + tok) * o_ld + h * vdim + j0 + jj + 32 * cc] = sum;
                 }
             }
         }
@@ -280,13 +286,13 @@ recurrence_scan_kernel(const float* z, int ld, const float* fz, ScanCols at, flo
         for (int cc = 0; cc < CPT; ++cc)
 #pragma unroll
             for (int k = 0; k < ROWS; ++k)
-                if (live[cc] && i0 + k < dim) S[(size_t)(i0 + k) * vdim + j0 + jj + 32 * cc] = s[cc][k];
+                if (live[cc] && i0 + k < dim) S[(size_t)(i0 + k) * vdim + j0 + jj + 32 * cc] = k & 1 ? s[cc][k / 2].y : s[cc][k / 2].x;
     }
     if (mode == LOCAL && blockIdx.z == 0 && jj == 0) {
         float* G = piece_gates + ((size_t)blockIdx.x * heads + h) * dim;
 #pragma unroll
         for (int k = 0; k < ROWS; ++k)
-            if (i0 + k < dim) G[i0 + k] = g[k];
+            if (i0 + k < dim) G[i0 + k] = k & 1 ? g[k / 2].y : g[k / 2].x;
     }
 }
 
@@ -425,23 +431,24 @@ keyed_prepare_kernel(float* z, int ld, int q_col, int a_col, int rank, const flo
 }
 
 
-constexpr int SCAN_SMEM_LIMIT = 96 * 1024;       // two blocks to an SM
+constexpr int SCAN_SMEM_LIMIT = 112 * 1024;      // two blocks to an SM
 
-template <int ROWS, bool KEYED>
+template <int ROWS, bool KEYED, int CPT>
 int launch_scan(bool vec, dim3 grid, cudaStream_t stream, const float* z, int ld, const float* fz, ScanCols at, float* o_raw,
                 float* state, float* piece_state, float* piece_gates, const int* cu_seqlens, const int* seq_slot, int heads,
                 int dim, int vdim, int mode, int piece, int max_pieces, int longest, const float* prep_bias,
                 const float* prep_low, KeyedPrep keyed) {
-    const int token_bytes = ScanTile<ROWS, KEYED>::TOKEN * (int)sizeof(float);
+    const int token_bytes = ScanTile<ROWS, KEYED, CPT>::TOKEN * (int)sizeof(float);
     int tile_t = SCAN_SMEM_LIMIT / token_bytes;
     if (tile_t > 64) tile_t = 64;
     if (tile_t > longest) tile_t = longest;                      // a decode step brings one token
+    if (tile_t > 0) tile_t = (longest + (longest + tile_t - 1) / tile_t - 1) / ((longest + tile_t - 1) / tile_t);       // tiles of equal length
     if (tile_t < 1) return fail("gated_recurrence: a token's %d bytes of gates do not fit shared memory", token_bytes);
     const size_t smem = (size_t)tile_t * token_bytes;
     cudaError_t e = cudaSuccess;
 #define RI_LAUNCH(V, M)                                                                                                   \
     {                                                                                                                     \
-        auto kernel = recurrence_scan_kernel<ROWS, V, M, KEYED>;                                                          \
+        auto kernel = recurrence_scan_kernel<ROWS, V, M, KEYED, CPT>;                                                          \
         static PerDeviceOnce once;                                                                                        \
         if (int rc = raise_dynamic_smem(kernel, SCAN_SMEM_LIMIT, once, "gated_recurrence")) return rc;                    \
         e = launch_dependent(kernel, grid, SCAN_THREADS, smem, stream, z, ld, fz, at, o_raw, state, piece_state,          \
@@ -449,9 +456,14 @@ int launch_scan(bool vec, dim3 grid, cudaStream_t stream, const float* z, int ld
                              prep_low, keyed);                                                                            \
     }
     if (vec) {
-        if (mode == WHOLE) RI_LAUNCH(true, WHOLE) else if (mode == LOCAL) RI_LAUNCH(true, LOCAL) else RI_LAUNCH(true, FINAL)
+        if (mode == LOCAL) RI_LAUNCH(true, LOCAL) else if (mode == FINAL) RI_LAUNCH(true, FINAL)
     } else {
-        if (mode == WHOLE) RI_LAUNCH(false, WHOLE) else if (mode == LOCAL) RI_LAUNCH(false, LOCAL) else RI_LAUNCH(false, FINAL)
+        if (mode == LOCAL) RI_LAUNCH(false, LOCAL) else if (mode == FINAL) RI_LAUNCH(false, FINAL)
+    }
+    if constexpr (CPT == 2) {
+        if (mode == WHOLE) {
+            if (vec) RI_LAUNCH(true, WHOLE) else RI_LAUNCH(false, WHOLE)
+        }
     }
 #undef RI_LAUNCH
     return check_launch(e, "gated_recurrence (scan)");
@@ -470,21 +482,23 @@ int scan_and_norm(const float* z, int ld, const float* fz, ScanCols at, const fl
     const bool vec = dim % 4 == 0 && vdim % 4 == 0 && ld % 4 == 0 && at.f_ld % 4 == 0 && (uintptr_t)z % 16 == 0 &&
                      (uintptr_t)fz % 16 == 0 && at.q_col % 4 == 0 && at.f_col % 4 == 0 && at.v_col % 4 == 0 &&
                      at.k_col % 4 == 0;
-    const int col_tiles = (vdim + COLS - 1) / COLS;
     float* piece_state = scratch;
     float* piece_gates = piece > 0 ? scratch + (size_t)n_seqs * max_pieces * heads * dim * vdim : nullptr;
     auto scan = [&](int mode) -> int {
         const int mp = mode == WHOLE ? 1 : max_pieces;
-        dim3 grid(n_seqs * mp, heads, col_tiles);
+        // four columns per thread for pieces, where the rows leave the registers and the blocks that are left fill the SMs
+        const int cpt = mode != WHOLE && rows <= 16 && vdim > 64 && (long long)n_seqs * mp * heads * ((vdim + 127) / 128) >= sm_count() ? 4 : 2;
+        dim3 grid(n_seqs * mp, heads, (vdim + 32 * cpt - 1) / (32 * cpt));
         const int longest = mode == WHOLE ? (longest_run > 0 ? longest_run : n_tokens) : piece;
-#define RI_SCAN(ROWS) launch_scan<ROWS, KEYED>(vec, grid, stream, z, ld, fz, at, o_raw, state, piece_state, piece_gates,        \
-                                               cu_seqlens, seq_slot, heads, dim, vdim, mode, piece > 0 ? piece : 1, mp, longest, \
-                                               mode == WHOLE ? prep_bias : nullptr, mode == WHOLE ? prep_low : nullptr, keyed)
-        if (rows == 4) return RI_SCAN(4);
-        if (rows == 8) return RI_SCAN(8);
-        if (rows == 16) return RI_SCAN(16);
-        if (rows == 32) return RI_SCAN(32);
-        return RI_SCAN(64);
+#define RI_SCAN(ROWS, CPT) launch_scan<ROWS, KEYED, CPT>(vec, grid, stream, z, ld, fz, at, o_raw, state, piece_state, piece_gates,    \
+                                                         cu_seqlens, seq_slot, heads, dim, vdim, mode, piece > 0 ? piece : 1, mp,      \
+                                                         longest, mode == WHOLE ? prep_bias : nullptr,                                 \
+                                                         mode == WHOLE ? prep_low : nullptr, keyed)
+        if (rows == 4) return cpt == 4 ? RI_SCAN(4, 4) : RI_SCAN(4, 2);
+        if (rows == 8) return cpt == 4 ? RI_SCAN(8, 4) : RI_SCAN(8, 2);
+        if (rows == 16) return cpt == 4 ? RI_SCAN(16, 4) : RI_SCAN(16, 2);
+        if (rows == 32) return RI_SCAN(32, 2);
+        return RI_SCAN(64, 2);
 #undef RI_SCAN
     };
     if (piece <= 0) {
