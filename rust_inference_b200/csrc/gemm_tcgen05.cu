@@ -132,9 +132,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;     // swizzled tiles want 1024-byte alignment
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int total_kb = (K + BLOCK_K - 1) / BLOCK_K;
-    // The gated product of a few tokens may have its K cut over the CTAs of a cluster (`cluster` > 1; one tile per
-    // cluster, one token tile): see the end of the kernel.
-    const bool clustered = DUAL && cluster > 1;
+    // A product of a few tokens that does not add onto sums may have its K cut over the CTAs of a cluster (`cluster` > 1; one
+    // tile per cluster, one token tile): see the end of the kernel.
+    constexpr bool CLUSTERS = MODE != 2 && TN == 16;
+    const bool clustered = CLUSTERS && cluster > 1;
     const int rank = clustered ? (int)cluster_rank() : 0;
     // Tiles are numbered with the token tile fastest, so that CTAs running together share a weight
     // tile in L2; a CTA takes tiles blockIdx.x, blockIdx.x + gridDim.x, ...
@@ -351,11 +352,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         }
     }
 
-    if constexpr (DUAL) {
+    if constexpr (CLUSTERS) {
         if (clustered) {
-            // Token c is finished by the CTA of rank c % cluster: everybody sends it its sums of that token, gate and up, into
-            // `recv` [rank of the sender][c / cluster][gate, up][128] (behind the ring), and it adds them in the order of the
+            // Token c is finished by the CTA of rank c % cluster: everybody sends it its sums of that token (gate and up), into
+            // `recv` [rank of the sender][c / cluster][(gate, up)][128] (behind the ring), and it adds them in the order of the
             // ranks.  A CTA that gave up says so first; then none of the cluster writes.
+            constexpr int SENT = (DUAL ? 2 : 1) * BLOCK_F;         // floats per token
             const int held = (n_tok + cluster - 1) / cluster;
             float* recv = reinterpret_cast<float*>(smem_raw + (smem_base - smem_u32(smem_raw)) + (size_t)stages * STAGE_BYTES);
             const int fl = (warp & 3) * 32 + lane;
@@ -364,20 +366,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             if (abort_flag && lane == 0) set_in_all(&any_failed, cluster);
             if (warp >= 2 && !abort_flag) {
                 const uint32_t trow = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
-                const float* mine = recv + (size_t)rank * held * 2 * BLOCK_F + fl;
+                const float* mine = recv + (size_t)rank * held * SENT + fl;
 #pragma unroll 1
                 for (int c0 = 0; c0 < n_tok; c0 += 16) {
                     uint32_t v[16], u[16];
                     tmem_ld16(trow + c0, v);
-                    tmem_ld16(trow + TN + c0, u);
+                    if (DUAL) tmem_ld16(trow + TN + c0, u);
                     tmem_wait_ld();
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
                         const int c = c0 + j;
                         if (c >= n_tok) break;
-                        const int to = c % cluster, at = (c / cluster) * 2 * BLOCK_F;
+                        const int to = c % cluster, at = (c / cluster) * SENT;
                         store_peer_float(mine + at, (uint32_t)to, __uint_as_float(v[j]));
-                        store_peer_float(mine + at + BLOCK_F, (uint32_t)to, __uint_as_float(u[j]));
+                        if (DUAL) store_peer_float(mine + at + BLOCK_F, (uint32_t)to, __uint_as_float(u[j]));
                     }
                 }
             }
@@ -386,14 +388,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             const int f = ((int)blockIdx.x / cluster) * BLOCK_F + fl;
             if (warp >= 2 && !any_failed && f < n_feat) {
                 const GateForm gf = load_gate_form(MODE == 3 ? bias : nullptr);
+                const ActForm af = MODE == 4 ? load_act_form(bias) : ActForm{0.f, 0.f, 0.f};
+                const float b = MODE == 5 ? (f < (int)bias[0] ? 1.f : 0.f) : (MODE != 3 && MODE != 4 && bias != nullptr) ? bias[f] : 0.f;
                 for (int i = 0, c = rank; c < n_tok; ++i, c += cluster) {
-                    const float* from = recv + (size_t)i * 2 * BLOCK_F + fl;
+                    const float* from = recv + (size_t)i * SENT + fl;
                     float g = 0.f, up = 0.f;
-                    for (int p = 0; p < cluster; ++p, from += (size_t)held * 2 * BLOCK_F) {
+                    for (int p = 0; p < cluster; ++p, from += (size_t)held * SENT) {
                         g += from[0];
-                        up += from[BLOCK_F];
+                        if (DUAL) up += from[BLOCK_F];
                     }
-                    store_result<MODE>(out_, (size_t)c * n_feat + f, g, 0.f, up, gf, ActForm{0.f, 0.f, 0.f});
+                    store_result<MODE>(out_, (size_t)c * n_feat + f, g, b, up, gf, af);
                 }
             }
         }
@@ -926,9 +930,9 @@ int launch(int tn, const CUtensorMap& mw, const CUtensorMap& mw2, const CUtensor
     const int total_kb = (K + BLOCK_K - 1) / BLOCK_K;
     if (split_k < 1) split_k = 1;
     if (split_k > total_kb) split_k = total_kb;
-    const int cluster = DUAL ? split_k : 1;                          // the gated epilogue's pieces of K meet in a cluster
+    const int cluster = MODE != 2 ? split_k : 1;                     // pieces of K that are not added onto sums meet in a cluster
     const long long cluster_ctas = (long long)((n_feat + BLOCK_F - 1) / BLOCK_F) * cluster;
-    const int recv = cluster > 1 ? cluster * ((n_tok + cluster - 1) / cluster) * 2 * BLOCK_F * 4 : 0;
+    const int recv = cluster > 1 ? cluster * ((n_tok + cluster - 1) / cluster) * (DUAL ? 2 : 1) * BLOCK_F * 4 : 0;
     // Small token tiles (decode) leave room for a second CTA on the SM, so that the next kernel's
     // CTAs can settle in and prefetch their weights while this one drains.
     int budget = (3 * STAGE_BYTES <= 108 * 1024 && TN <= 64) ? 108 * 1024 : SMEM_BUDGET;
@@ -939,7 +943,7 @@ int launch(int tn, const CUtensorMap& mw, const CUtensorMap& mw2, const CUtensor
     if (stages < 1) stages = 1;
     const size_t smem = (size_t)stages * STAGE_BYTES + 1024 + recv;
     int kb_per_split = (total_kb + split_k - 1) / split_k;
-    if (!DUAL) split_k = (total_kb + kb_per_split - 1) / kb_per_split;          // no empty split
+    if (MODE == 2) split_k = (total_kb + kb_per_split - 1) / kb_per_split;      // no empty split
     auto kernel = gemm_tc_kernel<TN, DUAL, MODE>;
     static PerDeviceOnce configured;       // per device: the attribute belongs to a device's copy of the kernel
     if (int rc = raise_dynamic_smem(kernel, SMEM_BUDGET + 1024 + CLUSTER_RECV_MAX, configured, "gemm_tcgen05")) return rc;
@@ -1078,14 +1082,14 @@ int pick_tile(int tn, const CUtensorMap& mw, const CUtensorMap& mw2, const CUten
 
 }  // namespace
 
-// Over how many CTAs of a cluster K is cut for the gated product of a few tokens.  Such a product is a read of its weights, and a CTA,
+// Over how many CTAs of a cluster K is cut for a product of a few tokens that is not added onto sums.  It is a read of its weights, and a CTA,
 // whose ring holds 102 KB of them on their way, takes about 64 GB/s, so a product with few tiles leaves most of the memory's rate
 // unused.  Cut in four where that makes about one CTA per SM: most of a CTA's weights are then asked for before its wait.  Otherwise
 // in two or three, whichever leaves the SMs more evenly filled, as long as all CTAs are resident together (two to an SM).
 // Whole decode steps, us, not cut / 2 / 3 / 4: 38 tiles of K = 896 (24 layers), 1 token 690 / 648 / 650 / 633, 8 tokens 757 / 713 / 692 /
 // 675; 70 tiles of 1,536 (28), 1 token 1,059 / 985 / 1,025 / 1,000, 12 tokens 1,140 / 1,130 / 1,144 / 1,203; 86 tiles of 2,048 (36), 1 token
 // 1,629 / 1,604 / 1,576 / 1,758; 112 tiles of 4,096 (32), 1 token 2,835 / 2,670 / 2,925 / 2,828.
-int gated_cluster(int n_tok, int n_feat, int K) {
+int cluster_split(int n_tok, int n_feat, int K) {
     const int total_kb = (K + BLOCK_K - 1) / BLOCK_K, sms = sm_count();
     const long long tiles = (n_feat + BLOCK_F - 1) / BLOCK_F;
     if (n_tok > CLUSTER_MAX_TOK || total_kb < 8) return 1;
@@ -1135,7 +1139,7 @@ RI_API int ri_gemm_tcgen05_plan(int n_tok, int n_feat, int K, int mode, int* til
         if (mode == 2) sp = pair_split(n_tok, n_feat, K);
     } else if (n_tok <= 128) {
         tn = n_tok <= 16 ? 16 : (n_tok + 15) / 16 * 16;
-        if (mode == 3) sp = gated_cluster(n_tok, n_feat, K);
+        if (mode != 2) sp = cluster_split(n_tok, n_feat, K);
         if (can_split && feat_tiles < ctas) {
             // every piece ends in tn x 128 atomic adds, so wider steps want longer pieces: at least a tenth of
             // the tile's width in k-blocks (128 tokens, K = 3584: 4-5 pieces, 11 us, against 10 pieces, 13 us)
@@ -1190,9 +1194,8 @@ RI_API int ri_gemm_tcgen05(const void* map_x, const void* map_w, const void* map
     if (mode == 5 && bias == nullptr) return fail("gemm_tcgen05: the partly activated epilogue needs its number of features");
     if (mode == 3 && map_w2 == nullptr) return fail("gemm_tcgen05: the SiLU-gate epilogue needs a second matrix");
     if (mode == 2 && bias != nullptr) return fail("gemm_tcgen05: the residual epilogue takes no bias");
-    if (mode == 3 && split_k > 1 && (split_k > 8 || n_tok > CLUSTER_MAX_TOK))
-        return fail("gemm_tcgen05: no cluster of %d CTAs for the gated epilogue of %d tokens", split_k, n_tok);
-    if (mode != 2 && mode != 3 && split_k > 1) return fail("gemm_tcgen05: only the residual and the gated epilogue can split K");
+    if (mode != 2 && split_k > 1 && (split_k > 8 || n_tok > CLUSTER_MAX_TOK))
+        return fail("gemm_tcgen05: no cluster of %d CTAs for %d tokens", split_k, n_tok);
     const bool dual = mode == 3;
     int tn = 0, planned_split = 1;
     ri_gemm_tcgen05_plan(n_tok, n_feat, K, mode, &tn, &planned_split);

@@ -31,3 +31,25 @@ def test_gated_product_refuses_clusters_it_cannot_form():
         x = torch.zeros(m, 1024, device=DEV, dtype=torch.bfloat16)
         with pytest.raises(ops.KernelError, match="no cluster"):
             tcgen05.gemm(x, w, torch.zeros(m, 128, device=DEV, dtype=torch.bfloat16), ops.EPI_SILU_MUL, w2=w, split_k=cluster)
+
+
+@pytest.mark.parametrize("m", [1, 5, 16])
+@pytest.mark.parametrize("n, k, cluster", [(128, 512, 2), (391, 1000, 3), (72, 2056, 8), (1000, 640, 4)])
+def test_plain_products_cut_over_a_cluster(m, n, k, cluster):
+    from rust_inference_b200.kernels import linear, ops, tcgen05
+    x = (torch.randn(m, k, device=DEV) * 0.5).bfloat16()
+    w = linear.Weight((torch.randn(n, k, device=DEV) * 0.1).bfloat16())
+    bias, cols = torch.randn(n, device=DEV), torch.tensor([n // 2], dtype=torch.float32, device=DEV)
+    ref = x.double() @ w.t.double().t()
+    out32, part = torch.full((m, n), 9.0, device=DEV), torch.full((m, n), 9.0, device=DEV)
+    out = torch.full((m, n), 9.0, device=DEV, dtype=torch.bfloat16)
+    tcgen05.gemm(x, w, out32, ops.EPI_STORE_F32, split_k=cluster)
+    tcgen05.gemm(x, w, out, ops.EPI_STORE, bias=bias, split_k=cluster)
+    tcgen05.gemm(x, w, part, ops.EPI_SILU_F32, silu_cols=cols, split_k=cluster)
+    # float32 sums of k products; one rounding to bfloat16; the quick exponential and division of the activated columns
+    assert float((out32.double() - ref).norm() / ref.norm()) <= 1e-5
+    assert float((out.double() - ref - bias).norm() / (ref + bias).norm()) <= 2.0 ** -8
+    want = torch.cat([ref[:, :n // 2] * torch.sigmoid(ref[:, :n // 2]), ref[:, n // 2:]], dim=1)
+    assert float((part.double() - want).norm() / want.norm()) <= 1e-5
+    torch.cuda.synchronize()
+    tcgen05.check_status()
