@@ -2,8 +2,8 @@
 // every M (K a multiple of 4 and 16-byte aligned operands: rows are read 16 bytes at a time; `gemm_simt.cu` has the rest).
 //
 // Few rows of X (a decode step, up to FEW_MAX): the product is a read of W.  A warp owns a few rows of W, its lanes run
-// along K with 16-byte loads straight into registers, several steps ahead, and every loaded weight meets all rows of X,
-// which lie in shared memory; FFMA, float32 sums.  K is cut over the thread blocks of a cluster when N alone has too few
+// along K with 16-byte asynchronous copies into a ring of their own, several steps ahead, and every weight meets all rows of X,
+// which lie in shared memory too; FFMA, float32 sums.  K is cut over the thread blocks of a cluster when N alone has too few
 // rows to keep the memory busy; the pieces meet through distributed shared memory in a fixed order, so a product's bits do
 // not change from run to run.
 //
@@ -37,13 +37,29 @@ namespace {
 // ---------------------------------------------------------------------------------------------------------------------
 // Few rows of X.
 //
-// Bound by the read of W.  Two blocks' worth of loads in flight per SM cover the memory's latency (8 warps x 4 KiB per
-// block).  A weight costs one FFMA per row of X and a 16-byte read of X from shared memory per RW of them: with RW = 2 up
-// to four rows and 4 beyond, both stay below what the memory delivers (23 bytes per clock and SM).
+// Bound by the read of W.  Every lane copies its 16 bytes of a row and step into a ring in shared memory and reads only what it
+// copied itself, so no warp waits for another: 3 to 7 steps of 512 bytes a row are on their way per warp (24 to 56 KiB per block),
+// across groups of rows and before the wait for the kernel before.  Loads into registers did the same on paper, but how many of
+// them a use waited for hung on how the compiler shared its scoreboards out (one more unused branch in the kernel changed a step
+// of a 0.5B-sized decoder from 887 to 797 us); X comes by such copies too.  Where K is cut over a cluster the pieces go straight to
+// the block that finishes an output, which reads them behind one meeting point.  A decode step of a 1.5B-sized decoder and 4 sequences:
+// 1,988 -> about 1,885 us, 0.5B-sized 933 -> 790 (1 sequence), 1,406 -> 1,270 (8).  Asking for the following weights to come into the L2
+// before the wait as well cost 1%.  A weight costs one FFMA per row of X and a 16-byte read of X from shared memory per RW of them:
+// with RW = 2 up to four rows and 4 beyond, both stay below what the memory delivers (23 bytes per clock and SM).
 // ---------------------------------------------------------------------------------------------------------------------
 constexpr int FEW_MAX = 16;
 constexpr int FEW_THREADS = 256, FEW_WARPS = FEW_THREADS / 32;
 constexpr int STEP = 128;                      // floats of K that a warp reads per step and row: 16 bytes per lane
+
+// 16 bytes into shared memory; not `in`: zeros, and nothing is read
+__device__ __forceinline__ void copy16_or_zeros(float* dst, const float* src, bool in) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(in ? 16 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+__host__ __device__ constexpr int few_ring_floats(int rw, int u) { return FEW_WARPS * u * rw * STEP; }
 
 // a[0 .. n) of every lane, summed over the lanes: afterwards lane l holds in a[0 .. n/32) (n < 32: in a[0]) the sums number
 // `lane_first` .. ; every exchange halves what a lane still carries
@@ -78,115 +94,153 @@ gemm_f32_few_kernel(const float* X, const float* __restrict__ W, const float* __
     constexpr int FEATS = DUAL ? RW / 2 : RW;                // features per warp (gated: a gate row and an up row each)
     constexpr int GROUP = FEW_WARPS * FEATS;                 // features per block
     constexpr int SUMS = FEW_WARPS * RW * MT;
-    extern __shared__ __align__(16) float xs[];              // [MT][this block's stretch of K]
-    __shared__ float sums[2][SUMS];
+    extern __shared__ __align__(16) float smem[];
+    __shared__ float sums[2][SUMS + 16];                     // whole products; K cut: the pieces of this block's outputs, block by block
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float* ring = smem + warp * (U * RW * STEP) + lane * 4;  // [U][RW][STEP] per warp; a lane reads only what it copied itself
+    float* xs = smem + few_ring_floats(RW, U);               // [MT][this block's stretch of K]
     const int rank = splits > 1 ? (int)cluster_rank() : 0;
     const int first_step = (int)((long long)steps * rank / splits);
     const int ns = (int)((long long)steps * (rank + 1) / splits) - first_step;      // >= 1: splits <= steps
-    const int ns_up = (ns + U - 1) / U * U;
     const int k0 = first_step * STEP, width = ns * STEP;
     const int groups = (N + GROUP - 1) / GROUP, stride = (int)gridDim.x / splits;
 
-    auto load = [&](float4 (&w)[RW], int group, int step) {
-        const int k = k0 + step * STEP + lane * 4;
-        const int f = group * GROUP + warp * FEATS;
-        const bool in = step < ns && k < K && group < groups;
+    // the next step's weights on their way into a slot of the ring: steps of this group of rows, then of the block's next group
+    int group = (int)blockIdx.x / splits, copy_group = group, copy_step = 0;
+    auto copy_next = [&](int slot) {
+        if (copy_group < groups) {
+            const int k = k0 + copy_step * STEP + lane * 4;
 #pragma unroll
-        for (int r = 0; r < RW; ++r) {
-            const int row = min(DUAL ? f + r / 2 : f + r, N - 1);
-            const float* base = (DUAL && (r & 1)) ? W2 : W;
-            w[r] = in ? load_weight(base + (size_t)row * K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int r = 0; r < RW; ++r) {
+                const int f = copy_group * GROUP + warp * FEATS, row = min(DUAL ? f + r / 2 : f + r, N - 1);
+                const float* base = (DUAL && (r & 1)) ? W2 : W;
+                copy16_or_zeros(ring + (slot * RW + r) * STEP, base + (k < K ? (size_t)row * K + k : 0), k < K);
+            }
+            if (++copy_step == ns) {
+                copy_step = 0;
+                copy_group += stride;
+            }
         }
+        copies_commit();
     };
 
     let_next_kernel_start();
-    float4 w[U][RW];
-    int group = (int)blockIdx.x / splits;
+    if (splits > 1) cluster_arrive();
 #pragma unroll
-    for (int u = 0; u < U; ++u) load(w[u], group, u);        // weights: written by no kernel
+    for (int u = 0; u < U - 1; ++u) copy_next(u);            // weights: written by no kernel
     wait_for_previous_kernels();
-    for (int i = threadIdx.x * 4; i < MT * width; i += FEW_THREADS * 4) {
-        const int m = i / width, k = k0 + i - m * width;     // width is a multiple of 4: the four belong to one row
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (m < M && k < K) v = load_written(X + (size_t)m * K + k);
-        *reinterpret_cast<float4*>(xs + i) = v;
+    // X: asynchronous copies too, all on their way at once (rows and columns beyond X become zeros)
+    for (int m = 0, k = threadIdx.x * 4;; k += FEW_THREADS * 4) {
+        while (k >= width && m < MT) {
+            k -= width;
+            ++m;
+        }
+        if (m == MT) break;
+        const bool in = m < M && k0 + k < K;                 // width is a multiple of 4: the four belong to one row
+        copy16_or_zeros(xs + m * width + k, in ? X + (size_t)m * K + k0 + k : X, in);
     }
+    copies_commit();
+    copies_wait<0>();
     const Forms forms = load_forms<MODE>(bias);
+    // outputs (feature of the group, row of X), the feature fastest; the cluster's blocks share them out
+    constexpr int TOTAL = GROUP * MT;
+    const int each = (TOTAL + splits - 1) / splits, from = min(TOTAL, each * rank), to = min(TOTAL, from + each);
     __syncthreads();
+    if (splits > 1) cluster_wait();              // every block of the cluster is there: its shared memory may be written
 
+    int slot = 0, used = U - 1;                  // this step's slot, and the one of the step before it: free
     for (int turn = 0; group < groups; group += stride, turn ^= 1) {
+        float old = 0.f;                         // what this thread's output is added to
+        if (MODE == 2) {
+            const int i = from + threadIdx.x, m = i / GROUP, f = group * GROUP + i - m * GROUP;
+            if (i < to && m < M && f < N) old = out[(size_t)m * N + f];
+        }
         float acc[RW * MT];
 #pragma unroll
         for (int i = 0; i < RW * MT; ++i) acc[i] = 0.f;
-        for (int s0 = 0; s0 < ns_up; s0 += U) {
+        const float* x0 = xs + lane * 4;
+        for (int s = 0; s < ns; ++s, x0 += STEP) {
+            copies_wait<U - 2>();
+            float4 w[RW];
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                if (s0 + u < ns) {
-                    const float* x0 = xs + (s0 + u) * STEP + lane * 4;
+            for (int r = 0; r < RW; ++r) w[r] = *reinterpret_cast<const float4*>(ring + (slot * RW + r) * STEP);
+            copy_next(used);
+            used = slot;
+            slot = slot == U - 1 ? 0 : slot + 1;
 #pragma unroll
-                    for (int m = 0; m < MT; ++m) {
-                        const float4 x = *reinterpret_cast<const float4*>(x0 + m * width);
+            for (int m = 0; m < MT; ++m) {
+                const float4 x = *reinterpret_cast<const float4*>(x0 + m * width);
 #pragma unroll
-                        for (int r = 0; r < RW; ++r) {
-                            float a = acc[r * MT + m];
-                            a = fmaf(w[u][r].x, x.x, a);
-                            a = fmaf(w[u][r].y, x.y, a);
-                            a = fmaf(w[u][r].z, x.z, a);
-                            a = fmaf(w[u][r].w, x.w, a);
-                            acc[r * MT + m] = a;
-                        }
-                    }
+                for (int r = 0; r < RW; ++r) {
+                    float a = acc[r * MT + m];
+                    a = fmaf(w[r].x, x.x, a);
+                    a = fmaf(w[r].y, x.y, a);
+                    a = fmaf(w[r].z, x.z, a);
+                    a = fmaf(w[r].w, x.w, a);
+                    acc[r * MT + m] = a;
                 }
-                // the registers just used take the step U further on, of this group of rows or of the next
-                const int next = s0 + u + U;
-                if (next < ns_up) load(w[u], group, next);
-                else load(w[u], group + stride, next - ns_up);
             }
         }
         const int at = reduce_lanes(acc, lane);
         constexpr int HELD = RW * MT >= 32 ? RW * MT / 32 : 1;
         if (RW * MT >= 32 || (lane & (32 / (RW * MT) - 1)) == 0) {
 #pragma unroll
-            for (int i = 0; i < HELD; ++i) sums[turn][warp * RW * MT + at + i] = acc[i];
+            for (int i = 0; i < HELD; ++i) {
+                if (splits == 1) {
+                    sums[turn][warp * RW * MT + at + i] = acc[i];
+                } else {                         // to the block that finishes this output
+                    const int r = (at + i) / MT, m = (at + i) % MT;
+                    const int o = m * GROUP + warp * FEATS + (DUAL ? r / 2 : r), owner = o / each;
+                    store_peer_float(&sums[turn][(DUAL ? 2 : 1) * (rank * each + o - owner * each) + (DUAL ? r & 1 : 0)], (uint32_t)owner, acc[i]);
+                }
+            }
         }
         if (splits > 1) cluster_sync(); else __syncthreads();
-        // outputs (feature of the group, row of X), the feature fastest; the cluster's blocks share them out
-        const int total = GROUP * MT, from = total * rank / splits, to = total * (rank + 1) / splits;
         for (int i = from + threadIdx.x; i < to; i += FEW_THREADS) {
             const int m = i / GROUP, fl = i - m * GROUP, f = group * GROUP + fl;
             if (m >= M || f >= N) continue;
-            const int slot = ((fl / FEATS) * RW + (fl % FEATS) * (DUAL ? 2 : 1)) * MT + m;
             float v = 0.f, up = 0.f;
             if (splits > 1) {
                 for (int p = 0; p < splits; ++p) {
-                    v += peer_float(&sums[turn][slot], (uint32_t)p);
-                    if (DUAL) up += peer_float(&sums[turn][slot + MT], (uint32_t)p);
+                    const float* piece = &sums[turn][(DUAL ? 2 : 1) * (p * each + i - from)];
+                    v += piece[0];
+                    if (DUAL) up += piece[1];
                 }
             } else {
+                const int slot = ((fl / FEATS) * RW + (fl % FEATS) * (DUAL ? 2 : 1)) * MT + m;
                 v = sums[turn][slot];
                 if (DUAL) up = sums[turn][slot + MT];
             }
-            finish<MODE>(out, (size_t)m * N + f, f, v, up, bias, forms);
+            const size_t o = (size_t)m * N + f;
+            if (MODE == 2) out[o] = (i < from + FEW_THREADS ? old : out[o]) + v;
+            else finish<MODE>(out, o, f, v, up, bias, forms);
         }
         // the other half of `sums` is next: whoever writes this half again has passed the barrier of the turn between
     }
-    if (splits > 1) cluster_sync();              // a peer may still be reading this block's sums
 }
 
-constexpr int FEW_SMEM_MAX = 200 * 1024;
+constexpr int FEW_SMEM_MAX = 200 * 1024, SM_SMEM = 227 * 1024;
+
+// Slots of a warp's ring, with the X of a block in `x_bytes`, and blocks per SM: the deeper ring while three blocks still fit an SM (one row
+// of X: 887 -> 760 us a step as above with 8 slots).
+constexpr int few_slots_least(int rw) { return rw == 2 ? 4 : 3; }
+constexpr int few_slots_most(int rw) { return rw == 2 ? 8 : 4; }
+int few_slots(int rw, long long x_bytes) {
+    return x_bytes + 4ll * few_ring_floats(rw, few_slots_most(rw)) <= 74 * 1024 ? few_slots_most(rw) : few_slots_least(rw);
+}
+int few_per_sm(int rows, long long smem) { return max(1, min(rows > 8 ? 2 : 3, (int)(SM_SMEM / (smem + (rows > 8 ? 6 : 3) * 1024)))); }
 
 // How a product of few rows is cut: blocks along K (0: X does not fit shared memory in any cut).
-int few_splits(int rows, int group, int N, int K) {
+int few_splits(int rows, int rw, int group, int N, int K) {
     const int steps = (K + STEP - 1) / STEP, groups = (N + group - 1) / group;
     int best = 0;
     long long best_cost = 0;
     for (int s = 1; s <= 8 && s <= steps; s *= 2) {
         const int per = (steps + s - 1) / s;
-        const long long smem = (long long)rows * per * STEP * 4;
+        const long long x_bytes = (long long)rows * per * STEP * 4, smem = x_bytes + 4ll * few_ring_floats(rw, few_slots(rw, x_bytes));
         if (smem > FEW_SMEM_MAX) continue;
-        const int resident = (smem > 100 * 1024 ? 1 : smem > 66 * 1024 || rows > 8 ? 2 : 3) * sm_count() / s;      // clusters
+        const int resident = few_per_sm(rows, smem) * sm_count() / s;      // clusters
         // rounds of the persistent grid times the steps of one, and what a round costs besides (about two steps; four
         // where the pieces meet across blocks)
         const long long rounds = (groups + resident - 1) / resident;
@@ -201,11 +255,13 @@ int launch_few(const float* X, const float* W, const float* W2, const float* bia
                cudaStream_t stream) {
     constexpr int GROUP = FEW_WARPS * (MODE == 3 ? RW / 2 : RW);
     const int steps = (K + STEP - 1) / STEP, groups = (N + GROUP - 1) / GROUP;
-    const size_t smem = (size_t)MT * ((steps + splits - 1) / splits) * STEP * 4;
+    const long long x_bytes = (long long)MT * ((steps + splits - 1) / splits) * STEP * 4;
+    if constexpr (U == few_slots_least(RW))
+        if (few_slots(RW, x_bytes) != U) return launch_few<MT, RW, few_slots_most(RW), MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
+    const size_t smem = (size_t)x_bytes + 4 * few_ring_floats(RW, U);
     static PerDeviceOnce once;
     if (int rc = raise_dynamic_smem(gemm_f32_few_kernel<MT, RW, U, MODE>, FEW_SMEM_MAX, once, "gemm_f32")) return rc;
-    const int per_sm = smem > 100 * 1024 ? 1 : smem > 66 * 1024 || MT > 8 ? 2 : 3;
-    const int clusters = max(1, min(groups, per_sm * sm_count() / splits));
+    const int clusters = max(1, min(groups, few_per_sm(MT, smem) * sm_count() / splits));
     return launch_cluster("gemm_f32 (few rows)", gemm_f32_few_kernel<MT, RW, U, MODE>, dim3(clusters * splits), FEW_THREADS, smem, splits,
                           stream, X, W, W2, bias, out, M, N, K, steps, splits);
 }
@@ -537,13 +593,13 @@ int dispatch(const float* X, const float* W, const float* W2, const float* bias,
     if (M <= few_max) {
         const int rows = M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : M <= 8 ? 8 : 16;
         const int rw = rows <= 4 ? 2 : 4;
-        const int splits = few_splits(rows, FEW_WARPS * (MODE == 3 ? rw / 2 : rw), N, K);
+        const int splits = few_splits(rows, rw, FEW_WARPS * (MODE == 3 ? rw / 2 : rw), N, K);
         if (splits > 0) {
-            if (rows == 1) return launch_few<1, 2, 4, MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
-            if (rows == 2) return launch_few<2, 2, 4, MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
-            if (rows == 4) return launch_few<4, 2, 4, MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
-            if (rows == 8) return launch_few<8, 4, 2, MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
-            return launch_few<16, 4, 2, MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
+            if (rows == 1) return launch_few<1, 2, few_slots_least(2), MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
+            if (rows == 2) return launch_few<2, 2, few_slots_least(2), MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
+            if (rows == 4) return launch_few<4, 2, few_slots_least(2), MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
+            if (rows == 8) return launch_few<8, 4, few_slots_least(4), MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
+            return launch_few<16, 4, few_slots_least(4), MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
         }
     }
     if (M <= 32) return launch_split<32, MODE>(X, W, W2, bias, out, M, N, K, status, stream);
