@@ -280,7 +280,9 @@ attn_f32_kernel(const float* q, int q_ld, const float* __restrict__ kcache, cons
 // owns four channels of a few keys' values.  What bounds a step is the latency of a block's few pages: 16-row tiles of the kernel
 // above, which read every key through shared memory for all of their rows, took 17.1 us for four sequences of up to 700 positions
 // (6 query heads per kv head of 128, eight blocks each; the generic kernel 112); with this one the 28-layer step around it went
-// from 2,286 to 1,989 us.
+// from 2,286 to 1,989 us.  Positions, slots, pages and a first page that lies wholly before the step are read before the wait for the
+// kernel before: the chain of four dependent reads and the page's own is over when the queries come (with the float32 rotary kernel's
+// reads done likewise, 1,963 -> 1,894 us, products as they were).
 template <int HD, int ROWS>
 constexpr int few_smem_floats() { return ROWS * HD + 2 * ROWS * (KEYS + 4) + 4 * ROWS + 1024 / HD * ROWS * HD; }
 
@@ -306,10 +308,13 @@ attn_f32_few_kernel(const float* q, int q_ld, const float* __restrict__ kcache, 
     const int rank = splits > 1 ? (int)cluster_rank() : 0;
     const int kvh = blockIdx.y, seq = blockIdx.z;
     let_next_kernel_start();
-    wait_for_previous_kernels();
+    // positions, slots and pages are fixed before the step, and so are the keys and values of pages that lie wholly before it
     const int first_tok = cu_seqlens[seq], n_tok = cu_seqlens[seq + 1] - first_tok;
     const int n_rows = n_tok * n_rep;            // at most ROWS
-    if (n_rows == 0) return;                     // a whole cluster at once
+    if (n_rows == 0) {                           // a whole cluster at once
+        wait_for_previous_kernels();             // (who waits for this kernel waits for those before it too)
+        return;
+    }
     const int start = seq_start[seq];
     const int* pages = page_table + (size_t)seq_slot[seq] * max_pages;
     const int page_end = (start + n_tok - 1) / KEYS + 1;
@@ -334,8 +339,16 @@ attn_f32_few_kernel(const float* q, int q_ld, const float* __restrict__ kcache, 
 #pragma unroll
         for (int i = 0; i < VN; ++i) vr[i] = load_written(src + i * HD);
     };
-    fetch_keys(page);
-    fetch_values(page);
+    const bool older = (page + 1) * KEYS <= start;
+    if (older) {
+        fetch_keys(page);
+        fetch_values(page);
+    }
+    wait_for_previous_kernels();
+    if (!older) {
+        fetch_keys(page);
+        fetch_values(page);
+    }
     for (int i = tid * 4; i < ROWS * HD; i += THREADS * 4) {
         const int r = i / HD, d = i % HD;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);

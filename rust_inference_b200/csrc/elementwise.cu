@@ -3,6 +3,7 @@
 //
 // The residual stream is float32 in both precisions; `T` is the activation/storage
 // type (float or bf16).  Statistics, rotation and SiLU are computed in float32.
+#include <type_traits>
 #include "common.cuh"
 
 using namespace ri;
@@ -523,15 +524,36 @@ __global__ void rope_cache_write_kernel(T* __restrict__ qkv, int ld, const float
     }
 }
 
-// The same for bf16 rows whose head size and rotated channels are multiples of 16 (values: of 8), moved 16 bytes at a time: a
+// eight elements: as floats, back, and from one place to another
+__device__ __forceinline__ void load8(const __nv_bfloat16* p, float* f) { unpack8(*reinterpret_cast<const uint4*>(p), f); }
+__device__ __forceinline__ void store8(__nv_bfloat16* p, const float* f) { *reinterpret_cast<uint4*>(p) = pack8(f); }
+__device__ __forceinline__ void copy8(__nv_bfloat16* to, const __nv_bfloat16* from) {
+    *reinterpret_cast<uint4*>(to) = *reinterpret_cast<const uint4*>(from);
+}
+__device__ __forceinline__ void load8(const float* p, float* f) {
+    *reinterpret_cast<float4*>(f) = *reinterpret_cast<const float4*>(p);
+    *reinterpret_cast<float4*>(f + 4) = *reinterpret_cast<const float4*>(p + 4);
+}
+__device__ __forceinline__ void store8(float* p, const float* f) {
+    *reinterpret_cast<float4*>(p) = *reinterpret_cast<const float4*>(f);
+    *reinterpret_cast<float4*>(p + 4) = *reinterpret_cast<const float4*>(f + 4);
+}
+__device__ __forceinline__ void copy8(float* to, const float* from) {
+    __align__(16) float f[8];
+    load8(from, f);
+    store8(to, f);
+}
+
+// The same for rows whose head size and rotated channels are multiples of 16 (values: of 8), moved 8 elements at a time: a
 // thread takes 8 consecutive elements of a head (and, for the half-split pairing, their 8 partners half the rotated channels
 // on), rotates them in float32 and writes them back the same way; channels behind the rotated ones are copied for keys and
-// stay where they are for queries.  (2,048 tokens of 16 + 4 heads of 128 with 64 rotated channels: 7.9 us, 11.5 element by element.)
-__global__ void rope_cache_write_vec_kernel(__nv_bfloat16* __restrict__ qkv, int ld, const float* __restrict__ cos_t,
+// stay where they are for queries.  (2,048 tokens of 16 + 4 heads of 128 with 64 rotated channels in bfloat16: 7.9 us, 11.5 element by element.)
+template <typename T>
+__global__ void rope_cache_write_vec_kernel(T* __restrict__ qkv, int ld, const float* __restrict__ cos_t,
                                             const float* __restrict__ sin_t, const int* __restrict__ token_pos,
                                             const int* __restrict__ token_seq, const int* __restrict__ seq_slot,
                                             const int* __restrict__ page_table, int max_pages,
-                                            __nv_bfloat16* __restrict__ kcache, __nv_bfloat16* __restrict__ vcache,
+                                            T* __restrict__ kcache, T* __restrict__ vcache,
                                             int n_heads, int n_kv_heads, int hd, int page_size, int style,
                                             int write_kv, int rot, int v_hd) {
     const int t = blockIdx.x;
@@ -556,17 +578,17 @@ __global__ void rope_cache_write_vec_kernel(__nv_bfloat16* __restrict__ qkv, int
     const size_t cache_base = cache_row * hd, head_stride = (size_t)page_size * hd;
     const size_t v_base = cache_row * v_hd, v_head_stride = (size_t)page_size * v_hd;
     wait_for_previous_kernels();          // the projections come from the previous kernel
-    __nv_bfloat16* row = qkv + (size_t)t * ld;
+    T* row = qkv + (size_t)t * ld;
 
     const int heads = n_heads + (write_kv ? n_kv_heads : 0);
     if (style == 0) {
         const int per_head = half / 8;                // rotated chunk pairs of a head
         for (int idx = threadIdx.x; idx < heads * per_head; idx += blockDim.x) {
             const int h = idx / per_head, j = idx % per_head;
-            const __nv_bfloat16* src = row + (size_t)h * hd + 8 * j;      // q heads, then k heads: one run of columns
-            float lo[8], hi[8], cs[8], sn[8], ylo[8], yhi[8];
-            unpack8(*reinterpret_cast<const uint4*>(src), lo);
-            unpack8(*reinterpret_cast<const uint4*>(src + half), hi);
+            const T* src = row + (size_t)h * hd + 8 * j;      // q heads, then k heads: one run of columns
+            __align__(16) float lo[8], hi[8], cs[8], sn[8], ylo[8], yhi[8];
+            load8(src, lo);
+            load8(src + half, hi);
             *reinterpret_cast<float4*>(cs) = *reinterpret_cast<const float4*>(c + 8 * j);
             *reinterpret_cast<float4*>(cs + 4) = *reinterpret_cast<const float4*>(c + 8 * j + 4);
             *reinterpret_cast<float4*>(sn) = *reinterpret_cast<const float4*>(s + 8 * j);
@@ -576,18 +598,18 @@ __global__ void rope_cache_write_vec_kernel(__nv_bfloat16* __restrict__ qkv, int
                 ylo[i] = lo[i] * cs[i] - hi[i] * sn[i];
                 yhi[i] = lo[i] * sn[i] + hi[i] * cs[i];
             }
-            __nv_bfloat16* dst = h < n_heads ? row + (size_t)h * hd + 8 * j
+            T* dst = h < n_heads ? row + (size_t)h * hd + 8 * j
                                              : kcache + cache_base + (size_t)(h - n_heads) * head_stride + 8 * j;
-            *reinterpret_cast<uint4*>(dst) = pack8(ylo);
-            *reinterpret_cast<uint4*>(dst + half) = pack8(yhi);
+            store8(dst, ylo);
+            store8(dst + half, yhi);
         }
     } else {
         const int per_head = rot / 8;                 // rotated chunks of a head, 4 adjacent pairs each
         for (int idx = threadIdx.x; idx < heads * per_head; idx += blockDim.x) {
             const int h = idx / per_head, j = idx % per_head;
-            const __nv_bfloat16* src = row + (size_t)h * hd + 8 * j;
-            float x[8], y[8], cs[4], sn[4];
-            unpack8(*reinterpret_cast<const uint4*>(src), x);
+            const T* src = row + (size_t)h * hd + 8 * j;
+            __align__(16) float x[8], y[8], cs[4], sn[4];
+            load8(src, x);
             *reinterpret_cast<float4*>(cs) = *reinterpret_cast<const float4*>(c + 4 * j);
             *reinterpret_cast<float4*>(sn) = *reinterpret_cast<const float4*>(s + 4 * j);
 #pragma unroll
@@ -595,22 +617,20 @@ __global__ void rope_cache_write_vec_kernel(__nv_bfloat16* __restrict__ qkv, int
                 y[2 * i] = x[2 * i] * cs[i] - x[2 * i + 1] * sn[i];
                 y[2 * i + 1] = x[2 * i] * sn[i] + x[2 * i + 1] * cs[i];
             }
-            __nv_bfloat16* dst = h < n_heads ? row + (size_t)h * hd + 8 * j
+            T* dst = h < n_heads ? row + (size_t)h * hd + 8 * j
                                              : kcache + cache_base + (size_t)(h - n_heads) * head_stride + 8 * j;
-            *reinterpret_cast<uint4*>(dst) = pack8(y);
+            store8(dst, y);
         }
     }
     if (!write_kv) return;
     const int rest = (hd - rot) / 8, v_chunks = v_hd / 8;
     for (int idx = threadIdx.x; idx < n_kv_heads * rest; idx += blockDim.x) {
         const int h = idx / rest, j = rot + 8 * (idx % rest);
-        *reinterpret_cast<uint4*>(kcache + cache_base + (size_t)h * head_stride + j) =
-            *reinterpret_cast<const uint4*>(row + q_dim + (size_t)h * hd + j);
+        copy8(kcache + cache_base + (size_t)h * head_stride + j, row + q_dim + (size_t)h * hd + j);
     }
     for (int idx = threadIdx.x; idx < n_kv_heads * v_chunks; idx += blockDim.x) {
         const int h = idx / v_chunks, j = idx % v_chunks;
-        *reinterpret_cast<uint4*>(vcache + v_base + (size_t)h * v_head_stride + 8 * j) =
-            *reinterpret_cast<const uint4*>(row + q_dim + kv_dim + (size_t)h * v_hd + 8 * j);
+        copy8(vcache + v_base + (size_t)h * v_head_stride + 8 * j, row + q_dim + kv_dim + (size_t)h * v_hd + 8 * j);
     }
 }
 
@@ -629,12 +649,16 @@ RI_API int ri_rope_cache_write(void* qkv, int dtype, int ld, const float* cos_t,
     cudaError_t e = cudaSuccess;
     const bool aligned = rot % 16 == 0 && v_hd % 8 == 0 && hd % 16 == 0 && ld % 8 == 0 && (uintptr_t)qkv % 16 == 0 && (uintptr_t)kcache % 16 == 0 &&
                          (uintptr_t)vcache % 16 == 0 && (uintptr_t)cos_t % 16 == 0 && (uintptr_t)sin_t % 16 == 0;
-    if (dtype == RI_BF16 && aligned) {
+    if (aligned && (dtype == RI_BF16 || dtype == RI_F32)) {
         const int items = (n_heads + n_kv_heads) * hd / 16;
         const int vthreads = items >= 256 ? 256 : (items >= 128 ? 128 : 64);
-        e = launch_dependent(rope_cache_write_vec_kernel, n_tokens, vthreads, 0, stream,
-            (__nv_bfloat16*)qkv, ld, cos_t, sin_t, token_pos, token_seq, seq_slot, page_table, max_pages,
-            (__nv_bfloat16*)kcache, (__nv_bfloat16*)vcache, n_heads, n_kv_heads, hd, page_size, style, write_kv, rot, v_hd);
+        auto launch = [&](auto* rows) {
+            using T = std::remove_pointer_t<decltype(rows)>;
+            return launch_dependent(rope_cache_write_vec_kernel<T>, n_tokens, vthreads, 0, stream,
+                rows, ld, cos_t, sin_t, token_pos, token_seq, seq_slot, page_table, max_pages,
+                (T*)kcache, (T*)vcache, n_heads, n_kv_heads, hd, page_size, style, write_kv, rot, v_hd);
+        };
+        e = dtype == RI_F32 ? launch((float*)qkv) : launch((__nv_bfloat16*)qkv);
         return check_launch(e, "rope_cache_write");
     }
     if (dtype == RI_F32)
