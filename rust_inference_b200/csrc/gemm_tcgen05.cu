@@ -16,11 +16,12 @@
 // The grid is persistent: as many CTAs as fit the GPU at once, each walking its share of
 // the output tiles (token tile fastest, so CTAs that run together share a weight tile in
 // L2).  Warp 0 issues the TMA loads, warp 1 allocates tensor memory and issues the MMAs
-// (one elected thread), warps 2-5 run the epilogue: each reads its 32 lanes of the
+// (one elected lane of a warp that stays together), warps 2-5 run the epilogue: each reads its 32 lanes of the
 // accumulator with tcgen05.ld and writes the result.  There are two accumulator buffers
 // in tensor memory, so the epilogue of one tile runs while the MMAs of the next fill the
 // other.  K can be split over tiles; the split pieces are combined with float32 atomic
-// adds, which only the residual epilogue allows.
+// adds, which only the residual epilogue allows.  The other epilogues cut K over the CTAs of
+// a cluster for steps of up to 16 tokens, the pieces meeting in shared memory.
 //
 // Epilogues (float32 arithmetic):
 //   0  out<bf16> = acc + bias                         (q/k/v projection, attention.rs:66-76)
@@ -1088,7 +1089,8 @@ int pick_tile(int tn, const CUtensorMap& mw, const CUtensorMap& mw2, const CUten
 // in two or three, whichever leaves the SMs more evenly filled, as long as all CTAs are resident together (two to an SM).
 // Whole decode steps, us, not cut / 2 / 3 / 4: 38 tiles of K = 896 (24 layers), 1 token 690 / 648 / 650 / 633, 8 tokens 757 / 713 / 692 /
 // 675; 70 tiles of 1,536 (28), 1 token 1,059 / 985 / 1,025 / 1,000, 12 tokens 1,140 / 1,130 / 1,144 / 1,203; 86 tiles of 2,048 (36), 1 token
-// 1,629 / 1,604 / 1,576 / 1,758; 112 tiles of 4,096 (32), 1 token 2,835 / 2,670 / 2,925 / 2,828.
+// 1,629 / 1,604 / 1,576 / 1,758; 112 tiles of 4,096 (32), 1 token 2,835 / 2,670 / 2,925 / 2,828.  (Gated products.  With those that store
+// their results cut likewise: decode steps of 8 sequences of a 2,048-wide routed decoder 486 -> 448, of a latent one 271 -> 261.)
 int cluster_split(int n_tok, int n_feat, int K) {
     const int total_kb = (K + BLOCK_K - 1) / BLOCK_K, sms = sm_count();
     const long long tiles = (n_feat + BLOCK_F - 1) / BLOCK_F;
@@ -1114,20 +1116,21 @@ RI_API int ri_gemm_tcgen05_set_pairs(int n_tok, int always) {
 }
 
 // How a product of n_tok tokens, n_feat features and inner size K is cut: the token tile (rows of the
-// activation box, written to *tile) and, for the residual epilogue (mode 2, the only one that can
-// add partial sums), over how many pieces K is split (*split; 1 for the other modes).
+// activation box, written to *tile) and over how many pieces K is split (*split): tiles
+// whose pieces are added to the residual stream (mode 2), CTAs of a cluster in the other modes (`cluster_split`; 1 beyond 16 tokens).
 //
 //  up to 128 tokens   one token tile, as narrow as the step allows.  Such steps stream weights:
 //                     measured in a replayed graph at 8 tokens, the o, q/k/v and down projections of
 //                     a 3584-wide model are fastest with about two CTAs per SM (7-10 pieces) and at
 //                     least 4 k-blocks per piece (more for wider steps, whose pieces end in more atomics).
 //  beyond, SiLU-gate  the token-major kernel, 128 tokens per tile.
-//  beyond, others     the feature-major kernel.  Measured at 192..4,096 tokens: a k-block takes about
-//                     as long whatever the tile's width (128..256), so what counts is how many rounds
-//                     the persistent grid makes and how long a work item's K run is.  Every width of
-//                     128..256 and every split is tried on depth x (k-blocks per item + a dozen for
-//                     the item's epilogue and ramp); ties go to the narrower tile.  (Down projection
-//                     of 512 tokens: 256 x 5 pieces, 63.5 us, against 128 x 2, 100 us.)
+//  beyond, others     the feature-major kernel.  What counts is how many rounds the persistent grid
+//                     makes and how long a work item's K run is.  Every width of 128..256 and every
+//                     split is tried on depth x (k-blocks per item + a dozen for the item's epilogue
+//                     and ramp); ties go to the narrower tile.  Products onto the residual stream of
+//                     200..1,000 tokens would gain from narrower tiles in fewer pieces (512 x 1,536 x
+//                     1,536: 256 tokens in 6 pieces 12.2 us, 64 in 3 8.7; 512 x 896 x 4,864: 13.4
+//                     against 10.1); the plan does not try them.
 RI_API int ri_gemm_tcgen05_plan(int n_tok, int n_feat, int K, int mode, int* tile, int* split) {
     const long long feat_tiles = (n_feat + BLOCK_F - 1) / BLOCK_F;
     const long long ctas = sm_count();

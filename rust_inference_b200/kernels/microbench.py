@@ -407,13 +407,16 @@ def step_parts(model: dict, batch: int, prompt_min: int = 128, prompt_max: int =
         return gemm
 
     noop = lambda *a, **k: None
+    real_rope = ops.rope_cache_write_acc
+    no_rope = lambda *a, attend=None, **k: real_rope(*a, attend=attend, **k) if attend is not None else None
     qd, kvd, h, inter = cfg.q_dim, cfg.kv_dim, cfg.hidden_size, cfg.intermediate_size
     full = time_step()
     out = {"kernel": "step_parts", "tokens": batch, "layers": cfg.num_hidden_layers, "step_us": full, "without_us": {}}
     cases = {
         "sampler": lambda: time_step(sampler=None),
-        "attention": lambda: without([(attention_part.attn_kernels, "attention", noop)]),
-        "rope_cache_write": lambda: without([(ops, "rope_cache_write_acc", noop), (ops, "rope_cache_write", noop)]),
+        # (where the attention forms the heads itself, leaving it out leaves out the rotary encoding and the cache write too)
+        "attention": lambda: without([(attention_part.attn_kernels, "attention", noop), (attention_part.attn_kernels.FormedHeads, "run", noop)]),
+        "rope_cache_write": lambda: without([(ops, "rope_cache_write_acc", no_rope), (ops, "rope_cache_write", noop)]),
         "rmsnorm": lambda: without([(ops, "rmsnorm", lambda x, w, eps, out, rows=None: out)]),
         "qkv_gemm": lambda: without([(tcgen05, "gemm", gemm_except(lambda w, mode: w.n == qd + 2 * kvd and w.k == h))]),
         "o_gemm": lambda: without([(tcgen05, "gemm", gemm_except(lambda w, mode: w.n == h and w.k == qd and mode == ops.EPI_RESIDUAL))]),
