@@ -237,7 +237,12 @@ __device__ __forceinline__ void let_next_kernel_start(int line = __builtin_LINE(
     timeline_entry(line);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// the two halves, for a kernel that holds the next one back until it is done
+__device__ __forceinline__ void note_kernel_start(int line = __builtin_LINE()) { timeline_entry(line); }
+__device__ __forceinline__ void release_next_kernel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #else
+__device__ __forceinline__ void note_kernel_start() {}
+__device__ __forceinline__ void release_next_kernel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #define RI_PHASE(k) ((void)0)
 #define RI_PHASE_LATEST(k) ((void)0)
 __device__ __forceinline__ void wait_for_previous_kernels() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

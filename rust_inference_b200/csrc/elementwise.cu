@@ -1275,6 +1275,7 @@ __global__ void advance_decode_kernel(int* __restrict__ token_pos, int* __restri
                                       int* __restrict__ draw_counter, int* __restrict__ turn,
                                       int* __restrict__ host_ring, int host_slots, int* __restrict__ log_ring,
                                       int log_slots) {
+    note_kernel_start();
     wait_for_previous_kernels();          // every kernel of the step has read the arrays; the sampler has written the tokens
     const int t = turn ? *turn : 0;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -1292,7 +1293,7 @@ __global__ void advance_decode_kernel(int* __restrict__ token_pos, int* __restri
     __syncthreads();                      // everyone has read *turn
     if (threadIdx.x == 0 && turn) *turn = t + 1;
     __threadfence();
-    let_next_kernel_start();
+    release_next_kernel();
 }
 
 RI_API int ri_advance_decode(int* token_pos, int* seq_start, int* seq_len, int n, const int* token_ids,
