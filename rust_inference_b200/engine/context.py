@@ -85,6 +85,7 @@ class StepContext:
     device: torch.device
     workspace: Workspace
     extras: dict = field(default_factory=dict)
+    routed: bool = False          # the decoder chooses experts token by token (`DecoderModel.routed`)
     # host copies of the per-sequence arrays (None inside a captured graph, whose arrays change
     # between replays): for parts that are not graph_safe
     host_slots: list | None = None

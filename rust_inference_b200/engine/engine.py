@@ -197,6 +197,7 @@ class Engine:
             logit_rows=view("logit_rows"), n_logit_rows=sc["n_logit_rows"], max_new=sc["max_new"],
             max_len=sc["max_len"], all_single=sc["all_single"], page_table=self.cache.page_table,
             page_size=self.cache.page_size, dtype=self.dtype, device=self.device, workspace=self.workspace,
+            routed=self.model.routed,
             host_slots=sc["host"][0], host_starts=sc["host"][1], host_counts=sc["host"][2])
 
     def step(self, slots: list, tokens: list, wants="last", borrow: bool = False, probe=None):

@@ -84,7 +84,7 @@ class DecodeGraph:
             seq_len=view("seq_len"), cu_seqlens=view("cu_seqlens"), logit_rows=view("logit_rows"),
             n_logit_rows=n_seqs, max_new=1, max_len=engine.max_seq_len, all_single=True,
             page_table=engine.cache.page_table, page_size=engine.cache.page_size, dtype=engine.dtype,
-            device=dev, workspace=engine.workspace, extras={"graph": True})
+            device=dev, workspace=engine.workspace, extras={"graph": True}, routed=engine.model.routed)
 
     # ---- what the static arrays hold ------------------------------------------------------
     def holds(self, slots: list, starts: list, streams=None, counters=None, seed=None) -> bool:

@@ -90,6 +90,8 @@ class DecoderModel:
         self.head = _build("head", self._head_spec, **kw)
         self.stream_parts = [_build("stream", ps, **kw) for ps in spec.stream_parts]
 
+        self.routed = any(part.routes for layer in self.layers for part in layer.parts.values())
+
         # the schedule: who writes which cache layer
         seen = set()
         self.schedule = []

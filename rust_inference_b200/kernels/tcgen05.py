@@ -183,7 +183,9 @@ def gemm(x: torch.Tensor, w, out: torch.Tensor, mode: int, ctx=None, bias=None, 
         return out
     tile, planned = plan(m, n, k, mode)
     if split_k is None:
-        split_k = planned
+        # a decoder that routes has K cut only where the pieces meet on the residual stream: in a cluster they make other sums than
+        # the uncut product, and a near tie of a router's scores turns them into another expert
+        split_k = 1 if getattr(ctx, "routed", False) and mode != ops.EPI_RESIDUAL else planned
     map_x = _x_map(x, tile)
     st = status_word()
     _call("gemm_tcgen05", "ri_gemm_tcgen05", c_void_p(map_x.data_ptr()), c_void_p(weight_map(w).data_ptr()),

@@ -333,6 +333,8 @@ class GQAttention(Mixer):
         if (not ctx.all_single or self.extended or self.value_mix is not None or not writes_cache or self.v_head_dim != self.head_dim
                 or not hasattr(self.position, "apply_and_store_from_accumulators") or not linear.wants_split(x, self.w_qkv)):
             return False
+        if getattr(ctx, "routed", False) and (getattr(self.position, "partial", False) or self.qk_norm_eps is not None or self.values_from_keys or self.out_scale != 1.0):
+            return False                # not the bits of the kernels it replaces: see `Part.routes`
         mixed = ctx.buffer("attn_out", (x.shape[0], self.o_dim), self.dtype)
         attend = attn_kernels.formed_heads(
             mixed, ctx, width, n_heads=self.n_heads, n_kv_heads=self.n_kv_heads, head_dim=self.head_dim,

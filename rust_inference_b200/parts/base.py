@@ -21,6 +21,10 @@ class Part:
     # False if `forward` needs the host between kernels (reads a tensor back, loops in Python
     # over device data): the engine then runs decode steps eagerly instead of replaying a graph.
     graph_safe = True
+    # True if the part chooses by comparing what it computes (a router): where two scores nearly tie, a difference of rounding
+    # before it becomes another choice, so a decoder with such a part keeps its products' sums and its heads' roundings as they are
+    # for any number of tokens (`StepContext.routed`).
+    routes = False
 
     def __init__(self, *, hidden_size: int, dtype: torch.dtype, device):
         self.hidden_size = hidden_size

@@ -159,6 +159,8 @@ class RoutedExperts(FeedForward):
                 out[nm["shared_mix"]] = self.shared_mix.view(1, -1)
         return out
 
+    routes = True
+
     # steps of more tokens than this run the experts' products on the tensor cores (tiles of 128 rows of one
     # expert, their weights streamed by TMA) when the sizes allow; the FFMA form is the 32-bit path and
     # the fallback for other sizes
