@@ -56,6 +56,21 @@ def test_wide_products_with_infinities_keep_their_neighbours(splits):
     assert torch.equal(got[rows][:, cols], clean[rows][:, cols])
 
 
+@pytest.mark.parametrize("splits", [1, 2])
+@pytest.mark.parametrize("size", [0.0, 2.0 ** -70, 2.0 ** -50, 2.0 ** -48])
+def test_wide_products_add_to_subnormal_numbers(size, splits):
+    """Sums of nothing, of 2^-140, and on both sides of 2^-100, added to subnormal numbers and to what nearly cancels them."""
+    ops = _ops()
+    x, w = torch.zeros(70, 192, device=DEV), torch.zeros(130, 192, device=DEV)
+    x[:, 0], w[:, 0] = size, size * 1.25
+    v = torch.tensor(size).float() * (size * 1.25)
+    out = torch.full((70, 130), 2.0 ** -139, device=DEV)
+    out[:, 1::3], out[:, 2::3] = 3 * 2.0 ** -149, -v.item() * (1.0 + 2.0 ** -23)
+    want = out.cpu().clone() + v
+    ops.gemm_f32_wide(x, w, out, ops.EPI_RESIDUAL, splits=splits)
+    assert torch.equal(out.cpu(), want)
+
+
 def test_wide_products_refuse_what_they_cannot_cut():
     ops = _ops()
     x, w, out = torch.zeros(70, 64, device=DEV), torch.zeros(8, 64, device=DEV), torch.zeros(70, 8, device=DEV)
