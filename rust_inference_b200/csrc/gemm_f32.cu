@@ -2,7 +2,7 @@
 // every M (K a multiple of 4 and 16-byte aligned operands: rows are read 16 bytes at a time; `gemm_simt.cu` has the rest).
 //
 // Few rows of X (a decode step, up to FEW_MAX): the product is a read of W.  A warp owns a few rows of W, its lanes run
-// along K with 16-byte asynchronous copies into a ring of their own, several steps ahead, and every weight meets all rows of X,
+// along K with 16-byte asynchronous copies into a ring of their own (or loads), several steps ahead, and every weight meets all rows of X,
 // which lie in shared memory too; FFMA, float32 sums.  K is cut over the thread blocks of a cluster when N alone has too few
 // rows to keep the memory busy; the pieces meet through distributed shared memory in a fixed order, so a product's bits do
 // not change from run to run.
@@ -38,10 +38,10 @@ namespace {
 // Few rows of X.
 //
 // Bound by the read of W.  Every lane copies its 16 bytes of a row and step into a ring in shared memory and reads only what it
-// copied itself, so no warp waits for another: 3 to 7 steps of 512 bytes a row are on their way per warp (24 to 56 KiB per block),
-// across groups of rows and before the wait for the kernel before.  Loads into registers did the same on paper, but how many of
-// them a use waited for hung on how the compiler shared its scoreboards out (one more unused branch in the kernel changed a step
-// of a 0.5B-sized decoder from 887 to 797 us); X comes by such copies too.  Where K is cut over a cluster the pieces go straight to
+// copied itself, so no warp waits for another: 3 or 7 steps of 512 bytes a row are on their way per warp (up to four rows of X; 2 or 3
+// beyond; 24 to 56 KiB per block), across groups of rows and before the wait for the kernel before.  Loads into registers (4 or 2 steps of
+// them; RING false) do the same on paper and took a step of a 0.5B-sized decoder from 797 to 887 us, depending on an unused branch; they
+// are left where X leaves a ring too little room (`few_plan`).  X comes by such copies too.  Where K is cut over a cluster the pieces go straight to
 // the block that finishes an output, which reads them behind one meeting point.  A decode step of a 1.5B-sized decoder and 4 sequences:
 // 1,988 -> about 1,885 us, 0.5B-sized 933 -> 790 (1 sequence), 1,406 -> 1,270 (8).  Asking for the following weights to come into the L2
 // before the wait as well cost 1%.  A weight costs one FFMA per row of X and a 16-byte read of X from shared memory per RW of them:
@@ -86,7 +86,7 @@ __device__ __forceinline__ int reduce_lanes(float (&a)[N], int lane) {
     return first;
 }
 
-template <int MT, int RW, int U, int MODE>
+template <int MT, int RW, int U, int MODE, bool RING>
 __global__ void __launch_bounds__(FEW_THREADS, MT > 8 ? 2 : 3)
 gemm_f32_few_kernel(const float* X, const float* __restrict__ W, const float* __restrict__ W2,
                     const float* __restrict__ bias, float* out, int M, int N, int K, int steps, int splits) {
@@ -99,7 +99,7 @@ gemm_f32_few_kernel(const float* X, const float* __restrict__ W, const float* __
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float* ring = smem + warp * (U * RW * STEP) + lane * 4;  // [U][RW][STEP] per warp; a lane reads only what it copied itself
-    float* xs = smem + few_ring_floats(RW, U);               // [MT][this block's stretch of K]
+    float* xs = smem + (RING ? few_ring_floats(RW, U) : 0);  // [MT][this block's stretch of K]
     const int rank = splits > 1 ? (int)cluster_rank() : 0;
     const int first_step = (int)((long long)steps * rank / splits);
     const int ns = (int)((long long)steps * (rank + 1) / splits) - first_step;      // >= 1: splits <= steps
@@ -124,11 +124,25 @@ gemm_f32_few_kernel(const float* X, const float* __restrict__ W, const float* __
         }
         copies_commit();
     };
+    // without the ring: U steps in registers
+    float4 held[RING ? 1 : U][RW];
+    auto load = [&](float4 (&w)[RW], int group, int step) {
+        const int k = k0 + step * STEP + lane * 4, f = group * GROUP + warp * FEATS;
+        const bool in = step < ns && k < K && group < groups;
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+            const int row = min(DUAL ? f + r / 2 : f + r, N - 1);
+            const float* base = (DUAL && (r & 1)) ? W2 : W;
+            w[r] = in ? load_weight(base + (size_t)row * K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
 
     let_next_kernel_start();
     if (splits > 1) cluster_arrive();
 #pragma unroll
-    for (int u = 0; u < U - 1; ++u) copy_next(u);            // weights: written by no kernel
+    for (int u = 0; u < (RING ? U - 1 : U); ++u) {           // weights: written by no kernel
+        if constexpr (RING) copy_next(u); else load(held[u], group, u);
+    }
     wait_for_previous_kernels();
     // X: asynchronous copies too, all on their way at once (rows and columns beyond X become zeros)
     for (int m = 0, k = threadIdx.x * 4;; k += FEW_THREADS * 4) {
@@ -152,7 +166,7 @@ gemm_f32_few_kernel(const float* X, const float* __restrict__ W, const float* __
     int slot = 0, used = U - 1;                  // this step's slot, and the one of the step before it: free
     for (int turn = 0; group < groups; group += stride, turn ^= 1) {
         float old = 0.f;                         // what this thread's output is added to
-        if (MODE == 2) {
+        if (MODE == 2 && RING) {
             const int i = from + threadIdx.x, m = i / GROUP, f = group * GROUP + i - m * GROUP;
             if (i < to && m < M && f < N) old = out[(size_t)m * N + f];
         }
@@ -160,14 +174,7 @@ gemm_f32_few_kernel(const float* X, const float* __restrict__ W, const float* __
 #pragma unroll
         for (int i = 0; i < RW * MT; ++i) acc[i] = 0.f;
         const float* x0 = xs + lane * 4;
-        for (int s = 0; s < ns; ++s, x0 += STEP) {
-            copies_wait<U - 2>();
-            float4 w[RW];
-#pragma unroll
-            for (int r = 0; r < RW; ++r) w[r] = *reinterpret_cast<const float4*>(ring + (slot * RW + r) * STEP);
-            copy_next(used);
-            used = slot;
-            slot = slot == U - 1 ? 0 : slot + 1;
+        auto multiply = [&](const float4 (&w)[RW], const float* x0) {
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
                 const float4 x = *reinterpret_cast<const float4*>(x0 + m * width);
@@ -179,6 +186,30 @@ gemm_f32_few_kernel(const float* X, const float* __restrict__ W, const float* __
                     a = fmaf(w[r].z, x.z, a);
                     a = fmaf(w[r].w, x.w, a);
                     acc[r * MT + m] = a;
+                }
+            }
+        };
+        if constexpr (RING) {
+            for (int s = 0; s < ns; ++s, x0 += STEP) {
+                copies_wait<U - 2>();
+                float4 w[RW];
+#pragma unroll
+                for (int r = 0; r < RW; ++r) w[r] = *reinterpret_cast<const float4*>(ring + (slot * RW + r) * STEP);
+                copy_next(used);
+                used = slot;
+                slot = slot == U - 1 ? 0 : slot + 1;
+                multiply(w, x0);
+            }
+        } else {
+            const int ns_up = (ns + U - 1) / U * U;
+            for (int s0 = 0; s0 < ns_up; s0 += U) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (s0 + u < ns) multiply(held[u], x0 + (s0 + u) * STEP);
+                    // the registers just used take the step U further on, of this group of rows or of the next
+                    const int next = s0 + u + U;
+                    if (next < ns_up) load(held[u], group, next);
+                    else load(held[u], group + stride, next - ns_up);
                 }
             }
         }
@@ -213,14 +244,14 @@ gemm_f32_few_kernel(const float* X, const float* __restrict__ W, const float* __
                 if (DUAL) up = sums[turn][slot + MT];
             }
             const size_t o = (size_t)m * N + f;
-            if (MODE == 2) out[o] = (i < from + FEW_THREADS ? old : out[o]) + v;
+            if (MODE == 2) out[o] = (RING && i < from + FEW_THREADS ? old : out[o]) + v;
             else finish<MODE>(out, o, f, v, up, bias, forms);
         }
         // the other half of `sums` is next: whoever writes this half again has passed the barrier of the turn between
     }
 }
 
-constexpr int FEW_SMEM_MAX = 200 * 1024, SM_SMEM = 227 * 1024;
+constexpr int FEW_SMEM_MAX = 200 * 1024, SM_SMEM = 228 * 1024;
 
 // Slots of a warp's ring, with the X of a block in `x_bytes`, and blocks per SM: the deeper ring while three blocks still fit an SM (one row
 // of X: 887 -> 760 us a step as above with 8 slots).
@@ -229,41 +260,63 @@ constexpr int few_slots_most(int rw) { return rw == 2 ? 8 : 4; }
 int few_slots(int rw, long long x_bytes) {
     return x_bytes + 4ll * few_ring_floats(rw, few_slots_most(rw)) <= 74 * 1024 ? few_slots_most(rw) : few_slots_least(rw);
 }
-int few_per_sm(int rows, long long smem) { return max(1, min(rows > 8 ? 2 : 3, (int)(SM_SMEM / (smem + (rows > 8 ? 6 : 3) * 1024)))); }
+constexpr int few_held(int rw) { return rw == 2 ? 4 : 2; }            // steps in registers, without a ring
+int few_per_sm(int rows, int rw, long long smem) {         // (its own sums and 1 KB of the system's lie in a block's shared memory too)
+    return max(1, min(rows > 8 ? 2 : 3, (int)(SM_SMEM / (smem + 8 * (FEW_WARPS * rw * rows + 16) + 1024))));
+}
 
-// How a product of few rows is cut: blocks along K (0: X does not fit shared memory in any cut).
-int few_splits(int rows, int rw, int group, int N, int K) {
+// How a product of few rows is cut: blocks along K (0: another kernel), and whether the weights come through the ring.  A ring takes 32 or
+// 48 KB of a block that X may need; where fewer blocks fit an SM for it, registers are the better place.  us, ring / registers: 8 x 14,336
+// x 4,096 gated 150 / 105, 16 x 11,008 x 2,048 gated 91 / 61, 8 x 3,584 x 18,944 123 / 104, 16 x 32,000 x 2,048 127 / 82, 4 x 2,048 x
+// 40,960 123 / 86; where as many fit it is the ring: 8 x 8,960 x 1,536 gated 23 / 32, 8 x 4,608 x 3,584 15 / 22.  Over 230 shapes of 1 to
+// 16 rows the plan is on average within 5% of the best of both and all cuts.  (9 rows and more of which one block fills an SM without a
+// ring go to the tensor cores: 16 x 4,096 x 22,016 139 us, 270 from registers.)
+struct FewPlan { int splits; bool ring; };
+FewPlan few_plan(int rows, int rw, int group, int N, int K) {
     const int steps = (K + STEP - 1) / STEP, groups = (N + group - 1) / group;
-    int best = 0;
+    FewPlan best{0, true};
     long long best_cost = 0;
-    for (int s = 1; s <= 8 && s <= steps; s *= 2) {
-        const int per = (steps + s - 1) / s;
-        const long long x_bytes = (long long)rows * per * STEP * 4, smem = x_bytes + 4ll * few_ring_floats(rw, few_slots(rw, x_bytes));
-        if (smem > FEW_SMEM_MAX) continue;
-        const int resident = few_per_sm(rows, smem) * sm_count() / s;      // clusters
-        // rounds of the persistent grid times the steps of one, and what a round costs besides (about two steps; four
-        // where the pieces meet across blocks)
-        const long long rounds = (groups + resident - 1) / resident;
-        const long long cost = rounds * (per + (s > 1 ? 4 : 2));
-        if (best == 0 || cost < best_cost) { best = s; best_cost = cost; }
-    }
+    for (int ring = 1; ring >= 0; --ring)
+        for (int s = 1; s <= 8 && s <= steps; s *= 2) {
+            const int per = (steps + s - 1) / s;
+            const long long x_bytes = (long long)rows * per * STEP * 4;
+            const long long smem = x_bytes + (ring ? 4ll * few_ring_floats(rw, few_slots(rw, x_bytes)) : 0);
+            const int per_sm = few_per_sm(rows, rw, smem);
+            if (smem > FEW_SMEM_MAX || (!ring && rows > 8 && per_sm == 1)) continue;
+            const int resident = per_sm * sm_count() / s;      // clusters
+            // rounds of the persistent grid times the steps of one, and what a round costs besides (about three steps; four where the
+            // pieces meet across blocks); registers for 5% less
+            const long long rounds = (groups + resident - 1) / resident;
+            const long long cost = rounds * (per + (s > 1 ? 4 : 3)) * (ring ? 95 : 100);
+            if (best.splits == 0 || cost < best_cost) {
+                best = FewPlan{s, ring != 0};
+                best_cost = cost;
+            }
+        }
     return best;
 }
 
-template <int MT, int RW, int U, int MODE>
+template <int MT, int RW, int U, int MODE, bool RING>
 int launch_few(const float* X, const float* W, const float* W2, const float* bias, float* out, int M, int N, int K, int splits,
                cudaStream_t stream) {
     constexpr int GROUP = FEW_WARPS * (MODE == 3 ? RW / 2 : RW);
     const int steps = (K + STEP - 1) / STEP, groups = (N + GROUP - 1) / GROUP;
     const long long x_bytes = (long long)MT * ((steps + splits - 1) / splits) * STEP * 4;
-    if constexpr (U == few_slots_least(RW))
-        if (few_slots(RW, x_bytes) != U) return launch_few<MT, RW, few_slots_most(RW), MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
-    const size_t smem = (size_t)x_bytes + 4 * few_ring_floats(RW, U);
+    if constexpr (RING && U == few_slots_least(RW))
+        if (few_slots(RW, x_bytes) != U) return launch_few<MT, RW, few_slots_most(RW), MODE, true>(X, W, W2, bias, out, M, N, K, splits, stream);
+    const size_t smem = (size_t)x_bytes + (RING ? 4 * few_ring_floats(RW, U) : 0);
+    auto kernel = gemm_f32_few_kernel<MT, RW, U, MODE, RING>;
     static PerDeviceOnce once;
-    if (int rc = raise_dynamic_smem(gemm_f32_few_kernel<MT, RW, U, MODE>, FEW_SMEM_MAX, once, "gemm_f32")) return rc;
-    const int clusters = max(1, min(groups, few_per_sm(MT, smem) * sm_count() / splits));
-    return launch_cluster("gemm_f32 (few rows)", gemm_f32_few_kernel<MT, RW, U, MODE>, dim3(clusters * splits), FEW_THREADS, smem, splits,
-                          stream, X, W, W2, bias, out, M, N, K, steps, splits);
+    if (int rc = raise_dynamic_smem(kernel, FEW_SMEM_MAX, once, "gemm_f32")) return rc;
+    const int clusters = max(1, min(groups, few_per_sm(MT, RW, smem) * sm_count() / splits));
+    return launch_cluster("gemm_f32 (few rows)", kernel, dim3(clusters * splits), FEW_THREADS, smem, splits, stream, X, W, W2, bias, out, M, N,
+                          K, steps, splits);
+}
+template <int MT, int RW, int MODE>
+int launch_few(const FewPlan& p, const float* X, const float* W, const float* W2, const float* bias, float* out, int M, int N, int K,
+               cudaStream_t stream) {
+    return p.ring ? launch_few<MT, RW, few_slots_least(RW), MODE, true>(X, W, W2, bias, out, M, N, K, p.splits, stream)
+                  : launch_few<MT, RW, few_held(RW), MODE, false>(X, W, W2, bias, out, M, N, K, p.splits, stream);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -593,13 +646,13 @@ int dispatch(const float* X, const float* W, const float* W2, const float* bias,
     if (M <= few_max) {
         const int rows = M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : M <= 8 ? 8 : 16;
         const int rw = rows <= 4 ? 2 : 4;
-        const int splits = few_splits(rows, rw, FEW_WARPS * (MODE == 3 ? rw / 2 : rw), N, K);
-        if (splits > 0) {
-            if (rows == 1) return launch_few<1, 2, few_slots_least(2), MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
-            if (rows == 2) return launch_few<2, 2, few_slots_least(2), MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
-            if (rows == 4) return launch_few<4, 2, few_slots_least(2), MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
-            if (rows == 8) return launch_few<8, 4, few_slots_least(4), MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
-            return launch_few<16, 4, few_slots_least(4), MODE>(X, W, W2, bias, out, M, N, K, splits, stream);
+        const FewPlan p = few_plan(rows, rw, FEW_WARPS * (MODE == 3 ? rw / 2 : rw), N, K);
+        if (p.splits > 0) {
+            if (rows == 1) return launch_few<1, 2, MODE>(p, X, W, W2, bias, out, M, N, K, stream);
+            if (rows == 2) return launch_few<2, 2, MODE>(p, X, W, W2, bias, out, M, N, K, stream);
+            if (rows == 4) return launch_few<4, 2, MODE>(p, X, W, W2, bias, out, M, N, K, stream);
+            if (rows == 8) return launch_few<8, 4, MODE>(p, X, W, W2, bias, out, M, N, K, stream);
+            return launch_few<16, 4, MODE>(p, X, W, W2, bias, out, M, N, K, stream);
         }
     }
     if (M <= 32) return launch_split<32, MODE>(X, W, W2, bias, out, M, N, K, status, stream);

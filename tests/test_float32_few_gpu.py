@@ -13,6 +13,8 @@ DEV = "cuda:0"
     (1, 40, 4), (8, 8200, 1040), (16, 5000, 2052),
     (3, 130, 18944), (8, 30, 18944), (16, 40, 18944),      # K over the most blocks; the largest X that fits
     (16, 40, 30000),                       # and one that does not
+    # weights in registers, where a ring would leave room for fewer blocks: steps that do not fill the registers, several groups
+    (8, 4100, 2052), (16, 3000, 2052), (5, 900, 18948), (4, 620, 40964), (2, 620, 45004), (1, 620, 90004), (8, 70, 40964),
 ])
 def test_few_rows(m, n, k):
     from rust_inference_b200.kernels import ops, tcgen05
