@@ -49,6 +49,36 @@ __device__ __forceinline__ void set_in_all(volatile int* own, int blocks) {
     }
 }
 
+// How many blocks the device holds at once in clusters of `size` (2 to 8) when a block has an SM to itself: clusters lie within groups of
+// SMs, whose numbers of SMs leave some over (148 SMs: less than 138 blocks in clusters of three, 144 in clusters of four).
+// Asked once per device and size, with a kernel that may have the `smem` bytes, more than half of an SM's.
+inline int blocks_alone(const void* kernel, int threads, size_t smem, int size) {
+    static std::atomic<int> known[64][9];
+    if (size <= 1) return sm_count();
+    int dev = 0, n = 0;
+    if (size > 8 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sm_count() - 20;
+    n = known[dev][size].load(std::memory_order_relaxed);
+    if (n == 0) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)size);
+        cfg.blockDim = dim3((unsigned)threads);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)size;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
+            cudaGetLastError();
+            n = (sm_count() - 20) / size;
+        }
+        n *= size;
+        known[dev][size].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
 // A launch that may start under the kernel before it (`launch_dependent`), its blocks in clusters of `cluster` along x.
 template <typename... KArgs, typename... Args>
 int launch_cluster(const char* what, void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, int cluster, cudaStream_t stream,

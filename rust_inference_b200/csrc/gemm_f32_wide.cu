@@ -468,35 +468,10 @@ constexpr int smem_bytes(int tn) { return 1024 + STAGES * (W_STAGE + 3 * tn * BK
 // but no less than 1,220; a tile's epilogue 2,000 (gated 4,500); one whose pieces meet in a cluster 6,000.  Over 14 shapes of 33 to 512
 // rows the plan is within 3% of the best of all widths and cuts.
 struct Plan { int tn, splits; long long cost; };
-// Blocks of clusters of `splits` that the device holds at once (asked once per device; a block has an SM to itself).
 int blocks_at_once(int splits) {
-    static std::atomic<int> known[64][4];
-    const int which = splits == 2 ? 1 : splits == 4 ? 2 : splits == 8 ? 3 : 0;
-    if (which == 0) return sm_count();
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 128;
-    n = known[dev][which].load(std::memory_order_relaxed);
-    if (n == 0) {
-        static PerDeviceOnce once;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(splits);
-        cfg.blockDim = dim3(THREADS);
-        cfg.dynamicSmemBytes = smem_bytes(MAX_TN);
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)splits;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        if (raise_dynamic_smem(gemm_f32_wide_kernel<1>, smem_bytes(MAX_TN), once, "gemm_f32") != 0 ||
-            cudaOccupancyMaxActiveClusters(&n, gemm_f32_wide_kernel<1>, &cfg) != cudaSuccess || n <= 0) {
-            cudaGetLastError();
-            n = 128 / splits;
-        }
-        n *= splits;
-        known[dev][which].store(n, std::memory_order_relaxed);
-    }
-    return n;
+    static PerDeviceOnce once;
+    if (raise_dynamic_smem(gemm_f32_wide_kernel<1>, smem_bytes(MAX_TN), once, "gemm_f32") != 0) return 128;
+    return blocks_alone((const void*)gemm_f32_wide_kernel<1>, THREADS, smem_bytes(MAX_TN), splits);
 }
 Plan plan(int M, int N, int K, bool dual) {
     const int feats = dual ? ROWS / 2 : ROWS, total_kb = (K + BK - 1) / BK;

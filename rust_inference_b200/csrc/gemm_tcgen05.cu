@@ -934,10 +934,16 @@ int launch(int tn, const CUtensorMap& mw, const CUtensorMap& mw2, const CUtensor
     const int cluster = MODE != 2 ? split_k : 1;                     // pieces of K that are not added onto sums meet in a cluster
     const long long cluster_ctas = (long long)((n_feat + BLOCK_F - 1) / BLOCK_F) * cluster;
     const int recv = cluster > 1 ? cluster * ((n_tok + cluster - 1) / cluster) * (DUAL ? 2 : 1) * BLOCK_F * 4 : 0;
+    auto kernel = gemm_tc_kernel<TN, DUAL, MODE>;
+    static PerDeviceOnce configured;       // per device: the attribute belongs to a device's copy of the kernel
+    if (int rc = raise_dynamic_smem(kernel, SMEM_BUDGET + 1024 + CLUSTER_RECV_MAX, configured, "gemm_tcgen05")) return rc;
     // Small token tiles (decode) leave room for a second CTA on the SM, so that the next kernel's
     // CTAs can settle in and prefetch their weights while this one drains.
     int budget = (3 * STAGE_BYTES <= 108 * 1024 && TN <= 64) ? 108 * 1024 : SMEM_BUDGET;
-    if (cluster > 1 && cluster_ctas > sm_count()) budget = 111 * 1024 - recv;         // two of these CTAs on an SM
+    // What a CTA receives from its cluster comes on top, and from a few tokens on one CTA fills the SM.  Where not all of the clusters are
+    // resident so, two of their CTAs share an SM, with less of a ring (two instead of three gated stages from 10 tokens on, in clusters of 2
+    // or 4 from 9): 48 tiles of 2,048 in clusters of 3, 8 tokens 13.5 us in two rounds, 7.5 so.
+    if (cluster > 1 && cluster_ctas > blocks_alone((const void*)kernel, THREADS, SMEM_BUDGET, cluster)) budget = 111 * 1024 - recv;
     int stages = budget / STAGE_BYTES;
     if (stages > MAX_STAGES) stages = MAX_STAGES;
     if (stages > total_kb) stages = total_kb;
@@ -945,9 +951,6 @@ int launch(int tn, const CUtensorMap& mw, const CUtensorMap& mw2, const CUtensor
     const size_t smem = (size_t)stages * STAGE_BYTES + 1024 + recv;
     int kb_per_split = (total_kb + split_k - 1) / split_k;
     if (MODE == 2) split_k = (total_kb + kb_per_split - 1) / kb_per_split;      // no empty split
-    auto kernel = gemm_tc_kernel<TN, DUAL, MODE>;
-    static PerDeviceOnce configured;       // per device: the attribute belongs to a device's copy of the kernel
-    if (int rc = raise_dynamic_smem(kernel, SMEM_BUDGET + 1024 + CLUSTER_RECV_MAX, configured, "gemm_tcgen05")) return rc;
     if (cluster > 1) {
         if (cluster_ctas > 0x7fffffffLL) return fail("gemm_tcgen05: %lld CTAs exceed the grid limit", cluster_ctas);
         return launch_cluster("gemm_tcgen05 (cluster)", kernel, dim3((unsigned)cluster_ctas), THREADS, smem, cluster, stream, mw, mw2, mx, bias,
@@ -1084,13 +1087,16 @@ int pick_tile(int tn, const CUtensorMap& mw, const CUtensorMap& mw2, const CUten
 }  // namespace
 
 // Over how many CTAs of a cluster K is cut for a product of a few tokens that is not added onto sums.  It is a read of its weights, and a CTA,
-// whose ring holds 102 KB of them on their way, takes about 64 GB/s, so a product with few tiles leaves most of the memory's rate
-// unused.  Cut in four where that makes about one CTA per SM: most of a CTA's weights are then asked for before its wait.  Otherwise
+// whose ring holds 96 KB of them on their way (64 to 96 where two share an SM with what they receive, see `launch`), takes about 64 GB/s,
+// so a product with few tiles leaves most of the memory's rate unused.  Cut in four where that makes about one CTA per SM: most of a
+// CTA's weights are then asked for before its wait.  Otherwise
 // in two or three, whichever leaves the SMs more evenly filled, as long as all CTAs are resident together (two to an SM).
 // Whole decode steps, us, not cut / 2 / 3 / 4: 38 tiles of K = 896 (24 layers), 1 token 690 / 648 / 650 / 633, 8 tokens 757 / 713 / 692 /
 // 675; 70 tiles of 1,536 (28), 1 token 1,059 / 985 / 1,025 / 1,000, 12 tokens 1,140 / 1,130 / 1,144 / 1,203; 86 tiles of 2,048 (36), 1 token
 // 1,629 / 1,604 / 1,576 / 1,758; 112 tiles of 4,096 (32), 1 token 2,835 / 2,670 / 2,925 / 2,828.  (Gated products.  With those that store
-// their results cut likewise: decode steps of 8 sequences of a 2,048-wide routed decoder 486 -> 448, of a latent one 271 -> 261.)
+// their results cut likewise a decode step of 8 sequences of a 2,048-wide decoder of latent attention went from 271 to 261.)  The products
+// alone at 9 to 16 tokens, not cut / as planned: 70 tiles of 1,536 14.5-15.3 / 12.8-13.7, 86 of 2,048 20.0-21.1 / 18.1-20.1, 112 of 4,096
+// 42.8-43.3 / 42.3-43.5.
 int cluster_split(int n_tok, int n_feat, int K) {
     const int total_kb = (K + BLOCK_K - 1) / BLOCK_K, sms = sm_count();
     const long long tiles = (n_feat + BLOCK_F - 1) / BLOCK_F;

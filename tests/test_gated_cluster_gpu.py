@@ -53,3 +53,29 @@ def test_plain_products_cut_over_a_cluster(m, n, k, cluster):
     assert float((part.double() - want).norm() / want.norm()) <= 1e-5
     torch.cuda.synchronize()
     tcgen05.check_status()
+
+
+@pytest.mark.parametrize("m", [1, 8, 9, 12, 16, 17])
+@pytest.mark.parametrize("n, k, cluster", [
+    (4096, 1032, 4), (4736, 1024, 4),                # 32 tiles, and 37: more clusters of four than SMs hold one by one
+    (5120, 1024, 3), (6144, 1024, 3),                # 40 tiles, and 48: the same for clusters of three
+    (8960, 640, 2), (18944, 512, 1), (1024, 448, 1)])
+def test_planned_clusters(n, k, cluster, m):
+    """The plan's own cut, whose sums are the same on every run and those of the cut asked for by number."""
+    from rust_inference_b200.kernels import linear, ops, tcgen05
+    x = (torch.randn(m, k, device=DEV) * 0.5).bfloat16()
+    w, w2 = (linear.Weight((torch.randn(n, k, device=DEV) * 0.1).bfloat16()) for _ in range(2))
+    cluster = 1 if m > 16 else cluster
+    ref, up = (x.double() @ t.t.double().t() for t in (w, w2))
+    # gated: one rounding to bfloat16; stored: float32 sums of k products
+    for mode, extra, want, tol in ((ops.EPI_SILU_MUL, dict(w2=w2), ref * torch.sigmoid(ref) * up, 2.0 ** -8), (ops.EPI_STORE_F32, {}, ref, 1e-5)):
+        assert tcgen05.plan(m, n, k, mode)[1] == cluster
+        out = torch.full((m, n), 9.0, device=DEV, dtype=torch.bfloat16 if extra else torch.float32)
+        again, asked = out.clone(), out.clone()
+        tcgen05.gemm(x, w, out, mode, **extra)
+        tcgen05.gemm(x, w, again, mode, **extra)
+        tcgen05.gemm(x, w, asked, mode, split_k=cluster, **extra)
+        assert torch.equal(out, again) and torch.equal(out, asked)
+        assert float((out.double() - want).norm() / want.norm()) <= tol
+    torch.cuda.synchronize()
+    tcgen05.check_status()
