@@ -486,8 +486,12 @@ int scan_and_norm(const float* z, int ld, const float* fz, ScanCols at, const fl
     float* piece_gates = piece > 0 ? scratch + (size_t)n_seqs * max_pieces * heads * dim * vdim : nullptr;
     auto scan = [&](int mode) -> int {
         const int mp = mode == WHOLE ? 1 : max_pieces;
-        // four columns per thread for pieces, where the rows leave the registers and the blocks that are left fill the SMs
-        const int cpt = mode != WHOLE && rows <= 16 && vdim > 64 && (long long)n_seqs * mp * heads * ((vdim + 127) / 128) >= sm_count() ? 4 : 2;
+        // four columns per thread for pieces, where the rows leave the registers and the blocks with two columns, two or (few rows) three
+        // to an SM, would no longer be resident together, but for a few that hang over (us, two / four columns: 16 heads of 64 x 128,
+        // 416 or 208 blocks 58.9 / 63.6, 480 or 240 78 / 64; 8 of 128 x 128, 256 or 128 66 / 93, 304 or 152 83 / 95 and, the last pieces whole,
+        // 98 / 96, 320 or 160 99 / 96, 512 or 256 124 / 101)
+        const long long wide = (long long)n_seqs * mp * heads * ((vdim + 127) / 128);
+        const int cpt = mode != WHOLE && rows <= 16 && vdim > 64 && 200 * wide > 103LL * (rows <= 8 ? 3 : 2) * sm_count() ? 4 : 2;
         dim3 grid(n_seqs * mp, heads, (vdim + 32 * cpt - 1) / (32 * cpt));
         const int longest = mode == WHOLE ? (longest_run > 0 ? longest_run : n_tokens) : piece;
 #define RI_SCAN(ROWS, CPT) launch_scan<ROWS, KEYED, CPT>(vec, grid, stream, z, ld, fz, at, o_raw, state, piece_state, piece_gates,    \

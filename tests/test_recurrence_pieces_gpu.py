@@ -11,7 +11,9 @@ def _i32(v):
 
 
 @pytest.mark.parametrize("lengths, heads, dim, vdim", [([1300], 8, 128, 128), ([200, 1, 513, 64], 16, 100, 72), ([400, 130], 20, 24, 130),
-                                                       ([300], 2, 128, 128), ([257], 3, 250, 65)])
+                                                       ([300], 2, 128, 128), ([257], 3, 250, 65),
+                                                       # blocks of two columns that just fit the SMs together, and that do not
+                                                       ([770], 16, 64, 128), ([900], 16, 64, 128), ([1180], 8, 128, 128)])
 def test_pieces_are_the_one_pass(lengths, heads, dim, vdim):
     from rust_inference_b200.kernels import ops
     n, b, piece = sum(lengths), len(lengths), 64
