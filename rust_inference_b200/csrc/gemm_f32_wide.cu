@@ -524,10 +524,11 @@ int launch(const Plan& p, const CUtensorMap& map, const float* X, const float* W
 // Columns of the three bfloat16 matrices that a product of K takes as scratch, [3][M][that many].
 RI_API int ri_gemm_f32_wide_ld(int K) { return (K + 7) / 8 * 8; }
 
-// `mode`: the epilogue, as in `ri_gemm_f32`; parts: bfloat16 [3][M][ri_gemm_f32_wide_ld(K)], 16-byte aligned, overwritten.
-// tn, splits (0: the plan's): rows of X per tile, a multiple of 16 up to 176, and blocks along K, 1, 2, 4 or 8; for tests.
-RI_API int ri_gemm_f32_wide(const float* X, const float* W, const float* W2, const float* bias, float* out, void* parts, int mode, int M,
-                            int N, int K, int tn, int splits, int* status, cudaStream_t stream) {
+// `mode`: the epilogue, as in `ri_gemm_f32`; parts: bfloat16 [3][part_rows][ri_gemm_f32_wide_ld(K)], 16-byte aligned, overwritten: so many
+// rows of X are cut and multiplied at a time, in stretches of about equal length.
+// tn, splits (0: the plan's): rows of X per tile, a multiple of 16 up to 128, and blocks along K, 1, 2, 4 or 8; for tests.
+RI_API int ri_gemm_f32_wide(const float* X, const float* W, const float* W2, const float* bias, float* out, void* parts, int part_rows,
+                            int mode, int M, int N, int K, int tn, int splits, int* status, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || K % 4) return fail("gemm_f32: K must be a positive multiple of 4, found %d", K);
     if (((uintptr_t)X | (uintptr_t)W | (uintptr_t)W2 | (uintptr_t)parts) % 16) return fail("gemm_f32: operands must be 16-byte aligned");
@@ -535,26 +536,37 @@ RI_API int ri_gemm_f32_wide(const float* X, const float* W, const float* W2, con
     if (mode == 2 && bias != nullptr) return fail("gemm_f32: the residual epilogue takes no bias");
     if ((mode == 4 || mode == 5) && bias == nullptr) return fail("gemm_f32: epilogue %d needs its constants", mode);
     if (mode < 0 || mode > 5) return fail("gemm_f32: unknown epilogue mode %d", mode);
+    if (part_rows <= 0) return fail("gemm_f32: parts of %d rows", part_rows);
     const int ld = ri_gemm_f32_wide_ld(K), total_kb = (K + BK - 1) / BK;
-    Plan p = plan(M, N, K, mode == 3);
-    if (tn > 0) p.tn = tn;
-    if (splits > 0) p.splits = splits;
-    if (p.tn % 16 || p.tn > MAX_TN || p.splits > total_kb || (p.splits != 1 && p.splits != 2 && p.splits != 4 && p.splits != 8))
-        return fail("gemm_f32: no tiles of %d rows cut into %d", p.tn, p.splits);
-    CUtensorMap map;
-    if (int rc = encode_parts(&map, parts, M, ld, p.tn)) return rc;
-    const long long items = (long long)M * (ld / 4);
-    const cudaError_t e = launch_dependent(cut_rows_kernel, dim3((unsigned)(items + 255 < 256LL * 4096 ? (items + 255) / 256 : 4096)), 256, 0,
-                                           stream, X, (__nv_bfloat16*)parts, M, K, ld);
-    if (int rc = check_launch(e, "gemm_f32 (cut)")) return rc;
-    switch (mode) {
-        case 0:
-        case 1: return launch<1>(p, map, X, W, W2, bias, out, M, N, K, status, stream);
-        case 2: return launch<2>(p, map, X, W, W2, bias, out, M, N, K, status, stream);
-        case 3: return launch<3>(p, map, X, W, W2, bias, out, M, N, K, status, stream);
-        case 4: return launch<4>(p, map, X, W, W2, bias, out, M, N, K, status, stream);
-        default: return launch<5>(p, map, X, W, W2, bias, out, M, N, K, status, stream);
+    const int stretches = M / part_rows + (M % part_rows != 0), most = M / stretches + (M % stretches != 0);
+    for (int m0 = 0; m0 < M; m0 += most) {
+        const int rows = M - m0 < most ? M - m0 : most;
+        const float* x = X + (size_t)m0 * K;
+        float* to = out + (size_t)m0 * N;
+        Plan p = plan(rows, N, K, mode == 3);
+        if (tn > 0) p.tn = tn;
+        if (splits > 0) p.splits = splits;
+        if (p.tn % 16 || p.tn > MAX_TN || p.splits > total_kb || (p.splits != 1 && p.splits != 2 && p.splits != 4 && p.splits != 8))
+            return fail("gemm_f32: no tiles of %d rows cut into %d", p.tn, p.splits);
+        CUtensorMap map;
+        if (int rc = encode_parts(&map, parts, rows, ld, p.tn)) return rc;
+        // (waits for the products of the stretch before, which read the parts)
+        const long long items = (long long)rows * (ld / 4);
+        const cudaError_t e = launch_dependent(cut_rows_kernel, dim3((unsigned)(items + 255 < 256LL * 4096 ? (items + 255) / 256 : 4096)), 256,
+                                               0, stream, x, (__nv_bfloat16*)parts, rows, K, ld);
+        if (int rc = check_launch(e, "gemm_f32 (cut)")) return rc;
+        int rc = 0;
+        switch (mode) {
+            case 0:
+            case 1: rc = launch<1>(p, map, x, W, W2, bias, to, rows, N, K, status, stream); break;
+            case 2: rc = launch<2>(p, map, x, W, W2, bias, to, rows, N, K, status, stream); break;
+            case 3: rc = launch<3>(p, map, x, W, W2, bias, to, rows, N, K, status, stream); break;
+            case 4: rc = launch<4>(p, map, x, W, W2, bias, to, rows, N, K, status, stream); break;
+            default: rc = launch<5>(p, map, x, W, W2, bias, to, rows, N, K, status, stream);
+        }
+        if (rc) return rc;
     }
+    return 0;
 }
 
 RI_DEFINE_LAST_ERROR()

@@ -508,28 +508,35 @@ def gemm_f32_takes_wide(m: int, n: int, k: int) -> bool:
     return m > F32_WIDE_MANY_ROWS or (m > F32_WIDE_ROWS and n * k >= F32_WIDE_WEIGHTS)
 
 
+# Bytes of the scratch below, which a workspace keeps: more rows are cut and multiplied in stretches (of at least 128 rows, a whole tile).
+# us, all rows at once / in stretches: 8,000 x 3,584 x 18,944 8,870 / 8,290 (four of 2,000), 2,500 of them 2,560 / 2,630, 8,000 x 1,536 x
+# 8,960 1,790 / 1,825.  Half of it, and 8,000 x 896 x 4,864 in two stretches of rounds that do not fill: 514 / 624.
+F32_PARTS_BYTES = 256 << 20
+
+
 def gemm_f32_wide_scratch(m: int, k: int) -> tuple:
-    """Shape of the bfloat16 scratch that `gemm_f32_wide` cuts x into."""
-    return 3, m, -(-k // 8) * 8
+    """Shape of the bfloat16 scratch that `gemm_f32_wide` cuts x into, so many rows at a time."""
+    ld = -(-k // 8) * 8
+    return 3, min(m, max(128, F32_PARTS_BYTES // (6 * ld) // 128 * 128)), ld
 
 
 def gemm_f32_wide(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, *, bias: torch.Tensor | None = None,
                   w2: torch.Tensor | None = None, gate_form: torch.Tensor | None = None, act_form: torch.Tensor | None = None,
                   silu_cols: torch.Tensor | None = None, parts: torch.Tensor | None = None, tile: int = 0, splits: int = 0) -> torch.Tensor:
     """`gemm_f32` for many rows of x, which are cut into their bfloat16 parts once, in memory (csrc/gemm_f32_wide.cu).  parts: bfloat16
-    scratch (`gemm_f32_wide_scratch`; made here if None); tile, splits: rows of x per tile and blocks along K (0: the kernel's own
+    scratch (`gemm_f32_wide_scratch`, or with fewer rows: that many of x's are multiplied at a time; made here if None); tile, splits: rows of x per tile and blocks along K (0: the kernel's own
     plan), for comparisons and tests."""
     bias = _gemm_constants(x, w, out, mode, bias, w2, gate_form, act_form, silu_cols)
     _need(x.dtype == torch.float32, "gemm_f32: float32 operands")
     m, k = x.shape
     if parts is None:
         parts = torch.empty(gemm_f32_wide_scratch(m, k), dtype=torch.bfloat16, device=x.device)
-    _need(parts.dtype == torch.bfloat16 and parts.is_contiguous() and tuple(parts.shape) == gemm_f32_wide_scratch(m, k) and parts.is_cuda,
-          "gemm_f32: scratch for the parts of x")
+    _need(parts.dtype == torch.bfloat16 and parts.is_contiguous() and parts.dim() == 3 and parts.shape[0] == 3 and parts.shape[1] > 0
+          and parts.shape[2] == gemm_f32_wide_scratch(m, k)[2] and parts.is_cuda, "gemm_f32: scratch for the parts of x")
     from . import tcgen05
     st = tcgen05.f32_status_word()
-    _call("gemm_f32_wide", "ri_gemm_f32_wide", _p(x), _p(w), _p(w2), _p(bias), _p(out), _p(parts), c_int(mode), c_int(m),
-          c_int(w.shape[0]), c_int(k), c_int(tile), c_int(splits), c_void_p(st.data_ptr()), _stream())
+    _call("gemm_f32_wide", "ri_gemm_f32_wide", _p(x), _p(w), _p(w2), _p(bias), _p(out), _p(parts), c_int(parts.shape[1]), c_int(mode),
+          c_int(m), c_int(w.shape[0]), c_int(k), c_int(tile), c_int(splits), c_void_p(st.data_ptr()), _stream())
     return out
 
 

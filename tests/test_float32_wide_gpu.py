@@ -71,6 +71,27 @@ def test_wide_products_add_to_subnormal_numbers(size, splits):
     assert torch.equal(out.cpu(), want)
 
 
+@pytest.mark.parametrize("m, rows", [(300, 128), (257, 256), (100, 1), (64, 64), (300, 299)])
+def test_wide_products_in_stretches_of_rows(m, rows):
+    """Fewer rows of scratch than x has: cut and multiplied a stretch at a time, with the sums of the whole."""
+    ops = _ops()
+    n, k = 200, 260
+    x, w = torch.randn(m, k, device=DEV), torch.randn(n, k, device=DEV) / 16
+    whole, out = torch.ones(m, n, device=DEV), torch.ones(m + 1, n, device=DEV)
+    ops.gemm_f32_wide(x, w, whole, ops.EPI_RESIDUAL, splits=1)
+    parts = torch.empty(3, rows, 264, device=DEV, dtype=torch.bfloat16)
+    ops.gemm_f32_wide(x, w, out[:m], ops.EPI_RESIDUAL, splits=1, parts=parts)
+    assert torch.equal(out[:m], whole) and bool((out[m] == 1).all())
+
+
+def test_the_scratch_of_wide_products_is_bounded():
+    ops = _ops()
+    for m, k in ((8000, 18944), (100000, 896), (500, 262144), (70, 64)):
+        planes, rows, ld = ops.gemm_f32_wide_scratch(m, k)
+        assert planes == 3 and ld >= k and (rows == m or rows % 128 == 0)
+        assert 6 * rows * ld <= max(ops.F32_PARTS_BYTES, 128 * 6 * ld)
+
+
 def test_wide_products_refuse_what_they_cannot_cut():
     ops = _ops()
     x, w, out = torch.zeros(70, 64, device=DEV), torch.zeros(8, 64, device=DEV), torch.zeros(70, 8, device=DEV)
