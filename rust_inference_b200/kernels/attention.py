@@ -245,13 +245,15 @@ class FormedHeads:
 
 
 def formed_heads(out, ctx, width, *, n_heads, n_kv_heads, head_dim, rot_dims, scale, window=0, chunk=0, out_scale=1.0,
-                 norm=(None, None, 0.0), values_from_keys=False):
+                 norm=(None, None, 0.0), values_from_keys=False, arrays=()):
     """What runs a decode step's attention straight from its projection's sums (rows of `width` floats), or None where the kernel that
     does so takes no such step: bfloat16 steps of one token per sequence whose runs of pages meet in a cluster (or that have one
-    run), plain scores, heads of 64 or 128."""
+    run), plain scores, heads of 64 or 128, and whatever else it reads (`arrays`: tensors or None) on 16-byte boundaries."""
     if not ctx.all_single or ctx.dtype != torch.bfloat16 or (window and chunk) or rot_dims <= 0 or rot_dims % 8 or width % 8:
         return None
     if not ops.attention_mma_supports(head_dim, ctx.page_size, n_heads, n_kv_heads, True):
+        return None
+    if any(t is not None and t.data_ptr() % 16 for t in (*arrays, *norm[:2])):
         return None
     name, splits = decode_plan(ctx.n_seqs, n_kv_heads, ctx.page_table.shape[1] * ctx.page_size, ctx.page_size, head_dim)
     if not (name == "cluster" or (name == "tma" and splits == 1)):

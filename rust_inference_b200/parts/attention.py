@@ -340,6 +340,7 @@ class GQAttention(Mixer):
             mixed, ctx, width, n_heads=self.n_heads, n_kv_heads=self.n_kv_heads, head_dim=self.head_dim,
             rot_dims=self.position.rot_dims, scale=self.scale, window=self.window or 0, chunk=self.chunk or 0,
             out_scale=self.out_scale, values_from_keys=self.values_from_keys,
+            arrays=(self.b_qkv, self.position.cos, self.position.sin, cache_layer.k, cache_layer.v),
             norm=(None, None, 0.0) if self.qk_norm_eps is None else (self.q_norm, self.k_norm, self.qk_norm_eps))
         if attend is None:
             return False

@@ -20,14 +20,14 @@ SEPARATE = {"gated": dict(out_gate=True), "a gate per head": dict(head_gate=True
             "values of another size": dict(v_head_dim=64), "odd rotation": dict(rot_dims=36)}
 
 
-def _layer(form, seed=0):
+def _layer(form, seed=0, kind="rope"):
     from rust_inference_b200.parts.registry import lookup
     from rust_inference_b200.parts.spec import PartSpec
     form = dict(form)
     rot = form.pop("rot_dims", 128)
     part = lookup("mixer", "gqa_attention")(
         n_heads=8, n_kv_heads=2, head_dim=128, qkv_bias=form.pop("qkv_bias", False),
-        position=PartSpec("rope", {"head_dim": 128, "base": 10000.0, "rot_dims": rot}), hidden_size=WIDTH, dtype=torch.bfloat16, device=DEV,
+        position=PartSpec(kind, {"head_dim": 128, "base": 10000.0, "rot_dims": rot}), hidden_size=WIDTH, dtype=torch.bfloat16, device=DEV,
         **form)
     g = torch.Generator(device=DEV).manual_seed(seed)
     part.set_tensors({name: torch.randn(ts.shape, device=DEV, generator=g) * 0.1 + (1.0 if "norm" in name else 0.0) if ts.role == "vector"
@@ -37,9 +37,17 @@ def _layer(form, seed=0):
     return part
 
 
-def _step(part, monkeypatch, *, separate, routed=False, writes_cache=True):
+def _off(t, floats):
+    """t's numbers in memory that begins `floats` numbers behind a boundary."""
+    room = torch.empty(t.numel() + 4, dtype=t.dtype, device=t.device)
+    view = room[floats:floats + t.numel()].view(t.shape)
+    view.copy_(t)
+    return view
+
+
+def _step(part, monkeypatch, *, separate, routed=False, writes_cache=True, shift=0):
     """One decode step of sequences that end before, at and behind a page's edge: (times the attention formed the heads, its
-    result, the cache's keys and values)."""
+    result, the cache's keys and values).  shift: the angle tables lie so many floats off a 16-byte boundary."""
     from test_vadodra_gpu import make_ctx
     from rust_inference_b200.cache.sequence_cache import SequenceCache
     from rust_inference_b200.engine.context import Workspace
@@ -55,6 +63,8 @@ def _step(part, monkeypatch, *, separate, routed=False, writes_cache=True):
     ctx.routed = routed
     x = torch.randn(len(starts), WIDTH, device=DEV, generator=g).bfloat16()
     residual = torch.zeros(len(starts), WIDTH, device=DEV)
+    if shift:
+        part.position.cos, part.position.sin = (_off(t, shift) for t in (part.position.cos, part.position.sin))
     runs = []
     with monkeypatch.context() as m:
         # sums in one order, whichever pieces of K arrive first
@@ -95,3 +105,15 @@ def test_a_decoder_that_routes_keeps_its_roundings(name, monkeypatch):
 @pytest.mark.parametrize("name", SEPARATE)
 def test_what_the_attention_does_not_form(name, monkeypatch):
     assert _step(_layer(SEPARATE[name]), monkeypatch, separate=False, writes_cache=SEPARATE[name].get("own_kv", True))[0] == 0
+
+
+@pytest.mark.parametrize("array", ["bias", "angles", "norms"])
+def test_arrays_off_a_boundary_go_to_the_separate_kernels(array, monkeypatch):
+    part = _layer({"bias": dict(qkv_bias=True), "angles": {}, "norms": dict(qk_norm_eps=1e-5)}[array])
+    _, want, k, v = _step(part, monkeypatch, separate=True)
+    if array == "bias":
+        part.b_qkv = _off(part.b_qkv, 1)
+    if array == "norms":
+        part.k_norm = _off(part.k_norm, 3)
+    formed, out, k2, v2 = _step(part, monkeypatch, separate=False, shift=2 if array == "angles" else 0)
+    assert formed == 0 and torch.equal(out, want) and torch.equal(k, k2) and torch.equal(v, v2)
