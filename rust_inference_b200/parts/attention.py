@@ -9,6 +9,7 @@ from ..cache.sequence_cache import KVRequest, StateRequest
 from ..kernels import linear, ops, attention as attn_kernels
 from .base import Mixer
 from .registry import register, lookup
+from .rope import RotaryEncoding
 from .spec import TensorSpec, PartSpec
 
 
@@ -331,9 +332,9 @@ class GQAttention(Mixer):
         """A decode step whose projection is split over K: the attention's own kernel adds the bias to the sums, norms and turns the
         heads and writes the cache.  False (nothing done) where it does not take the step."""
         if (not ctx.all_single or self.extended or self.value_mix is not None or not writes_cache or self.v_head_dim != self.head_dim
-                or not hasattr(self.position, "apply_and_store_from_accumulators") or not linear.wants_split(x, self.w_qkv)):
-            return False
-        if getattr(ctx, "routed", False) and (getattr(self.position, "partial", False) or self.qk_norm_eps is not None or self.values_from_keys or self.out_scale != 1.0):
+                or type(self.position) is not RotaryEncoding or not linear.wants_split(x, self.w_qkv)):
+            return False                # (a position encoding of a caller's own has steps of its own)
+        if getattr(ctx, "routed", False) and (self.position.partial or self.qk_norm_eps is not None or self.values_from_keys or self.out_scale != 1.0):
             return False                # not the bits of the kernels it replaces: see `Part.routes`
         mixed = ctx.buffer("attn_out", (x.shape[0], self.o_dim), self.dtype)
         attend = attn_kernels.formed_heads(

@@ -117,3 +117,32 @@ def test_arrays_off_a_boundary_go_to_the_separate_kernels(array, monkeypatch):
         part.k_norm = _off(part.k_norm, 3)
     formed, out, k2, v2 = _step(part, monkeypatch, separate=False, shift=2 if array == "angles" else 0)
     assert formed == 0 and torch.equal(out, want) and torch.equal(k, k2) and torch.equal(v, v2)
+
+
+def test_a_position_encoding_of_ones_own_keeps_its_interface(monkeypatch):
+    """A registered encoding whose methods know nothing of an attention that forms heads is called as it was, and one that changes a
+    method of the rotary one is not passed by."""
+    from rust_inference_b200.parts.registry import lookup, register, unregister
+    base = lookup("position", "rope")
+    called = []
+
+    @register("position", "toy_rope")
+    class Toy(base):
+        def apply_and_store_from_accumulators(self, acc, bias, q_out, ctx, cache_layer, *, n_heads, n_kv_heads, head_dim, write_kv):
+            called.append("sums")
+            super().apply_and_store_from_accumulators(acc, bias, q_out, ctx, cache_layer, n_heads=n_heads, n_kv_heads=n_kv_heads,
+                                                      head_dim=head_dim, write_kv=write_kv)
+
+        def apply_and_store(self, *args, **kw):
+            called.append("rows")
+            super().apply_and_store(*args, **kw)
+
+    try:
+        for form, way in (({}, "sums"), (dict(rot_dims=64), "rows")):
+            _, want, k, v = _step(_layer(form), monkeypatch, separate=True)
+            called.clear()
+            formed, out, k2, v2 = _step(_layer(form, kind="toy_rope"), monkeypatch, separate=False)
+            assert formed == 0 and called == [way]
+            assert torch.equal(out, want) and torch.equal(k, k2) and torch.equal(v, v2)
+    finally:
+        unregister("position", "toy_rope")
