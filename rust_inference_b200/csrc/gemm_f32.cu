@@ -1,5 +1,5 @@
 // out[M, N] = X[M, K] * W[N, K]^T for float32 operands with float32 results, in two kernels that between them take
-// every M (K a multiple of 4 and 16-byte aligned operands: rows are read 16 bytes at a time; `gemm_simt.cu` has the rest).
+// M up to 64 (K a multiple of 4 and 16-byte aligned operands: rows are read 16 bytes at a time; `gemm_simt.cu` has the rest).
 //
 // Few rows of X (a decode step, up to FEW_MAX): the product is a read of W.  A warp owns a few rows of W, its lanes run
 // along K with 16-byte asynchronous copies into a ring of their own (or loads), several steps ahead, and every weight meets all rows of X,
@@ -329,10 +329,23 @@ int launch_few(const FewPlan& p, const float* X, const float* W, const float* W2
 // 64 x 4,864 x 896 gated takes 29 us, 64 x 896 x 4,864 24.  Parts rounded instead of cut off, with six products, took as long and left
 // a single product off by up to 1.4 x 2^-24.
 // ---------------------------------------------------------------------------------------------------------------------
-constexpr int ROWS = 128, BK = 64, PART = ROWS * BK * 2, STAGES = 2;
+constexpr int ROWS = 128, BK = 64, PART = ROWS * BK * 2, STAGES = 2, SPLIT_MAX = 64;
 constexpr int CUT_WARPS = 8, CUT_THREADS = CUT_WARPS * 32, ADD_WARPS = 8;
 constexpr int SPLIT_THREADS = CUT_THREADS + ADD_WARPS * 32;
 enum Status { ST_CUT_TIMEOUT = 41, ST_MMA_TIMEOUT = 42, ST_ADD_TIMEOUT = 43 };
+
+// Infinite or NaN sums of a tile computed again over the block's piece of K: a warp takes 32 neighbouring features and four rows of X.
+// (A call of its own: inside the kernel it takes registers from the loops that always run.)
+template <int TN, bool DUAL>
+__device__ __noinline__ void sums_again(float* pieces, const float* X, const float* W, const float* W2, int M, int N, int K, int f0, int k_begin,
+                                        int k_end) {
+    constexpr int FEATS = DUAL ? ROWS / 2 : ROWS;
+    for (int g = threadIdx.x >> 5; g < TN / 4 * (ROWS / 32); g += SPLIT_THREADS / 32) {
+        const int c0 = g / (ROWS / 32) * 4, r0 = g % (ROWS / 32) * 32;
+        sum_again(pieces + c0 * ROWS + r0, ROWS, X, c0, min(4, M - c0), f0 + (r0 + (int)(threadIdx.x & 31)) % FEATS < N, K, k_begin, k_end,
+                  [&](int r) { return (DUAL && r0 + r >= FEATS ? W2 : W) + (size_t)(f0 + (DUAL ? (r0 + r) % FEATS : r0 + r)) * K; });
+    }
+}
 
 template <int TN, int MODE>
 __global__ void __launch_bounds__(SPLIT_THREADS, 1)
@@ -354,8 +367,7 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
     float* pieces = reinterpret_cast<float*>(smem_raw + (base - smem_u32(smem_raw)));      // [TN][128], over the stages at the end
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = splits > 1 ? (int)cluster_rank() : 0;
-    const int tok_tiles = (M + TN - 1) / TN, tile = (int)blockIdx.x / splits;
-    const int t0 = (tile % tok_tiles) * TN, f0 = (tile / tok_tiles) * FEATS;        // rows of X fastest: W stays in L2
+    const int f0 = (int)blockIdx.x / splits * FEATS;             // one tile holds all rows of X: M <= TN
     const int total_kb = (K + BK - 1) / BK;
     const int kb0 = (int)((long long)total_kb * rank / splits);
     const int n_kb = (int)((long long)total_kb * (rank + 1) / splits) - kb0;        // >= 1: splits <= total_kb
@@ -385,9 +397,6 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
     if (splits > 1) cluster_arrive();            // flags and barriers are set up
     let_next_kernel_start();
 
-    // row r of the tile (one that exists): which row of which matrix
-    auto weight_row = [&](int r) { return (DUAL && r >= FEATS ? W2 : W) + (size_t)(f0 + (DUAL ? r % FEATS : r)) * K; };
-
     if (warp < CUT_WARPS) {
         // ---- read, cut, store: 16 threads per row of 64 floats ----
         const int k4 = threadIdx.x & 15, row = threadIdx.x >> 4;             // rows row, row + 16, ...
@@ -395,14 +404,14 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
         constexpr int WN = ROWS / 16, XN = TN / 16;
         // a thread's rows are 16 apart: one address per matrix, and a bit for every row that exists
         const size_t stride = (size_t)16 * K;
-        const float* xp = X + (size_t)(t0 + row) * K;
+        const float* xp = X + (size_t)row * K;
         const float* wp = W + (size_t)(f0 + row) * K;
         const float* wp2 = DUAL ? W2 + (size_t)(f0 + row) * K : nullptr;
         uint32_t w_has = 0, x_has = 0;
 #pragma unroll
         for (int i = 0; i < WN; ++i) w_has |= (f0 + (row + 16 * i) % FEATS < N ? 1u : 0u) << i;
 #pragma unroll
-        for (int i = 0; i < XN; ++i) x_has |= (t0 + row + 16 * i < M ? 1u : 0u) << i;
+        for (int i = 0; i < XN; ++i) x_has |= (row + 16 * i < M ? 1u : 0u) << i;
         const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
         int k = kb0 * BK + k4 * 4;
         auto load_w = [&](int i, bool in) {
@@ -518,7 +527,7 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
 #pragma unroll
             for (int c = 0; c < COLS; ++c) {
                 pieces[(part * COLS + c) * ROWS + q * 32 + lane] = acc[c] * DOWN;
-                finite &= fabsf(acc[c]) <= 3.402823466e38f;
+                finite &= fabsf(acc[c]) <= LARGEST;
             }
             if (!finite) odd_flag = 1;
         }
@@ -533,57 +542,7 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
     }
     bool failed = abort_flag != 0;
     if (odd_flag && !failed) {
-        // infinite or NaN sums are computed again, as plain float32 sums over this block's piece of K; the others stay what they
-        // are.  A warp looks at 32 neighbouring features of four rows of X and takes four features at a time that are to be done
-        // for any of the rows, its lanes along K, so that both operands are read in whole lines and each once for four sums
-        // (333 x 151,936 x 896 with one row of NaN: 1,262 us, 986 without; with NaN in every row 7,505, the FFMA kernel 2,962).
-        const int k_end = min(K, (kb0 + n_kb) * BK);
-        for (int g = warp; g < TN / 4 * (ROWS / 32); g += SPLIT_THREADS / 32) {
-            const int c0 = g / (ROWS / 32) * 4, r0 = g % (ROWS / 32) * 32;
-            const bool exists = f0 + (r0 + lane) % FEATS < N;        // zeros in the place of a row may have met an infinity too
-            const float* x[4];
-            uint32_t odd[4], todo = 0;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const bool row = t0 + c0 + i < M;
-                x[i] = X + (size_t)(row ? t0 + c0 + i : t0) * K;
-                odd[i] = __ballot_sync(0xffffffffu, row && exists && !(fabsf(pieces[(c0 + i) * ROWS + r0 + lane]) <= 3.402823466e38f));
-                todo |= odd[i];
-            }
-            while (todo != 0) {
-                const float* w[4];
-                int r[4];
-                float sum[4][4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {                        // fewer than four left: the first again
-                    r[j] = todo != 0 ? __ffs(todo) - 1 : r[0];
-                    w[j] = weight_row(r0 + r[j]);
-                    todo &= todo - 1;
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) sum[i][j] = 0.f;
-                }
-#pragma unroll 2
-                for (int k = kb0 * BK + lane * 4; k < k_end; k += 128) {
-                    float4 a[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) a[i] = load_written(x[i] + k);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const float4 b = load_weight(w[j] + k);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            sum[i][j] = fmaf(a[i].w, b.w, fmaf(a[i].z, b.z, fmaf(a[i].y, b.y, fmaf(a[i].x, b.x, sum[i][j]))));
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const float v = warp_sum(sum[i][j]);
-                        if (lane == 0 && ((odd[i] >> r[j]) & 1)) pieces[(c0 + i) * ROWS + r0 + r[j]] = v;
-                    }
-            }
-        }
+        sums_again<TN, DUAL>(pieces, X, W, W2, M, N, K, f0, kb0 * BK, min(K, (kb0 + n_kb) * BK));
         __syncthreads();
     }
     if (splits > 1) {
@@ -596,7 +555,7 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
     const int from = TN * FEATS / splits * rank, to = from + TN * FEATS / splits;      // TN * FEATS is a multiple of 8
     for (int i = from + (int)threadIdx.x; i < to && !failed; i += SPLIT_THREADS) {
         const int c = i / FEATS, fl = i - c * FEATS, f = f0 + fl;
-        if (t0 + c >= M || f >= N) continue;
+        if (c >= M || f >= N) continue;
         const int at = c * ROWS + fl;
         float v = 0.f, up = 0.f;
         if (splits > 1) {
@@ -608,7 +567,7 @@ gemm_f32_split_kernel(const float* X, const float* __restrict__ W, const float* 
             v = pieces[at];
             if (DUAL) up = pieces[at + FEATS];
         }
-        finish<MODE>(out, (size_t)(t0 + c) * N + f, f, v, up, bias, forms);
+        finish<MODE>(out, (size_t)c * N + f, f, v, up, bias, forms);
     }
     if (splits > 1) cluster_sync();          // a peer may still be reading this block's pieces
 }
@@ -620,7 +579,7 @@ int launch_split(const float* X, const float* W, const float* W2, const float* b
     constexpr int SMEM = STAGES * 3 * (PART + TN * BK * 2) + 1024;
     static PerDeviceOnce once;
     if (int rc = raise_dynamic_smem(gemm_f32_split_kernel<TN, MODE>, SMEM, once, "gemm_f32")) return rc;
-    const long long tiles = (long long)((M + TN - 1) / TN) * ((N + FEATS - 1) / FEATS);
+    const long long tiles = (N + FEATS - 1) / FEATS;
     const int total_kb = (K + BK - 1) / BK;
     // K over the blocks of a cluster while that shortens the run of the fullest SM: rounds of the grid (one block per SM;
     // clusters of eight leave some SMs out) times blocks of K, plus what a tile costs besides (about three blocks of K, one
@@ -671,6 +630,7 @@ RI_API int ri_gemm_f32(const float* X, const float* W, const float* W2, const fl
     if (mode == 3 && W2 == nullptr) return fail("gemm_f32: the gated epilogue needs a second matrix");
     if (mode == 2 && bias != nullptr) return fail("gemm_f32: the residual epilogue takes no bias");
     if ((mode == 4 || mode == 5) && bias == nullptr) return fail("gemm_f32: epilogue %d needs its constants", mode);
+    if (M > SPLIT_MAX) return fail("gemm_f32: %d rows exceed %d", M, SPLIT_MAX);
     if (few_max < 0 || few_max > FEW_MAX) few_max = FEW_MAX;
     switch (mode) {
         case 0:

@@ -67,5 +67,58 @@ __device__ __forceinline__ void put(uint32_t addr, uint32_t part_bytes, const fl
     store8(addr + 2 * part_bytes, l[0], l[1]);
 }
 
+constexpr float LARGEST = 3.402823466e38f;
+// The sums of up to four rows of X (from t0 on) and 32 rows of W, at buf[i * ld + lane] for a warp: those that are infinite or NaN are computed
+// again, as plain float32 sums over k_begin .. k_end; the others stay what they are.  `exists`: the lane's row of W does (zeros in its place
+// may have met an infinity too); weight_row(r): the memory of row r.  The warp takes four rows of W at a time that are to be done for
+// any of the rows of X, its lanes along K, so that both operands are read in whole lines and each once for four sums.
+template <typename Row>
+__device__ __forceinline__ void sum_again(float* buf, int ld, const float* X, int t0, int columns, bool exists, int K, int k_begin, int k_end,
+                                          Row weight_row) {
+    const int lane = threadIdx.x & 31;
+    const float* x[4];
+    uint32_t odd[4], todo = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        x[i] = X + (size_t)(i < columns ? t0 + i : t0) * K;
+        odd[i] = __ballot_sync(0xffffffffu, i < columns && exists && !(fabsf(buf[i * ld + lane]) <= LARGEST));
+        todo |= odd[i];
+    }
+    while (todo != 0) {
+        const float* w[4];
+        int r[4];
+        float sum[4][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {                                // fewer than four left: the first again
+            r[j] = todo != 0 ? __ffs(todo) - 1 : r[0];
+            w[j] = weight_row(r[j]);
+            todo &= todo - 1;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) sum[i][j] = 0.f;
+        }
+#pragma unroll 2
+        for (int k = k_begin + lane * 4; k < k_end; k += 128) {
+            float4 a[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i] = load_written(x[i] + k);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float4 b = load_weight(w[j] + k);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    sum[i][j] = fmaf(a[i].w, b.w, fmaf(a[i].z, b.z, fmaf(a[i].y, b.y, fmaf(a[i].x, b.x, sum[i][j]))));
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float v = warp_sum(sum[i][j]);
+                if (lane == 0 && ((odd[i] >> r[j]) & 1)) buf[i * ld + r[j]] = v;
+            }
+    }
+    __syncwarp();
+}
+
 }  // namespace f32
 }  // namespace ri

@@ -40,7 +40,6 @@ constexpr int ADD_WARPS = 8, CUT_WARPS = 4, TMA_WARP = ADD_WARPS + CUT_WARPS, MM
 constexpr int THREADS = 16 * 32, LAUNCH_REGS = 128, ADD_REGS = 176, CUT_REGS = 96, ISSUE_REGS = 64;
 static_assert(8 * ADD_REGS + 4 * CUT_REGS + 4 * ISSUE_REGS <= 16 * LAUNCH_REGS, "a warp waits for registers that the block does not have");
 constexpr int S_COL = MAX_TN, SUM_COL = 3 * MAX_TN;          // tensor memory: the large products' sums, two buffers of the small ones', the groups' sum
-constexpr float LARGEST = 3.402823466e38f;
 enum Status { ST_CUT_TIMEOUT = 41, ST_MMA_TIMEOUT = 42, ST_ADD_TIMEOUT = 43 };
 
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
@@ -78,57 +77,6 @@ __device__ __forceinline__ int feature_of(int f0, int r) { return f0 + (DUAL ? (
 template <bool DUAL>
 __device__ __forceinline__ const float* weight_row(const float* W, const float* W2, int f0, int r, int K) {
     return (DUAL && (r & 16) ? W2 : W) + (size_t)feature_of<DUAL>(f0, r) * K;
-}
-
-// The sums of up to four columns (rows of X from t0 on) and this warp's 32 rows of W, in buf [4][32]: those that are infinite or NaN
-// are computed again, as plain float32 sums over k_begin .. k_end.  The warp's lanes run along K, up to four rows of W and four of X at a time.
-template <bool DUAL>
-__device__ __forceinline__ void sum_again(float* buf, const float* X, const float* W, const float* W2, int t0, int columns, int N, int K,
-                                          int f0, int r0, int k_begin, int k_end) {
-    const int lane = threadIdx.x & 31;
-    const bool exists = feature_of<DUAL>(f0, r0 + lane) < N;         // zeros in the place of a row may have met an infinity too
-    const float* x[4];
-    uint32_t odd[4], todo = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        x[i] = X + (size_t)(i < columns ? t0 + i : t0) * K;
-        odd[i] = __ballot_sync(0xffffffffu, i < columns && exists && !(fabsf(buf[i * 32 + lane]) <= LARGEST));
-        todo |= odd[i];
-    }
-    while (todo != 0) {
-        const float* w[4];
-        int r[4];
-        float sum[4][4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {                                // fewer than four left: the first again
-            r[j] = todo != 0 ? __ffs(todo) - 1 : r[0];
-            w[j] = weight_row<DUAL>(W, W2, f0, r0 + r[j], K);
-            todo &= todo - 1;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) sum[i][j] = 0.f;
-        }
-#pragma unroll 2
-        for (int k = k_begin + lane * 4; k < k_end; k += 128) {
-            float4 a[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = load_written(x[i] + k);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float4 b = load_weight(w[j] + k);
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    sum[i][j] = fmaf(a[i].w, b.w, fmaf(a[i].z, b.z, fmaf(a[i].y, b.y, fmaf(a[i].x, b.x, sum[i][j]))));
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float v = warp_sum(sum[i][j]);
-                if (lane == 0 && ((odd[i] >> r[j]) & 1)) buf[i * 32 + r[j]] = v;
-            }
-    }
-    __syncwarp();
 }
 
 // `finish`; an element that is added to is added to once, by an instruction that returns nothing, so that nobody waits for its old value
@@ -388,7 +336,8 @@ gemm_f32_wide_kernel(const __grid_constant__ CUtensorMap map_x, const float* X, 
                     for (int j = 0; j < 4; ++j) buf[j * 32 + lane] = acc[j];
                     __syncwarp();
                     if (c0 < columns)
-                        sum_again<DUAL>(buf, X, W, W2, t0 + c0, min(4, columns - c0), N, K, f0, q * 32, kb0 * BK, min(K, (kb0 + n_kb) * BK));
+                        sum_again(buf, 32, X, t0 + c0, min(4, columns - c0), f < N, K, kb0 * BK, min(K, (kb0 + n_kb) * BK),
+                                  [&](int r) { return weight_row<DUAL>(W, W2, f0, q * 32 + r, K); });
 #pragma unroll
                     for (int c = 0; c < HALF_MAX - 4; ++c) acc[c] = acc[c + 4];
 #pragma unroll

@@ -68,20 +68,9 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t addr) {
     return d;
 }
 
-__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-// The same for a warp that stays together: every lane calls, the one whose `leader` is set issues.  In a branch that one lane takes,
-// descriptors lie in that lane's registers and every MMA has them fetched from there, which takes 135 clocks from one MMA to the next
-// whatever its size (as long as 256 columns take); values that are the same in a whole warp are at hand.
+// An MMA and the arrival behind those issued so far, for a warp that stays together: every lane calls, the one whose `leader` is set issues.
+// In a branch that one lane takes, an MMA followed the one before after 135 clocks whatever its size (as long as 256 columns take); so
+// a small one follows as soon as it can.
 __device__ __forceinline__ uint32_t elect_one() {
     uint32_t leader;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(leader));
