@@ -146,3 +146,34 @@ def test_a_position_encoding_of_ones_own_keeps_its_interface(monkeypatch):
             assert torch.equal(out, want) and torch.equal(k, k2) and torch.equal(v, v2)
     finally:
         unregister("position", "toy_rope")
+
+
+@pytest.mark.parametrize("graphs", [True, False])
+def test_an_engine_decodes_over_a_page_edge(graphs, monkeypatch):
+    """Steps of a dense decoder from before a page's edge to behind it: every layer's attention forms its heads, and the logits are
+    those of the separate kernels."""
+    from rust_inference_b200 import Engine, config_from_dict
+    from rust_inference_b200.kernels import attention
+    config = config_from_dict({
+        "architectures": ["Qwen2ForCausalLM"], "hidden_size": 1024, "num_hidden_layers": 3, "num_attention_heads": 8, "num_key_value_heads": 2,
+        "head_dim": 128, "intermediate_size": 512, "vocab_size": 264, "rope_theta": 1e6, "rms_norm_eps": 1e-6, "attention_bias": True,
+        "tie_word_embeddings": False, "max_position_embeddings": 512})
+    tokens = [[(7 * i + 3 * b) % 264 for i in range(70)] for b in range(2)]
+    rows, counts = [], []
+    real, rule = attention.FormedHeads.run, attention.formed_heads
+    for separate in (False, True):
+        runs = []
+        monkeypatch.setattr(attention.FormedHeads, "run", lambda self, *a, **k: (runs.append(1), real(self, *a, **k))[1])
+        monkeypatch.setattr(attention, "formed_heads", (lambda *a, **k: None) if separate else rule)
+        eng = Engine.from_random(config, std=0.03, max_tokens=1024, n_slots=3, use_graphs=graphs)
+        slots = [eng.alloc_slot(), eng.alloc_slot()]
+        eng.step(slots, [t[:62 - b] for b, t in enumerate(tokens)], "none")
+        got = [eng.step(slots, [[t[62 - b + i]] for b, t in enumerate(tokens)], "last").clone() for i in range(6)]
+        torch.cuda.synchronize()
+        eng.check_device_status()
+        rows.append(torch.cat(got))
+        counts.append(len(runs))
+    # a captured step passes here when it is warmed up and captured, the others every time
+    assert counts[1] == 0 and counts[0] % 3 == 0 and counts[0] >= (3 if graphs else 18)
+    # the same sums and roundings but for the order in which pieces of K are added
+    assert float((rows[0] - rows[1]).norm() / rows[1].norm()) <= 1e-2

@@ -4,6 +4,8 @@ import pytest
 import torch
 
 import lulisun_models
+import plain_lulisun
+from conftest import random_tokens
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -47,3 +49,46 @@ def test_products_of_a_routed_step_keep_their_sums(m):
     assert all(torch.equal(got, want) for got, want in pairs)
     ctx.routed = False
     assert not torch.equal(linear.logits(x, w, f32(), ctx), pairs[0][1])          # (cut, the sums are others)
+
+
+@pytest.mark.parametrize("width, heads", [(1024, 8), (512, 4)])
+def test_routed_steps_away_from_near_ties(width, heads, monkeypatch, tmp_path):
+    """A decode step whose products are as large as served ones, routers undisturbed, against 64 bits: compared are the sequences
+    in which no token's choice, of groups or of experts, hangs on bfloat16's rounding of the router's input."""
+    layer = lulisun_models._layer(heads=heads, kv=2, dim=128, vdim=128, scale=0.088, chunk=16, base=10000.0, rot=64, rh=4, rdim=64, rvdim=64,
+                                  ls=0.7, rs=0.7, mlp=lulisun_models._moe(16, 2, 128, groups=(4, 2), shared=256))
+    cfg = {"architecture": "Lulisun", "vocab": 300, "width": width, "norm": {"eps": 1e-5}, "layers": [layer] * 2}
+    model = lulisun_models.make(tmp_path, f"w{width}", cfg=cfg)
+    margins, route = [], plain_lulisun.route
+
+    def recorded(h, w, pre, *, experts, top, groups, keep):
+        ids, weights, s = route(h, w, pre, experts=experts, top=top, groups=groups, keep=keep)
+        choice = (s + w[pre + "correction"]).view(len(h), groups, -1)
+        of_groups = choice.topk(2, -1).values.sum(-1).sort(-1, descending=True)
+        kept = torch.zeros(len(h), groups, dtype=torch.bool).scatter_(1, of_groups.indices[:, :keep], True)
+        best = choice.masked_fill(~kept[..., None], -9.0).view(len(h), -1).sort(-1, descending=True).values
+        margins.append(torch.minimum(of_groups.values[:, keep - 1] - of_groups.values[:, keep], best[:, top - 1] - best[:, top]))
+        return ids, weights, s
+
+    monkeypatch.setattr(plain_lulisun, "route", recorded)
+    n = 32
+    prompts = [random_tokens(3 + i % 5, 300, 100 + i) for i in range(n)]
+    want, decided = [], []
+    for p in prompts:
+        margins.clear()
+        want.append(model.plain_logits(p)[-1])
+        # a rounding to bfloat16 moves a router's score, a sigmoid of a sum of N(0, 1) terms, by about 2e-3
+        decided.append(min(float(m.min()) for m in margins) > 1e-2)
+    assert sum(decided) >= n // 4
+    from rust_inference_b200.engine.engine import Engine
+    eng = Engine.from_pretrained(model.folder, dtype="bfloat16", max_tokens=n * 64, n_slots=n)
+    for i in range(0, n, 8):
+        slots = [eng.alloc_slot() for _ in range(8)]
+        eng.step(slots, [p[:-1] for p in prompts[i:i + 8]], "none")
+        got = eng.step(slots, [p[-1:] for p in prompts[i:i + 8]], "last").double().cpu()
+        for j in range(8):
+            if decided[i + j]:
+                w = want[i + j]
+                # eight roundings to bfloat16 (2^-9) a layer one after the other; a wrong expert costs 0.1 and more
+                assert float((got[j] - w).norm() / w.norm()) <= 2e-2
+    eng.check_device_status()
